@@ -148,7 +148,8 @@ void free_batch(wc_batch* b) {
                     d.unordered, d.perm,         d.counts,     d.start,  d.cell_list,    d.num_nonempty,
                     d.scan_desc, d.scan_tile_counter, d.err,   d.hits,   b->d_scenes,    b->d_poff,
                     b->d_coff,   b->d_diag,      b->staging,   b->flush_buf, b->flush_sink, d.ids_a,
-                    d.ids_b,     d.accel,        d.xyz};
+                    d.ids_b,     d.accel,        d.xyz,        d.pstart, d.cidx,         d.rec,
+                    d.info};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (b->h_err) cudaFreeHost(b->h_err);
@@ -195,7 +196,7 @@ void apply_geometry(wc_batch* b, const wc_tuning& t) {
     const int variant = t.pass_variant == WC_PASSES_TEAM ? PASSES_TEAM : PASSES_LANE;
     if (variant != b->ld.pass_variant) {
         b->ld.pass_variant = variant;
-        sph_occupancy(true, &b->max_density_blocks, &b->max_force_blocks, variant);
+        sph_occupancy(true, &b->max_density_blocks, &b->max_force_blocks, variant, b->d.n);
     }
     b->tuning.pass_variant = (uint32_t)variant;
     b->ld.grid_density = b->ld.sms * (int)std::max(1u, std::min(t.density_blocks_per_sm, (uint32_t)b->max_density_blocks));
@@ -210,9 +211,10 @@ void apply_geometry(wc_batch* b, const wc_tuning& t) {
 void enqueue_step(wc_batch* b, const StepInputs& in) {
     const BatchTables bt = tables(b);
     launch_bin_count_batched(b->d, bt, b->ld, b->stream);
-    launch_scan_cells(b->d, b->stream);
+    const bool lane = b->ld.pass_variant == PASSES_LANE;
+    launch_scan_cells(b->d, b->stream, lane);
     launch_scatter(b->d, b->ld, b->stream);
-    launch_rank_gather(b->d, b->ld, b->stream);
+    launch_rank_gather(b->d, b->ld, b->stream, lane);
     launch_density_batched(b->d, bt, b->ld, b->stream);
     launch_force_batched(b->d, bt, in, b->ld, b->stream);
 }
@@ -259,6 +261,7 @@ wc_status capture(wc_batch* b, const StepInputs& in) {
     a.hits = b->d.hits;
     a.accel = b->d.accel;
     a.err = b->d.err;
+    a.lane = lane_tables(b->d);
     a.bind();
     b->graph_in = in;
     return WC_OK;
@@ -536,9 +539,13 @@ WC_API wc_status wc_batch_create(const wc_params* scenes, uint32_t num_scenes, w
     if (st == WC_OK) st = dalloc(&d.perm, n);
     if (st == WC_OK) st = dalloc(&d.ids_a, n);
     if (st == WC_OK) st = dalloc(&d.ids_b, n);
-    if (st == WC_OK) st = dalloc(&d.hits, (size_t)n * MASK_WORDS);
-    d.xyz_stride = xyz_stride_for((uint32_t)n);
-    if (st == WC_OK) st = dalloc(&d.xyz, 3 * (size_t)d.xyz_stride);
+    if (st == WC_OK) st = dalloc(&d.hits, hits_words(n));
+    d.pcap = padded_capacity(n, cells);
+    if (st == WC_OK) st = dalloc(&d.xyz, 3 * (size_t)d.pcap);
+    if (st == WC_OK) st = dalloc(&d.cidx, d.pcap);
+    if (st == WC_OK) st = dalloc(&d.rec, 2 * (size_t)d.pcap);
+    if (st == WC_OK) st = dalloc(&d.info, n);
+    if (st == WC_OK) st = dalloc(&d.pstart, cells + 1);
     if (st == WC_OK) st = dalloc(&d.counts, cells);
     if (st == WC_OK) st = dalloc(&d.start, cells + 1);
     if (st == WC_OK) st = dalloc(&d.cell_list, cells);
@@ -559,13 +566,14 @@ WC_API wc_status wc_batch_create(const wc_params* scenes, uint32_t num_scenes, w
         cudaMemsetAsync(d.err, 0, sizeof(uint32_t), b->stream);
         cudaMemsetAsync(d.num_nonempty, 0, 3 * sizeof(uint32_t), b->stream);
         cudaMemsetAsync(d.start, 0, sizeof(uint32_t) * (cells + 1), b->stream);
-        if (n) cudaMemsetAsync(d.hits, 0, sizeof(uint32_t) * MASK_WORDS * (size_t)n, b->stream);
-        cudaMemsetAsync(d.xyz, 0, sizeof(float) * 3 * (size_t)d.xyz_stride, b->stream);
+        cudaMemsetAsync(d.pstart, 0, sizeof(uint32_t) * (cells + 1), b->stream);
+        if (n) cudaMemsetAsync(d.hits, 0, sizeof(uint32_t) * hits_words(n), b->stream);
+        if (n) cudaMemsetAsync(d.info, 0, sizeof(uint2) * n, b->stream);
         // the force pass variant of the scenes' flags (a fluid with the same flags gives each scene's
         // result bit for bit)
         const int variant = (b->base[0].flags & WC_FLAG_CELL_TEAMS) ? PASSES_TEAM : PASSES_LANE;
-        b->ld = compute_launch_dims(b->device, variant);
-        sph_occupancy(true, &b->max_density_blocks, &b->max_force_blocks, variant);
+        b->ld = compute_launch_dims(b->device, variant, d.n);
+        sph_occupancy(true, &b->max_density_blocks, &b->max_force_blocks, variant, b->d.n);
         b->ld.grid_density = b->ld.sms * b->max_density_blocks;
         b->ld.grid_force = b->ld.sms * b->max_force_blocks;
         b->tuning = wc_tuning{(uint32_t)b->max_density_blocks, (uint32_t)b->max_force_blocks, 8u, 1.0f, 0.f, 0u,

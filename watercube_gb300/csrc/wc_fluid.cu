@@ -65,7 +65,8 @@ void free_all(wc_fluid* f) {
     void* ptrs[] = {d.pos_a,     d.vel_a,        d.pos_b,     d.vel_b,    d.ids_a,           d.ids_b,
                     d.keys,      d.ranks,        d.unordered, d.perm,     d.counts,          d.start,
                     d.cell_list, d.num_nonempty, d.scan_desc, d.ncount,   d.scan_tile_counter, d.err,
-                    d.hits,      f->staging,     f->flush_buf, f->flush_sink, d.accel,  d.xyz};
+                    d.hits,      f->staging,     f->flush_buf, f->flush_sink, d.accel,  d.xyz,
+                    d.pstart,    d.cidx,         d.rec,       d.info};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (f->h_err) cudaFreeHost(f->h_err);
@@ -95,9 +96,13 @@ wc_status allocate(wc_fluid* f) {
     WC_TRY(dalloc(&d.unordered, n));
     WC_TRY(dalloc(&d.perm, n));
     if (f->params.flags & WC_FLAG_NEIGHBOR_COUNTS) WC_TRY(dalloc(&d.ncount, n));
-    WC_TRY(dalloc(&d.hits, (size_t)n * MASK_WORDS));
-    d.xyz_stride = xyz_stride_for(n);
-    WC_TRY(dalloc(&d.xyz, 3 * (size_t)d.xyz_stride));
+    WC_TRY(dalloc(&d.hits, hits_words(n)));
+    d.pcap = padded_capacity(n, d.num_cells);
+    WC_TRY(dalloc(&d.xyz, 3 * (size_t)d.pcap));
+    WC_TRY(dalloc(&d.cidx, d.pcap));
+    WC_TRY(dalloc(&d.rec, 2 * (size_t)d.pcap));
+    WC_TRY(dalloc(&d.info, n));
+    WC_TRY(dalloc(&d.pstart, (size_t)d.num_cells + 1));
     WC_TRY(dalloc(&d.counts, d.num_cells));
     WC_TRY(dalloc(&d.start, (size_t)d.num_cells + 1));
     WC_TRY(dalloc(&d.cell_list, d.num_cells));
@@ -110,7 +115,7 @@ wc_status allocate(wc_fluid* f) {
     WC_CUDA_TRY(cudaMemsetAsync(d.start, 0, sizeof(uint32_t) * ((size_t)d.num_cells + 1), f->stream));
     WC_CUDA_TRY(cudaMemsetAsync(d.num_nonempty, 0, 3 * sizeof(uint32_t), f->stream));
     WC_CUDA_TRY(cudaMemsetAsync(d.err, 0, sizeof(uint32_t), f->stream));
-    WC_CUDA_TRY(cudaMemsetAsync(d.xyz, 0, sizeof(float) * 3 * (size_t)d.xyz_stride, f->stream));
+    WC_CUDA_TRY(cudaMemsetAsync(d.pstart, 0, sizeof(uint32_t) * ((size_t)d.num_cells + 1), f->stream));
     if (n) {
         WC_CUDA_TRY(cudaMemsetAsync(d.pos_a, 0, sizeof(float4) * n, f->stream));
         WC_CUDA_TRY(cudaMemsetAsync(d.vel_a, 0, sizeof(float4) * n, f->stream));
@@ -119,7 +124,8 @@ wc_status allocate(wc_fluid* f) {
         WC_CUDA_TRY(cudaMemsetAsync(d.perm, 0, sizeof(uint32_t) * n, f->stream));
         WC_CUDA_TRY(cudaMemsetAsync(d.keys, 0, sizeof(uint32_t) * n, f->stream));
         if (d.ncount) WC_CUDA_TRY(cudaMemsetAsync(d.ncount, 0, sizeof(uint32_t) * n, f->stream));
-        WC_CUDA_TRY(cudaMemsetAsync(d.hits, 0, sizeof(uint32_t) * MASK_WORDS * (size_t)n, f->stream));
+        WC_CUDA_TRY(cudaMemsetAsync(d.hits, 0, sizeof(uint32_t) * hits_words(n), f->stream));
+        WC_CUDA_TRY(cudaMemsetAsync(d.info, 0, sizeof(uint2) * n, f->stream));
     }
     WC_CUDA_TRY(cudaStreamSynchronize(f->stream));
     return WC_OK;
@@ -148,12 +154,14 @@ wc_status enqueue_upload(wc_fluid* f, bool state, const wc_particle* in, uint32_
     return WC_OK;
 }
 
-void enqueue_sort(wc_fluid* f) {
+void enqueue_sort(wc_fluid* f, int pass_variant) {
+    const bool lane = pass_variant == PASSES_LANE;
     launch_bin_count(f->d, f->sc, f->ld, f->stream);
-    launch_scan_cells(f->d, f->stream);
+    launch_scan_cells(f->d, f->stream, lane);
     launch_scatter(f->d, f->ld, f->stream);
-    launch_rank_gather(f->d, f->ld, f->stream);
+    launch_rank_gather(f->d, f->ld, f->stream, lane);
 }
+void enqueue_sort(wc_fluid* f) { enqueue_sort(f, f->ld.pass_variant); }
 
 void enqueue_step(wc_fluid* f, const StepInputs& in) {
     enqueue_sort(f);
@@ -210,6 +218,7 @@ wc_status capture_graph(wc_fluid* f, const StepInputs& in) {
     a.hits = f->d.hits;
     a.accel = f->d.accel;
     a.err = f->d.err;
+    a.lane = lane_tables(f->d);
     a.bind();
     f->graph_in = in;
     return WC_OK;
@@ -313,7 +322,9 @@ FluidInternals fluid_internals(wc_fluid* f) {
     return FluidInternals{&f->d, &f->sc, &f->in, &f->params, f->stream};
 }
 
-void fluid_enqueue_sort(wc_fluid* f) { enqueue_sort(f); }
+void fluid_enqueue_sort(wc_fluid* f, int pass_variant) {
+    enqueue_sort(f, pass_variant < 0 ? f->ld.pass_variant : pass_variant);
+}
 
 StepTarget fluid_target(wc_fluid* f) {
     StepTarget t{};
@@ -372,7 +383,7 @@ WC_API wc_status wc_fluid_create(const wc_params* p, wc_fluid** out) {
         delete f;
         return s;
     }
-    f->ld = compute_launch_dims(f->device, (f->params.flags & WC_FLAG_CELL_TEAMS) ? PASSES_TEAM : PASSES_LANE);
+    f->ld = compute_launch_dims(f->device, (f->params.flags & WC_FLAG_CELL_TEAMS) ? PASSES_TEAM : PASSES_LANE, f->d.n);
     f->sc = make_scene_consts(prm);
     f->in = make_step_inputs(prm, 0.0f);
     *out = f;
@@ -438,6 +449,7 @@ WC_API wc_status wc_fluid_integrate(wc_fluid* f, float dt) {
     WC_TRY(require(f, true));
     StepInputs in = f->in;
     in.dt = dt;
+    launch_pack_records(f->d, f->ld, f->stream);  // the caller may have written the sorted buffer
     launch_force(f->d, f->sc, in, f->ld, f->stream);
     WC_TRY(check_launch());
     ++f->steps;
@@ -667,11 +679,11 @@ WC_API wc_status wc_fluid_time_steps(wc_fluid* f, float dt, uint32_t nsteps, int
             cudaEventRecord(ke[0], f->stream);
             launch_bin_count(f->d, f->sc, f->ld, f->stream);
             cudaEventRecord(ke[1], f->stream);
-            launch_scan_cells(f->d, f->stream);
+            launch_scan_cells(f->d, f->stream, f->ld.pass_variant == PASSES_LANE);
             cudaEventRecord(ke[2], f->stream);
             launch_scatter(f->d, f->ld, f->stream);
             cudaEventRecord(ke[3], f->stream);
-            launch_rank_gather(f->d, f->ld, f->stream);
+            launch_rank_gather(f->d, f->ld, f->stream, f->ld.pass_variant == PASSES_LANE);
             cudaEventRecord(ke[4], f->stream);
             launch_density(f->d, f->sc, f->ld, f->stream);
             cudaEventRecord(ke[5], f->stream);

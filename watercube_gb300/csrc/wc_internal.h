@@ -141,8 +141,28 @@ constexpr int MASK_WORDS = 128;
 // Force kernel dense path: per-lane neighbour list capacity ([CAP][32] words per warp).
 constexpr int FORCE_LIST_CAP = 16;
 
-// The stride of DevBuffers::xyz for n particles.
-inline uint32_t xyz_stride_for(uint32_t n) { return ((n + 3u) & ~3u) + 4u; }
+// Lane passes: a target's neighbours as (first candidate, bit mask) entries of 8 bytes in the space of
+// its MASK_WORDS words; the mask's top bit is candidate `first`, and entries of empty masks are
+// not written. A target with more non-empty blocks than LANE_ENTRIES tests its candidates again
+// in the force pass. Entries lie transposed in chunks of 32 targets (entry e of slot ti at
+// (ti / 32 * LANE_ENTRIES + e) * 32 + ti % 32), so a warp's accesses are contiguous.
+constexpr uint32_t LANE_ENTRIES = MASK_WORDS / 2;
+// DevBuffers::info.x beyond an entry count: more blocks than fit, and a slot of an overfull cell.
+constexpr uint32_t INFO_DENSE = 0xfffffffeu, INFO_OVERFULL = 0xffffffffu;
+
+// Words of DevBuffers::hits for n particles: whole chunks of 32.
+inline size_t hits_words(uint64_t n) { return (size_t)((n + 31u) & ~31ull) * MASK_WORDS; }
+
+// The padded slots of the lane passes: every cell's particles start at a multiple of 4 and the
+// places up to the next multiple hold PAD_POSITION in x, y and z, so that four consecutive slots
+// are one aligned 16-byte load per coordinate and never belong to two cells.
+// Far beyond any kernel radius, with a finite squared distance (a padding place contributes
+// 0 x finite = 0 to every sum, where an infinite one would contribute 0 x infinity).
+constexpr float PAD_POSITION = 3e18f;
+inline uint32_t padded_capacity(uint64_t n, uint64_t cells) {
+    const uint64_t c = n + 3u * (n < cells ? n : cells);
+    return (uint32_t)((c + 7u) & ~7ull) + 8u;
+}
 
 struct DevBuffers {
     uint32_t n;          // particles
@@ -163,11 +183,19 @@ struct DevBuffers {
     uint32_t* scan_tile_counter;
     uint32_t* ncount;  // [n] or null
     uint32_t* hits;    // [n * MASK_WORDS] neighbour bit strings
-    // x, y, z of the sorted positions as three float arrays of xyz_stride (a multiple of 4 that
-    // is >= n) elements each, written by the gather for the lane density pass's 16-byte loads of
-    // four consecutive candidates; the padding past n is zero
+    // The lane passes' padded slots (see padded_capacity), written by the lane variant's scan and
+    // gather: pstart is the exclusive prefix of the cells' counts rounded up to 4 (+ total), xyz the
+    // sorted positions' x, y, z as three arrays of pcap elements, cidx the sorted slot of a padded
+    // one (all ones: padding). rec: per padded slot (x, y, z, 1 / density) (v, pressure), 32 bytes
+    // written by the density pass and read by the force pass's neighbour gathers. info: per sorted
+    // slot (entries of its neighbour masks or INFO_*, its padded slot), from the density pass. Only
+    // pstart and info need a first value (zero: no candidates, no neighbours, nothing else read).
+    uint32_t* pstart;  // [C+1]
     float* xyz;
-    uint32_t xyz_stride;
+    uint32_t* cidx;
+    float4* rec;  // [2 pcap]
+    uint2* info;  // [n]
+    uint32_t pcap;
     float4* accel;     // [n] acceleration of each particle in the last force pass, or null
     uint32_t* err;
 };
@@ -189,10 +217,12 @@ struct LaunchDims {
     int pass_variant;
 };
 
-LaunchDims compute_launch_dims(int device, int pass_variant = PASSES_LANE);
+LaunchDims compute_launch_dims(int device, int pass_variant = PASSES_LANE, uint32_t n = 0);
 
 // The learned rollout's judge-step buffers of the force pass (sorted order): `out` receives
 // (J, density rate) per particle, `rate` holds the density pass's (density rate, pressure rate).
+// `rate` has one entry per padded slot; the density pass leaves the slot's own rates in out[ti].zw
+// (pressure rate, density rate) until the force pass overwrites it.
 struct FeatureBuffers {
     float4* out;
     const float2* rate;
@@ -201,14 +231,20 @@ struct FeatureBuffers {
 
 // Stage launchers (wc_sort.cu, wc_sph.cu). All enqueue on `s` and never synchronise.
 void launch_bin_count(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, cudaStream_t s);
-void launch_scan_cells(const DevBuffers& d, cudaStream_t s);
+// lane: the tables of the lane passes (pstart, and the gather's padded arrays) instead of the team
+// passes' list of non-empty cells.
+void launch_scan_cells(const DevBuffers& d, cudaStream_t s, bool lane = false);
 void launch_scatter(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s);
 // vxyz (optional, the learned rollout's judge steps): also the sorted velocities' x, y, z as three
-// arrays of d.xyz_stride elements.
-void launch_rank_gather(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s, float* vxyz = nullptr);
+// arrays of d.pcap elements, in padded slots.
+void launch_rank_gather(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s, bool lane = false,
+                        float* vxyz = nullptr);
 void launch_density(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, cudaStream_t s);
 void launch_force(const DevBuffers& d, const SceneConsts& sc, const StepInputs& in, const LaunchDims& ld,
                   cudaStream_t s);
+// The lane force pass's records again from the sorted buffer, for a force pass that does not
+// directly follow its density pass (the caller may have written the sorted buffer in between).
+void launch_pack_records(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s);
 // Feature levels of the judge step's passes: FEAT_RATE (the stale mode's judge) — the density
 // pass's judge sums and the force pass's own density rate; FEAT_FULL (the Taylor and network
 // modes, and sample recording) — also the density and pressure rates from the density pass
@@ -216,15 +252,15 @@ void launch_force(const DevBuffers& d, const SceneConsts& sc, const StepInputs& 
 enum : int { FEAT_NONE = 0, FEAT_RATE = 1, FEAT_FULL = 2 };
 
 // The learned rollout's judge step runs the lane passes with their feature outputs, whatever
-// ld.pass_variant says: the density pass also writes rate[ti] = (density rate, pressure rate)
+// ld.pass_variant says: the density pass also writes the density and pressure rates (FeatureBuffers)
 // from the gather's velocity arrays vxyz and, when judge_part is given, the judge's sums
-// judge_part[m] = sum over the 32 slots of chunk m of |rho_carried / rho_SPH - 1| (rho_carried:
+// judge_part[m] = sum over the slots of chunk m (lane_chunks) of |rho_carried / rho_SPH - 1| (rho_carried:
 // the sorted buffer's .w before the pass); the force pass reads the neighbours' rates and writes
 // feat[ti] = (J, density rate), J the time derivative of the SPH acceleration (sorted order).
 void launch_density_feat(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, int level,
-                         const float* vxyz, float2* rate, float* judge_part, cudaStream_t s);
+                         const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s);
 void launch_density_batched_feat(const DevBuffers& d, const BatchTables& bt, const LaunchDims& ld, int level,
-                                 const float* vxyz, float2* rate, float* judge_part, cudaStream_t s);
+                                 const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s);
 void launch_force_feat(const DevBuffers& d, const SceneConsts& sc, const StepInputs& in, const LaunchDims& ld,
                        int level, FeatureBuffers fb, cudaStream_t s);
 void launch_force_batched_feat(const DevBuffers& d, const BatchTables& bt, const StepInputs& in, const LaunchDims& ld,
@@ -263,6 +299,32 @@ void launch_density_batched(const DevBuffers& d, const BatchTables& bt, const La
 void launch_force_batched(const DevBuffers& d, const BatchTables& bt, const StepInputs& in, const LaunchDims& ld,
                           cudaStream_t s);
 
+// Targets per lane of the lane density pass over n particles: one, or the two of a pair of padded
+// slots, which share every candidate load and loop step (with ~1.2 padded slots per particle a
+// warp of pairs covers 1.65 times the targets in 1.5 times the time). Pairs halve the warps, so
+// the choice is by waves of the 152 x 32 resident ones, a last partial wave counted as half a
+// wave. Measured per step: 100,000 particles 94 us with one, 97 with pairs; 200,000 121 and 109;
+// 400,000 156 and 165; 1,048,576 (the pass alone) 138 and 125.
+inline uint32_t lane_targets(uint32_t n) {
+    const double resident = 152.0 * 32.0, one = n / (32.0 * resident), pairs = 1.2 * n / (64.0 * resident);
+    auto waves = [](double w) { return w <= 1.0 ? 1.0 : w + 0.5; };
+    return 1.5 * waves(pairs) < waves(one) ? 2u : 1u;
+}
+// Chunks of 32 lanes of that pass, at most (the judge's partial sums are per chunk).
+inline uint32_t lane_chunks(uint32_t n, uint32_t pcap) {
+    return lane_targets(n) == 2u ? (pcap + 63u) / 64u : (n + 31u) / 32u;
+}
+
+// What the lane force pass reads of the padded slots (DevBuffers).
+struct LaneTables {
+    const float4* rec;
+    const uint2* info;
+    const float* xyz;
+    const uint32_t* pstart;
+    uint32_t pcap;
+};
+inline LaneTables lane_tables(const DevBuffers& d) { return LaneTables{d.rec, d.info, d.xyz, d.pstart, d.pcap}; }
+
 // Host copies of the force kernel's arguments, in declaration order, so that a captured step
 // graph's force node can be re-parameterised (dt, gravity, mouse ray) without re-capture.
 struct ForceKernelArgs {
@@ -283,12 +345,13 @@ struct ForceKernelArgs {
     const uint32_t* hits;
     float4* accel;
     uint32_t* err;
+    LaneTables lane{};
     FeatureBuffers feat{};  // the feature buffers of the learned rollout's judge steps (unused here)
-    static constexpr int COUNT = 18;  // every parameter of force_lane_kernel, in order
+    static constexpr int COUNT = 19;  // every parameter of force_lane_kernel, in order
     void* ptrs[COUNT];
     void bind() {
         void* p[COUNT] = {&sc,    &bt,    &in,    &n,     &num_cells, &pos_b,        &vel_b, &ids_b, &pos_a,
-                          &vel_a, &ids_a, &start, &cell_list, &num_nonempty, &hits, &accel, &err, &feat};
+                          &vel_a, &ids_a, &start, &cell_list, &num_nonempty, &hits, &accel, &err, &lane, &feat};
         for (int i = 0; i < COUNT; ++i) ptrs[i] = p[i];
     }
 };
@@ -297,7 +360,7 @@ struct ForceKernelArgs {
 const void* force_kernel_symbol(int pass_variant);
 const void* force_kernel_batched_symbol(int pass_variant);
 // Resident blocks per SM of the two neighbour passes (single-scene or batched variant).
-void sph_occupancy(bool batched, int* density_blocks, int* force_blocks, int pass_variant);
+void sph_occupancy(bool batched, int* density_blocks, int* force_blocks, int pass_variant, uint32_t n);
 
 // Internals of a wc_fluid, for the surrogate (wc_surrogate.cu), which works on a fluid's buffers.
 struct FluidInternals {
@@ -329,7 +392,7 @@ wc_status batch_check(wc_batch* b);                 // launch errors and device 
 wc_status fluid_check(wc_fluid* f);
 // FP64 totals of a fluid's state buffer: mass, momentum x/y/z, kinetic and potential energy.
 wc_status fluid_diagnostics(wc_fluid* f, double out[6]);
-void fluid_enqueue_sort(wc_fluid* f);
+void fluid_enqueue_sort(wc_fluid* f, int pass_variant = -1);  // -1: the fluid's own
 wc_status fluid_graph_step(wc_fluid* f, float dt);  // one plain SPH step (graph replay)
 void fluid_count_step(wc_fluid* f);
 void fluid_set_step_count(wc_fluid* f, uint64_t steps);

@@ -579,12 +579,21 @@ __global__ void __launch_bounds__(32 * OUT) output_mean_kernel(uint32_t ctas, ui
 
 // ---- rollout kernels ----------------------------------------------------------------------------
 
-// Judge: the judge step's density pass sums |rho_carried / rho_SPH - 1| per chunk of 32 sorted
-// slots; this kernel adds the chunk sums in a fixed order, FP32 per thread and warp (a relative
+// Judge: the judge step's density pass sums |rho_carried / rho_SPH - 1| per chunk of 32 lanes; this
+// kernel adds the chunk sums in a fixed order, FP32 per thread and warp (a relative
 // rounding of order 1e-6 against a tolerance of order 1e-2), FP64 across the warps.
 constexpr uint32_t JUDGE_THREADS = 1024;
-__global__ void __launch_bounds__(JUDGE_THREADS) judge_final_kernel(uint32_t chunks, const float* __restrict__ part,
+// padded: with two targets per lane, the number of padded slots (device memory), 64 to a chunk.
+struct JudgeChunks {
+    uint32_t chunks;
+    const uint32_t* padded;
+};
+JudgeChunks judge_chunks(const DevBuffers& d) {
+    return JudgeChunks{lane_chunks(d.n, d.pcap), lane_targets(d.n) == 2u ? d.pstart + d.num_cells : nullptr};
+}
+__global__ void __launch_bounds__(JUDGE_THREADS) judge_final_kernel(const JudgeChunks jc, const float* __restrict__ part,
                                                                     double* __restrict__ out) {
+    const uint32_t chunks = jc.padded ? min(jc.chunks, (*jc.padded + 63u) / 64u) : jc.chunks;
     __shared__ float s[JUDGE_THREADS / 32];
     float a = 0.f;
     for (uint32_t b = threadIdx.x; b < chunks; b += JUDGE_THREADS) a += part[b];
@@ -775,7 +784,7 @@ struct wc_local {
     float4* j0_id = nullptr;  // the judge step's J by particle id (recording)
     float4* feat = nullptr;   // judge step: (J, density rate) per sorted slot
     float2* rate = nullptr;   // judge step's density pass: (density rate, pressure rate) per sorted slot
-    uint32_t cap_n = 0;
+    uint32_t cap_n = 0, cap_p = 0;
     // training scratch
     uint32_t cap_rows = 0;
     __nv_bfloat16 *xb = nullptr, *h1 = nullptr, *h2 = nullptr, *dy16 = nullptr, *dz16 = nullptr;
@@ -789,7 +798,7 @@ struct wc_local {
     float* vxyz = nullptr;  // judge steps: the gather's sorted velocities (x, y, z arrays)
     float4 *save_pos[2] = {nullptr, nullptr}, *save_vel[2] = {nullptr, nullptr};
     uint32_t* save_ids[2] = {nullptr, nullptr};
-    float* judge_part = nullptr;  // per chunk of 32 sorted slots
+    float* judge_part = nullptr;  // per chunk of the density pass (lane_chunks)
     double *judge_out = nullptr, *h_judge = nullptr;
     uint32_t cap_roll = 0;
 };
@@ -914,14 +923,14 @@ void enqueue_closing_judge(wc_local* s, const StepTarget& t) {
         launch_bin_count_batched(d, t.bt, t.ld, t.stream);
     else
         launch_bin_count(d, t.sc, t.ld, t.stream);
-    launch_scan_cells(d, t.stream);
+    launch_scan_cells(d, t.stream, true);
     launch_scatter(d, t.ld, t.stream);
-    launch_rank_gather(d, t.ld, t.stream);
+    launch_rank_gather(d, t.ld, t.stream, true);
     if (t.bt.num_scenes)
-        launch_density_batched_feat(d, t.bt, t.ld, FEAT_RATE, nullptr, nullptr, s->judge_part, t.stream);
+        launch_density_batched_feat(d, t.bt, t.ld, FEAT_RATE, nullptr, nullptr, nullptr, s->judge_part, t.stream);
     else
-        launch_density_feat(d, t.sc, t.ld, FEAT_RATE, nullptr, nullptr, s->judge_part, t.stream);
-    judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(blocks_for(d.n, 32), s->judge_part, s->judge_out);
+        launch_density_feat(d, t.sc, t.ld, FEAT_RATE, nullptr, nullptr, nullptr, s->judge_part, t.stream);
+    judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(judge_chunks(d), s->judge_part, s->judge_out);
 }
 
 // The judge step, on the target's stream: a plain SPH step whose force pass also writes s->feat
@@ -938,20 +947,20 @@ void enqueue_judge_step(wc_local* s, const StepTarget& t, float dt, bool judge, 
     } else {
         launch_bin_count(d, t.sc, t.ld, t.stream);
     }
-    launch_scan_cells(d, t.stream);
+    launch_scan_cells(d, t.stream, true);
     launch_scatter(d, t.ld, t.stream);
     const bool full = level == FEAT_FULL;
-    launch_rank_gather(d, t.ld, t.stream, full ? s->vxyz : nullptr);
+    launch_rank_gather(d, t.ld, t.stream, true, full ? s->vxyz : nullptr);
     const FeatureBuffers fb{s->feat, s->rate};
     float* jp = judge && d.n ? s->judge_part : nullptr;
     if (t.bt.num_scenes) {
-        launch_density_batched_feat(d, t.bt, t.ld, level, s->vxyz, s->rate, jp, t.stream);
+        launch_density_batched_feat(d, t.bt, t.ld, level, s->vxyz, s->rate, s->feat, jp, t.stream);
         launch_force_batched_feat(d, t.bt, in, t.ld, level, fb, t.stream);
     } else {
-        launch_density_feat(d, t.sc, t.ld, level, s->vxyz, s->rate, jp, t.stream);
+        launch_density_feat(d, t.sc, t.ld, level, s->vxyz, s->rate, s->feat, jp, t.stream);
         launch_force_feat(d, t.sc, in, t.ld, level, fb, t.stream);
     }
-    if (jp) judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(blocks_for(d.n, 32), jp, s->judge_out);
+    if (jp) judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(judge_chunks(d), jp, s->judge_out);
 }
 
 wc_status plain_step(const StepTarget& t, float dt) {
@@ -964,8 +973,10 @@ wc_status set_recording(const StepTarget& t, bool on) {
 
 wc_status target_check(const StepTarget& t) { return t.fluid ? fluid_check(t.fluid) : batch_check(t.batch); }
 
-wc_status ensure_n(wc_local* s, uint32_t n) {
-    if (n <= s->cap_n) return WC_OK;
+wc_status ensure_n(wc_local* s, uint32_t n, uint32_t pcap) {
+    if (n <= s->cap_n && pcap <= s->cap_p) return WC_OK;
+    n = std::max(n, s->cap_n);
+    pcap = std::max(pcap, s->cap_p);
     dfree(s->x_id);
     dfree(s->y_id);
     dfree(s->a0_id);
@@ -973,15 +984,18 @@ wc_status ensure_n(wc_local* s, uint32_t n) {
     dfree(s->feat);
     dfree(s->rate);
     dfree(s->vxyz);
-    s->cap_n = 0;
+    dfree(s->judge_part);
+    s->cap_n = s->cap_p = 0;
     WC_TRY(dalloc(&s->x_id, (size_t)n * IN));
     WC_TRY(dalloc(&s->y_id, (size_t)n * YW));
     WC_TRY(dalloc(&s->a0_id, n));
     WC_TRY(dalloc(&s->j0_id, n));
     WC_TRY(dalloc(&s->feat, n));
-    WC_TRY(dalloc(&s->rate, n));
-    WC_TRY(dalloc(&s->vxyz, 3 * (size_t)xyz_stride_for(n)));
+    WC_TRY(dalloc(&s->rate, pcap));
+    WC_TRY(dalloc(&s->judge_part, std::max(blocks_for(n, 32), blocks_for(pcap, 64))));
+    WC_TRY(dalloc(&s->vxyz, 3 * (size_t)pcap));
     s->cap_n = n;
+    s->cap_p = pcap;
     return WC_OK;
 }
 
@@ -1000,7 +1014,7 @@ wc_status record(wc_local* s, const StepTarget& t0, float dt, uint32_t cycles, i
     StepTarget t = t0;
     const uint32_t n = t.d->n;
     if (!t.d->ids_a || !t.d->ids_b) return fail(WC_ERR_STATE, "recording samples needs particle ids (WC_FLAG_TRACK_IDS)");
-    WC_TRY(ensure_n(s, n));
+    WC_TRY(ensure_n(s, n, t.d->pcap));
     WC_TRY(ensure_samples(s, set));
     const bool had_accel = t.d->accel != nullptr;
     if (!had_accel) WC_TRY(set_recording(t, true));
@@ -1203,7 +1217,6 @@ wc_status ensure_roll(wc_local* s, uint32_t n) {
     dfree(s->change);
     dfree(s->mean_part);
     dfree(s->mean);
-    dfree(s->judge_part);
     for (int q = 0; q < 2; ++q) {
         dfree(s->save_pos[q]);
         dfree(s->save_vel[q]);
@@ -1213,7 +1226,6 @@ wc_status ensure_roll(wc_local* s, uint32_t n) {
     WC_TRY(dalloc(&s->change, (size_t)n * CHANGE_LD));
     if (!s->mean_part) WC_TRY(dalloc(&s->mean_part, (size_t)s->sms * MLP_CTAS_PER_SM * OUT));
     if (!s->mean) WC_TRY(dalloc(&s->mean, OUT));
-    WC_TRY(dalloc(&s->judge_part, blocks_for(n, 32)));
     for (int q = 0; q < 2; ++q) {
         WC_TRY(dalloc(&s->save_pos[q], n));
         WC_TRY(dalloc(&s->save_vel[q], n));
@@ -1448,7 +1460,7 @@ WC_API wc_status wc_local_predict(wc_local* s, wc_fluid* f, float dt, float* inp
     if (!s || !f) return fail(WC_ERR_INVALID_ARG, "null argument");
     StepTarget t = fluid_target(f);
     const uint32_t n = t.d->n;
-    WC_TRY(ensure_n(s, n));
+    WC_TRY(ensure_n(s, n, t.d->pcap));
     WC_TRY(ensure_roll(s, n));
     const bool had_accel = t.d->accel != nullptr;
     if (!had_accel) WC_TRY(wc_fluid_set_recording(f, 1));
@@ -1522,7 +1534,7 @@ WC_API wc_status wc_local_rollout_mode(wc_local* s, wc_fluid* f, float dt, uint3
     wc_local* w = s ? s : own;
     StepTarget t = fluid_target(f);
     const uint32_t n = t.d->n;
-    wc_status rc = ensure_n(w, n);
+    wc_status rc = ensure_n(w, n, t.d->pcap);
     if (rc == WC_OK) rc = ensure_roll(w, n);
     const bool had_accel = t.d->accel != nullptr;
     if (rc == WC_OK && !had_accel) rc = wc_fluid_set_recording(f, 1);

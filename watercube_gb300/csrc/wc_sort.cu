@@ -33,7 +33,8 @@ __device__ uint32_t g_scan_stall = 0;
 constexpr unsigned long long DESC_AGG = 1ull << 62;      // tile aggregate published
 constexpr unsigned long long DESC_PREFIX = 2ull << 62;   // inclusive prefix published
 constexpr unsigned long long DESC_VALUE = (1ull << 62) - 1;
-// Packed scan value: bits [0,31) particle count, bits [31,62) non-empty cell count.
+// Packed scan value: bits [0,31) particle count, bits [31,62) non-empty cell count (LANE: the cells'
+// counts rounded up to 4, the padded slots of the lane passes).
 constexpr int NZ_SHIFT = 31;
 constexpr unsigned long long COUNT_MASK = (1ull << NZ_SHIFT) - 1;
 
@@ -121,9 +122,11 @@ __global__ void __launch_bounds__(256) bin_count_kernel(const float4* __restrict
     }
 }
 
+// second: LANE ? the padded starts (+ total) : the list of non-empty cells.
+template <bool LANE>
 __global__ void __launch_bounds__(SCAN_THREADS) scan_cells_kernel(uint32_t* __restrict__ counts, uint32_t C,
                                                                   uint32_t* __restrict__ start,
-                                                                  uint32_t* __restrict__ cell_list,
+                                                                  uint32_t* __restrict__ second,
                                                                   uint32_t* __restrict__ num_nonempty,
                                                                   unsigned long long* desc, uint32_t* tile_counter,
                                                                   uint32_t num_tiles, uint32_t* err) {
@@ -161,7 +164,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_cells_kernel(uint32_t* __re
     }
     unsigned long long tv = 0;
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) tv += ((unsigned long long)(v[k] != 0u) << NZ_SHIFT) | v[k];
+    for (int k = 0; k < SCAN_ITEMS; ++k)
+        tv += ((unsigned long long)(LANE ? ((v[k] + 3u) & ~3u) : (v[k] != 0u ? 1u : 0u)) << NZ_SHIFT) | v[k];
 
     unsigned long long x = tv;
 #pragma unroll
@@ -233,13 +237,19 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_cells_kernel(uint32_t* __re
         const uint32_t c = base + k;
         if (c < C) {
             start[c] = run;
-            if (v[k]) cell_list[nz++] = c;
+            if (LANE) {
+                second[c] = nz;
+                nz += (v[k] + 3u) & ~3u;
+            } else if (v[k]) {
+                second[nz++] = c;
+            }
             run += v[k];
         }
     }
     if (tile == num_tiles - 1 && tid == SCAN_THREADS - 1) {
         start[C] = run;
-        *num_nonempty = nz;
+        if (LANE) second[C] = nz;
+        else *num_nonempty = nz;
     }
 }
 
@@ -260,7 +270,10 @@ __global__ void __launch_bounds__(256) scatter_cells_kernel(uint32_t n, const ui
 // its members in arrival order instead: the stable rank costs O(k) per member, O(k^2) per cell,
 // and an all-NaN state puts every particle in cell 0. Arrival ranks are unique in the cell, so
 // the permutation stays a permutation; the step reports the cell through DEVERR_CELL_OVERFLOW.
-template <bool IDS, bool VEL>
+// LANE: also the lane passes' padded slots (positions, slot index, and velocities with vxyz); the
+// cell's last particle writes the places up to the next multiple of 4: a position far away, whose
+// distance never passes the neighbour test.
+template <bool IDS, bool VEL, bool LANE>
 __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint32_t* __restrict__ keys,
                                                           const uint32_t* __restrict__ ranks,
                                                           const uint32_t* __restrict__ unordered,
@@ -270,8 +283,10 @@ __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint
                                                           const uint32_t* __restrict__ ids_in,
                                                           float4* __restrict__ pos_out, float4* __restrict__ vel_out,
                                                           uint32_t* __restrict__ ids_out, uint32_t* __restrict__ perm,
-                                                          uint32_t* __restrict__ err, float* __restrict__ xyz,
-                                                          uint32_t xyz_stride, float* __restrict__ vxyz) {
+                                                          uint32_t* __restrict__ err,
+                                                          const uint32_t* __restrict__ pstart,
+                                                          uint32_t* __restrict__ cidx, float* __restrict__ xyz,
+                                                          uint32_t pcap, float* __restrict__ vxyz) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t key = keys[i];
         const uint32_t s = start[key], e = min(start[key + 1], n);
@@ -287,16 +302,27 @@ __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint
         perm[dst] = i;
         const float4 p = pos_in[i];
         pos_out[dst] = p;
-        if (xyz) {
-            xyz[dst] = p.x;
-            xyz[xyz_stride + dst] = p.y;
-            xyz[2 * (size_t)xyz_stride + dst] = p.z;
-        }
-        if (VEL && vxyz) {
-            const float4 v = vel_in[i];
-            vxyz[dst] = v.x;
-            vxyz[xyz_stride + dst] = v.y;
-            vxyz[2 * (size_t)xyz_stride + dst] = v.z;
+        if (LANE) {
+            const uint32_t pd = pstart[key] + r;
+            const uint32_t last = s + r + 1u == e ? ((r + 4u) & ~3u) - r : 1u;  // places this thread writes
+            if (pd + last <= pcap) {
+                cidx[pd] = dst;
+                xyz[pd] = p.x;
+                xyz[pcap + pd] = p.y;
+                xyz[2 * (size_t)pcap + pd] = p.z;
+                for (uint32_t q = 1; q < last; ++q) {
+                    cidx[pd + q] = 0xffffffffu;
+                    xyz[pd + q] = xyz[pcap + pd + q] = xyz[2 * (size_t)pcap + pd + q] = PAD_POSITION;
+                }
+                if (VEL && vxyz) {
+                    const float4 v = vel_in[i];
+                    vxyz[pd] = v.x;
+                    vxyz[pcap + pd] = v.y;
+                    vxyz[2 * (size_t)pcap + pd] = v.z;
+                    for (uint32_t q = 1; q < last; ++q)
+                        vxyz[pd + q] = vxyz[pcap + pd + q] = vxyz[2 * (size_t)pcap + pd + q] = 0.f;
+                }
+            }
         }
         if (VEL) vel_out[dst] = vel_in[i];
         if (IDS) ids_out[dst] = ids_in[i];
@@ -352,30 +378,33 @@ void launch_bin_count_batched(const DevBuffers& d, const BatchTables& bt, const 
                                                 d.scan_tile_counter, d.num_tiles, d.err);
 }
 
-void launch_scan_cells(const DevBuffers& d, cudaStream_t s) {
-    scan_cells_kernel<<<d.num_tiles, SCAN_THREADS, 0, s>>>(d.counts, d.num_cells, d.start, d.cell_list,
-                                                           d.num_nonempty, d.scan_desc, d.scan_tile_counter,
-                                                           d.num_tiles, d.err);
+void launch_scan_cells(const DevBuffers& d, cudaStream_t s, bool lane) {
+    if (lane)
+        scan_cells_kernel<true><<<d.num_tiles, SCAN_THREADS, 0, s>>>(d.counts, d.num_cells, d.start, d.pstart,
+                                                                     d.num_nonempty, d.scan_desc, d.scan_tile_counter,
+                                                                     d.num_tiles, d.err);
+    else
+        scan_cells_kernel<false><<<d.num_tiles, SCAN_THREADS, 0, s>>>(d.counts, d.num_cells, d.start, d.cell_list,
+                                                                      d.num_nonempty, d.scan_desc, d.scan_tile_counter,
+                                                                      d.num_tiles, d.err);
 }
 
 void launch_scatter(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s) {
     scatter_cells_kernel<<<grid_for(d.n, ld.grid_stream), 256, 0, s>>>(d.n, d.keys, d.ranks, d.start, d.unordered);
 }
 
-void launch_rank_gather(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s, float* vxyz) {
+template <bool IDS, bool VEL, bool LANE>
+static void launch_gather(const DevBuffers& d, int grid, cudaStream_t s, float* vxyz) {
+    rank_gather_kernel<IDS, VEL, LANE><<<grid, 256, 0, s>>>(d.n, d.keys, d.ranks, d.unordered, d.start, d.pos_a, d.vel_a,
+                                                            d.ids_a, d.pos_b, d.vel_b, d.ids_b, d.perm, d.err, d.pstart,
+                                                            d.cidx, d.xyz, d.pcap, vxyz);
+}
+
+void launch_rank_gather(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s, bool lane, float* vxyz) {
     const int g = grid_for(d.n, ld.grid_stream);
-    if (!d.vel_a)
-        rank_gather_kernel<false, false><<<g, 256, 0, s>>>(d.n, d.keys, d.ranks, d.unordered, d.start, d.pos_a, nullptr,
-                                                           nullptr, d.pos_b, nullptr, nullptr, d.perm, d.err, d.xyz,
-                                                           d.xyz_stride, nullptr);
-    else if (d.ids_a)
-        rank_gather_kernel<true, true><<<g, 256, 0, s>>>(d.n, d.keys, d.ranks, d.unordered, d.start, d.pos_a, d.vel_a,
-                                                         d.ids_a, d.pos_b, d.vel_b, d.ids_b, d.perm, d.err, d.xyz,
-                                                         d.xyz_stride, vxyz);
-    else
-        rank_gather_kernel<false, true><<<g, 256, 0, s>>>(d.n, d.keys, d.ranks, d.unordered, d.start, d.pos_a,
-                                                          d.vel_a, nullptr, d.pos_b, d.vel_b, nullptr, d.perm, d.err,
-                                                          d.xyz, d.xyz_stride, vxyz);
+    if (!d.vel_a) launch_gather<false, false, false>(d, g, s, nullptr);
+    else if (d.ids_a) lane ? launch_gather<true, true, true>(d, g, s, vxyz) : launch_gather<true, true, false>(d, g, s, nullptr);
+    else lane ? launch_gather<false, true, true>(d, g, s, vxyz) : launch_gather<false, true, false>(d, g, s, nullptr);
 }
 
 void launch_aos_to_soa(const float4* aos, float4* pos, float4* vel, uint32_t n, cudaStream_t s) {

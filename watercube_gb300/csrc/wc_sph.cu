@@ -6,7 +6,10 @@
 //                                        and mouse forces), fused with symplectic Euler and the
 //                                        box-wall collision
 //
-// Work decomposition (both kernels): a warp owns one non-empty cell at a time, taking the next
+// Each pass has two variants (PASSES_*): one or two targets per lane (density_lane_kernel,
+// force_lane_kernel, the default, described where they stand) and a warp per cell, as follows.
+//
+// Work decomposition (both team kernels): a warp owns one non-empty cell at a time, taking the next
 // index into the cell list the scan produced from a counter (dynamic scheduling). The 27 neighbour cells of a cell form 9 rows of 3 cells
 // that are contiguous in key order, hence 9 contiguous ranges of the sorted particle buffer;
 // lanes 0..8 look them up once per cell and a 9-lane scan numbers the concatenated candidate
@@ -383,7 +386,8 @@ __device__ __forceinline__ void wall_weight_push(const SceneConsts& c, const flo
 }
 
 __device__ __forceinline__ float write_density(const SceneConsts& sc, float sum, uint32_t hits, const float4& pi,
-                                               uint32_t ti, float* rho_out, float* p_out, uint32_t* ncount) {
+                                               uint32_t ti, float* rho_out, float* p_out, uint32_t* ncount,
+                                               float* pressure_out = nullptr) {
     // The sum includes the particle itself (w = h^2): the reference's m*W(0) term.
     float rho = (sc.m * sc.c6) * sum;
     if (sc.flags & WC_FLAG_WALL_WEIGHTS) rho += wall_weight_density(sc, pi.x, pi.y, pi.z);
@@ -399,15 +403,15 @@ __device__ __forceinline__ float write_density(const SceneConsts& sc, float sum,
     rho_out[4 * (size_t)ti] = total;
     p_out[4 * (size_t)ti] = pressure;
     if (ncount) ncount[ti] = hits - 1u;
+    if (pressure_out) *pressure_out = pressure;
     return total;
 }
 
-// The judge step's rates of one particle from its density-pass sums: the Poly6 density rate
+// The judge step's (density rate, pressure rate) of one particle from its density-pass sums: the Poly6 density rate
 // -6 m c6 sum (cull - d2)^2 (r . u) (the time derivative of m c6 sum (cull - d2)^3 with
 // d(d2)/dt = 2 r . u), and the pressure rate dp/drho times it for the equation of state. The
 // wall terms (wall weights, pseudo wall density) are left out of both.
-__device__ __forceinline__ void write_rates(const SceneConsts& sc, float sum, float rr, uint32_t ti,
-                                            float2* rate_out) {
+__device__ __forceinline__ float2 density_rates(const SceneConsts& sc, float sum, float rr) {
     const float rho = (sc.m * sc.c6) * sum;
     const float rate = -6.f * sc.m * sc.c6 * rr;
     float dp;
@@ -417,7 +421,7 @@ __device__ __forceinline__ void write_rates(const SceneConsts& sc, float sum, fl
         const float x = rho / sc.rho0;
         dp = 3.f * sc.k * x * x / sc.rho0;
     }
-    rate_out[ti] = make_float2(rate, dp * rate);
+    return make_float2(rate, dp * rate);
 }
 
 // Dynamic cell scheduling: every warp takes cells from a counter until it draws an index >= M,
@@ -617,54 +621,74 @@ __global__ void __launch_bounds__(SPH_THREADS, 5) density_kernel(const SceneCons
     release_counter(counter, m, M, lane);
 }
 
-// ---- density, one lane per target -------------------------------------------------------------
+// ---- density, one or two targets per lane ---------------------------------------------------------
 //
-// A warp takes 32 consecutive sorted slots (dynamic scheduling over chunks of 32); each lane owns
-// one target, recomputes its cell from its position (the sort's binning) and walks the 9 row
-// ranges of the cell's 27 neighbour cells, testing every candidate. Lanes of the same cell walk
-// the same candidates in step, so their loads coincide. The target's hits form its bit string in
-// its own candidate numbering (bit b of word w: candidate 32 w + b of the rows concatenated),
-// kept when it fits the slot (at most 32 MASK_WORDS candidates); the lane force pass reads it.
+// A lane owns one target (TARGETS = 1: a warp takes 32 consecutive sorted slots) or the two of a pair
+// of padded slots (TARGETS = 2: a warp takes 64 consecutive padded slots), dynamically scheduled
+// over chunks of 32 lanes. It recomputes its cell from the position (the sort's binning) and walks
+// the 9 row ranges of the cell's 27 neighbour cells in padded slots, four candidates per 16-byte
+// load and coordinate; every cell starts at a multiple of 4 and its padding lies far away, so
+// no place needs a mask, and the sums do not depend on where a cell lies (a scene of a batch sees
+// the same sums as the scene alone, and a pair of targets the same as one).
+// Per block of up to 32 candidates of a row, the misses' sign bits form a word, one funnel shift per
+// candidate; a block with hits other than the target itself becomes an entry (first candidate,
+// mask with candidate j at bit 31 - j) for the force pass.
+// Bound by issue slots (62 % busy) and the latency of the candidate loads at the occupancy its
+// registers leave. 1,048,576 particles at the rest spacing: 172 us with masked quads of the
+// unpadded slots and one target per lane, 138 us with padded cells, 125 us with pairs (130 -> 85 M
+// warp-instructions, 56 -> 41 % of the L1's wavefronts); a fifth of them settled to 5.7 times the
+// density: 371 -> 269 us.
 // FEAT (the learned rollout's judge steps): each hit also adds (cull - d2)^2 (r . u), u = v_i - v_j,
 // to the Poly6 density rate (the candidates' velocities from the gather's arrays vxyz, four at a
-// time like the positions), and the pass writes rate_out[ti] = (density rate, pressure rate);
-// with judge_part it also sums |rho_carried / rho - 1| over each chunk of 32 slots into
-// judge_part[m] (rho_carried: the slot's .w before this pass; a non-finite ratio counts 1).
+// time like the positions), and the pass writes the slot's rates (FeatureBuffers);
+// with judge_part it also sums |rho_carried / rho - 1| over each chunk into judge_part[m]
+// (rho_carried: the slot's .w before this pass; a non-finite ratio counts 1).
 
-// Rows of the 27 neighbour cells of cell (cx, cy, cz): P[r] = first candidate of row r in the
-// concatenated numbering, D[r] = first slot of row r - P[r]; returns the candidate total.
-__device__ __forceinline__ uint32_t lane_rows(const uint32_t* __restrict__ tab, uint32_t n, int32_t R, int cx, int cy,
-                                              int cz, uint32_t P[9], uint32_t D[9]) {
-    uint32_t total = 0;
-#pragma unroll
-    for (int r = 0; r < 9; ++r) {
-        const int yy = cy + (r % 3) - 1, zz = cz + (r / 3) - 1;
-        uint32_t lo = 0, hi = 0;
-        if (yy >= 0 && yy < R && zz >= 0 && zz < R) {
-            const int x0 = cx > 0 ? cx - 1 : 0;
-            const int x1 = cx + 1 < R ? cx + 1 : R - 1;
-            const uint32_t row = (uint32_t)((zz * R + yy) * R);
-            hi = min(__ldg(tab + row + x1 + 1), n);
-            lo = min(__ldg(tab + row + x0), hi);
-        }
-        P[r] = total;
-        D[r] = lo - total;
-        total += hi - lo;
-    }
-    return total;
+// max(v, 0) that keeps a NaN (a non-finite position must not look like an empty neighbourhood).
+__device__ __forceinline__ float relu_nan(float v) {
+    float r;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(v));
+    return r;
 }
 
-template <bool BATCHED, int FEAT = FEAT_NONE>
-__global__ void __launch_bounds__(SPH_THREADS, (FEAT == FEAT_FULL && BATCHED) ? 3 : 4) density_lane_kernel(
+__device__ __forceinline__ void store_record(float4* rec, uint32_t pslot, const float4& pi, float inv_rho, const float4& vi,
+                                             float pressure) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(rec + 2 * (size_t)pslot), "f"(pi.x), "f"(pi.y),
+                 "f"(pi.z), "f"(inv_rho), "f"(vi.x), "f"(vi.y), "f"(vi.z), "f"(pressure)
+                 : "memory");
+}
+__device__ __forceinline__ void load_record(const float4* rec, uint32_t pslot, float4& p, float4& v) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(rec + 2 * (size_t)pslot));
+}
+
+// Slot ti's entry 0; its entry e lies 32 e further.
+__device__ __forceinline__ size_t entry_index(uint32_t ti) { return (size_t)(ti >> 5) * (LANE_ENTRIES * 32u) + (ti & 31u); }
+
+// Row r = (dy, dz) = (r % 3 - 1, r / 3 - 1) of cell (cx, cy, cz): the padded slots [lo, hi) of its three
+// cells. A timed-out scan (reported) leaves inconsistent tables; the range stays in the buffers.
+__device__ __forceinline__ void padded_row(const uint32_t* __restrict__ ptab, uint32_t pcap, int32_t R, int cx, int cy,
+                                           int cz, int r, uint32_t& lo, uint32_t& hi) {
+    const int yy = cy + (r % 3) - 1, zz = cz + (r / 3) - 1;
+    lo = hi = 0;
+    if (yy >= 0 && yy < R && zz >= 0 && zz < R) {
+        const uint32_t row = (uint32_t)((zz * R + yy) * R);
+        hi = min(__ldg(ptab + row + (cx + 1 < R ? cx + 1 : R - 1) + 1), pcap) & ~3u;
+        lo = min(__ldg(ptab + row + (cx > 0 ? cx - 1 : 0)) & ~3u, hi);
+    }
+}
+
+template <bool BATCHED, int FEAT, int TARGETS>
+__global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL ? 2 : 4) density_lane_kernel(
     const SceneConsts sc0, const BatchTables bt, const uint32_t n, const uint32_t num_cells,
     const float4* pos_in,  // its .w lanes are the density output: read with coherent loads
-    float* rho_out, float* p_out, const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_list,
-    uint32_t* __restrict__ num_nonempty,  // [1]: this pass's chunk counter
-    uint32_t* __restrict__ ncount, uint32_t* __restrict__ hits, uint32_t* __restrict__ err,
-    const float* __restrict__ xyz, const uint32_t xyz_stride,  // the gather's x, y, z arrays
-    const float4* vel_in = nullptr,  // FEAT: velocities (their .w lanes are the pressure output)
-    const float* __restrict__ vxyz = nullptr, float2* __restrict__ rate_out = nullptr,
-    float* __restrict__ judge_part = nullptr) {
+    const float4* vel_in,  // its .w lanes are the pressure output
+    float* rho_out, float* p_out, const uint32_t* __restrict__ start, const uint32_t* __restrict__ pstart,
+    const uint32_t* __restrict__ cidx, uint32_t* __restrict__ counter, uint32_t* __restrict__ ncount,
+    uint2* __restrict__ entries, uint2* __restrict__ info, uint32_t* __restrict__ err, const float* __restrict__ xyz,
+    const uint32_t pcap, float4* __restrict__ rec, const float* __restrict__ vxyz = nullptr,
+    float2* __restrict__ rate_out = nullptr, float4* __restrict__ feat = nullptr, float* __restrict__ judge_part = nullptr) {
     __shared__ uint32_t s_poff[BATCHED ? MAX_SCENES + 1 : 1];
     __shared__ uint32_t s_coff[BATCHED ? MAX_SCENES + 1 : 1];
     if (BATCHED) {
@@ -674,136 +698,174 @@ __global__ void __launch_bounds__(SPH_THREADS, (FEAT == FEAT_FULL && BATCHED) ? 
         }
         __syncthreads();
     }
-    (void)cell_list;
-    (void)num_cells;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t M = (n + 31u) >> 5;
-    uint32_t* const counter = num_nonempty + 1;
+    const uint32_t padded = TARGETS == 2 ? min(__ldg(pstart + num_cells), pcap) : 0u;
+    const uint32_t M = TARGETS == 2 ? (padded + 63u) >> 6 : (n + 31u) >> 5;
+    const float* const X = xyz;
+    const float* const Y = xyz + pcap;
+    const float* const Z = xyz + 2 * (size_t)pcap;
     uint32_t m_next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
     uint32_t m = __shfl_sync(FULL, m_next, 0);
     for (; m < M; m = __shfl_sync(FULL, m_next, 0)) {
         if (lane == 0) m_next = atomicAdd(counter, 1u);
-        const uint32_t ti = (m << 5) + lane;
-        float judge = 0.f;  // FEAT with judge_part: this slot's |rho_carried / rho - 1|
+        float judge = 0.f;  // FEAT with judge_part: this lane's |rho_carried / rho - 1|
         do {
-        if (ti >= n) break;
-        SceneConsts sc;
-        uint32_t coff = 0;
-        if (BATCHED) {
-            const uint32_t s = find_scene(s_poff, bt.num_scenes, ti);
-            sc = bt.scenes[s];
-            coff = s_coff[s];
-        } else {
-            sc = sc0;
-        }
-        const uint32_t* tab = start + coff;
-        const float4 pi = pos_in[ti];
-        int32_t cx, cy, cz;
-        const uint32_t c = bin_key(pi.x, pi.y, pi.z, sc.bin, sc.R, &cx, &cy, &cz);
-        const uint32_t cend = min(__ldg(tab + c + 1), n);
-        const uint32_t cbeg = min(__ldg(tab + c), cend);
-        if (cend - cbeg > MAX_CELL_PARTICLES) {
-            // not evaluated (see MAX_CELL_PARTICLES): NaN density and pressure, reported
-            rho_out[4 * (size_t)ti] = __int_as_float(0x7fc00000);
-            p_out[4 * (size_t)ti] = __int_as_float(0x7fc00000);
-            if (ncount) ncount[ti] = 0u;
-            if (FEAT == FEAT_FULL) rate_out[ti] = make_float2(0.f, 0.f);
-            if (ti == cbeg && err) atomicOr(err, DEVERR_CELL_OVERFLOW);
-            judge = 1.f;
-            break;
-        }
-        uint32_t P[9], D[9];
-        const uint32_t total = lane_rows(tab, n, sc.R, cx, cy, cz, P, D);
-        const bool keep = hits != nullptr && total <= 32u * (uint32_t)MASK_WORDS;
-        uint32_t* my_hits = hits ? hits + (size_t)ti * MASK_WORDS : nullptr;
-        float4 vi = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (FEAT == FEAT_FULL) vi = vel_in[ti];
-        float rr = 0.f;  // FEAT: sum of (cull - d2)^2 (r . u)
-        const float* X = xyz;
-        const float* Y = xyz + xyz_stride;
-        const float* Z = xyz + 2 * (size_t)xyz_stride;
-        const float* VX = vxyz;
-        const float* VY = vxyz + xyz_stride;
-        const float* VZ = vxyz + 2 * (size_t)xyz_stride;
-        const f2 px = pk(pi.x, pi.x), py = pk(pi.y, pi.y), pz = pk(pi.z, pi.z), cull2 = pk(sc.cull, sc.cull);
-        const f2 pvx = pk(vi.x, vi.x), pvy = pk(vi.y, vi.y), pvz = pk(vi.z, vi.z);
-        // the weights are added one by one in candidate order, so that the sum does not depend on
-        // where the quads fall (a scene of a batch sees the same sums as the scene alone)
-        float acc = 0.f;
-        uint32_t nh = 0, nbits = 0, wout = 0;
-        unsigned long long buf = 0ull;  // hit bits not yet stored, candidate order
+            uint32_t ti[TARGETS];  // sorted slots (>= n: none)
+            if (TARGETS == 2) {
+                const uint32_t p0 = (m << 6) + 2u * lane;
+                if (p0 >= padded) break;
+                const uint2 c2 = __ldg(reinterpret_cast<const uint2*>(cidx + p0));
+                ti[0] = c2.x;
+                ti[TARGETS - 1] = c2.y;
+            } else {
+                ti[0] = (m << 5) + lane;
+            }
+            if (ti[0] >= n) break;
+            uint32_t coff = 0, s = 0;
+            if (BATCHED) {
+                s = find_scene(s_poff, bt.num_scenes, ti[0]);
+                coff = s_coff[s];
+            }
+            const SceneConsts& sc = BATCHED ? bt.scenes[s] : sc0;
+            float4 pi[TARGETS];
+            pi[0] = pos_in[ti[0]];
+            if (TARGETS == 2) pi[TARGETS - 1] = ti[TARGETS - 1] < n ? pos_in[ti[TARGETS - 1]] : pi[0];
+            int32_t cx, cy, cz;
+            const int32_t R = sc.R;
+            const uint32_t c = bin_key(pi[0].x, pi[0].y, pi[0].z, sc.bin, R, &cx, &cy, &cz);
+            const uint32_t* const ptab = pstart + coff;
+            const uint32_t cend = min(__ldg(start + coff + c + 1), n);
+            const uint32_t cbeg = min(__ldg(start + coff + c), cend);
+            // the lane's first padded slot (a slot outside its cell's range, which only a caller
+            // who overwrote the sorted buffer leaves, is clamped into the buffers)
+            const uint32_t pself = TARGETS == 2 ? (m << 6) + 2u * lane : min(__ldg(ptab + c) + (ti[0] - cbeg), pcap - 1u);
+            if (cend - cbeg > MAX_CELL_PARTICLES) {
+                // not evaluated (see MAX_CELL_PARTICLES): NaN density and pressure, reported
+                const float nan = __int_as_float(0x7fc00000);
 #pragma unroll
-        for (int r = 0; r < 9; ++r) {
-            const uint32_t lo = P[r] + D[r];
-            const uint32_t end = lo + ((r < 8 ? P[r + 1] : total) - P[r]);
-            // the aligned quads of the x, y, z arrays that cover [lo, end), one 16-byte load per
-            // coordinate and the packed f32x2 test (the same fused operations per element as the
-            // scalar test); quad places outside the row are masked out
-            for (uint32_t k = lo & ~3u; k < end; k += 4u) {
-                const ulonglong2 qx = *reinterpret_cast<const ulonglong2*>(X + k);
-                const ulonglong2 qy = *reinterpret_cast<const ulonglong2*>(Y + k);
-                const ulonglong2 qz = *reinterpret_cast<const ulonglong2*>(Z + k);
-                const f2 dx01 = sub2(px, qx.x), dx23 = sub2(px, qx.y);
-                const f2 dy01 = sub2(py, qy.x), dy23 = sub2(py, qy.y);
-                const f2 dz01 = sub2(pz, qz.x), dz23 = sub2(pz, qz.y);
-                const f2 d01 = fma2(dz01, dz01, fma2(dy01, dy01, mul2(dx01, dx01)));
-                const f2 d23 = fma2(dz23, dz23, fma2(dy23, dy23, mul2(dx23, dx23)));
-                // w = cull - d2 >= 0 exactly when d2 <= cull (the reference's sqrtf(d2) < h; a tie
-                // gives +0), and (cull - d2)^3 is Poly6's (h^2 - r^2)^3 with h^2 to the ulp
-                float w0, w1, w2, w3;
-                upk(sub2(cull2, d01), w0, w1);
-                upk(sub2(cull2, d23), w2, w3);
-                const uint32_t s0 = lo > k ? lo - k : 0u;
-                const uint32_t e0 = min(end - k, 4u);
-                const uint32_t valid = (0xFu >> (4u - e0)) & (0xFu << s0);
-                const uint32_t miss = (__float_as_uint(w0) >> 31) | ((__float_as_uint(w1) >> 30) & 2u) |
-                                      ((__float_as_uint(w2) >> 29) & 4u) | ((__float_as_uint(w3) >> 28) & 8u);
-                const uint32_t hit = ~miss & valid;
-                const float g0 = (hit & 1u) ? w0 : 0.f, g1 = (hit & 2u) ? w1 : 0.f;
-                const float g2 = (hit & 4u) ? w2 : 0.f, g3 = (hit & 8u) ? w3 : 0.f;
-                float q0, q1, q2, q3;
-                upk(mul2(pk(g0, g1), pk(g0, g1)), q0, q1);
-                upk(mul2(pk(g2, g3), pk(g2, g3)), q2, q3);
-                acc = fmaf(q0, g0, acc);
-                acc = fmaf(q1, g1, acc);
-                acc = fmaf(q2, g2, acc);
-                acc = fmaf(q3, g3, acc);
-                nh += (uint32_t)__popc(hit);
-                if (FEAT == FEAT_FULL) {
-                    // r . u of the four candidates (packed), added as (cull - d2)^2 (r . u) in order
-                    // (loaded for every quad: skipping the quads without hits diverges and was
-                    // slower)
-                    const ulonglong2 ux = *reinterpret_cast<const ulonglong2*>(VX + k);
-                    const ulonglong2 uy = *reinterpret_cast<const ulonglong2*>(VY + k);
-                    const ulonglong2 uz = *reinterpret_cast<const ulonglong2*>(VZ + k);
-                    const f2 ru01 = fma2(dz01, sub2(pvz, uz.x), fma2(dy01, sub2(pvy, uy.x), mul2(dx01, sub2(pvx, ux.x))));
-                    const f2 ru23 = fma2(dz23, sub2(pvz, uz.y), fma2(dy23, sub2(pvy, uy.y), mul2(dx23, sub2(pvx, ux.y))));
-                    float r0, r1, r2, r3;
-                    upk(ru01, r0, r1);
-                    upk(ru23, r2, r3);
-                    rr = fmaf(q0, r0, rr);
-                    rr = fmaf(q1, r1, rr);
-                    rr = fmaf(q2, r2, rr);
-                    rr = fmaf(q3, r3, rr);
+                for (int t = 0; t < TARGETS; ++t) {
+                    if (ti[t] >= n) continue;
+                    store_record(rec, pself + t, pi[t], nan, vel_in[ti[t]], nan);
+                    rho_out[4 * (size_t)ti[t]] = nan;
+                    p_out[4 * (size_t)ti[t]] = nan;
+                    info[ti[t]] = make_uint2(INFO_OVERFULL, pself + t);
+                    if (ncount) ncount[ti[t]] = 0u;
+                    if (FEAT == FEAT_FULL) {
+                        rate_out[pself + t] = make_float2(0.f, 0.f);
+                        feat[ti[t]] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                    if (ti[t] == cbeg && err) atomicOr(err, DEVERR_CELL_OVERFLOW);
+                    judge += 1.f;
                 }
-                buf |= (unsigned long long)(hit >> s0) << nbits;
-                nbits += e0 - s0;
-                if (nbits >= 32u) {
-                    if (keep) my_hits[wout] = (uint32_t)buf;
-                    ++wout;
-                    buf >>= 32;
-                    nbits -= 32u;
+                break;
+            }
+            const float cull = sc.cull;
+            const f2 cull2 = pk(cull, cull);
+            f2 px[TARGETS], py[TARGETS], pz[TARGETS];
+            float acc[TARGETS], rr[TARGETS];  // Poly6 sum; FEAT_FULL: sum of (cull - d2)^2 (r . u)
+            uint32_t nh[TARGETS], ne[TARGETS];
+            uint2* at[TARGETS];
+            float4 vi[TARGETS];
+#pragma unroll
+            for (int t = 0; t < TARGETS; ++t) {
+                px[t] = pk(pi[t].x, pi[t].x);
+                py[t] = pk(pi[t].y, pi[t].y);
+                pz[t] = pk(pi[t].z, pi[t].z);
+                acc[t] = rr[t] = 0.f;
+                nh[t] = ne[t] = 0;
+                at[t] = entries + entry_index(ti[t] < n ? ti[t] : ti[0]);
+                if (FEAT == FEAT_FULL) vi[t] = vel_in[ti[t] < n ? ti[t] : ti[0]];
+            }
+            uint32_t lo, hi;
+            padded_row(ptab, pcap, R, cx, cy, cz, 0, lo, hi);
+#pragma unroll 1
+            for (int r = 0; r < 9; ++r) {
+                uint32_t k = lo;
+                const uint32_t end = hi;
+                if (r < 8) padded_row(ptab, pcap, R, cx, cy, cz, r + 1, lo, hi);  // overlaps this row's tests
+                while (k < end) {
+                    const uint32_t base = k, stop = min(k + 32u, end);
+                    uint32_t word[TARGETS];
+#pragma unroll
+                    for (int t = 0; t < TARGETS; ++t) word[t] = 0u;
+#pragma unroll 1
+                    for (; k < stop; k += 4u) {
+                        const ulonglong2 qx = *reinterpret_cast<const ulonglong2*>(X + k);
+                        const ulonglong2 qy = *reinterpret_cast<const ulonglong2*>(Y + k);
+                        const ulonglong2 qz = *reinterpret_cast<const ulonglong2*>(Z + k);
+                        ulonglong2 ux, uy, uz;
+                        if (FEAT == FEAT_FULL) {
+                            ux = *reinterpret_cast<const ulonglong2*>(vxyz + k);
+                            uy = *reinterpret_cast<const ulonglong2*>(vxyz + pcap + k);
+                            uz = *reinterpret_cast<const ulonglong2*>(vxyz + 2 * (size_t)pcap + k);
+                        }
+#pragma unroll
+                        for (int t = 0; t < TARGETS; ++t) {
+                            const f2 dx01 = sub2(px[t], qx.x), dx23 = sub2(px[t], qx.y);
+                            const f2 dy01 = sub2(py[t], qy.x), dy23 = sub2(py[t], qy.y);
+                            const f2 dz01 = sub2(pz[t], qz.x), dz23 = sub2(pz[t], qz.y);
+                            const f2 d01 = fma2(dz01, dz01, fma2(dy01, dy01, mul2(dx01, dx01)));
+                            const f2 d23 = fma2(dz23, dz23, fma2(dy23, dy23, mul2(dx23, dx23)));
+                            // w = cull - d2 >= 0 exactly when d2 <= cull (the reference's sqrtf(d2) < h;
+                            // a tie gives +0), and (cull - d2)^3 is Poly6's (h^2 - r^2)^3 with h^2 to
+                            // the ulp
+                            float w0, w1, w2, w3;
+                            upk(sub2(cull2, d01), w0, w1);
+                            upk(sub2(cull2, d23), w2, w3);
+                            word[t] = __funnelshift_l(__float_as_uint(w0), word[t], 1);
+                            word[t] = __funnelshift_l(__float_as_uint(w1), word[t], 1);
+                            word[t] = __funnelshift_l(__float_as_uint(w2), word[t], 1);
+                            word[t] = __funnelshift_l(__float_as_uint(w3), word[t], 1);
+                            // added one by one in candidate order
+                            const float g0 = relu_nan(w0), g1 = relu_nan(w1), g2 = relu_nan(w2), g3 = relu_nan(w3);
+                            float q0, q1, q2, q3;
+                            upk(mul2(pk(g0, g1), pk(g0, g1)), q0, q1);
+                            upk(mul2(pk(g2, g3), pk(g2, g3)), q2, q3);
+                            acc[t] = fmaf(q3, g3, fmaf(q2, g2, fmaf(q1, g1, fmaf(q0, g0, acc[t]))));
+                            if (FEAT == FEAT_FULL) {
+                                const f2 vx = pk(vi[t].x, vi[t].x), vy = pk(vi[t].y, vi[t].y), vz = pk(vi[t].z, vi[t].z);
+                                const f2 ru01 = fma2(dz01, sub2(vz, uz.x), fma2(dy01, sub2(vy, uy.x), mul2(dx01, sub2(vx, ux.x))));
+                                const f2 ru23 = fma2(dz23, sub2(vz, uz.y), fma2(dy23, sub2(vy, uy.y), mul2(dx23, sub2(vx, ux.y))));
+                                float r0, r1, r2, r3;
+                                upk(ru01, r0, r1);
+                                upk(ru23, r2, r3);
+                                rr[t] = fmaf(q3, r3, fmaf(q2, r2, fmaf(q1, r1, fmaf(q0, r0, rr[t]))));
+                            }
+                        }
+                    }
+                    const uint32_t bits = stop - base;
+#pragma unroll
+                    for (int t = 0; t < TARGETS; ++t) {
+                        uint32_t mask = ~word[t] << (32u - bits);
+                        nh[t] += (uint32_t)__popc(mask);
+                        const uint32_t self = pself + t - base;
+                        if (self < 32u) mask &= ~(0x80000000u >> self);
+                        if (mask && ti[t] < n) {
+                            if (ne[t] < LANE_ENTRIES) at[t][32u * ne[t]] = make_uint2(base, mask);
+                            ++ne[t];
+                        }
+                    }
                 }
             }
-        }
-        if (keep && nbits) my_hits[wout] = (uint32_t)buf;
-        if (FEAT == FEAT_FULL) write_rates(sc, acc, rr, ti, rate_out);
-        const float rho_t = write_density(sc, acc, nh, pi, ti, rho_out, p_out, ncount);
-        if (FEAT && judge_part) {
-            // the ratio in FP32 (relative rounding 1e-7 against a tolerance of order 1e-2)
-            const float q = rho_t != 0.f ? fabsf(__fdividef(pi.w, rho_t) - 1.f) : 0.f;
-            judge = isfinite(q) ? q : 1.f;
-        }
+#pragma unroll
+            for (int t = 0; t < TARGETS; ++t) {
+                if (ti[t] >= n) continue;
+                const float4 v = FEAT == FEAT_FULL ? vi[t] : vel_in[ti[t]];
+                float pressure;
+                const float rho_t = write_density(sc, acc[t], nh[t], pi[t], ti[t], rho_out, p_out, ncount, &pressure);
+                store_record(rec, pself + t, pi[t], __fdividef(1.0f, rho_t), v, pressure);
+                info[ti[t]] = make_uint2(ne[t] <= LANE_ENTRIES ? ne[t] : INFO_DENSE, pself + t);
+                if (FEAT == FEAT_FULL) {
+                    const float2 rates = density_rates(sc, acc[t], rr[t]);
+                    rate_out[pself + t] = rates;
+                    feat[ti[t]] = make_float4(0.f, 0.f, rates.y, rates.x);
+                }
+                if (FEAT && judge_part) {
+                    // the ratio in FP32 (relative rounding 1e-7 against a tolerance of order 1e-2)
+                    const float q = rho_t != 0.f ? fabsf(__fdividef(pi[t].w, rho_t) - 1.f) : 0.f;
+                    judge += isfinite(q) ? q : 1.f;
+                }
+            }
         } while (false);
         if (FEAT && judge_part) {
 #pragma unroll
@@ -812,6 +874,20 @@ __global__ void __launch_bounds__(SPH_THREADS, (FEAT == FEAT_FULL && BATCHED) ? 
         }
     }
     if (lane == 0 && m == M + gridDim.x * (uint32_t)WARPS - 1u) atomicExch(counter, 0u);
+}
+
+// The records of the padded slots again from the sorted buffer, for a force pass that does not
+// directly follow its density pass.
+__global__ void __launch_bounds__(256) pack_records_kernel(uint32_t n, const float4* __restrict__ pos,
+                                                           const float4* __restrict__ vel,
+                                                           const uint2* __restrict__ info, uint32_t pcap,
+                                                           float4* __restrict__ rec) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint2 in = info[i];
+        if (in.x == 0u || in.y >= pcap) continue;  // no neighbours: nobody reads its record
+        const float4 p = pos[i], v = vel[i];
+        store_record(rec, in.y, p, __fdividef(1.0f, p.w), v, v.w);
+    }
 }
 
 // ---- force + integration ------------------------------------------------------------------------
@@ -824,7 +900,7 @@ constexpr int force_accumulators() {
     return FEAT == FEAT_FULL ? NF_FEAT : (FEAT == FEAT_RATE ? NF_RATE : NF_PLAIN);
 }
 
-// One neighbour's pressure and viscosity terms. f[0..2] collects pres*(h-d)^2*r/d and f[3..5]
+// One neighbour's pressure and viscosity terms, inv_rho = 1 / rho_j. f[0..2] collects pres*(h-d)^2*r/d and f[3..5]
 // collects (v_j - v_i)*(h-d)/rho_j; the constant factors are applied once per particle.
 // FEAT_FULL (the fast rollout's judge steps): the time derivative of the pressure term, with
 // u = v_i - v_j the rate of r, d' = r.u/d the rate of d and the density pass's rates (rho_j',
@@ -838,13 +914,12 @@ constexpr int force_accumulators() {
 // (cull - d2)^2 (r . u) (times -6 m c6 per particle).
 template <int FEAT = FEAT_NONE>
 __device__ __forceinline__ void pair_terms(const float4& pi, const float4& vi, const float4& pj, const float4& vj,
-                                           float h, float cull, float* f, float pdot_i = 0.f,
+                                           float inv_rho, float h, float cull, float* f, float pdot_i = 0.f,
                                            float2 rj = make_float2(0.f, 0.f)) {
     const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
     const float d2 = dist2(rx, ry, rz);
     const float rsq = d2 > 0.f ? rsqrtf(d2) : 0.f;  // coincident pair (or self): r = 0, no push
     const float d = d2 * rsq;
-    const float inv_rho = __fdividef(1.0f, pj.w);
     const float hd = h - d;
     const float pres = (vi.w + vj.w) * (0.5f * inv_rho);  // (p_i + p_j) / (2 rho_j)
     if (pres > 0.f) {
@@ -879,28 +954,45 @@ __device__ __forceinline__ void pair_terms(const float4& pi, const float4& vi, c
     }
 }
 
-// A lane's list (entries list[e * 32 + lane], e < cnt), four entries per round so their loads
-// overlap; an empty place takes the particle itself (slot self), whose terms are exactly zero.
-// FEAT_FULL: also the neighbours' rates (rate[k]) and the target's pressure rate pdot_i.
-template <int FEAT, int ROUND = 4>
+// The team pass's list of a lane (entries list[e * 32 + lane], e < cnt), four entries per round so
+// their loads overlap; an empty place takes the particle itself (slot self), whose terms are
+// exactly zero.
 __device__ __forceinline__ void accumulate_list(const uint32_t* list, uint32_t cnt, uint32_t lane, uint32_t self,
                                                 const float4& pi, const float4& vi, const float4* __restrict__ pos,
-                                                const float4* __restrict__ vel, float h, float cull, float* f,
-                                                const float2* __restrict__ rate = nullptr, float pdot_i = 0.f) {
-    for (uint32_t e = 0; e < cnt; e += (uint32_t)ROUND) {
-        uint32_t k[ROUND];
+                                                const float4* __restrict__ vel, float h, float cull, float* f) {
+    for (uint32_t e = 0; e < cnt; e += 4u) {
+        uint32_t k[4];
 #pragma unroll
-        for (int u = 0; u < ROUND; ++u) k[u] = e + (uint32_t)u < cnt ? list[(e + (uint32_t)u) * 32u + lane] : self;
+        for (int u = 0; u < 4; ++u) k[u] = e + (uint32_t)u < cnt ? list[(e + (uint32_t)u) * 32u + lane] : self;
+        float4 pj[4], vj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            pj[u] = __ldg(pos + k[u]);
+            vj[u] = __ldg(vel + k[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            pair_terms<FEAT_NONE>(pi, vi, pj[u], vj[u], __fdividef(1.0f, pj[u].w), h, cull, f);
+    }
+}
+
+// The lane pass's: the neighbours' records (padded slots), one 32-byte load each. FEAT_FULL: also
+// their rates and the target's pressure rate pdot_i.
+template <int FEAT, int ROUND>
+__device__ __forceinline__ void accumulate_records(const uint32_t* list, uint32_t cnt, uint32_t self, const float4& pi,
+                                                   const float4& vi, const float4* __restrict__ rec, float h, float cull,
+                                                   float* f, const float2* __restrict__ rate, float pdot_i) {
+    for (uint32_t e = 0; e < cnt; e += (uint32_t)ROUND) {
         float4 pj[ROUND], vj[ROUND];
         float2 rj[ROUND];
 #pragma unroll
         for (int u = 0; u < ROUND; ++u) {
-            pj[u] = __ldg(pos + k[u]);
-            vj[u] = __ldg(vel + k[u]);
-            rj[u] = FEAT == FEAT_FULL ? __ldg(rate + k[u]) : make_float2(0.f, 0.f);
+            const uint32_t k = e + (uint32_t)u < cnt ? list[(e + (uint32_t)u) * 32u] : self;
+            load_record(rec, k, pj[u], vj[u]);
+            rj[u] = FEAT == FEAT_FULL ? __ldg(rate + k) : make_float2(0.f, 0.f);
         }
 #pragma unroll
-        for (int u = 0; u < ROUND; ++u) pair_terms<FEAT>(pi, vi, pj[u], vj[u], h, cull, f, pdot_i, rj[u]);
+        for (int u = 0; u < ROUND; ++u) pair_terms<FEAT>(pi, vi, pj[u], vj[u], pj[u].w, h, cull, f, pdot_i, rj[u]);
     }
 }
 
@@ -978,8 +1070,8 @@ __device__ __forceinline__ void integrate_store(const SceneConsts& sc, const Ste
     }
 }
 
-// The learned rollout's judge steps use the lane force pass (force_lane_kernel<.., true>); `fb`
-// keeps this kernel's parameters those of the lane kernel (one argument list re-parameterises
+// The learned rollout's judge steps use the lane force pass (force_lane_kernel<.., true>); `lt` and `fb`
+// keep this kernel's parameters those of the lane kernel (one argument list re-parameterises
 // the captured force node of either variant).
 template <bool BATCHED>
 __global__ void __launch_bounds__(SPH_THREADS, 4) force_kernel(const SceneConsts sc0, const BatchTables bt,
@@ -995,9 +1087,10 @@ __global__ void __launch_bounds__(SPH_THREADS, 4) force_kernel(const SceneConsts
                                                                uint32_t* __restrict__ num_nonempty,  // [0] cells, [1]/[2] counters
                                                                const uint32_t* __restrict__ hits,
                                                                float4* __restrict__ accel,
-                                                               uint32_t* __restrict__ err,
+                                                               uint32_t* __restrict__ err, const LaneTables lt = {},
                                                                FeatureBuffers fb = {}) {
     (void)fb;
+    (void)lt;
     constexpr int FEAT = FEAT_NONE;
     constexpr int NF = NF_PLAIN;
     // Per warp: the slot table (candidate number -> sorted slot), then the dense path's per-lane
@@ -1127,7 +1220,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 4) force_kernel(const SceneConsts
                             vj[u] = __ldg(vel_b + k[u]);
                         }
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) pair_terms<FEAT>(pi, vi, pj[u], vj[u], sc.h, sc.cull, f);
+                        for (int u = 0; u < 4; ++u) pair_terms<FEAT>(pi, vi, pj[u], vj[u], __fdividef(1.0f, pj[u].w), sc.h, sc.cull, f);
                     }
                 }
             } else if (tm.active) {
@@ -1161,7 +1254,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 4) force_kernel(const SceneConsts
                             vj[u] = __ldg(vel_b + k[u]);
                         }
 #pragma unroll
-                        for (int u = 0; u < 2; ++u) pair_terms<FEAT>(pi, vi, pj[u], vj[u], sc.h, sc.cull, f);
+                        for (int u = 0; u < 2; ++u) pair_terms<FEAT>(pi, vi, pj[u], vj[u], __fdividef(1.0f, pj[u].w), sc.h, sc.cull, f);
                     }
                 }
             }
@@ -1211,7 +1304,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 4) force_kernel(const SceneConsts
                                 list[(cnt++) * 32u + lane] = q < len ? slot[q] : ti;
                             }
                             if (!__any_sync(FULL, word != 0u)) break;
-                            accumulate_list<FEAT>(list, cnt, lane, ti, pi, vi, pos_b, vel_b, sc.h, sc.cull, f);
+                            accumulate_list(list, cnt, lane, ti, pi, vi, pos_b, vel_b, sc.h, sc.cull, f);
                             cnt = 0;
                         }
                     }
@@ -1233,7 +1326,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 4) force_kernel(const SceneConsts
                     const ulonglong2* qx = reinterpret_cast<const ulonglong2*>(fx) + rsl;
                     for (uint32_t j = 0; j < IT; ++j, qx += tm.S) {
                         if (__any_sync(FULL, cnt + 4u > (uint32_t)FORCE_LIST_CAP)) {
-                            accumulate_list<FEAT>(list, cnt, lane, ti, pi, vi, pos_b, vel_b, sc.h, sc.cull, f);
+                            accumulate_list(list, cnt, lane, ti, pi, vi, pos_b, vel_b, sc.h, sc.cull, f);
                             cnt = 0;
                         }
                         uint32_t bits = quad_test<FORCE_STAGE>(qx, px, py, pz, cull2);
@@ -1250,7 +1343,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 4) force_kernel(const SceneConsts
                     }
                 }
             }
-            accumulate_list<FEAT>(list, cnt, lane, ti, pi, vi, pos_b, vel_b, sc.h, sc.cull, f);
+            accumulate_list(list, cnt, lane, ti, pi, vi, pos_b, vel_b, sc.h, sc.cull, f);
 #pragma unroll
             for (int q = 0; q < NF; ++q) f[q] = slice_sum(f[q], tm.S, nt, tm.sl);
             if (tm.sl == 0u) integrate_store<FEAT>(sc, in, pi, vi, f, ti, pos_a, vel_a, ids_b, ids_a, accel);
@@ -1263,14 +1356,19 @@ __global__ void __launch_bounds__(SPH_THREADS, 4) force_kernel(const SceneConsts
 // ---- force + integration, one lane per target ------------------------------------------------
 //
 // A warp takes 32 consecutive sorted slots (dynamic scheduling over chunks of 32) and each lane
-// owns one target. The lane recomputes its cell from its position (the sort's binning) and the 9
-// row ranges of the cell's 27 neighbour cells in the density pass's candidate numbering, and
-// decodes the target's bit string from the lane density pass (bit b of word w: candidate
-// 32 w + b) into a per-lane list of neighbour slots; the list is evaluated four neighbours per
-// round whenever it fills. Targets whose bit string was not kept (more than 32 MASK_WORDS
-// candidates) test their candidates directly.
+// owns one target. The lane decodes the density pass's entries (first candidate, mask) into a
+// per-lane list of neighbour slots, all lanes entry by entry, and the list is evaluated four
+// neighbours per round whenever an entry might not fit: one 32-byte load per neighbour brings
+// its position, reciprocal density, velocity and pressure. No cell table is read and no candidate
+// number mapped to a slot. Bound by the L1's data path (81 % of its wavefronts: the 32 lanes of a load
+// hit ~19 different lines) at three blocks per SM (four fit, but their lists leave half the L1:
+// 354 instead of 372 us in the settled state, 37 instead of 45 us at 80,000 particles).
+// 1,048,576 particles at the rest spacing: 176 -> 121 us against the bit strings in candidate
+// numbering and two 16-byte loads per neighbour (135 -> 82 M warp-instructions); a fifth settled to
+// 5.7 times the density: 408 -> 352 us. A target whose blocks did not fit (INFO_DENSE) tests its candidates
+// again, with the density pass's packed test.
 
-constexpr uint32_t LANE_LIST = 48;  // neighbour slots a lane collects before evaluating them (48: 32 and 64 were slower)
+constexpr uint32_t LANE_LIST = 48;  // neighbour slots a lane collects before evaluating them
 
 // Readback progress (StepInputs part fields): after chunk m every lane fences its stores, and the
 // warp that brings its part's count to the part's size publishes the part: the counter goes back
@@ -1290,41 +1388,28 @@ __device__ __forceinline__ void report_chunk(const StepInputs& in, uint32_t m, u
     }
 }
 
-// The row of candidate q (the last row whose first candidate is <= q) and its slot, from the row
-// starts P[0..8] (P[0] = 0, non-decreasing) and offsets D[r] = first slot of row r - P[r].
-__device__ __forceinline__ uint32_t slot_of(uint32_t q, const uint32_t P[9], const uint32_t D[9]) {
-    const bool b4 = q >= P[4];
-    const bool b2 = q >= (b4 ? P[6] : P[2]);
-    const bool b1 = q >= (b4 ? (b2 ? P[7] : P[5]) : (b2 ? P[3] : P[1]));
-    uint32_t d = b4 ? (b2 ? (b1 ? D[7] : D[6]) : (b1 ? D[5] : D[4])) : (b2 ? (b1 ? D[3] : D[2]) : (b1 ? D[1] : D[0]));
-    if (b4 && b2 && b1 && q >= P[8]) d = D[8];
-    return q + d;
-}
-
 template <bool BATCHED, int FEAT = FEAT_NONE>
-__global__ void __launch_bounds__(SPH_THREADS, (FEAT == FEAT_FULL && BATCHED) ? 2 : 3) force_lane_kernel(
+__global__ void __launch_bounds__(SPH_THREADS, 3) force_lane_kernel(
     const SceneConsts sc0, const BatchTables bt, const StepInputs in, const uint32_t n, const uint32_t num_cells,
     const float4* __restrict__ pos_b, const float4* __restrict__ vel_b, const uint32_t* __restrict__ ids_b,
     float4* __restrict__ pos_a, float4* __restrict__ vel_a, uint32_t* __restrict__ ids_a,
     const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_list,
     uint32_t* __restrict__ num_nonempty,  // [2]: this pass's chunk counter
     const uint32_t* __restrict__ hits, float4* __restrict__ accel, uint32_t* __restrict__ err,
-    FeatureBuffers fb = {}) {  // FEAT: the judge step's rates and feature output
+    const LaneTables lt = {}, FeatureBuffers fb = {}) {  // FEAT: the judge step's rates and feature output
     constexpr int NF = force_accumulators<FEAT>();
     __shared__ uint32_t s_list[WARPS][LANE_LIST * 32];
     __shared__ uint32_t s_poff[BATCHED ? MAX_SCENES + 1 : 1];
-    __shared__ uint32_t s_coff[BATCHED ? MAX_SCENES + 1 : 1];
     if (BATCHED) {
-        for (uint32_t t = threadIdx.x; t <= bt.num_scenes; t += blockDim.x) {
-            s_poff[t] = bt.poff[t];
-            s_coff[t] = bt.coff[t];
-        }
+        for (uint32_t t = threadIdx.x; t <= bt.num_scenes; t += blockDim.x) s_poff[t] = bt.poff[t];
         __syncthreads();
     }
+    (void)start;
     (void)cell_list;
     (void)num_cells;
+    const uint2* const entries = reinterpret_cast<const uint2*>(hits);
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t* list = s_list[threadIdx.x >> 5];
+    uint32_t* const list = s_list[threadIdx.x >> 5] + lane;
     const uint32_t M = (n + 31u) >> 5;  // chunks of 32 slots
     uint32_t* const counter = num_nonempty + 2;
     uint32_t m_next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
@@ -1334,81 +1419,85 @@ __global__ void __launch_bounds__(SPH_THREADS, (FEAT == FEAT_FULL && BATCHED) ? 
         const uint32_t ti = (m << 5) + lane;
         const bool live = ti < n;
         const uint32_t tself = live ? ti : n - 1u;
-        SceneConsts sc;
-        uint32_t coff = 0;
-        if (BATCHED) {
-            const uint32_t s = find_scene(s_poff, bt.num_scenes, tself);
-            sc = bt.scenes[s];
-            coff = s_coff[s];
-        } else {
-            sc = sc0;
-        }
-        const uint32_t* tab = start + coff;
+        const uint32_t s = BATCHED ? find_scene(s_poff, bt.num_scenes, tself) : 0u;
+        const SceneConsts& sc = BATCHED ? bt.scenes[s] : sc0;
+        const uint2 info = __ldg(lt.info + tself);
         const float4 pi = pos_b[tself];
         const float4 vi = vel_b[tself];
-        const float2 ri = FEAT == FEAT_FULL ? fb.rate[tself] : make_float2(0.f, 0.f);
-        int32_t cx, cy, cz;
-        const uint32_t c = bin_key(pi.x, pi.y, pi.z, sc.bin, sc.R, &cx, &cy, &cz);
-        const uint32_t cend = min(__ldg(tab + c + 1), n);
-        const uint32_t cbeg = min(__ldg(tab + c), cend);
-        const uint32_t ncell = cend - cbeg;
-        // rows of the 27 neighbour cells, in the density pass's candidate numbering
-        uint32_t P[9], D[9];
-        const uint32_t total = lane_rows(tab, n, sc.R, cx, cy, cz, P, D);
-        const bool overfull = ncell > MAX_CELL_PARTICLES;
-        // the lane density pass's bit string: word w, bit b is candidate 32 w + b; kept when the
-        // candidates fit the slot
-        const uint32_t inchunk = live && !overfull && ti >= cbeg && ti < cend;
-        const bool kept = hits != nullptr && total <= 32u * (uint32_t)MASK_WORDS;
-        const uint32_t nwords = (total + 31u) >> 5;
+        // the density pass left the slot's rates here: (pressure rate, density rate)
+        const float2 ri = FEAT == FEAT_FULL ? make_float2(fb.out[tself].z, fb.out[tself].w) : make_float2(0.f, 0.f);
+        const float h = sc.h, cull = sc.cull;
+        const uint32_t self = min(info.y, lt.pcap - 1u);
         float f[NF] = {};
-        // candidate generator state: bit strings (w, word) or direct tests (q)
-        bool more = inchunk && total > 0;
-        uint32_t w = 0, word = 0, q = 0;
-        if (more && kept) word = __ldg(hits + (size_t)ti * MASK_WORDS);
-        for (;;) {
-            uint32_t cnt = 0;
-            while (more && cnt < LANE_LIST) {
-                if (kept) {
-                    if (word == 0u) {
-                        if (++w >= nwords) {
-                            more = false;
-                            break;
+        uint32_t cnt = 0;
+        auto flush = [&]() {
+            // J (FEAT_FULL): two neighbours per round, so that the pass fits 80 registers
+            accumulate_records<FEAT, FEAT == FEAT_FULL ? 2 : 4>(list, cnt, self, pi, vi, lt.rec, h, cull, f, fb.rate, ri.x);
+            cnt = 0;
+        };
+        // one entry per lane (mask 0: none), taken by the whole warp together
+        auto take = [&](uint32_t base, uint32_t mask) {
+            if (__any_sync(FULL, cnt + (uint32_t)__popc(mask) > LANE_LIST)) flush();
+            while (mask) {
+                const uint32_t j = (uint32_t)__clz((int)mask);
+                mask ^= 0x80000000u >> j;
+                list[(cnt++) * 32u] = base + j;
+            }
+        };
+        const bool fits = live && info.x <= LANE_ENTRIES;
+        const uint32_t mine = fits ? info.x : 0u;
+        const uint32_t most = __reduce_max_sync(FULL, mine);
+        const uint2* const my = entries + entry_index(tself);
+        uint2 next = mine ? __ldg(my) : make_uint2(0u, 0u);
+        for (uint32_t e = 0; e < most; ++e) {
+            const uint2 cur = next;
+            next = e + 1u < mine ? __ldg(my + 32u * (e + 1u)) : make_uint2(0u, 0u);
+            take(cur.x, cur.y);
+        }
+        const bool dense = live && info.x == INFO_DENSE;
+        if (__any_sync(FULL, dense)) {
+            const uint32_t coff = BATCHED ? __ldg(bt.coff + s) : 0u;
+            int32_t cx, cy, cz;
+            bin_key(pi.x, pi.y, pi.z, sc.bin, sc.R, &cx, &cy, &cz);
+            const f2 px = pk(pi.x, pi.x), py = pk(pi.y, pi.y), pz = pk(pi.z, pi.z), cull2 = pk(cull, cull);
+#pragma unroll 1
+            for (int r = 0; r < 9; ++r) {
+                uint32_t lo = 0, hi = 0;
+                if (dense) padded_row(lt.pstart + coff, lt.pcap, sc.R, cx, cy, cz, r, lo, hi);
+                const uint32_t blocks = __reduce_max_sync(FULL, (hi - lo + 31u) >> 5);
+#pragma unroll 1
+                for (uint32_t b = 0; b < blocks; ++b, lo += 32u) {
+                    uint32_t mask = 0;
+                    if (lo < hi) {
+                        const uint32_t stop = min(lo + 32u, hi);
+                        uint32_t word = 0;
+#pragma unroll 1
+                        for (uint32_t k = lo; k < stop; k += 4u) {
+                            const ulonglong2 qx = *reinterpret_cast<const ulonglong2*>(lt.xyz + k);
+                            const ulonglong2 qy = *reinterpret_cast<const ulonglong2*>(lt.xyz + lt.pcap + k);
+                            const ulonglong2 qz = *reinterpret_cast<const ulonglong2*>(lt.xyz + 2 * (size_t)lt.pcap + k);
+                            const f2 dx01 = sub2(px, qx.x), dx23 = sub2(px, qx.y);
+                            const f2 dy01 = sub2(py, qy.x), dy23 = sub2(py, qy.y);
+                            const f2 dz01 = sub2(pz, qz.x), dz23 = sub2(pz, qz.y);
+                            float w0, w1, w2, w3;
+                            upk(sub2(cull2, fma2(dz01, dz01, fma2(dy01, dy01, mul2(dx01, dx01)))), w0, w1);
+                            upk(sub2(cull2, fma2(dz23, dz23, fma2(dy23, dy23, mul2(dx23, dx23)))), w2, w3);
+                            word = __funnelshift_l(__float_as_uint(w0), word, 1);
+                            word = __funnelshift_l(__float_as_uint(w1), word, 1);
+                            word = __funnelshift_l(__float_as_uint(w2), word, 1);
+                            word = __funnelshift_l(__float_as_uint(w3), word, 1);
                         }
-                        word = __ldg(hits + (size_t)ti * MASK_WORDS + w);
-                        continue;
+                        mask = ~word << (32u - (stop - lo));
+                        if (self - lo < 32u) mask &= ~(0x80000000u >> (self - lo));
                     }
-                    const uint32_t b = (uint32_t)__ffs(word) - 1u;
-                    word &= word - 1u;
-                    const uint32_t cq = 32u * w + b;
-                    // bits always come from this step's density pass over the same tables; the
-                    // check only keeps a stage-by-stage caller's stale bits in bounds
-                    if (cq < total) {
-                        const uint32_t k = slot_of(cq, P, D);
-                        list[cnt * 32u + lane] = k < n ? k : ti;
-                        ++cnt;
-                    }
-                } else {
-                    if (q >= total) {
-                        more = false;
-                        break;
-                    }
-                    const uint32_t k = min(slot_of(q, P, D), n - 1u);
-                    ++q;
-                    const float4 pj = __ldg(pos_b + k);
-                    const float d2 = dist2(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z);
-                    if (d2 <= sc.cull) list[(cnt++) * 32u + lane] = k;  // the target itself adds zero
+                    take(lo, mask);
                 }
             }
-            if (!__any_sync(FULL, cnt > 0u)) break;
-            // J (FEAT_FULL) of a single scene: two neighbours per round, so that the pass fits 80
-            // registers and three blocks per SM (the batched one keeps four and two blocks)
-            accumulate_list<FEAT, (FEAT == FEAT_FULL && !BATCHED) ? 2 : 4>(list, cnt, lane, tself, pi, vi, pos_b, vel_b,
-                                                                          sc.h, sc.cull, f, fb.rate, ri.y);
-            if (!__any_sync(FULL, more)) break;
         }
+        if (__any_sync(FULL, cnt > 0u)) flush();
+        if (__any_sync(FULL, live && info.x == INFO_OVERFULL) && lane == 0 && err) atomicOr(err, DEVERR_CELL_OVERFLOW);
         if (live) {
-            if (overfull) {
+            if (info.x == INFO_OVERFULL) {
                 // not evaluated (see MAX_CELL_PARTICLES): the particle keeps its state, reported
                 pos_a[ti] = pi;
                 vel_a[ti] = vi;
@@ -1419,9 +1508,8 @@ __global__ void __launch_bounds__(SPH_THREADS, (FEAT == FEAT_FULL && BATCHED) ? 
                 if (ids_a) ids_a[ti] = ids_b[ti];
                 if (accel) accel[ti] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (FEAT) fb.out[ti] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (ti == cbeg && err) atomicOr(err, DEVERR_CELL_OVERFLOW);
             } else {
-                integrate_store<FEAT>(sc, in, pi, vi, f, ti, pos_a, vel_a, ids_b, ids_a, accel, fb, ri.x);
+                integrate_store<FEAT>(sc, in, pi, vi, f, ti, pos_a, vel_a, ids_b, ids_a, accel, fb, ri.y);
             }
         }
         if (in.part_done) report_chunk(in, m, M, lane);
@@ -1442,37 +1530,34 @@ static_assert(arity(&force_lane_kernel<true, FEAT_NONE>) == ForceKernelArgs::COU
 
 }  // namespace
 
-void sph_occupancy(bool batched, int* density_blocks, int* force_blocks, int pass_variant) {
-    int bd = 0, bf = 0;
-    if (batched) {
-        if (pass_variant == PASSES_LANE)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, density_lane_kernel<true>, SPH_THREADS, 0);
+template <bool BATCHED>
+static void occupancy(int* bd, int* bf, int pass_variant, uint32_t n) {
+    if (pass_variant == PASSES_LANE) {
+        if (lane_targets(n) == 2u)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(bd, density_lane_kernel<BATCHED, FEAT_NONE, 2>, SPH_THREADS, 0);
         else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, density_kernel<true>, SPH_THREADS, 0);
-        if (pass_variant == PASSES_LANE)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bf, force_lane_kernel<true>, SPH_THREADS, 0);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bf, force_kernel<true>, SPH_THREADS, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(bd, density_lane_kernel<BATCHED, FEAT_NONE, 1>, SPH_THREADS, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(bf, force_lane_kernel<BATCHED>, SPH_THREADS, 0);
     } else {
-        if (pass_variant == PASSES_LANE)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, density_lane_kernel<false>, SPH_THREADS, 0);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, density_kernel<false>, SPH_THREADS, 0);
-        if (pass_variant == PASSES_LANE)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bf, force_lane_kernel<false>, SPH_THREADS, 0);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bf, force_kernel<false>, SPH_THREADS, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(bd, density_kernel<BATCHED>, SPH_THREADS, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(bf, force_kernel<BATCHED>, SPH_THREADS, 0);
     }
+}
+
+void sph_occupancy(bool batched, int* density_blocks, int* force_blocks, int pass_variant, uint32_t n) {
+    int bd = 0, bf = 0;
+    if (batched) occupancy<true>(&bd, &bf, pass_variant, n);
+    else occupancy<false>(&bd, &bf, pass_variant, n);
     *density_blocks = bd > 0 ? bd : 1;
     *force_blocks = bf > 0 ? bf : 1;
 }
 
-LaunchDims compute_launch_dims(int device, int pass_variant) {
+LaunchDims compute_launch_dims(int device, int pass_variant, uint32_t n) {
     LaunchDims ld;
     cudaDeviceGetAttribute(&ld.sms, cudaDevAttrMultiProcessorCount, device);
     if (ld.sms <= 0) ld.sms = 1;
     int bd = 1, bf = 1;
-    sph_occupancy(false, &bd, &bf, pass_variant);
+    sph_occupancy(false, &bd, &bf, pass_variant, n);
     ld.grid_density = ld.sms * bd;
     ld.grid_force = ld.sms * bf;
     ld.grid_stream = ld.sms * 8;
@@ -1480,31 +1565,44 @@ LaunchDims compute_launch_dims(int device, int pass_variant) {
     return ld;
 }
 
-// The density pass of variant `ld.pass_variant`: its bit strings are laid out for the force pass
+namespace {
+template <bool BATCHED, int FEAT, int TARGETS>
+void launch_density_lane(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, int grid, uint32_t* ncount,
+                         const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
+    density_lane_kernel<BATCHED, FEAT, TARGETS><<<grid, SPH_THREADS, 0, s>>>(
+        sc, bt, d.n, d.num_cells, d.pos_b, d.vel_b, reinterpret_cast<float*>(d.pos_b) + 3,
+        reinterpret_cast<float*>(d.vel_b) + 3, d.start, d.pstart, d.cidx, d.num_nonempty + 1, ncount,
+        reinterpret_cast<uint2*>(d.hits), d.info, d.err, d.xyz, d.pcap, d.rec, vxyz, rate, feat, judge_part);
+}
+template <bool BATCHED>
+void launch_density_any(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
+                        uint32_t* ncount, cudaStream_t s) {
+    if (ld.pass_variant != PASSES_LANE)
+        density_kernel<BATCHED><<<ld.grid_density, SPH_THREADS, 0, s>>>(
+            sc, bt, d.n, d.num_cells, d.pos_b, reinterpret_cast<float*>(d.pos_b) + 3,
+            reinterpret_cast<float*>(d.vel_b) + 3, d.start, d.cell_list, d.num_nonempty, ncount, d.hits, d.err);
+    else if (lane_targets(d.n) == 2u)
+        launch_density_lane<BATCHED, FEAT_NONE, 2>(d, sc, bt, ld.grid_density, ncount, nullptr, nullptr, nullptr, nullptr, s);
+    else
+        launch_density_lane<BATCHED, FEAT_NONE, 1>(d, sc, bt, ld.grid_density, ncount, nullptr, nullptr, nullptr, nullptr, s);
+}
+}  // namespace
+
+// The density pass of variant `ld.pass_variant`: its neighbour masks are laid out for the force pass
 // of the same variant.
 void launch_density(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, cudaStream_t s) {
-    uint32_t* nc = (sc.flags & WC_FLAG_NEIGHBOR_COUNTS) ? d.ncount : nullptr;
-    if (ld.pass_variant == PASSES_LANE)
-        density_lane_kernel<false><<<ld.grid_density, SPH_THREADS, 0, s>>>(
-            sc, BatchTables{}, d.n, d.num_cells, d.pos_b, reinterpret_cast<float*>(d.pos_b) + 3,
-            reinterpret_cast<float*>(d.vel_b) + 3, d.start, d.cell_list, d.num_nonempty, nc, d.hits, d.err, d.xyz,
-            d.xyz_stride);
-    else
-        density_kernel<false><<<ld.grid_density, SPH_THREADS, 0, s>>>(
-            sc, BatchTables{}, d.n, d.num_cells, d.pos_b, reinterpret_cast<float*>(d.pos_b) + 3,
-            reinterpret_cast<float*>(d.vel_b) + 3, d.start, d.cell_list, d.num_nonempty, nc, d.hits, d.err);
+    launch_density_any<false>(d, sc, BatchTables{}, ld, (sc.flags & WC_FLAG_NEIGHBOR_COUNTS) ? d.ncount : nullptr, s);
 }
 
 void launch_density_batched(const DevBuffers& d, const BatchTables& bt, const LaunchDims& ld, cudaStream_t s) {
-    if (ld.pass_variant == PASSES_LANE)
-        density_lane_kernel<true><<<ld.grid_density, SPH_THREADS, 0, s>>>(
-            SceneConsts{}, bt, d.n, d.num_cells, d.pos_b, reinterpret_cast<float*>(d.pos_b) + 3,
-            reinterpret_cast<float*>(d.vel_b) + 3, d.start, d.cell_list, d.num_nonempty, d.ncount, d.hits, d.err,
-            d.xyz, d.xyz_stride);
-    else
-        density_kernel<true><<<ld.grid_density, SPH_THREADS, 0, s>>>(
-            SceneConsts{}, bt, d.n, d.num_cells, d.pos_b, reinterpret_cast<float*>(d.pos_b) + 3,
-            reinterpret_cast<float*>(d.vel_b) + 3, d.start, d.cell_list, d.num_nonempty, d.ncount, d.hits, d.err);
+    launch_density_any<true>(d, SceneConsts{}, bt, ld, d.ncount, s);
+}
+
+void launch_pack_records(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s) {
+    if (ld.pass_variant != PASSES_LANE || !d.n) return;
+    const uint32_t blocks = (d.n + 255u) / 256u;
+    pack_records_kernel<<<blocks < (uint32_t)ld.grid_stream ? blocks : (uint32_t)ld.grid_stream, 256, 0, s>>>(
+        d.n, d.pos_b, d.vel_b, d.info, d.pcap, d.rec);
 }
 
 // The force pass of variant `ld.pass_variant` on a persistent grid sized from that kernel's
@@ -1526,11 +1624,11 @@ void launch_force_any(const DevBuffers& d, const SceneConsts& sc, const BatchTab
     if (lane)
         force_lane_kernel<BATCHED, FEAT><<<grid, SPH_THREADS, 0, s>>>(
             sc, bt, in, d.n, d.num_cells, d.pos_b, d.vel_b, d.ids_b, d.pos_a, d.vel_a, d.ids_a, d.start, d.cell_list,
-            d.num_nonempty, d.hits, d.accel, d.err, fb);
+            d.num_nonempty, d.hits, d.accel, d.err, lane_tables(d), fb);
     else
         force_kernel<BATCHED><<<grid, SPH_THREADS, 0, s>>>(sc, bt, in, d.n, d.num_cells, d.pos_b, d.vel_b, d.ids_b,
                                                           d.pos_a, d.vel_a, d.ids_a, d.start, d.cell_list,
-                                                          d.num_nonempty, d.hits, d.accel, d.err, fb);
+                                                          d.num_nonempty, d.hits, d.accel, d.err, lane_tables(d), fb);
 }
 
 void launch_force(const DevBuffers& d, const SceneConsts& sc, const StepInputs& in, const LaunchDims& ld,
@@ -1560,36 +1658,41 @@ void launch_force_batched_feat(const DevBuffers& d, const BatchTables& bt, const
 }
 
 // The judge steps' density pass: the lane kernel with its judge sums (and, FEAT_FULL, rate)
-// output, on a grid of its own occupancy, whatever ld.pass_variant says (its bit strings are the
-// lane force pass's).
-template <bool BATCHED, int FEAT>
-void launch_density_any_feat(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
-                             const float* vxyz, float2* rate, float* judge_part, cudaStream_t s) {
+// output, on a grid of its own occupancy, whatever ld.pass_variant says (its masks are the lane
+// force pass's).
+template <bool BATCHED, int FEAT, int TARGETS>
+void launch_density_feat_as(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
+                            const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
     static int blocks = 0;
     if (!blocks) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, density_lane_kernel<BATCHED, FEAT>, SPH_THREADS, 0);
-        if (blocks <= 0) blocks = 1;
+        int b = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, density_lane_kernel<BATCHED, FEAT, TARGETS>, SPH_THREADS, 0);
+        blocks = b > 0 ? b : 1;
     }
     uint32_t* nc = BATCHED ? d.ncount : ((sc.flags & WC_FLAG_NEIGHBOR_COUNTS) ? d.ncount : nullptr);
-    density_lane_kernel<BATCHED, FEAT><<<ld.sms * blocks, SPH_THREADS, 0, s>>>(
-        sc, bt, d.n, d.num_cells, d.pos_b, reinterpret_cast<float*>(d.pos_b) + 3, reinterpret_cast<float*>(d.vel_b) + 3,
-        d.start, d.cell_list, d.num_nonempty, nc, d.hits, d.err, d.xyz, d.xyz_stride, d.vel_b, vxyz, rate, judge_part);
+    launch_density_lane<BATCHED, FEAT, TARGETS>(d, sc, bt, ld.sms * blocks, nc, vxyz, rate, feat, judge_part, s);
+}
+
+template <bool BATCHED>
+void launch_density_feat_any(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
+                             int level, const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
+    const bool pairs = lane_targets(d.n) == 2u;
+    if (level == FEAT_FULL)
+        pairs ? launch_density_feat_as<BATCHED, FEAT_FULL, 2>(d, sc, bt, ld, vxyz, rate, feat, judge_part, s)
+              : launch_density_feat_as<BATCHED, FEAT_FULL, 1>(d, sc, bt, ld, vxyz, rate, feat, judge_part, s);
+    else
+        pairs ? launch_density_feat_as<BATCHED, FEAT_RATE, 2>(d, sc, bt, ld, vxyz, rate, feat, judge_part, s)
+              : launch_density_feat_as<BATCHED, FEAT_RATE, 1>(d, sc, bt, ld, vxyz, rate, feat, judge_part, s);
 }
 
 void launch_density_feat(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, int level,
-                         const float* vxyz, float2* rate, float* judge_part, cudaStream_t s) {
-    if (level == FEAT_FULL)
-        launch_density_any_feat<false, FEAT_FULL>(d, sc, BatchTables{}, ld, vxyz, rate, judge_part, s);
-    else
-        launch_density_any_feat<false, FEAT_RATE>(d, sc, BatchTables{}, ld, vxyz, rate, judge_part, s);
+                         const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
+    launch_density_feat_any<false>(d, sc, BatchTables{}, ld, level, vxyz, rate, feat, judge_part, s);
 }
 
 void launch_density_batched_feat(const DevBuffers& d, const BatchTables& bt, const LaunchDims& ld, int level,
-                                 const float* vxyz, float2* rate, float* judge_part, cudaStream_t s) {
-    if (level == FEAT_FULL)
-        launch_density_any_feat<true, FEAT_FULL>(d, SceneConsts{}, bt, ld, vxyz, rate, judge_part, s);
-    else
-        launch_density_any_feat<true, FEAT_RATE>(d, SceneConsts{}, bt, ld, vxyz, rate, judge_part, s);
+                                 const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
+    launch_density_feat_any<true>(d, SceneConsts{}, bt, ld, level, vxyz, rate, feat, judge_part, s);
 }
 
 const void* force_kernel_symbol(int pass_variant) {

@@ -771,7 +771,7 @@ struct RolloutRun {
     // SPH density of the state buffer, per state slot.
     void densities(float* rho) {
         DevBuffers& D = *fi.d;
-        fluid_enqueue_sort(f);
+        fluid_enqueue_sort(f, PASSES_LANE);
         launch_density(D, *fi.sc, dims, fi.stream);
         scatter_density(D.n, D.perm, D.pos_b, rho, fi.stream);
     }
@@ -824,7 +824,7 @@ struct RolloutRun {
         const uint32_t n = D.n;
         int device = 0;
         WC_CUDA_TRY(cudaGetDevice(&device));
-        dims = compute_launch_dims(device);
+        dims = compute_launch_dims(device, PASSES_LANE, fi.d->n);
         if (host_hist) {
             WC_CUDA_TRY(cudaMemcpyAsync(s->hist_in, host_hist, sizeof(float4) * 5 * (size_t)n, cudaMemcpyHostToDevice,
                                         fi.stream));
