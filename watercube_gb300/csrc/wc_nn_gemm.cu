@@ -19,13 +19,17 @@
 // Every wait on the mbarrier is bounded; a wait that runs out sets an error flag, and the
 // kernel still releases its tensor memory before it returns.
 //
-// Two kernels: gemm_pipe_kernel (persistent, warp-specialised, an operand ring, B resident in
-// shared memory when it fits, two accumulators, see below) for row-major operands without a
-// split of K — the forward layers and the input gradients; gemm_kernel (one tile per CTA, two operand buffers) for the transposed
-// weight-gradient operands and split-K.
+// Three kernels: gemm_tma_kernel (persistent, operands and results by TMA, see below) for the plain
+// forward layers and input gradients, gemm_pipe_kernel (persistent, warp-specialised, a cp.async
+// operand ring) for gathered or concatenated A, more than 128 columns and unaligned results, and
+// gemm_kernel (one tile per CTA, two operand buffers) for the transposed weight-gradient operands
+// and split-K.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <mutex>
 
 #include "wc_internal.h"
 #include "wc_nn.h"
@@ -508,135 +512,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t v[32]) {
         : "r"(taddr));
 }
 
-// The LayerNorm epilogue (GemmArgs::ln_gamma, n = 128, one column of tiles): the two warps that
-// read the same 32 accumulator lanes (`quarter`) hold a row's 128 columns between them, 64 each
-// (`half`). Each thread sums its 64 values, the pair exchanges the sums through shared memory at
-// a named barrier of its 64 threads (ids 1 .. 4), then the squared deviations from the mean the
-// same way, and each thread normalises, scales and shifts its own columns, adds the residual row
-// and stores BF16. Both warps of a pair pass both barriers of every tile: whether each warp's
-// accumulator wait succeeded is exchanged at the first barrier and the pair leaves together.
-__device__ __forceinline__ void pair_sync(uint32_t quarter) {
-    asm volatile("bar.sync %0, 64;" ::"r"(1u + quarter) : "memory");
-}
-
-__device__ __forceinline__ void drain_accumulators_ln(const GemmArgs& g, uint32_t tmem, uint64_t* acc_full,
-                                                      uint64_t* acc_empty, volatile int* failed, uint32_t ntiles,
-                                                      uint32_t nslices, uint32_t quarter, uint32_t half,
-                                                      uint32_t lane, float (*xs)[2][32], float (*xv)[2][32],
-                                                      int (*oks)[2]) {
-    constexpr float LN_EPSILON = 1e-5f;
-    const uint32_t col0 = 64u * half;
-    // bias, gamma and beta four at a time when all three allow 16-byte loads (uniform branch)
-    const bool vec = ((reinterpret_cast<uintptr_t>(g.ln_gamma) | reinterpret_cast<uintptr_t>(g.ln_beta) |
-                       reinterpret_cast<uintptr_t>(g.bias)) & 15u) == 0;
-    uint32_t t = 0;
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t) {
-        const uint32_t b = t & 1u;
-        bool ok = !*failed && mbar_wait(smem_addr(&acc_full[b]), (t >> 1) & 1u);
-        ok = __all_sync(0xffffffffu, ok);
-        float x[64];
-        if (ok) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t taddr = tmem + ((32u * quarter) << 16) + b * (uint32_t)BN + col0;
-            uint32_t v[32];
-            tmem_ld32(taddr, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = nslices ? __uint_as_float(v[j]) : 0.f;
-            tmem_ld32(taddr + 32u, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 32; ++j) x[32 + j] = nslices ? __uint_as_float(v[j]) : 0.f;
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[b]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 64; ++j) x[j] = 0.f;
-        }
-        if (g.bias) {
-            if (vec) {
-#pragma unroll
-                for (int j = 0; j < 64; j += 4) {
-                    const float4 bb = __ldg(reinterpret_cast<const float4*>(g.bias + col0 + j));
-                    x[j] += bb.x;
-                    x[j + 1] += bb.y;
-                    x[j + 2] += bb.z;
-                    x[j + 3] += bb.w;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 64; ++j) x[j] += __ldg(g.bias + col0 + j);
-            }
-        }
-        float sum = 0.f;
-#pragma unroll
-        for (int j = 0; j < 64; ++j) sum += x[j];
-        xs[quarter][half][lane] = sum;
-        if (lane == 0) oks[quarter][half] = ok ? 1 : 0;
-        pair_sync(quarter);
-        if (!(oks[quarter][0] && oks[quarter][1])) {
-            if (lane == 0) *failed = 1;
-            break;
-        }
-        const float mean = (xs[quarter][0][lane] + xs[quarter][1][lane]) * (1.f / 128.f);
-        float sq = 0.f;
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            x[j] -= mean;
-            sq += x[j] * x[j];
-        }
-        xv[quarter][half][lane] = sq;
-        pair_sync(quarter);
-        const float var = (xv[quarter][0][lane] + xv[quarter][1][lane]) * (1.f / 128.f);
-        const float rstd = rsqrtf(var + LN_EPSILON);
-        const uint32_t row = tile * BM + 32u * quarter + lane;
-        if (row >= g.m) continue;
-        const __nv_bfloat16* res = g.ln_resid ? g.ln_resid + (size_t)row * 128u + col0 : nullptr;
-        __nv_bfloat16* out = g.c_bf16 + (size_t)row * g.ldc + col0;
-#pragma unroll
-        for (int c = 0; c < 64; c += 8) {
-            float gm[8], bt[8];
-            if (vec) {
-#pragma unroll
-                for (int k = 0; k < 8; k += 4) {
-                    const float4 g4 = __ldg(reinterpret_cast<const float4*>(g.ln_gamma + col0 + c + k));
-                    const float4 b4 = __ldg(reinterpret_cast<const float4*>(g.ln_beta + col0 + c + k));
-                    gm[k] = g4.x, gm[k + 1] = g4.y, gm[k + 2] = g4.z, gm[k + 3] = g4.w;
-                    bt[k] = b4.x, bt[k + 1] = b4.y, bt[k + 2] = b4.z, bt[k + 3] = b4.w;
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    gm[k] = __ldg(g.ln_gamma + col0 + c + k);
-                    bt[k] = __ldg(g.ln_beta + col0 + c + k);
-                }
-            }
-            float o[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) o[k] = x[c + k] * rstd * gm[k] + bt[k];
-            if (res) {
-                const uint4 rv = __ldg(reinterpret_cast<const uint4*>(res + c));
-                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&rv);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float2 f = __bfloat1622float2(h[k]);
-                    o[2 * k] += f.x;
-                    o[2 * k + 1] += f.y;
-                }
-            }
-            uint4 w;
-            __nv_bfloat162 q0 = __floats2bfloat162_rn(o[0], o[1]), q1 = __floats2bfloat162_rn(o[2], o[3]);
-            __nv_bfloat162 q2 = __floats2bfloat162_rn(o[4], o[5]), q3 = __floats2bfloat162_rn(o[6], o[7]);
-            w.x = *reinterpret_cast<uint32_t*>(&q0);
-            w.y = *reinterpret_cast<uint32_t*>(&q1);
-            w.z = *reinterpret_cast<uint32_t*>(&q2);
-            w.w = *reinterpret_cast<uint32_t*>(&q3);
-            *reinterpret_cast<uint4*>(out + c) = w;
-        }
-    }
-}
-
 template <bool RB>
 __global__ void __launch_bounds__(PIPE_THREADS, 1) gemm_pipe_kernel(const GemmArgs g, uint32_t* err) {
     constexpr int STAGES = PipeShape<RB>::STAGES, LAG = PipeShape<RB>::LAG;
@@ -787,13 +662,28 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1) gemm_pipe_kernel(const GemmAr
 // For A without a row gather or a second source, and B^T of one column of tiles (n <= 128,
 // k <= 64 RB_MAX_SLICES): one thread of warp 0 copies the operands with cp.async.bulk.tensor
 // (TMA) in the 128-byte-swizzled K-major layout — B^T once per CTA (barrier `b_full`), then the
-// A slices of the CTA's tiles into a 6-slot ring, each copy completing its slot's `full` barrier
+// A slices of the CTA's tiles into a ring, each copy completing its slot's `full` barrier
 // by its byte count (mbarrier expect_tx); warp 1 issues the MMAs with 128-byte-swizzle
 // descriptors (a K step of 16 is a 32-byte advance inside the swizzle atom); warps 2..9 drain
-// the accumulators as in gemm_pipe_kernel. The tensor maps cover this GPU's own global memory;
-// no multicast.
-constexpr int TMA_STAGES = 6;
+// the accumulators, two warps per 32 rows, 64 columns each. The tensor maps cover this GPU's
+// own global memory; no multicast.
+//
+// The epilogue never touches global memory a row per thread (32 lines per instruction): results
+// leave through shared memory and TMA stores, a 32-row box per warp (FP32 accumulation into C as
+// a TMA add), and what it reads per element arrives there first, 128 columns by 128 rows in two
+// stages — the residual rows of a LayerNorm by TMA (AUX_TMA), the gathered rows added to a layer by
+// four more warps with cp.async, 16 lanes to a row (AUX_GATHER). BF16 results are written over
+// the place of the values read. Bound by the traffic it cannot avoid: 460,000 rows of 128 with two
+// gathered rows each take 59 us against 134 us with row-per-thread accesses (62 % of the copy
+// bandwidth for A and C alone, the gathered rows come from L2 on top).
 constexpr int TMA_THREADS = 32 * (2 + PIPE_EPILOGUE);
+constexpr int GATHER_WARPS = 4;
+constexpr int TMA_MAX_STAGES = 6;
+constexpr uint32_t TMA_SMEM_LIMIT = 224u * 1024u;  // dynamic; the barriers and row sums take up to 3 KB more
+enum : int { AUX_NONE = 0, AUX_TMA = 1, AUX_GATHER = 2 };
+constexpr uint32_t AUX_BYTES = BM * 128u * 2u;      // 128 rows of 128 BF16: two halves of 64 columns
+constexpr uint32_t HALF_BYTES = AUX_BYTES / 2u;     // a half's rows of 128 bytes, swizzled
+constexpr uint32_t F32_OUT_BYTES = BM * 128u * 4u;  // per warp two boxes of 32 rows x 32 columns
 
 // Shared-memory descriptor of a K-major operand tile in the 128-byte swizzle layout: rows of
 // 128 bytes, 8-row groups 1,024 bytes apart (SBO), the leading-byte offset unused, version 1.
@@ -821,13 +711,245 @@ __device__ __forceinline__ void tma_load_box(const CUtensorMap* map, void* dst, 
         : "memory");
 }
 
-template <bool LN>
-__global__ void __launch_bounds__(TMA_THREADS, 1) gemm_tma_kernel(const GemmArgs g,
-                                                                  const __grid_constant__ CUtensorMap map_a,
-                                                                  const __grid_constant__ CUtensorMap map_b,
-                                                                  uint32_t* err) {
+// A 32-row box from shared memory to the tensor of `map` (rows and columns outside it are not
+// written), as a store or as an addition to what is there.
+__device__ __forceinline__ void tma_store_box(const CUtensorMap* map, uint32_t src, uint32_t x, uint32_t y, bool add) {
+    if (add)
+        asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                         reinterpret_cast<uint64_t>(map)),
+                     "r"(x), "r"(y), "r"(src)
+                     : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                         reinterpret_cast<uint64_t>(map)),
+                     "r"(x), "r"(y), "r"(src)
+                     : "memory");
+}
+
+// Byte offset of 16-byte chunk c (0..7) of row r in a 128-byte-swizzled block.
+__device__ __forceinline__ uint32_t sw128(uint32_t r, uint32_t c) { return r * 128u + ((c ^ (r & 7u)) << 4); }
+
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+    const __nv_bfloat162 q = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&q);
+}
+// x[0..8) += the eight BF16 of v
+__device__ __forceinline__ void add8(float* x, const uint4& v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        x[2 * k] += __uint_as_float(w[k] << 16);
+        x[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u);
+    }
+}
+
+// Shared memory of the TMA kernel: [B^T slices][A ring][two aux / BF16 output stages][FP32 output].
+struct TmaPlan {
+    uint32_t stages;     // A ring slots
+    uint32_t aux_bytes;  // per stage: operands of 32 KB (AUX_GATHER with two: 64 KB), 0 without BF16 output or aux
+    uint32_t f32_bytes;
+    uint32_t smem;
+};
+
+struct TmaMaps {
+    CUtensorMap a, b, aux, cb, cf;
+};
+
+__device__ __forceinline__ void pair_sync(uint32_t quarter) {
+    asm volatile("bar.sync %0, 64;" ::"r"(1u + quarter) : "memory");
+}
+
+// The epilogue of one warp: rows 32 quarter .., columns 64 half .. of every tile of the CTA.
+// LN (n = 128): the two warps that read the same 32 accumulator lanes hold a row's 128 columns
+// between them. Each thread sums its 64 values, the pair exchanges the sums through shared memory at
+// a named barrier of its 64 threads (ids 1 .. 4), then the squared deviations from the mean the
+// same way, and each thread normalises, scales and shifts its own columns and adds the residual
+// row. Both warps of a pair pass both barriers of every tile: whether each warp's waits succeeded is
+// exchanged at the first barrier and the pair leaves together.
+template <int AUX, bool LN, bool F32, bool BF>
+__device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& maps, const TmaPlan& plan, uint32_t tmem,
+                                             uint64_t* acc_full, uint64_t* acc_empty, uint64_t* aux_full,
+                                             uint64_t* aux_empty, volatile int* failed, uint32_t ntiles, uint32_t quarter,
+                                             uint32_t half, uint32_t lane, uint32_t aux_base, uint32_t f32_base,
+                                             float (*xs)[2][32], float (*xv)[2][32], int (*oks)[2]) {
+    constexpr float LN_EPSILON = 1e-5f;
+    const uint32_t col0 = 64u * half, r = 32u * quarter + lane;
+    const uint32_t f32_buf = f32_base + (quarter * 2u + half) * (F32_OUT_BYTES / 8u);  // this warp's two boxes
+    // bias, gamma and beta four at a time when they allow 16-byte loads of whole tiles (uniform branch)
+    const bool vec = g.n == 128u && ((reinterpret_cast<uintptr_t>(g.bias) | (LN ? reinterpret_cast<uintptr_t>(g.ln_gamma) |
+                                      reinterpret_cast<uintptr_t>(g.ln_beta) : 0)) & 15u) == 0;
+    uint32_t t = 0;
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t) {
+        const uint32_t b = t & 1u;
+        bool ok = !*failed && mbar_wait(smem_addr(&acc_full[b]), (t >> 1) & 1u);
+        if (AUX != AUX_NONE) ok = ok && mbar_wait(smem_addr(&aux_full[b]), (t >> 1) & 1u);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!LN && !ok) {
+            if (lane == 0) *failed = 1;
+            break;
+        }
+        const uint32_t stage = aux_base + b * plan.aux_bytes + half * HALF_BYTES;
+        const uint32_t row0 = tile * BM + 32u * quarter;
+        // The staging this warp is about to write has been read by its earlier stores: two tiles ago
+        // (BF16, two stages), the previous tile's (FP32, one). With aux rows the previous tile's
+        // stage, read by then, goes back to the producer, who fills it during this tile.
+        if (lane == 0) {
+            if (F32 || (AUX != AUX_NONE && BF)) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            if (AUX != AUX_NONE && BF && t > 0) mbar_arrive(&aux_empty[b ^ 1u]);
+        }
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t taddr = tmem + ((32u * quarter) << 16) + b * (uint32_t)BN + col0;
+        auto bias_add = [&](float* x, uint32_t c) {  // 32 columns from c
+            if (!g.bias) return;
+            if (vec) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    const float4 bb = __ldg(reinterpret_cast<const float4*>(g.bias + c + j));
+                    x[j] += bb.x;
+                    x[j + 1] += bb.y;
+                    x[j + 2] += bb.z;
+                    x[j + 3] += bb.w;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (c + j < g.n) x[j] += __ldg(g.bias + c + j);
+            }
+        };
+        if constexpr (LN) {
+            float x[64];
+            if (ok) {
+                uint32_t v[32];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    tmem_ld32(taddr + 32u * q, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) x[32 * q + j] = g.k ? __uint_as_float(v[j]) : 0.f;
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[b]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 64; ++j) x[j] = 0.f;
+            }
+            bias_add(x, col0);
+            bias_add(x + 32, col0 + 32u);
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 64; ++j) sum += x[j];
+            xs[quarter][half][lane] = sum;
+            if (lane == 0) oks[quarter][half] = ok ? 1 : 0;
+            pair_sync(quarter);
+            if (!(oks[quarter][0] && oks[quarter][1])) {
+                if (lane == 0) *failed = 1;
+                break;
+            }
+            const float mean = (xs[quarter][0][lane] + xs[quarter][1][lane]) * (1.f / 128.f);
+            float sq = 0.f;
+#pragma unroll
+            for (int j = 0; j < 64; ++j) {
+                x[j] -= mean;
+                sq += x[j] * x[j];
+            }
+            xv[quarter][half][lane] = sq;
+            pair_sync(quarter);
+            const float var = (xv[quarter][0][lane] + xv[quarter][1][lane]) * (1.f / 128.f);
+            const float rstd = rsqrtf(var + LN_EPSILON);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                float gm[8], bt[8];
+                if (vec) {
+#pragma unroll
+                    for (int k = 0; k < 8; k += 4) {
+                        const float4 g4 = __ldg(reinterpret_cast<const float4*>(g.ln_gamma + col0 + 8 * c + k));
+                        const float4 b4 = __ldg(reinterpret_cast<const float4*>(g.ln_beta + col0 + 8 * c + k));
+                        gm[k] = g4.x, gm[k + 1] = g4.y, gm[k + 2] = g4.z, gm[k + 3] = g4.w;
+                        bt[k] = b4.x, bt[k + 1] = b4.y, bt[k + 2] = b4.z, bt[k + 3] = b4.w;
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        gm[k] = __ldg(g.ln_gamma + col0 + 8 * c + k);
+                        bt[k] = __ldg(g.ln_beta + col0 + 8 * c + k);
+                    }
+                }
+                float o[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) o[k] = x[8 * c + k] * rstd * gm[k] + bt[k];
+                const uint32_t at = stage + sw128(r, (uint32_t)c);
+                if (AUX == AUX_TMA) add8(o, lds128(at));
+                sts128(at, make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7])));
+            }
+        } else {
+#pragma unroll
+            for (uint32_t q = 0; q < 2; ++q) {
+                uint32_t v[32];
+                tmem_ld32(taddr + 32u * q, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                float x[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) x[j] = g.k ? __uint_as_float(v[j]) : 0.f;
+                bias_add(x, col0 + 32u * q);
+#pragma unroll
+                for (uint32_t c = 0; c < 4; ++c) {
+                    float* y = x + 8 * c;
+                    const uint32_t at = stage + sw128(r, 4u * q + c);
+                    if (AUX == AUX_GATHER) {
+                        if (g.add1) add8(y, lds128(at));
+                        if (g.add2) add8(y, lds128(at + (g.add1 ? AUX_BYTES : 0u)));
+                    }
+                    if (g.relu) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) y[k] = fmaxf(y[k], 0.f);
+                    }
+                    if (F32) {
+                        const uint32_t f = f32_buf + q * 4096u;  // columns 32 q .. of this warp's 64
+                        sts128(f + sw128(lane, 2u * c), make_uint4(__float_as_uint(y[0]), __float_as_uint(y[1]),
+                                                                  __float_as_uint(y[2]), __float_as_uint(y[3])));
+                        sts128(f + sw128(lane, 2u * c + 1u), make_uint4(__float_as_uint(y[4]), __float_as_uint(y[5]),
+                                                                       __float_as_uint(y[6]), __float_as_uint(y[7])));
+                    }
+                    if (BF) sts128(at, make_uint4(pack2(y[0], y[1]), pack2(y[2], y[3]), pack2(y[4], y[5]), pack2(y[6], y[7])));
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+            if (!LN) mbar_arrive(&acc_empty[b]);
+            if (row0 < g.m) {
+                if (BF && col0 < g.n) tma_store_box(&maps.cb, stage + 32u * quarter * 128u, col0, row0, false);
+                if (F32 && col0 < g.n) tma_store_box(&maps.cf, f32_buf, col0, row0, g.accumulate != 0);
+                if (F32 && col0 + 32u < g.n) tma_store_box(&maps.cf, f32_buf + 4096u, col0 + 32u, row0, g.accumulate != 0);
+            }
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            if (AUX != AUX_NONE && !BF) mbar_arrive(&aux_empty[b]);  // read, and nothing is stored from it
+        }
+        __syncwarp();
+    }
+    // the stores have left shared memory before the CTA gives it up
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
+}
+
+template <int AUX, bool LN, bool F32, bool BF>
+__global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER_WARPS : 0), 1)
+    gemm_tma_kernel(const GemmArgs g, const __grid_constant__ TmaMaps maps, const TmaPlan plan, uint32_t* err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ uint64_t full[TMA_STAGES], empty[TMA_STAGES], acc_full[2], acc_empty[2], b_full;
+    __shared__ uint64_t full[TMA_MAX_STAGES], empty[TMA_MAX_STAGES], acc_full[2], acc_empty[2], aux_full[2], aux_empty[2], b_full;
     // LN: the warp pairs' exchanged row sums, squared deviations and wait outcomes
     __shared__ float s_lnx[LN ? 4 : 1][2][32], s_lnv[LN ? 4 : 1][2][32];
     __shared__ int s_lnok[LN ? 4 : 1][2];
@@ -835,20 +957,23 @@ __global__ void __launch_bounds__(TMA_THREADS, 1) gemm_tma_kernel(const GemmArgs
     __shared__ int s_failed;
     volatile int* failed = &s_failed;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t tiles_m = (g.m + BM - 1) / BM, tiles_n = 1u;
-    const uint32_t ntiles = tiles_m;
+    const uint32_t ntiles = (g.m + BM - 1) / BM;
     const uint32_t nslices = (g.k + BK - 1) / BK;
-    // [B^T slices 0 .. nslices)[A ring], every slot 16 KB and 1,024-byte aligned
+    const uint32_t stages = plan.stages;
     unsigned char* const ring = smem_raw + nslices * TILE_BYTES;
+    const uint32_t aux_base = smem_addr(ring) + stages * TILE_BYTES;
+    const uint32_t f32_base = aux_base + 2u * plan.aux_bytes;
 
     if (threadIdx.x == 0) {
-        for (int q = 0; q < TMA_STAGES; ++q) {
+        for (uint32_t q = 0; q < stages; ++q) {
             mbar_init(&full[q], 1);
             mbar_init(&empty[q], 1);
         }
         for (int q = 0; q < 2; ++q) {
             mbar_init(&acc_full[q], 1);
             mbar_init(&acc_empty[q], PIPE_EPILOGUE);
+            mbar_init(&aux_full[q], AUX == AUX_GATHER ? 32 * GATHER_WARPS : 1);
+            mbar_init(&aux_empty[q], PIPE_EPILOGUE);
         }
         mbar_init(&b_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -866,21 +991,31 @@ __global__ void __launch_bounds__(TMA_THREADS, 1) gemm_tma_kernel(const GemmArgs
 
     if (warp == 0) {
         if (lane == 0) {
-            // B^T once, then the A slices of every tile through the ring
+            // B^T once, then the A slices (and the epilogue's rows) of every tile
             mbar_expect_tx(&b_full, nslices * TILE_BYTES);
-            for (uint32_t sl = 0; sl < nslices; ++sl) tma_load_box(&map_b, smem_raw + sl * TILE_BYTES, sl * BK, 0u, &b_full);
-            uint32_t it = 0;
-            for (uint32_t tile = blockIdx.x; tile < ntiles && !*failed; tile += gridDim.x) {
+            for (uint32_t sl = 0; sl < nslices; ++sl) tma_load_box(&maps.b, smem_raw + sl * TILE_BYTES, sl * BK, 0u, &b_full);
+            uint32_t it = 0, t = 0;
+            for (uint32_t tile = blockIdx.x; tile < ntiles && !*failed; tile += gridDim.x, ++t) {
                 const uint32_t m0 = tile * BM;
                 for (uint32_t sl = 0; sl < nslices; ++sl, ++it) {
-                    const uint32_t st = it % TMA_STAGES;
-                    if (it >= (uint32_t)TMA_STAGES &&
-                        !mbar_wait(smem_addr(&empty[st]), ((it / TMA_STAGES) - 1u) & 1u)) {
+                    const uint32_t st = it % stages;
+                    if (it >= stages && !mbar_wait(smem_addr(&empty[st]), ((it / stages) - 1u) & 1u)) {
                         *failed = 1;
                         break;
                     }
                     mbar_expect_tx(&full[st], TILE_BYTES);
-                    tma_load_box(&map_a, ring + st * TILE_BYTES, sl * BK, m0, &full[st]);
+                    tma_load_box(&maps.a, ring + st * TILE_BYTES, sl * BK, m0, &full[st]);
+                }
+                if (AUX == AUX_TMA && !*failed) {
+                    const uint32_t b = t & 1u;
+                    if (t >= 2 && !mbar_wait(smem_addr(&aux_empty[b]), ((t >> 1) - 1u) & 1u)) {
+                        *failed = 1;
+                        break;
+                    }
+                    unsigned char* dst = ring + stages * TILE_BYTES + b * plan.aux_bytes;
+                    mbar_expect_tx(&aux_full[b], AUX_BYTES);
+                    tma_load_box(&maps.aux, dst, 0u, m0, &aux_full[b]);
+                    tma_load_box(&maps.aux, dst + HALF_BYTES, 64u, m0, &aux_full[b]);
                 }
             }
         }
@@ -899,8 +1034,8 @@ __global__ void __launch_bounds__(TMA_THREADS, 1) gemm_tma_kernel(const GemmArgs
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc_addr = tmem + b * (uint32_t)BN;
                 for (uint32_t sl = 0; sl < nslices; ++sl, ++it) {
-                    const uint32_t st = it % TMA_STAGES;
-                    if (!mbar_wait(smem_addr(&full[st]), (it / TMA_STAGES) & 1u)) {
+                    const uint32_t st = it % stages;
+                    if (!mbar_wait(smem_addr(&full[st]), (it / stages) & 1u)) {
                         *failed = 1;
                         break;
                     }
@@ -928,14 +1063,48 @@ __global__ void __launch_bounds__(TMA_THREADS, 1) gemm_tma_kernel(const GemmArgs
             }
         }
         __syncwarp();
+    } else if (warp < 2u + PIPE_EPILOGUE) {
+        // warps 2..9: quarter w % 4 (the accumulator lanes its position in the warpgroup may
+        // address), columns 64 ((w - 2) / 4) ..
+        tma_epilogue<AUX, LN, F32, BF>(g, maps, plan, tmem, acc_full, acc_empty, aux_full, aux_empty, failed, ntiles,
+                                       warp & 3u, (warp - 2u) / 4u, lane, aux_base, f32_base, s_lnx, s_lnv, s_lnok);
     } else {
-        // warps 2..9: quarter w % 4, columns 64 ((w - 2) / 4) ..
-        if constexpr (LN)
-            drain_accumulators_ln(g, tmem, acc_full, acc_empty, failed, ntiles, nslices, warp & 3u, (warp - 2u) / 4u,
-                                  lane, s_lnx, s_lnv, s_lnok);
-        else
-            drain_accumulators(g, tmem, acc_full, acc_empty, failed, ntiles, tiles_n, nslices, warp & 3u,
-                               (warp - 2u) / 4u, lane);
+        // AUX_GATHER: warp w copies the gathered rows of tile rows 32 w .. + 31, two rows per
+        // instruction, 16 lanes of 16 bytes each; every thread's copies arrive on the stage's
+        // barrier as they complete. Rows past the matrix are zero-filled.
+        const uint32_t r0 = 32u * (warp - 2u - PIPE_EPILOGUE), chunk = lane & 15u;
+        const __nv_bfloat16* const src[2] = {g.add1, g.add2};
+        const uint32_t* const idx[2] = {g.add1_idx, g.add2_idx};
+        uint32_t t = 0;
+        for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t) {
+            const uint32_t b = t & 1u, row = tile * BM + r0 + lane;
+            uint32_t at[2];
+#pragma unroll
+            for (int o = 0; o < 2; ++o) at[o] = src[o] && row < g.m ? __ldg(idx[o] + row) : 0u;
+            bool ok = !*failed && (t < 2 || mbar_wait(smem_addr(&aux_empty[b]), ((t >> 1) - 1u) & 1u));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+                if (lane == 0) *failed = 1;
+                break;
+            }
+            uint32_t dst = aux_base + b * plan.aux_bytes + (chunk >> 3) * HALF_BYTES;
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                if (!src[o]) continue;
+#pragma unroll 8
+                for (uint32_t q = 0; q < 16u; ++q) {
+                    const uint32_t rr = 2u * q + (lane >> 4);
+                    const uint32_t k = __shfl_sync(0xffffffffu, at[o], (int)rr);
+                    const uint32_t bytes = tile * BM + r0 + rr < g.m ? 16u : 0u;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + sw128(r0 + rr, chunk & 7u)),
+                                 "l"(src[o] + (size_t)k * g.ld_add + 8u * chunk), "r"(bytes)
+                                 : "memory");
+                }
+                dst += AUX_BYTES;
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&aux_full[b])) : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
     }
     __syncthreads();
     if (*failed && threadIdx.x == 0 && err) atomicOr(err, DEVERR_MMA_TIMEOUT);
@@ -996,21 +1165,78 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// A 2-D BF16 row-major tensor [outer x inner] with rows `stride_bytes` apart, read in boxes of
-// 64 x 128 elements with the 128-byte swizzle, out-of-range elements as zeros.
-bool encode_operand(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t stride_bytes) {
+// A 2-D row-major tensor [outer x inner] of BF16 (or FP32) with rows `stride_bytes` apart, accessed in
+// boxes of 128 bytes x `rows` rows with the 128-byte swizzle, out-of-range elements read as zeros.
+bool encode_operand(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t stride_bytes,
+                    uint32_t rows = BM, bool f32 = false) {
     const EncodeTiledFn fn = encode_tiled();
     if (!fn || reinterpret_cast<uintptr_t>(base) % 16u || stride_bytes % 16u || inner == 0 || outer == 0) return false;
     const cuuint64_t dims[2] = {inner, outer};
     const cuuint64_t strides[1] = {stride_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)BM};
+    const cuuint32_t box[2] = {f32 ? 32u : 64u, rows};
     const cuuint32_t elem[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
+              dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 bool gemm_ln_available() { return encode_tiled() != nullptr; }
+
+namespace {
+
+template <int AUX, bool LN, bool F32, bool BF>
+wc_status launch_tma_as(const GemmArgs& g, const TmaMaps& maps, const TmaPlan& plan, uint32_t grid, uint32_t* err,
+                        cudaStream_t s) {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        cudaFuncSetAttribute(gemm_tma_kernel<AUX, LN, F32, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)TMA_SMEM_LIMIT);
+    });
+    const int threads = TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER_WARPS : 0);
+    gemm_tma_kernel<AUX, LN, F32, BF><<<grid, threads, plan.smem, s>>>(g, maps, plan, err);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(WC_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
+    return WC_OK;
+}
+
+// The TMA kernel for plain row-major A, n <= 128 and k <= 384, when every operand it moves by TMA has a
+// tensor map (16-byte aligned base and rows), the gathered rows are whole and aligned, and the shared
+// memory holds at least two A slots (all but k > 256 with two gathered operands, or with FP32 and
+// BF16 outputs together). Otherwise the caller runs the cp.async kernel.
+wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream_t s, bool* launched) {
+    *launched = false;
+    const bool gather = g.add1 || g.add2, aux = gather || g.ln_resid, f32 = g.c_f32 != nullptr, bf = g.c_bf16 != nullptr;
+    TmaMaps maps;
+    if (!encode_operand(&maps.a, g.a, g.k, g.m, 2ull * g.lda) || !encode_operand(&maps.b, g.b, g.k, g.n, 2ull * g.ldb))
+        return WC_OK;
+    if (bf && !encode_operand(&maps.cb, g.c_bf16, g.n, g.m, 2ull * g.ldc, 32)) return WC_OK;
+    if (f32 && !encode_operand(&maps.cf, g.c_f32, g.n, g.m, 4ull * g.ldc, 32, true)) return WC_OK;
+    if (g.ln_resid && !encode_operand(&maps.aux, g.ln_resid, 128, g.m, 256)) return WC_OK;
+    if (gather && (g.n != 128u || g.ld_add % 8u || reinterpret_cast<uintptr_t>(g.add1) % 16u ||
+                   reinterpret_cast<uintptr_t>(g.add2) % 16u))
+        return WC_OK;
+    const uint32_t nslices = (g.k + BK - 1) / BK;
+    TmaPlan plan{};
+    plan.aux_bytes = (g.add1 && g.add2) ? 2u * AUX_BYTES : (aux || bf) ? AUX_BYTES : 0u;
+    plan.f32_bytes = f32 ? F32_OUT_BYTES : 0u;
+    const uint32_t fixed = nslices * TILE_BYTES + 2u * plan.aux_bytes + plan.f32_bytes;
+    if (fixed + 2u * TILE_BYTES > TMA_SMEM_LIMIT) return WC_OK;
+    plan.stages = std::min<uint32_t>(TMA_MAX_STAGES, (TMA_SMEM_LIMIT - fixed) / TILE_BYTES);
+    plan.smem = fixed + plan.stages * TILE_BYTES;
+    *launched = true;
+    if (g.ln_gamma)
+        return aux ? launch_tma_as<AUX_TMA, true, false, true>(g, maps, plan, grid, err, s)
+                   : launch_tma_as<AUX_NONE, true, false, true>(g, maps, plan, grid, err, s);
+    if (gather)
+        return f32 ? (bf ? launch_tma_as<AUX_GATHER, false, true, true>(g, maps, plan, grid, err, s)
+                         : launch_tma_as<AUX_GATHER, false, true, false>(g, maps, plan, grid, err, s))
+                   : launch_tma_as<AUX_GATHER, false, false, true>(g, maps, plan, grid, err, s);
+    return f32 ? (bf ? launch_tma_as<AUX_NONE, false, true, true>(g, maps, plan, grid, err, s)
+                     : launch_tma_as<AUX_NONE, false, true, false>(g, maps, plan, grid, err, s))
+               : launch_tma_as<AUX_NONE, false, false, true>(g, maps, plan, grid, err, s);
+}
+
+}  // namespace
 
 wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s) {
     const wc_status st = check_gemm(g);
@@ -1033,25 +1259,9 @@ wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s) {
         const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
         const bool rb = g.n <= (uint32_t)BN && (g.k + BK - 1) / BK <= RB_MAX_SLICES;
         if (rb && !g.a_rows && !g.a2) {
-            // plain A: the TMA kernel, when both operands have tensor maps
-            CUtensorMap ma, mb;
-            if (encode_operand(&ma, g.a, g.k, g.m, 2ull * g.lda) && encode_operand(&mb, g.b, g.k, g.n, 2ull * g.ldb)) {
-                static bool tma_attr = false;
-                if (!tma_attr) {
-                    cudaFuncSetAttribute(gemm_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)pipe_smem_bytes(true, RB_MAX_SLICES * BK));
-                    cudaFuncSetAttribute(gemm_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)pipe_smem_bytes(true, RB_MAX_SLICES * BK));
-                    tma_attr = true;
-                }
-                if (g.ln_gamma)
-                    gemm_tma_kernel<true><<<grid, TMA_THREADS, pipe_smem_bytes(true, g.k), s>>>(g, ma, mb, err);
-                else
-                    gemm_tma_kernel<false><<<grid, TMA_THREADS, pipe_smem_bytes(true, g.k), s>>>(g, ma, mb, err);
-                const cudaError_t e = cudaGetLastError();
-                if (e != cudaSuccess) return fail(WC_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
-                return WC_OK;
-            }
+            bool launched = false;
+            WC_TRY(launch_tma(g, grid, err, s, &launched));
+            if (launched) return WC_OK;
         }
         if (g.ln_gamma) return fail(WC_ERR_STATE, "gemm: the LayerNorm epilogue needs the TMA kernel (plain A, k <= 384)");
         if (rb)
