@@ -63,3 +63,18 @@ def test_unaligned_result(wclib, torch):  # noqa: F811
     c = torch.zeros(m * 131 + 1, device="cuda")  # rows of 131 floats from an odd address
     run(wclib, torch, m=m, n=n, k=k, a=a, lda=k, b=wt, ldb=k, c_f32=c[1:], ldc=131)
     close(c[1:].view(m, 131)[:, :n], a.float() @ wt.float().t())
+
+
+@pytest.mark.parametrize("m,n", [(128, 128), (16, 128), (128, 16), (72, 40), (8, 8)])
+@pytest.mark.parametrize("k,chunk", [(1, 64), (63, 64), (65, 64), (1000, 128), (40003, 192)])
+def test_weight_gradient_splits(wclib, torch, m, n, k, chunk):  # noqa: F811
+    """X^T dY per split of the rows, the last one ragged; the tolerance is close()'s, of FP32 sums of
+    exact products in another order."""
+    x, dy = rnd(torch, k, m, seed=1), rnd(torch, k, n, seed=2)
+    parts = -(-k // chunk)
+    out = torch.full((parts + 1, m, n), 7.0, device="cuda")
+    run(wclib, torch, m=m, n=n, k=k, k_chunk=chunk, a=x, lda=m, a_transposed=1, b=dy, ldb=n, b_rowmajor=1, c_f32=out,
+        ldc=n, split_stride=m * n)
+    ref = torch.stack([p.float().t() @ q.float() for p, q in zip(x.split(chunk), dy.split(chunk))])
+    close(out[:parts], ref)
+    assert bool((out[parts] == 7.0).all())

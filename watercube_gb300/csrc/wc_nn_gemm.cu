@@ -1114,6 +1114,129 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
     }
 }
 
+// ---- weight gradients: C = X^T dY, both operands read along their rows ---------------------------
+//
+// A transposed and B row-major (m, n <= 128; X [k x m], dY [k x n]): a slice of 64 rows of either is
+// 64 x 64 boxes that TMA copies into shared memory as they lie, 128 bytes of columns per row,
+// 128-byte swizzle, which is the tensor core's MN-major operand layout (8-row groups 1,024 bytes
+// apart, the next 64 columns 8,192), so nothing is transposed on the way. One CTA per split of the
+// rows, three 32 KB slots, two CTAs per SM: one thread feeds the ring, one issues the MMAs, then
+// four warps drain the accumulator. Bound by the operands' bytes: 459,213 rows of 128 + 128 in 248
+// splits take 49 us (5.1 TB/s, 75 % of the copy bandwidth) against 127 us with register transposes
+// and two synchronous buffers (gemm_kernel, which keeps m or n > 128 and unaligned operands).
+constexpr int WG_STAGES = 3;
+constexpr uint32_t WG_SLOT = 2u * TILE_BYTES;
+constexpr uint32_t WG_SMEM = WG_STAGES * WG_SLOT;
+
+// Shared-memory descriptor of an MN-major operand in the 128-byte swizzle layout.
+__device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t saddr) {
+    uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
+    d |= (uint64_t)(8192u >> 4) << 16;  // the next 64 columns
+    d |= (uint64_t)(1024u >> 4) << 32;  // the next 8 rows of K
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+
+__global__ void __launch_bounds__(THREADS, 2) gemm_wgrad_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
+                                                                const __grid_constant__ CUtensorMap map_b, uint32_t* err) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ uint64_t full[WG_STAGES], empty[WG_STAGES], done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_failed;
+    volatile int* failed = &s_failed;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t k_begin = blockIdx.x * g.k_chunk, k_end = min(g.k, k_begin + g.k_chunk);
+    const uint32_t nslices = (k_end - k_begin + BK - 1) / BK;
+    const uint32_t boxes_a = (g.m + 63u) / 64u, boxes_b = (g.n + 63u) / 64u;
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < WG_STAGES; ++q) {
+            mbar_init(&full[q], 1);
+            mbar_init(&empty[q], 1);
+        }
+        mbar_init(&done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_failed = 0;
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
+                     "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    if (warp == 0 && lane == 0) {
+        for (uint32_t it = 0; it < nslices; ++it) {
+            const uint32_t st = it % WG_STAGES;
+            if (it >= (uint32_t)WG_STAGES && !mbar_wait(smem_addr(&empty[st]), ((it / WG_STAGES) - 1u) & 1u)) {
+                *failed = 1;
+                break;
+            }
+            unsigned char* const slot = smem_raw + st * WG_SLOT;
+            mbar_expect_tx(&full[st], (boxes_a + boxes_b) * (TILE_BYTES / 2u));
+            for (uint32_t q = 0; q < boxes_a; ++q)
+                tma_load_box(&map_a, slot + q * (TILE_BYTES / 2u), 64u * q, k_begin + it * BK, &full[st]);
+            for (uint32_t q = 0; q < boxes_b; ++q)
+                tma_load_box(&map_b, slot + TILE_BYTES + q * (TILE_BYTES / 2u), 64u * q, k_begin + it * BK, &full[st]);
+        }
+    } else if (warp == 1 && lane == 0) {
+        // both operands MN-major (bits 15 and 16), N the columns rounded up to 16; accumulator rows and
+        // columns past the matrix hold whatever their operands' places did and are not read
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                               (((g.n + 15u) / 16u * 2u) << 17) | ((uint32_t)(BM >> 4) << 24);
+        for (uint32_t it = 0; it < nslices; ++it) {
+            const uint32_t st = it % WG_STAGES;
+            if (!mbar_wait(smem_addr(&full[st]), (it / WG_STAGES) & 1u)) {
+                *failed = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t base = smem_addr(smem_raw + st * WG_SLOT);
+#pragma unroll
+            for (uint32_t j = 0; j < BK / 16; ++j) {
+                const uint64_t ad = sw128_mn_desc(base + 2048u * j);
+                const uint64_t bd = sw128_mn_desc(base + TILE_BYTES + 2048u * j);
+                const uint32_t acc = (it > 0 || j > 0) ? 1u : 0u;
+                asm volatile(
+                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_addr(&empty[st]))
+                         : "memory");
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&done))
+                     : "memory");
+    }
+    __syncwarp();
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&done), 0u));
+    if (!ok) *failed = 1;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncthreads();
+    const bool bad = *failed != 0;
+    if (bad && threadIdx.x == 0 && err) atomicOr(err, DEVERR_MMA_TIMEOUT);
+    const uint32_t row = 32u * warp + lane;
+    for (uint32_t c0 = 0; c0 < g.n; c0 += 32u) {
+        uint32_t v[32];
+        tmem_ld32(tmem + ((32u * warp) << 16) + c0, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (row >= g.m || bad) continue;
+        float x[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
+        epilogue_store(g, x, row, c0, min(32u, g.n - c0), blockIdx.x);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    }
+}
+
 }  // namespace
 
 // 64 KB of operand buffers: at most three CTAs per SM, 3 x 128 of the SM's 512 columns of
@@ -1271,6 +1394,20 @@ wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s) {
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return fail(WC_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
         return WC_OK;
+    }
+    if (g.a_transposed && g.b_rowmajor && g.m <= (uint32_t)BM && g.n <= (uint32_t)BN && g.k && !g.a2 && !g.a_rows) {
+        // the weight-gradient kernel where both operands have tensor maps
+        CUtensorMap ma, mb;
+        if (encode_operand(&ma, g.a, g.m, g.k, 2ull * g.lda, 64) && encode_operand(&mb, g.b, g.n, g.k, 2ull * g.ldb, 64)) {
+            static std::once_flag once;
+            std::call_once(once, [] {
+                cudaFuncSetAttribute(gemm_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM);
+            });
+            gemm_wgrad_kernel<<<(g.k + g.k_chunk - 1) / g.k_chunk, THREADS, WG_SMEM, s>>>(g, ma, mb, err);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return fail(WC_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
+            return WC_OK;
+        }
     }
     static bool attr_done = false;
     if (!attr_done) {
