@@ -38,11 +38,14 @@ struct GemmArgs {
     const float* ln_gamma;
     const float* ln_beta;
     const __nv_bfloat16* ln_resid;
+    // ReLU's backward (relu_z set, rows of n): the result where relu_z > 0, zero elsewhere; needs n = 128,
+    // both outputs and the TMA kernel
+    const __nv_bfloat16* relu_z;
 };
 
 size_t gemm_smem_bytes();
-// Whether launch_gemm can run a LayerNorm-epilogue GEMM (the TMA kernel's tensor maps exist).
-bool gemm_ln_available();
+// Whether launch_gemm can run the epilogues that only the TMA kernel has (its tensor maps exist).
+bool gemm_tma_available();
 wc_status check_gemm(const GemmArgs& g);
 wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s);
 
@@ -68,11 +71,12 @@ void edge_features(uint32_t e, const float4* pos, const uint32_t* recv, const ui
 void layernorm(uint32_t rows, const float* y, const float* gamma, const float* beta, const __nv_bfloat16* resid,
                __nv_bfloat16* out, float* mean, float* rstd, cudaStream_t s);
 uint32_t layernorm_backward_blocks(uint32_t rows);
-void layernorm_backward(uint32_t rows, const float* dout, const float* y, const float* mean, const float* rstd,
-                        const float* gamma, __nv_bfloat16* dy, float* dy_f32, float* part, cudaStream_t s);
+// add_src: dout += add_src[add_idx[row]] first (fresh: dout is taken as zero before that), see wc_nn_ops.cu.
+void layernorm_backward(uint32_t rows, float* dout, const float* y, const float* mean, const float* rstd,
+                        const float* gamma, const uint32_t* add_idx, const float* add_src, bool fresh, __nv_bfloat16* dy,
+                        float* part, float* part_dy, cudaStream_t s);
 void relu_mask(size_t count, float* g_inout, const __nv_bfloat16* z, __nv_bfloat16* out, cudaStream_t s);
 void cast_bf16(size_t count, const float* x, __nv_bfloat16* out, cudaStream_t s);
-void gather_add(uint32_t rows, const uint32_t* idx, const float* src, float* dst, cudaStream_t s);
 void segment_sum_bf16(uint32_t nodes, const uint32_t* rowptr, const uint32_t* idx, const __nv_bfloat16* src,
                       float* out_f32, __nv_bfloat16* out_bf16, cudaStream_t s);
 void segment_sum_f32(uint32_t nodes, const uint32_t* rowptr, const uint32_t* idx, const float* src, float* out_f32,

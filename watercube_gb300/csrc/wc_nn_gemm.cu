@@ -910,6 +910,15 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
                         if (g.add1) add8(y, lds128(at));
                         if (g.add2) add8(y, lds128(at + (g.add1 ? AUX_BYTES : 0u)));
                     }
+                    if (AUX == AUX_TMA) {  // relu_z
+                        const uint4 z = lds128(at);
+                        const uint32_t w[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            if (!(__uint_as_float(w[k] << 16) > 0.f)) y[2 * k] = 0.f;
+                            if (!(__uint_as_float(w[k] & 0xffff0000u) > 0.f)) y[2 * k + 1] = 0.f;
+                        }
+                    }
                     if (g.relu) {
 #pragma unroll
                         for (int k = 0; k < 8; ++k) y[k] = fmaxf(y[k], 0.f);
@@ -1261,6 +1270,9 @@ wc_status check_gemm(const GemmArgs& g) {
                        g.k_chunk < g.k))
         return fail(WC_ERR_INVALID_ARG,
                     "gemm: the LayerNorm epilogue needs n = ldc = 128, beta, a BF16 output only and plain operands");
+    if (g.relu_z && (g.n != 128u || !g.c_bf16 || !g.c_f32 || g.ln_gamma || g.relu || g.add1 || g.add2 || g.accumulate ||
+                     g.a_rows || g.a2 || g.a_transposed || g.b_rowmajor || g.k > 128u || g.k_chunk < g.k))
+        return fail(WC_ERR_INVALID_ARG, "gemm: the ReLU mask epilogue needs n = 128, k <= 128, both outputs and plain operands");
     return WC_OK;
 }
 
@@ -1303,7 +1315,7 @@ bool encode_operand(CUtensorMap* map, const void* base, uint64_t inner, uint64_t
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool gemm_ln_available() { return encode_tiled() != nullptr; }
+bool gemm_tma_available() { return encode_tiled() != nullptr; }
 
 namespace {
 
@@ -1328,13 +1340,14 @@ wc_status launch_tma_as(const GemmArgs& g, const TmaMaps& maps, const TmaPlan& p
 // BF16 outputs together). Otherwise the caller runs the cp.async kernel.
 wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream_t s, bool* launched) {
     *launched = false;
-    const bool gather = g.add1 || g.add2, aux = gather || g.ln_resid, f32 = g.c_f32 != nullptr, bf = g.c_bf16 != nullptr;
+    const bool gather = g.add1 || g.add2, aux = gather || g.ln_resid || g.relu_z, f32 = g.c_f32 != nullptr, bf = g.c_bf16 != nullptr;
     TmaMaps maps;
     if (!encode_operand(&maps.a, g.a, g.k, g.m, 2ull * g.lda) || !encode_operand(&maps.b, g.b, g.k, g.n, 2ull * g.ldb))
         return WC_OK;
     if (bf && !encode_operand(&maps.cb, g.c_bf16, g.n, g.m, 2ull * g.ldc, 32)) return WC_OK;
     if (f32 && !encode_operand(&maps.cf, g.c_f32, g.n, g.m, 4ull * g.ldc, 32, true)) return WC_OK;
     if (g.ln_resid && !encode_operand(&maps.aux, g.ln_resid, 128, g.m, 256)) return WC_OK;
+    if (g.relu_z && !encode_operand(&maps.aux, g.relu_z, 128, g.m, 256)) return WC_OK;
     if (gather && (g.n != 128u || g.ld_add % 8u || reinterpret_cast<uintptr_t>(g.add1) % 16u ||
                    reinterpret_cast<uintptr_t>(g.add2) % 16u))
         return WC_OK;
@@ -1350,6 +1363,7 @@ wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream
     if (g.ln_gamma)
         return aux ? launch_tma_as<AUX_TMA, true, false, true>(g, maps, plan, grid, err, s)
                    : launch_tma_as<AUX_NONE, true, false, true>(g, maps, plan, grid, err, s);
+    if (g.relu_z) return launch_tma_as<AUX_TMA, false, true, true>(g, maps, plan, grid, err, s);
     if (gather)
         return f32 ? (bf ? launch_tma_as<AUX_GATHER, false, true, true>(g, maps, plan, grid, err, s)
                          : launch_tma_as<AUX_GATHER, false, true, false>(g, maps, plan, grid, err, s))
@@ -1386,6 +1400,7 @@ wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s) {
             WC_TRY(launch_tma(g, grid, err, s, &launched));
             if (launched) return WC_OK;
         }
+        if (g.relu_z) return fail(WC_ERR_STATE, "gemm: the ReLU mask epilogue needs the TMA kernel (plain A, k <= 128)");
         if (g.ln_gamma) return fail(WC_ERR_STATE, "gemm: the LayerNorm epilogue needs the TMA kernel (plain A, k <= 384)");
         if (rb)
             gemm_pipe_kernel<true><<<grid, PIPE_THREADS, pipe_smem_bytes(true, g.k), s>>>(g, err);

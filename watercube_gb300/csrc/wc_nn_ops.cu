@@ -184,52 +184,79 @@ __global__ void layernorm_kernel(uint32_t rows, const float* __restrict__ y, con
     }
 }
 
-// dy = rstd (g - mean(g) - xhat mean(g xhat)), g = dout * gamma; per-block partial sums of
-// dgamma = sum dout xhat and dbeta = sum dout (rows of block b: [b*rpb, (b+1)*rpb)).
+// dy = rstd (g - mean(g) - xhat mean(g xhat)), g = dout * gamma, rows of 128, a warp per row and two
+// rows in flight; per-block partial sums of dgamma = sum dout xhat, dbeta = sum dout
+// (part[b][256]) and the bias gradient of the layer before, sum dy (part_dy[b][128]); rows of block
+// b: [b * rpb, (b+1) * rpb). With add_src, dout is dout (or zero, `fresh`) + add_src[add_idx[row]],
+// written back (the messages' gradient through the aggregation). Bound by its bytes: 1,792 per row
+// with the added rows (in L2), 1,280 without.
 constexpr int LNB_WARPS = 8;
+template <bool ADD>
 __global__ void __launch_bounds__(LNB_WARPS * 32) layernorm_backward_kernel(
-    uint32_t rows, uint32_t rows_per_block, const float* __restrict__ dout, const float* __restrict__ y,
+    uint32_t rows, uint32_t rows_per_block, float* __restrict__ dout, const float* __restrict__ y,
     const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ gamma,
-    __nv_bfloat16* __restrict__ dy, float* __restrict__ dy_f32, float* __restrict__ part) {
-    __shared__ float s_g[LNB_WARPS][128], s_b[LNB_WARPS][128];
+    const uint32_t* __restrict__ add_idx, const float* __restrict__ add_src, int fresh, __nv_bfloat16* __restrict__ dy,
+    float* __restrict__ part, float* __restrict__ part_dy) {
+    __shared__ float s_sum[3][LNB_WARPS][128];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
     const float4 gm = reinterpret_cast<const float4*>(gamma)[lane];
-    float pg[4] = {0.f, 0.f, 0.f, 0.f}, pb[4] = {0.f, 0.f, 0.f, 0.f};
-    for (uint32_t row = r0 + warp; row < r1; row += LNB_WARPS) {
-        const float4 d = reinterpret_cast<const float4*>(dout + (size_t)row * 128)[lane];
-        const float4 v = reinterpret_cast<const float4*>(y + (size_t)row * 128)[lane];
-        const float mu = mean[row], rs = rstd[row];
-        const float xh[4] = {(v.x - mu) * rs, (v.y - mu) * rs, (v.z - mu) * rs, (v.w - mu) * rs};
-        const float dd[4] = {d.x, d.y, d.z, d.w};
-        const float gg[4] = {d.x * gm.x, d.y * gm.y, d.z * gm.z, d.w * gm.w};
-        const float mg = warp_sum(gg[0] + gg[1] + gg[2] + gg[3]) * (1.f / 128.f);
-        const float mgx = warp_sum(gg[0] * xh[0] + gg[1] * xh[1] + gg[2] * xh[2] + gg[3] * xh[3]) * (1.f / 128.f);
-        __nv_bfloat16* o = dy + (size_t)row * 128 + 4 * lane;
-        float r[4];
+    float pg[4] = {0.f, 0.f, 0.f, 0.f}, pb[4] = {0.f, 0.f, 0.f, 0.f}, py[4] = {0.f, 0.f, 0.f, 0.f};
+    for (uint32_t row = r0 + warp; row < r1; row += 2u * LNB_WARPS) {
+        float4 d[2], v[2], s[2];
+        float mu[2], rs[2];
+        const bool two = row + LNB_WARPS < r1;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            r[k] = rs * (gg[k] - mg - xh[k] * mgx);
-            o[k] = __float2bfloat16_rn(r[k]);
-            pg[k] += dd[k] * xh[k];
-            pb[k] += dd[k];
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t i = u && two ? row + LNB_WARPS : row;
+            if (ADD) s[u] = __ldg(reinterpret_cast<const float4*>(add_src + (size_t)__ldg(add_idx + i) * 128) + lane);
+            d[u] = ADD && fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4*>(dout + (size_t)i * 128)[lane];
+            v[u] = __ldg(reinterpret_cast<const float4*>(y + (size_t)i * 128) + lane);
+            mu[u] = __ldg(mean + i);
+            rs[u] = __ldg(rstd + i);
         }
-        if (dy_f32) *reinterpret_cast<float4*>(dy_f32 + (size_t)row * 128 + 4 * lane) = make_float4(r[0], r[1], r[2], r[3]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (u && !two) break;
+            const uint32_t i = u ? row + LNB_WARPS : row;
+            if (ADD) {
+                d[u].x += s[u].x;
+                d[u].y += s[u].y;
+                d[u].z += s[u].z;
+                d[u].w += s[u].w;
+                reinterpret_cast<float4*>(dout + (size_t)i * 128)[lane] = d[u];
+            }
+            const float xh[4] = {(v[u].x - mu[u]) * rs[u], (v[u].y - mu[u]) * rs[u], (v[u].z - mu[u]) * rs[u],
+                                 (v[u].w - mu[u]) * rs[u]};
+            const float dd[4] = {d[u].x, d[u].y, d[u].z, d[u].w};
+            const float gg[4] = {dd[0] * gm.x, dd[1] * gm.y, dd[2] * gm.z, dd[3] * gm.w};
+            const float mg = warp_sum(gg[0] + gg[1] + gg[2] + gg[3]) * (1.f / 128.f);
+            const float mgx = warp_sum(gg[0] * xh[0] + gg[1] * xh[1] + gg[2] * xh[2] + gg[3] * xh[3]) * (1.f / 128.f);
+            float r[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                r[k] = rs[u] * (gg[k] - mg - xh[k] * mgx);
+                pg[k] += dd[k] * xh[k];
+                pb[k] += dd[k];
+                py[k] += r[k];
+            }
+            const __nv_bfloat162 q0 = __floats2bfloat162_rn(r[0], r[1]), q1 = __floats2bfloat162_rn(r[2], r[3]);
+            reinterpret_cast<uint2*>(dy + (size_t)i * 128)[lane] =
+                make_uint2(*reinterpret_cast<const uint32_t*>(&q0), *reinterpret_cast<const uint32_t*>(&q1));
+        }
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        s_g[warp][4 * lane + k] = pg[k];
-        s_b[warp][4 * lane + k] = pb[k];
+        s_sum[0][warp][4 * lane + k] = pg[k];
+        s_sum[1][warp][4 * lane + k] = pb[k];
+        s_sum[2][warp][4 * lane + k] = py[k];
     }
     __syncthreads();
-    if (threadIdx.x < 128) {
-        float a = 0.f, b = 0.f;
-        for (int w = 0; w < LNB_WARPS; ++w) {
-            a += s_g[w][threadIdx.x];
-            b += s_b[w][threadIdx.x];
-        }
-        part[(size_t)blockIdx.x * 256 + threadIdx.x] = a;
-        part[(size_t)blockIdx.x * 256 + 128 + threadIdx.x] = b;
+    for (uint32_t c = threadIdx.x; c < 384u; c += LNB_WARPS * 32) {
+        float a = 0.f;
+        for (int w = 0; w < LNB_WARPS; ++w) a += s_sum[c >> 7][w][c & 127u];
+        if (c < 256u) part[(size_t)blockIdx.x * 256 + c] = a;
+        else part_dy[(size_t)blockIdx.x * 128 + (c - 256u)] = a;
     }
 }
 
@@ -248,21 +275,6 @@ __global__ void relu_mask_kernel(size_t count, float* __restrict__ g, const __nv
 __global__ void cast_kernel(size_t count, const float* __restrict__ x, __nv_bfloat16* __restrict__ out) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
         out[i] = __float2bfloat16_rn(x[i]);
-}
-
-// dst[e] += src[idx[e]] (rows of 128).
-__global__ void gather_add_kernel(uint32_t rows, const uint32_t* __restrict__ idx, const float* __restrict__ src,
-                                  float* __restrict__ dst) {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (row >= rows) return;
-    const float4 s = reinterpret_cast<const float4*>(src + (size_t)idx[row] * 128)[lane];
-    float4* d = reinterpret_cast<float4*>(dst + (size_t)row * 128) + lane;
-    float4 v = *d;
-    v.x += s.x;
-    v.y += s.y;
-    v.z += s.z;
-    v.w += s.w;
-    *d = v;
 }
 
 // out[i] = sum over e in [rowptr[i], rowptr[i+1]) of src[idx ? idx[e] : e] (rows of 128).
@@ -558,22 +570,29 @@ void layernorm(uint32_t rows, const float* y, const float* gamma, const float* b
                __nv_bfloat16* out, float* mean, float* rstd, cudaStream_t s) {
     if (rows) layernorm_kernel<<<blocks_for((size_t)rows * 32, 256), 256, 0, s>>>(rows, y, gamma, beta, resid, out, mean, rstd);
 }
-uint32_t layernorm_backward_blocks(uint32_t rows) { return rows ? blocks_for(rows, 512) : 0; }
-void layernorm_backward(uint32_t rows, const float* dout, const float* y, const float* mean, const float* rstd,
-                        const float* gamma, __nv_bfloat16* dy, float* dy_f32, float* part, cudaStream_t s) {
-    const uint32_t blocks = layernorm_backward_blocks(rows);
-    if (blocks)
-        layernorm_backward_kernel<<<blocks, LNB_WARPS * 32, 0, s>>>(rows, 512, dout, y, mean, rstd, gamma, dy, dy_f32,
-                                                                    part);
+// Eight blocks of eight warps per SM when the rows fill them with two rows a warp at least.
+static uint32_t layernorm_backward_rows(uint32_t rows) {
+    const uint32_t per = (rows + 1215u) / 1216u;
+    return std::max(16u, (per + 15u) / 16u * 16u);
+}
+uint32_t layernorm_backward_blocks(uint32_t rows) { return rows ? blocks_for(rows, layernorm_backward_rows(rows)) : 0; }
+void layernorm_backward(uint32_t rows, float* dout, const float* y, const float* mean, const float* rstd,
+                        const float* gamma, const uint32_t* add_idx, const float* add_src, bool fresh, __nv_bfloat16* dy,
+                        float* part, float* part_dy, cudaStream_t s) {
+    const uint32_t blocks = layernorm_backward_blocks(rows), rpb = layernorm_backward_rows(rows);
+    if (!blocks) return;
+    if (add_src)
+        layernorm_backward_kernel<true><<<blocks, LNB_WARPS * 32, 0, s>>>(rows, rpb, dout, y, mean, rstd, gamma, add_idx,
+                                                                          add_src, fresh, dy, part, part_dy);
+    else
+        layernorm_backward_kernel<false><<<blocks, LNB_WARPS * 32, 0, s>>>(rows, rpb, dout, y, mean, rstd, gamma, nullptr,
+                                                                           nullptr, 0, dy, part, part_dy);
 }
 void relu_mask(size_t count, float* g, const __nv_bfloat16* z, __nv_bfloat16* out, cudaStream_t s) {
     if (count) relu_mask_kernel<<<(unsigned)std::min<size_t>(blocks_for(count, 256), 65535), 256, 0, s>>>(count, g, z, out);
 }
 void cast_bf16(size_t count, const float* x, __nv_bfloat16* out, cudaStream_t s) {
     if (count) cast_kernel<<<(unsigned)std::min<size_t>(blocks_for(count, 256), 65535), 256, 0, s>>>(count, x, out);
-}
-void gather_add(uint32_t rows, const uint32_t* idx, const float* src, float* dst, cudaStream_t s) {
-    if (rows) gather_add_kernel<<<blocks_for((size_t)rows * 32, 256), 256, 0, s>>>(rows, idx, src, dst);
 }
 void segment_sum_bf16(uint32_t nodes, const uint32_t* rowptr, const uint32_t* idx, const __nv_bfloat16* src,
                       float* out_f32, __nv_bfloat16* out_bf16, cudaStream_t s) {

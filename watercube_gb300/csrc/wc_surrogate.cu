@@ -327,13 +327,42 @@ wc_status bgrad(wc_surrogate* s, const Lin& l, uint32_t rows, const float* dy) {
     return WC_OK;
 }
 
-wc_status ln_back(wc_surrogate* s, const LNp& ln, uint32_t rows, const float* dout, const float* y, const float* st,
-                  __nv_bfloat16* dy, float* dy_f32) {
+// dX = (dY . W^T) masked by the ReLU that made z, FP32 and BF16 (which may overwrite dY: a tile's rows
+// are read before they are written).
+wc_status dgrad_relu(wc_surrogate* s, const Lin& l, uint32_t rows, const __nv_bfloat16* dy, const __nv_bfloat16* z,
+                     float* dx, __nv_bfloat16* dx_bf16) {
+    if (!gemm_tma_available()) {
+        WC_TRY(dgrad(s, l, rows, dy, 0, W, dx, false));
+        relu_mask((size_t)rows * W, dx, z, dx_bf16, s->stream);
+        return WC_OK;
+    }
+    GemmArgs g{};
+    g.m = rows;
+    g.n = W;
+    g.k = l.nout;
+    g.k_chunk = ((l.nout + 63) / 64) * 64;
+    g.a = dy;
+    g.lda = l.nout;
+    g.b = s->wb + l.wk;
+    g.ldb = l.nout;
+    g.c_f32 = dx;
+    g.c_bf16 = dx_bf16;
+    g.ldc = W;
+    g.relu_z = z;
+    return launch_gemm(g, s->d_err, s->stream);
+}
+
+// The LayerNorm's backward of the layer y = W z + b behind it: dy, and the gradients of gamma, beta
+// and l's bias. recv and dagg: dout += dagg[recv[row]] first (fresh: dout holds nothing yet).
+wc_status ln_back(wc_surrogate* s, const LNp& ln, const Lin& l, uint32_t rows, float* dout, const float* y, const float* st,
+                  __nv_bfloat16* dy, const uint32_t* recv = nullptr, const float* dagg = nullptr, bool fresh = false) {
     const uint32_t blocks = layernorm_backward_blocks(rows);
     if (!blocks) return WC_OK;
-    WC_TRY(ensure_part(s, (size_t)blocks * 256));
-    layernorm_backward(rows, dout, y, st, st + rows, s->w + ln.g, dy, dy_f32, s->work.part, s->stream);
+    WC_TRY(ensure_part(s, (size_t)blocks * 384));
+    float* const part_dy = s->work.part + (size_t)blocks * 256;
+    layernorm_backward(rows, dout, y, st, st + rows, s->w + ln.g, recv, dagg, fresh, dy, s->work.part, part_dy, s->stream);
     colsum_partials(blocks, 256, s->work.part, s->g + ln.g, 1, s->stream);
+    colsum_partials(blocks, 128, part_dy, s->g + l.b, 1, s->stream);
     return WC_OK;
 }
 
@@ -403,7 +432,7 @@ wc_status ensure_work(wc_surrogate* s, uint32_t n, uint32_t e, bool saved) {
     // split-K partials of the weight gradients (<= 304 splits of a 128 x 128 tile), column-sum
     // and LayerNorm-backward partials
     size_t need = std::max<size_t>(part_cap, 304u * (size_t)W * W);
-    need = std::max<size_t>(need, (size_t)layernorm_backward_blocks(ce) * 256);
+    need = std::max<size_t>(need, (size_t)layernorm_backward_blocks(ce) * 384);
     need = std::max<size_t>(need, (size_t)colsum_blocks(ce) * W);
     WC_TRY(ensure_part(s, need));
     return WC_OK;
@@ -500,7 +529,7 @@ wc_status forward(wc_surrogate* s, bool keep) {
     if (s->cast_dirty) cast_all(s);
     Work& w = s->work;
     const uint32_t n = s->n, e = s->e;
-    const bool fuse = !keep && gemm_ln_available();
+    const bool fuse = !keep && gemm_tma_available();
     float* st = w.stn0;
     WC_TRY(fwd(s, s->ne1, n, w.xn, nullptr, true, nullptr, w.zn0));
     if (fuse) {
@@ -558,12 +587,10 @@ wc_status backward(wc_surrogate* s) {
     // decoder
     WC_TRY(wgrad(s, s->d2, n, w.zd, W, 0, w.dout_b));
     WC_TRY(bgrad(s, s->d2, n, w.dout));
-    WC_TRY(dgrad(s, s->d2, n, w.dout_b, 0, W, w.dtmp_n, false));
-    relu_mask((size_t)n * W, w.dtmp_n, w.zd, w.gb_n, s->stream);
+    WC_TRY(dgrad_relu(s, s->d2, n, w.dout_b, w.zd, w.dtmp_n, w.gb_n));
     WC_TRY(wgrad(s, s->d1, n, hbuf(w, s->L), W, 0, w.gb_n));
     WC_TRY(bgrad(s, s->d1, n, w.dtmp_n));
     WC_TRY(dgrad(s, s->d1, n, w.gb_n, 0, W, w.dh, false));
-    WC_CUDA_TRY(cudaMemsetAsync(w.de, 0, sizeof(float) * (size_t)e * W, s->stream));
     for (int li = (int)s->L - 1; li >= 0; --li) {
         const uint32_t l = (uint32_t)li;
         const MPLayer& L = s->layers[l];
@@ -576,46 +603,38 @@ wc_status backward(wc_surrogate* s) {
         float* yn = lbuf(w, w.yn, l, pn);
         float* stn = lbuf(w, w.stn, l, 2 * (size_t)w.cap_n);
         // node block: h' = h + LN(yn); dh holds d h' and keeps flowing to h (residual)
-        WC_TRY(ln_back(s, L.lnn, n, w.dh, yn, stn, w.gb_n, w.dtmp_n));
+        WC_TRY(ln_back(s, L.lnn, L.n2, n, w.dh, yn, stn, w.gb_n));
         WC_TRY(wgrad(s, L.n2, n, zn, W, 0, w.gb_n));
-        WC_TRY(bgrad(s, L.n2, n, w.dtmp_n));
-        WC_TRY(dgrad(s, L.n2, n, w.gb_n, 0, W, w.dtmp_n, false));
-        relu_mask((size_t)n * W, w.dtmp_n, zn, w.gb_n2, s->stream);  // gb_n2 = d zn
+        WC_TRY(dgrad_relu(s, L.n2, n, w.gb_n, zn, w.dtmp_n, w.gb_n2));  // gb_n2 = d zn
         WC_TRY(wgrad(s, L.n1, n, h, W, 0, w.gb_n2));
         WC_TRY(wgrad(s, L.n1, n, agg, W, W, w.gb_n2));
         WC_TRY(bgrad(s, L.n1, n, w.dtmp_n));
         WC_TRY(dgrad(s, L.n1, n, w.gb_n2, 0, W, w.dh, true));
         WC_TRY(dgrad(s, L.n1, n, w.gb_n2, W, W, w.dagg, false));
-        // edge block: e' = e + LN(ye); de holds d e' from the next layer, plus the aggregation
-        gather_add(e, w.recv, w.dagg, w.de, s->stream);
-        WC_TRY(ln_back(s, L.lne, e, w.de, ye, ste, w.gb_e, w.dtmp_e));
+        // edge block: e' = e + LN(ye); de holds d e' from the next layer (nothing at the last), plus
+        // the aggregation's
+        WC_TRY(ln_back(s, L.lne, L.e2, e, w.de, ye, ste, w.gb_e, w.recv, w.dagg, l + 1 == s->L));
         WC_TRY(wgrad(s, L.e2, e, ze, W, 0, w.gb_e));
-        WC_TRY(bgrad(s, L.e2, e, w.dtmp_e));
-        WC_TRY(dgrad(s, L.e2, e, w.gb_e, 0, W, w.dtmp_e, false));
-        relu_mask((size_t)e * W, w.dtmp_e, ze, w.gb_e, s->stream);  // gb_e = d ze
+        WC_TRY(dgrad_relu(s, L.e2, e, w.gb_e, ze, w.dtmp_e, w.gb_e));  // gb_e = d ze
         WC_TRY(wgrad(s, L.e1e, e, el, W, 0, w.gb_e));
-        WC_TRY(bgrad(s, L.e1e, e, w.dtmp_e));
         WC_TRY(dgrad(s, L.e1e, e, w.gb_e, 0, W, w.de, true));
         segment_sum_f32(n, w.rowptr, nullptr, w.dtmp_e, w.dP, w.dPb, s->stream);
         segment_sum_f32(n, w.rowptr, w.rev, w.dtmp_e, w.dQ, w.dQb, s->stream);
+        WC_TRY(bgrad(s, L.e1e, n, w.dP));  // every edge is one node's incoming edge
         WC_TRY(wgrad(s, L.e1i, n, h, W, 0, w.dPb));
         WC_TRY(wgrad(s, L.e1s, n, h, W, 0, w.dQb));
         WC_TRY(dgrad(s, L.e1i, n, w.dPb, 0, W, w.dh, true));
         WC_TRY(dgrad(s, L.e1s, n, w.dQb, 0, W, w.dh, true));
     }
     // encoders
-    WC_TRY(ln_back(s, s->lnn0, n, w.dh, w.yn0, w.stn0, w.gb_n, w.dtmp_n));
+    WC_TRY(ln_back(s, s->lnn0, s->ne2, n, w.dh, w.yn0, w.stn0, w.gb_n));
     WC_TRY(wgrad(s, s->ne2, n, w.zn0, W, 0, w.gb_n));
-    WC_TRY(bgrad(s, s->ne2, n, w.dtmp_n));
-    WC_TRY(dgrad(s, s->ne2, n, w.gb_n, 0, W, w.dtmp_n, false));
-    relu_mask((size_t)n * W, w.dtmp_n, w.zn0, w.gb_n, s->stream);
+    WC_TRY(dgrad_relu(s, s->ne2, n, w.gb_n, w.zn0, w.dtmp_n, w.gb_n));
     WC_TRY(wgrad(s, s->ne1, n, w.xn, NODE_IN, 0, w.gb_n));
     WC_TRY(bgrad(s, s->ne1, n, w.dtmp_n));
-    WC_TRY(ln_back(s, s->lne0, e, w.de, w.ye0, w.ste0, w.gb_e, w.dtmp_e));
+    WC_TRY(ln_back(s, s->lne0, s->ee2, e, w.de, w.ye0, w.ste0, w.gb_e));
     WC_TRY(wgrad(s, s->ee2, e, w.ze0, W, 0, w.gb_e));
-    WC_TRY(bgrad(s, s->ee2, e, w.dtmp_e));
-    WC_TRY(dgrad(s, s->ee2, e, w.gb_e, 0, W, w.dtmp_e, false));
-    relu_mask((size_t)e * W, w.dtmp_e, w.ze0, w.gb_e, s->stream);
+    WC_TRY(dgrad_relu(s, s->ee2, e, w.gb_e, w.ze0, w.dtmp_e, w.gb_e));
     WC_TRY(wgrad(s, s->ee1, e, w.xe, EDGE_IN, 0, w.gb_e));
     WC_TRY(bgrad(s, s->ee1, e, w.dtmp_e));
     return WC_OK;
