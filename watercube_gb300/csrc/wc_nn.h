@@ -38,6 +38,9 @@ struct GemmArgs {
     const float* ln_gamma;
     const float* ln_beta;
     const __nv_bfloat16* ln_resid;
+    // training: c_f32 also receives the result before the LayerNorm, ln_mean and ln_rstd its row statistics
+    float* ln_mean;
+    float* ln_rstd;
     // ReLU's backward (relu_z set, rows of n): the result where relu_z > 0, zero elsewhere; needs n = 128,
     // both outputs and the TMA kernel
     const __nv_bfloat16* relu_z;

@@ -774,6 +774,11 @@ __device__ __forceinline__ void pair_sync(uint32_t quarter) {
 // same way, and each thread normalises, scales and shifts its own columns and adds the residual
 // row. Both warps of a pair pass both barriers of every tile: whether each warp's waits succeeded is
 // exchanged at the first barrier and the pair leaves together.
+// LN with F32 (training, which keeps the rows before the LayerNorm and its statistics): a thread takes
+// every second group of four columns, so that its sums and the pair's one exchange add in the order
+// of layernorm_kernel's warp (four columns per lane, lanes in pairs 16, 8, 4, 2, 1 apart), whose
+// results training had when it was a kernel of its own (the expressions are that kernel's too, so that
+// they contract alike): the layer and its LayerNorm took ~145 us at 460,000 rows.
 template <int AUX, bool LN, bool F32, bool BF>
 __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& maps, const TmaPlan& plan, uint32_t tmem,
                                              uint64_t* acc_full, uint64_t* acc_empty, uint64_t* aux_full,
@@ -826,7 +831,94 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
                     if (c + j < g.n) x[j] += __ldg(g.bias + c + j);
             }
         };
-        if constexpr (LN) {
+        if constexpr (LN && F32) {
+            float x[64];  // group j (0..15): columns 8 j + 4 half ..
+            if (ok) {
+                uint32_t v[64];
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j)
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(v[4 * j]), "=r"(v[4 * j + 1]), "=r"(v[4 * j + 2]), "=r"(v[4 * j + 3])
+                                 : "r"(taddr - col0 + 8u * j + 4u * half));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 64; ++j) x[j] = __uint_as_float(v[j]);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[b]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 64; ++j) x[j] = 0.f;
+            }
+            auto four = [&](const float* base, uint32_t j) {  // columns of group j
+                const float* q = base + 8u * j + 4u * half;
+                return vec ? __ldg(reinterpret_cast<const float4*>(q)) : make_float4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+            };
+            float s[16];
+            auto tree = [&]() {  // the sum of s[0..16) in pairs 8, 4, 2, 1 apart
+#pragma unroll
+                for (int h = 8; h > 0; h >>= 1)
+#pragma unroll
+                    for (int j = 0; j < h; ++j) s[j] += s[j + h];
+                return s[0];
+            };
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+                float* y = x + 4 * j;
+                if (g.bias) {
+                    const float4 bb = four(g.bias, j);
+                    y[0] += bb.x;
+                    y[1] += bb.y;
+                    y[2] += bb.z;
+                    y[3] += bb.w;
+                }
+                s[j] = ((y[0] + y[1]) + y[2]) + y[3];
+            }
+            xs[quarter][half][lane] = tree();
+            if (lane == 0) oks[quarter][half] = ok ? 1 : 0;
+            pair_sync(quarter);
+            if (!(oks[quarter][0] && oks[quarter][1])) {
+                if (lane == 0) *failed = 1;
+                break;
+            }
+            const float mean = (xs[quarter][0][lane] + xs[quarter][1][lane]) * (1.f / 128.f);
+            const uint32_t f32_rows = f32_base + quarter * (F32_OUT_BYTES / 4u);
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+                float* y = x + 4 * j;
+                sts128(f32_rows + (j >> 2) * 4096u + sw128(lane, 2u * (j & 3u) + half),
+                       make_uint4(__float_as_uint(y[0]), __float_as_uint(y[1]), __float_as_uint(y[2]), __float_as_uint(y[3])));
+#pragma unroll
+                for (int k = 0; k < 4; ++k) y[k] -= mean;
+                s[j] = y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
+            }
+            xv[quarter][half][lane] = tree();
+            pair_sync(quarter);
+            const float var = (xv[quarter][0][lane] + xv[quarter][1][lane]) * (1.f / 128.f);
+            const float rstd = rsqrtf(var + LN_EPSILON);
+            if (half == 0 && row0 + lane < g.m) {
+                g.ln_mean[row0 + lane] = mean;
+                g.ln_rstd[row0 + lane] = rstd;
+            }
+            const uint32_t rows = aux_base + b * plan.aux_bytes;
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+                const float* y = x + 4 * j;
+                const float4 gm = four(g.ln_gamma, j), bt = four(g.ln_beta, j);
+                float o[4] = {y[0] * rstd * gm.x + bt.x, y[1] * rstd * gm.y + bt.y, y[2] * rstd * gm.z + bt.z,
+                              y[3] * rstd * gm.w + bt.w};
+                const uint32_t at = rows + (j >> 3) * HALF_BYTES + sw128(r, j & 7u) + 8u * half;
+                if (AUX == AUX_TMA) {
+                    uint32_t w0, w1;
+                    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(w0), "=r"(w1) : "r"(at) : "memory");
+                    o[0] += __uint_as_float(w0 << 16);
+                    o[1] += __uint_as_float(w0 & 0xffff0000u);
+                    o[2] += __uint_as_float(w1 << 16);
+                    o[3] += __uint_as_float(w1 & 0xffff0000u);
+                }
+                asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(at), "r"(pack2(o[0], o[1])), "r"(pack2(o[2], o[3])) : "memory");
+            }
+        } else if constexpr (LN) {
             float x[64];
             if (ok) {
                 uint32_t v[32];
@@ -936,7 +1028,8 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
+        if (LN && F32) pair_sync(quarter);  // a box holds both warps' columns
+        else __syncwarp();
         if (lane == 0) {
             if (!LN) mbar_arrive(&acc_empty[b]);
             if (row0 < g.m) {
@@ -1265,7 +1358,7 @@ wc_status check_gemm(const GemmArgs& g) {
         return fail(WC_ERR_INVALID_ARG, "gemm: k must be a multiple of 8 (pad with zeros)");
     if ((g.add1 && !g.add1_idx) || (g.add2 && !g.add2_idx)) return fail(WC_ERR_INVALID_ARG, "gemm: gather without index");
     if (g.k_chunk == 0 || g.k_chunk % BK) return fail(WC_ERR_INVALID_ARG, "gemm: k_chunk must be a multiple of 64");
-    if (g.ln_gamma && (g.n != 128u || !g.ln_beta || !g.c_bf16 || g.c_f32 || g.relu || g.add1 || g.add2 ||
+    if (g.ln_gamma && (g.n != 128u || !g.ln_beta || !g.c_bf16 || (g.c_f32 && !(g.ln_mean && g.ln_rstd && g.k <= 128u)) || g.relu || g.add1 || g.add2 ||
                        g.accumulate || g.ldc != 128u || g.a_rows || g.a2 || g.a_transposed || g.b_rowmajor ||
                        g.k_chunk < g.k))
         return fail(WC_ERR_INVALID_ARG,
@@ -1360,6 +1453,9 @@ wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream
     plan.stages = std::min<uint32_t>(TMA_MAX_STAGES, (TMA_SMEM_LIMIT - fixed) / TILE_BYTES);
     plan.smem = fixed + plan.stages * TILE_BYTES;
     *launched = true;
+    if (g.ln_gamma && f32)
+        return aux ? launch_tma_as<AUX_TMA, true, true, true>(g, maps, plan, grid, err, s)
+                   : launch_tma_as<AUX_NONE, true, true, true>(g, maps, plan, grid, err, s);
     if (g.ln_gamma)
         return aux ? launch_tma_as<AUX_TMA, true, false, true>(g, maps, plan, grid, err, s)
                    : launch_tma_as<AUX_NONE, true, false, true>(g, maps, plan, grid, err, s);

@@ -242,10 +242,10 @@ wc_status fwd(wc_surrogate* s, const Lin& l, uint32_t rows, const __nv_bfloat16*
     return launch_gemm(g, s->d_err, s->stream);
 }
 
-// out = LN(a . W^T + b) * gamma + beta (+ resid) in one GEMM with the LayerNorm in its epilogue
-// (the forward pass of a rollout, which keeps no activations for a backward pass).
+// out = LN(a . W^T + b) * gamma + beta (+ resid) in one GEMM with the LayerNorm in its epilogue;
+// y and stats (training): also the rows before the LayerNorm and their means and 1 / deviations.
 wc_status fwd_ln(wc_surrogate* s, const Lin& l, uint32_t rows, const __nv_bfloat16* a, const float* gamma,
-                 const __nv_bfloat16* resid, __nv_bfloat16* out) {
+                 const __nv_bfloat16* resid, __nv_bfloat16* out, float* y, float* stats) {
     GemmArgs g{};
     g.m = rows;
     g.n = l.nout;
@@ -261,6 +261,11 @@ wc_status fwd_ln(wc_surrogate* s, const Lin& l, uint32_t rows, const __nv_bfloat
     g.ln_gamma = gamma;
     g.ln_beta = gamma + W;
     g.ln_resid = resid;
+    if (y) {
+        g.c_f32 = y;
+        g.ln_mean = stats;
+        g.ln_rstd = stats + rows;
+    }
     return launch_gemm(g, s->d_err, s->stream);
 }
 
@@ -523,57 +528,40 @@ wc_status prepare_sample(wc_surrogate* s, wc_fluid* f, bool saved, const float4*
 
 // ---- forward / backward ---------------------------------------------------------------------
 
-// keep: the activations and LayerNorm statistics the backward pass reads (training); without
-// it every second MLP layer and its LayerNorm run as one GEMM with the LayerNorm in the epilogue.
+// A second MLP layer and its LayerNorm, kept for the backward pass (y, stats) or not: one GEMM where
+// the LayerNorm's epilogue is available.
+wc_status layer_ln(wc_surrogate* s, bool keep, const Lin& l, uint32_t rows, const __nv_bfloat16* a, const LNp& ln,
+                   const __nv_bfloat16* resid, __nv_bfloat16* out, float* y, float* stats) {
+    if (gemm_tma_available())
+        return fwd_ln(s, l, rows, a, s->w + ln.g, resid, out, keep ? y : nullptr, keep ? stats : nullptr);
+    WC_TRY(fwd(s, l, rows, a, nullptr, false, y, nullptr));
+    layernorm(rows, y, s->w + ln.g, s->w + ln.g + W, resid, out, stats, stats + rows, s->stream);
+    return WC_OK;
+}
+
+// keep: the activations and LayerNorm statistics the backward pass reads (training).
 wc_status forward(wc_surrogate* s, bool keep) {
     if (s->cast_dirty) cast_all(s);
     Work& w = s->work;
     const uint32_t n = s->n, e = s->e;
-    const bool fuse = !keep && gemm_tma_available();
-    float* st = w.stn0;
     WC_TRY(fwd(s, s->ne1, n, w.xn, nullptr, true, nullptr, w.zn0));
-    if (fuse) {
-        WC_TRY(fwd_ln(s, s->ne2, n, w.zn0, s->w + s->lnn0.g, nullptr, hbuf(w, 0)));
-    } else {
-        WC_TRY(fwd(s, s->ne2, n, w.zn0, nullptr, false, w.yn0, nullptr));
-        layernorm(n, w.yn0, s->w + s->lnn0.g, s->w + s->lnn0.g + W, nullptr, hbuf(w, 0), st, st + n, s->stream);
-    }
+    WC_TRY(layer_ln(s, keep, s->ne2, n, w.zn0, s->lnn0, nullptr, hbuf(w, 0), w.yn0, w.stn0));
     WC_TRY(fwd(s, s->ee1, e, w.xe, nullptr, true, nullptr, w.ze0));
-    if (fuse) {
-        WC_TRY(fwd_ln(s, s->ee2, e, w.ze0, s->w + s->lne0.g, nullptr, ebuf(w, 0)));
-    } else {
-        WC_TRY(fwd(s, s->ee2, e, w.ze0, nullptr, false, w.ye0, nullptr));
-        layernorm(e, w.ye0, s->w + s->lne0.g, s->w + s->lne0.g + W, nullptr, ebuf(w, 0), w.ste0, w.ste0 + e,
-                  s->stream);
-    }
+    WC_TRY(layer_ln(s, keep, s->ee2, e, w.ze0, s->lne0, nullptr, ebuf(w, 0), w.ye0, w.ste0));
     const size_t pn = (size_t)w.cap_n * W, pe = (size_t)w.cap_e * W;
     for (uint32_t l = 0; l < s->L; ++l) {
         const MPLayer& L = s->layers[l];
         __nv_bfloat16 *h = hbuf(w, l), *h1 = hbuf(w, l + 1), *el = ebuf(w, l), *e1 = ebuf(w, l + 1);
         __nv_bfloat16* ze = lbuf(w, w.ze, l, pe);
-        float* ye = lbuf(w, w.ye, l, pe);
-        float* ste = lbuf(w, w.ste, l, 2 * (size_t)w.cap_e);
         __nv_bfloat16* agg = lbuf(w, w.agg, l, pn);
         __nv_bfloat16* zn = lbuf(w, w.zn, l, pn);
-        float* yn = lbuf(w, w.yn, l, pn);
-        float* stn = lbuf(w, w.stn, l, 2 * (size_t)w.cap_n);
         WC_TRY(fwd(s, L.e1i, n, h, nullptr, false, nullptr, w.P));
         WC_TRY(fwd(s, L.e1s, n, h, nullptr, false, nullptr, w.Q));
         WC_TRY(fwd(s, L.e1e, e, el, nullptr, true, nullptr, ze, w.P, w.recv, w.Q, w.col));
-        if (fuse) {
-            WC_TRY(fwd_ln(s, L.e2, e, ze, s->w + L.lne.g, el, e1));
-        } else {
-            WC_TRY(fwd(s, L.e2, e, ze, nullptr, false, ye, nullptr));
-            layernorm(e, ye, s->w + L.lne.g, s->w + L.lne.g + W, el, e1, ste, ste + e, s->stream);
-        }
+        WC_TRY(layer_ln(s, keep, L.e2, e, ze, L.lne, el, e1, lbuf(w, w.ye, l, pe), lbuf(w, w.ste, l, 2 * (size_t)w.cap_e)));
         segment_sum_bf16(n, w.rowptr, nullptr, e1, nullptr, agg, s->stream);
         WC_TRY(fwd(s, L.n1, n, h, agg, true, nullptr, zn));
-        if (fuse) {
-            WC_TRY(fwd_ln(s, L.n2, n, zn, s->w + L.lnn.g, h, h1));
-        } else {
-            WC_TRY(fwd(s, L.n2, n, zn, nullptr, false, yn, nullptr));
-            layernorm(n, yn, s->w + L.lnn.g, s->w + L.lnn.g + W, h, h1, stn, stn + n, s->stream);
-        }
+        WC_TRY(layer_ln(s, keep, L.n2, n, zn, L.lnn, h, h1, lbuf(w, w.yn, l, pn), lbuf(w, w.stn, l, 2 * (size_t)w.cap_n)));
     }
     WC_TRY(fwd(s, s->d1, n, hbuf(w, s->L), nullptr, true, nullptr, w.zd));
     WC_TRY(fwd(s, s->d2, n, w.zd, nullptr, false, w.out, nullptr));
