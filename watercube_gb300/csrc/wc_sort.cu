@@ -122,6 +122,24 @@ __global__ void __launch_bounds__(256) bin_count_kernel(const float4* __restrict
     }
 }
 
+// A tile's values (16 consecutive ones per thread) to out[first ..], below C, by way of shared memory
+// (rows of 16 words with one word of padding to every 32).
+__device__ __forceinline__ void store_tile(uint32_t* s, const uint32_t (&v)[SCAN_ITEMS], uint32_t* __restrict__ out,
+                                           uint32_t first, uint32_t C, uint32_t tid) {
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < SCAN_ITEMS; ++k) {
+        const uint32_t i = tid * SCAN_ITEMS + k;
+        s[i + (i >> 5)] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < SCAN_ITEMS; ++k) {
+        const uint32_t i = k * SCAN_THREADS + tid;
+        if (first + i < C) out[first + i] = s[i + (i >> 5)];
+    }
+}
+
 // second: LANE ? the padded starts (+ total) : the list of non-empty cells.
 template <bool LANE>
 __global__ void __launch_bounds__(SCAN_THREADS) scan_cells_kernel(uint32_t* __restrict__ counts, uint32_t C,
@@ -134,6 +152,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_cells_kernel(uint32_t* __re
     __shared__ uint32_t s_tile;
     __shared__ unsigned long long s_warp[NW];
     __shared__ unsigned long long s_excl;
+    __shared__ uint32_t s_tile_out[SCAN_TILE + SCAN_TILE / 32];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     // Tiles are numbered in arrival order, so every predecessor of a tile is already running:
     // the look-back below never waits on a block that has not been scheduled.
@@ -232,20 +251,22 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_cells_kernel(uint32_t* __re
     const unsigned long long pre = s_excl + thread_excl;
     uint32_t run = (uint32_t)(pre & COUNT_MASK);
     uint32_t nz = (uint32_t)(pre >> NZ_SHIFT);
+    // A thread's 16 results go through shared memory, so that the stores are whole 128-byte lines
+    // (written from the registers, each store of a warp touched 32 of them).
+    uint32_t r1[SCAN_ITEMS], r2[SCAN_ITEMS];
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
-        const uint32_t c = base + k;
-        if (c < C) {
-            start[c] = run;
-            if (LANE) {
-                second[c] = nz;
-                nz += (v[k] + 3u) & ~3u;
-            } else if (v[k]) {
-                second[nz++] = c;
-            }
-            run += v[k];
+        r1[k] = run;
+        run += v[k];
+        if (LANE) {
+            r2[k] = nz;
+            nz += (v[k] + 3u) & ~3u;
+        } else if (base + k < C && v[k]) {
+            second[nz++] = base + k;
         }
     }
+    store_tile(s_tile_out, r1, start, tile * (uint32_t)SCAN_TILE, C, tid);
+    if (LANE) store_tile(s_tile_out, r2, second, tile * (uint32_t)SCAN_TILE, C, tid);
     if (tile == num_tiles - 1 && tid == SCAN_THREADS - 1) {
         start[C] = run;
         if (LANE) second[C] = nz;

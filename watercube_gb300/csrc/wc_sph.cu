@@ -644,6 +644,26 @@ __global__ void __launch_bounds__(SPH_THREADS, 5) density_kernel(const SceneCons
 // with judge_part it also sums |rho_carried / rho - 1| over each chunk into judge_part[m]
 // (rho_carried: the slot's .w before this pass; a non-finite ratio counts 1).
 
+// Chunk scheduling of the lane kernels: a warp's first chunk is its place in the launch, blocks first
+// (so that few chunks spread over all SMs, and none waits for an atomic), the following ones come from a
+// counter, drawn one chunk ahead. With M chunks the active warps (those with a first chunk) draw M
+// values in all, each until one lies beyond the last chunk, so the warp that draws M - 1 draws last
+// and puts the counter back to zero for the next launch.
+struct LaneChunks {
+    uint32_t* counter;
+    uint32_t M, W, lane, drawn;
+    __device__ __forceinline__ LaneChunks(uint32_t* c, uint32_t m, uint32_t l)
+        : counter(c), M(m), W(gridDim.x * (uint32_t)WARPS), lane(l), drawn(0) {}
+    __device__ __forceinline__ uint32_t first() const { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }
+    __device__ __forceinline__ void prefetch() {
+        if (lane == 0) {
+            drawn = atomicAdd(counter, 1u);
+            if (drawn == M - 1u) atomicExch(counter, 0u);
+        }
+    }
+    __device__ __forceinline__ uint32_t next() const { return W + __shfl_sync(FULL, drawn, 0); }
+};
+
 // max(v, 0) that keeps a NaN (a non-finite position must not look like an empty neighbourhood).
 __device__ __forceinline__ float relu_nan(float v) {
     float r;
@@ -704,10 +724,9 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
     const float* const X = xyz;
     const float* const Y = xyz + pcap;
     const float* const Z = xyz + 2 * (size_t)pcap;
-    uint32_t m_next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
-    uint32_t m = __shfl_sync(FULL, m_next, 0);
-    for (; m < M; m = __shfl_sync(FULL, m_next, 0)) {
-        if (lane == 0) m_next = atomicAdd(counter, 1u);
+    LaneChunks chunks(counter, M, lane);
+    for (uint32_t m = chunks.first(); m < M; m = chunks.next()) {
+        chunks.prefetch();
         float judge = 0.f;  // FEAT with judge_part: this lane's |rho_carried / rho - 1|
         do {
             uint32_t ti[TARGETS];  // sorted slots (>= n: none)
@@ -873,7 +892,6 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
             if (lane == 0) judge_part[m] = judge;
         }
     }
-    if (lane == 0 && m == M + gridDim.x * (uint32_t)WARPS - 1u) atomicExch(counter, 0u);
 }
 
 // The records of the padded slots again from the sorted buffer, for a force pass that does not
@@ -1412,10 +1430,9 @@ __global__ void __launch_bounds__(SPH_THREADS, 3) force_lane_kernel(
     uint32_t* const list = s_list[threadIdx.x >> 5] + lane;
     const uint32_t M = (n + 31u) >> 5;  // chunks of 32 slots
     uint32_t* const counter = num_nonempty + 2;
-    uint32_t m_next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
-    uint32_t m = __shfl_sync(FULL, m_next, 0);
-    for (; m < M; m = __shfl_sync(FULL, m_next, 0)) {
-        if (lane == 0) m_next = atomicAdd(counter, 1u);
+    LaneChunks chunks(counter, M, lane);
+    for (uint32_t m = chunks.first(); m < M; m = chunks.next()) {
+        chunks.prefetch();
         const uint32_t ti = (m << 5) + lane;
         const bool live = ti < n;
         const uint32_t tself = live ? ti : n - 1u;
@@ -1514,8 +1531,6 @@ __global__ void __launch_bounds__(SPH_THREADS, 3) force_lane_kernel(
         }
         if (in.part_done) report_chunk(in, m, M, lane);
     }
-    // the chunk counter returns to zero for the next launch (see release_counter)
-    if (lane == 0 && m == M + gridDim.x * (uint32_t)WARPS - 1u) atomicExch(counter, 0u);
 }
 
 template <class... A>
