@@ -75,3 +75,26 @@ def test_rewritten_sorted_buffer(gpu, oracle, name):
     # terms, 500 x 2^-24 = 3e-5 of the largest change
     dv = np.abs(out[1][1]["velocity"] - out[1][0]["velocity"]).max()
     assert np.abs(out[0][1]["velocity"] - out[1][1]["velocity"]).max() <= 1e-4 * dv
+
+
+@pytest.mark.parametrize("G", [2, 5, 8, 33])
+@pytest.mark.parametrize("flags", [0, _abi.WC_FLAG_CELL_TEAMS])
+def test_surface_grid_edges(gpu, oracle, G, flags):
+    """The field's vertex blocks at ragged grids, on a fluid of either pass variant, bit for bit; the
+    same surface object then takes a larger and again the smaller mesh."""
+    from oracle import surface_ref as R
+    from watercube_gb300.surface import Surface
+
+    p, small = ragged(3001, 4, flags=flags)
+    big = small.copy()
+    big["position"] *= np.float32([1.6, 1.6, 1.0])
+    with fluid(p, small) as f, Surface(G, iso=0.3) as s:
+        for state in (small, big, small):
+            f.set_particles(state)
+            n = s.extract(f)
+            srt, _, _, counts, offsets = oracle.sort(p, state)
+            phi = R.field(srt["position"].astype(np.float32), np.append(offsets, np.uint32(len(state))), p.bin_size,
+                          p.grid_res, p.size, G, p.kernel_radius, p.particle_mass, p.rest_density)
+            assert np.array_equal(s.field(), phi)
+            ref = R.march(phi, p.size, 0.3)
+            assert n == ref.shape[0] and np.array_equal(s.triangles(), ref)
