@@ -44,6 +44,9 @@ struct wc_fluid {
     float4* staging = nullptr;
     uint32_t* h_err = nullptr;
     HostReadback readback{};  // wc_fluid_update_host
+    // kept from the first use: the recording's accelerations (d.accel while it is on), diagnostics
+    float4* accel_store = nullptr;
+    double *diag_part = nullptr, *h_diag = nullptr;
     // L2 flush for timing
     float4* flush_buf = nullptr;
     size_t flush_n4 = 0;
@@ -65,11 +68,13 @@ void free_all(wc_fluid* f) {
     void* ptrs[] = {d.pos_a,     d.vel_a,        d.pos_b,     d.vel_b,    d.ids_a,           d.ids_b,
                     d.keys,      d.ranks,        d.unordered, d.perm,     d.counts,          d.start,
                     d.cell_list, d.num_nonempty, d.scan_desc, d.ncount,   d.scan_tile_counter, d.err,
-                    d.hits,      f->staging,     f->flush_buf, f->flush_sink, d.accel,  d.xyz,
+                    d.hits,      f->staging,     f->flush_buf, f->flush_sink, f->accel_store, d.xyz,
+                    f->diag_part,
                     d.pstart,    d.cidx,         d.rec,       d.info};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (f->h_err) cudaFreeHost(f->h_err);
+    if (f->h_diag) cudaFreeHost(f->h_diag);
     if (f->exec) cudaGraphExecDestroy(f->exec);
     if (f->graph) cudaGraphDestroy(f->graph);
     f->readback.release();
@@ -351,6 +356,15 @@ wc_status fluid_graph_step(wc_fluid* f, float dt) {
     return rc;
 }
 
+wc_status fluid_diagnostics_buffers(wc_fluid* f, double** device, double** host) {
+    if (!f->diag_part) WC_TRY(dalloc(&f->diag_part, DIAG_BLOCKS * 5));
+    if (!f->h_diag && cudaMallocHost(reinterpret_cast<void**>(&f->h_diag), sizeof(double) * DIAG_BLOCKS * 5) != cudaSuccess)
+        return fail(WC_ERR_OOM, "pinned host allocation failed");
+    *device = f->diag_part;
+    *host = f->h_diag;
+    return WC_OK;
+}
+
 void fluid_count_step(wc_fluid* f) { ++f->steps; }
 void fluid_set_step_count(wc_fluid* f, uint64_t steps) { f->steps = steps; }
 
@@ -609,11 +623,11 @@ WC_API wc_status wc_fluid_set_recording(wc_fluid* f, int on) {
     clear_error();
     WC_TRY(require(f, false));
     if (on && !f->d.accel) {
-        WC_TRY(dalloc(&f->d.accel, f->d.n));
+        if (!f->accel_store) WC_TRY(dalloc(&f->accel_store, f->d.n));
+        f->d.accel = f->accel_store;
         if (f->d.n) WC_CUDA_TRY(cudaMemsetAsync(f->d.accel, 0, sizeof(float4) * f->d.n, f->stream));
     } else if (!on && f->d.accel) {
-        WC_CUDA_TRY(cudaStreamSynchronize(f->stream));
-        cudaFree(f->d.accel);
+        // the buffer stays with the fluid: a rollout switches recording on and off in every call
         f->d.accel = nullptr;
     }
     if (f->exec) cudaGraphExecDestroy(f->exec);

@@ -392,6 +392,13 @@ wc_status batch_check(wc_batch* b);                 // launch errors and device 
 wc_status fluid_check(wc_fluid* f);
 // FP64 totals of a fluid's state buffer: mass, momentum x/y/z, kinetic and potential energy.
 wc_status fluid_diagnostics(wc_fluid* f, double out[6]);
+// The same in two halves, for a caller that waits for the stream anyway: the totals' partial sums on
+// their way to the host, and the totals once the stream has been waited for.
+wc_status fluid_diagnostics_enqueue(wc_fluid* f);
+wc_status fluid_diagnostics_result(wc_fluid* f, double out[6]);
+// Their buffers (DIAG_BLOCKS x 5 sums on the device and in pinned memory), kept with the fluid.
+constexpr uint32_t DIAG_BLOCKS = 608;  // four per SM
+wc_status fluid_diagnostics_buffers(wc_fluid* f, double** device, double** host);
 void fluid_enqueue_sort(wc_fluid* f, int pass_variant = -1);  // -1: the fluid's own
 wc_status fluid_graph_step(wc_fluid* f, float dt);  // one plain SPH step (graph replay)
 void fluid_count_step(wc_fluid* f);

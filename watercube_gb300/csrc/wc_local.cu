@@ -1538,9 +1538,10 @@ WC_API wc_status wc_local_rollout_mode(wc_local* s, wc_fluid* f, float dt, uint3
     if (rc == WC_OK) rc = ensure_roll(w, n);
     const bool had_accel = t.d->accel != nullptr;
     if (rc == WC_OK && !had_accel) rc = wc_fluid_set_recording(f, 1);
-    if (rc == WC_OK) rc = fluid_check(f);
     double diag[6];
-    if (rc == WC_OK) rc = fluid_diagnostics(f, diag);
+    if (rc == WC_OK) rc = fluid_diagnostics_enqueue(f);
+    if (rc == WC_OK) rc = fluid_check(f);  // waits for the stream
+    if (rc == WC_OK) rc = fluid_diagnostics_result(f, diag);
     if (rc != WC_OK) {
         if (own) wc_local_destroy(own);
         return rc;
@@ -1654,13 +1655,14 @@ WC_API wc_status wc_local_rollout_mode(wc_local* s, wc_fluid* f, float dt, uint3
     cudaEventDestroy(e1);
     cudaEventDestroy(ej);
     if (rc == WC_OK && ce != cudaSuccess) rc = fail(WC_ERR_CUDA, "rollout: %s", cudaGetErrorString(ce));
-    if (rc == WC_OK) rc = fluid_check(f);
+    const bool closing = rc == WC_OK && fluid_diagnostics_enqueue(f) == WC_OK;
+    if (rc == WC_OK) rc = fluid_check(f);  // waits for the stream
     if (rc == WC_OK) rc = read_err(w);
     if (!had_accel) {
         const wc_status r2 = wc_fluid_set_recording(f, 0);
         if (rc == WC_OK) rc = r2;
     }
-    if (rc == WC_OK && fluid_diagnostics(f, diag) == WC_OK)
+    if (rc == WC_OK && closing && fluid_diagnostics_result(f, diag) == WC_OK)
         for (int q = 0; q < 6; ++q) out->diag_end[q] = diag[q];
     if (own) wc_local_destroy(own);
     if (rc != WC_OK) return rc;

@@ -679,24 +679,34 @@ __global__ void fluid_diag_kernel(uint32_t n, const float4* __restrict__ pos, co
 
 }  // namespace
 
-wc_status wc::fluid_diagnostics(wc_fluid* f, double out[6]) {
+wc_status wc::fluid_diagnostics_enqueue(wc_fluid* f) {
     FluidInternals fi = fluid_internals(f);
-    const uint32_t blocks = 256;
-    double* part = nullptr;
-    WC_TRY(dalloc(&part, blocks * 5));
-    fluid_diag_kernel<<<blocks, 256, 0, fi.stream>>>(fi.d->n, fi.d->pos_a, fi.d->vel_a, (double)fi.params->particle_mass,
-                                                     fi.in->g[0], fi.in->g[1], fi.in->g[2], part);
-    std::vector<double> h(blocks * 5);
-    cudaMemcpyAsync(h.data(), part, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, fi.stream);
-    cudaStreamSynchronize(fi.stream);
-    cudaFree(part);
+    double *part = nullptr, *host = nullptr;
+    WC_TRY(fluid_diagnostics_buffers(f, &part, &host));
+    fluid_diag_kernel<<<DIAG_BLOCKS, 256, 0, fi.stream>>>(fi.d->n, fi.d->pos_a, fi.d->vel_a,
+                                                          (double)fi.params->particle_mass, fi.in->g[0], fi.in->g[1],
+                                                          fi.in->g[2], part);
+    WC_CUDA_TRY(cudaMemcpyAsync(host, part, sizeof(double) * DIAG_BLOCKS * 5, cudaMemcpyDeviceToHost, fi.stream));
+    return WC_OK;
+}
+
+wc_status wc::fluid_diagnostics_result(wc_fluid* f, double out[6]) {
+    FluidInternals fi = fluid_internals(f);
+    double *part = nullptr, *host = nullptr;
+    WC_TRY(fluid_diagnostics_buffers(f, &part, &host));
     out[0] = (double)fi.params->particle_mass * fi.d->n;
     for (int q = 0; q < 5; ++q) {
         double a = 0.0;
-        for (uint32_t b = 0; b < blocks; ++b) a += h[(size_t)b * 5 + q];
+        for (uint32_t b = 0; b < DIAG_BLOCKS; ++b) a += host[(size_t)b * 5 + q];
         out[1 + q] = a;
     }
     return WC_OK;
+}
+
+wc_status wc::fluid_diagnostics(wc_fluid* f, double out[6]) {
+    WC_TRY(fluid_diagnostics_enqueue(f));
+    WC_CUDA_TRY(cudaStreamSynchronize(fluid_internals(f).stream));
+    return fluid_diagnostics_result(f, out);
 }
 
 namespace {
