@@ -96,6 +96,8 @@ void adam(size_t count, float* w, const float* g, float* m, float* v, float lr, 
 void cast_weight(const float* w, uint32_t k_in, uint32_t n_out, uint32_t k_pad, uint32_t n_pad, __nv_bfloat16* wt,
                  __nv_bfloat16* wk, cudaStream_t s);
 void gather4(uint32_t n, const uint32_t* perm, const float4* src, float4* dst, cudaStream_t s);
+void predictions(uint32_t n, const float* pred, uint32_t ldp, float scale, const float4* base, const uint32_t* perm,
+                 float4* out, cudaStream_t s);
 void sub_xyz(uint32_t n, float4* dst, const float4* sub, cudaStream_t s);
 void add_scaled(uint32_t n, const float* pred, uint32_t ldp, float scale, const float4* base, float4* dst,
                 cudaStream_t s);

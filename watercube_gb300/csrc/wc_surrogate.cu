@@ -1079,23 +1079,12 @@ WC_API wc_status wc_surrogate_forward_backward(wc_surrogate* s, int do_backward,
 WC_API wc_status wc_surrogate_predictions(wc_surrogate* s, float* host_out, uint32_t n) {
     clear_error();
     if (!s || !s->fluid || !host_out || n != s->n) return fail(WC_ERR_INVALID_ARG, "prediction buffer must hold n x 4");
-    // outputs are in sorted order: undo the sample's permutation on the host
-    FluidInternals fi = fluid_internals(s->fluid);
-    std::vector<float> out((size_t)n * OUT);
-    std::vector<uint32_t> perm(n);
-    std::vector<float4> base(s->has_stale ? n : 0);
-    WC_CUDA_TRY(cudaMemcpyAsync(out.data(), s->work.out, sizeof(float) * out.size(), cudaMemcpyDeviceToHost, s->stream));
-    WC_CUDA_TRY(cudaMemcpyAsync(perm.data(), fi.d->perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s->stream));
-    if (s->has_stale)
-        WC_CUDA_TRY(cudaMemcpyAsync(base.data(), s->work.stale_s, sizeof(float4) * n, cudaMemcpyDeviceToHost, s->stream));
-    WC_TRY(read_err(s));
-    for (uint32_t k = 0; k < n; ++k) {
-        const float b[3] = {s->has_stale ? base[k].x : 0.f, s->has_stale ? base[k].y : 0.f,
-                            s->has_stale ? base[k].z : 0.f};
-        for (int a = 0; a < 4; ++a)
-            host_out[(size_t)perm[k] * 4 + a] = a < 3 ? std::fmaf(out[(size_t)k * OUT + a], s->cfg.accel_scale, b[a]) : 0.f;
-    }
-    return WC_OK;
+    // outputs are in sorted order: the kernel undoes the sample's permutation (into the target's input
+    // buffer, which the sample has long gathered from)
+    nn::predictions(n, s->work.out, OUT, s->cfg.accel_scale, s->has_stale ? s->work.stale_s : nullptr,
+                    fluid_internals(s->fluid).d->perm, s->target_in, s->stream);
+    WC_CUDA_TRY(cudaMemcpyAsync(host_out, s->target_in, sizeof(float4) * n, cudaMemcpyDeviceToHost, s->stream));
+    return read_err(s);
 }
 
 WC_API wc_status wc_surrogate_adam(wc_surrogate* s, float lr, float grad_scale) {
