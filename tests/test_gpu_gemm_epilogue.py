@@ -78,3 +78,14 @@ def test_weight_gradient_splits(wclib, torch, m, n, k, chunk):  # noqa: F811
     ref = torch.stack([p.float().t() @ q.float() for p, q in zip(x.split(chunk), dy.split(chunk))])
     close(out[:parts], ref)
     assert bool((out[parts] == 7.0).all())
+
+
+@pytest.mark.parametrize("m", [1, 129, 20001])
+@pytest.mark.parametrize("split,k", [(128, 256), (64, 200), (40, 128)])  # 40: inside a slice, the cp.async kernel
+def test_two_sources(wclib, torch, m, split, k):  # noqa: F811
+    n = 128
+    x, y, wt = rnd(torch, m, split, seed=1), rnd(torch, m, k - split, seed=2), rnd(torch, n, k, seed=3)
+    c16 = torch.zeros(m, n, dtype=torch.bfloat16, device="cuda")
+    run(wclib, torch, m=m, n=n, k=k, a=x, lda=split, a2=y, lda2=k - split, k_split=split, b=wt, ldb=k, relu=1, c_bf16=c16,
+        ldc=n)
+    close(c16, torch.relu(torch.cat([x, y], 1).float() @ wt.float().t()), rel=BF16)

@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1) gemm_pipe_kernel(const GemmAr
 
 // ---- TMA variant: plain row-major A and B^T, B resident ----------------------------------------
 //
-// For A without a row gather or a second source, and B^T of one column of tiles (n <= 128,
+// For A without a row gather (a second source takes over at a whole slice), and B^T of one column of tiles (n <= 128,
 // k <= 64 RB_MAX_SLICES): one thread of warp 0 copies the operands with cp.async.bulk.tensor
 // (TMA) in the 128-byte-swizzled K-major layout — B^T once per CTA (barrier `b_full`), then the
 // A slices of the CTA's tiles into a ring, each copy completing its slot's `full` barrier
@@ -760,7 +760,7 @@ struct TmaPlan {
 };
 
 struct TmaMaps {
-    CUtensorMap a, b, aux, cb, cf;
+    CUtensorMap a, a2, b, aux, cb, cf;
 };
 
 __device__ __forceinline__ void pair_sync(uint32_t quarter) {
@@ -1106,7 +1106,10 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
                         break;
                     }
                     mbar_expect_tx(&full[st], TILE_BYTES);
-                    tma_load_box(&maps.a, ring + st * TILE_BYTES, sl * BK, m0, &full[st]);
+                    if (g.a2 && sl * BK >= g.k_split)
+                        tma_load_box(&maps.a2, ring + st * TILE_BYTES, sl * BK - g.k_split, m0, &full[st]);
+                    else
+                        tma_load_box(&maps.a, ring + st * TILE_BYTES, sl * BK, m0, &full[st]);
                 }
                 if (AUX == AUX_TMA && !*failed) {
                     const uint32_t b = t & 1u;
@@ -1427,7 +1430,8 @@ wc_status launch_tma_as(const GemmArgs& g, const TmaMaps& maps, const TmaPlan& p
     return WC_OK;
 }
 
-// The TMA kernel for plain row-major A, n <= 128 and k <= 384, when every operand it moves by TMA has a
+// The TMA kernel for row-major A (or [A | A2] split at a whole slice: the node layers' 65,536 x 256 take
+// 33 us with cp.async), n <= 128 and k <= 384, when every operand it moves by TMA has a
 // tensor map (16-byte aligned base and rows), the gathered rows are whole and aligned, and the shared
 // memory holds at least two A slots (all but k > 256 with two gathered operands, or with FP32 and
 // BF16 outputs together). Otherwise the caller runs the cp.async kernel.
@@ -1435,7 +1439,9 @@ wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream
     *launched = false;
     const bool gather = g.add1 || g.add2, aux = gather || g.ln_resid || g.relu_z, f32 = g.c_f32 != nullptr, bf = g.c_bf16 != nullptr;
     TmaMaps maps;
-    if (!encode_operand(&maps.a, g.a, g.k, g.m, 2ull * g.lda) || !encode_operand(&maps.b, g.b, g.k, g.n, 2ull * g.ldb))
+    if (g.a2 && (g.k_split % BK || g.k_split >= g.k || !encode_operand(&maps.a2, g.a2, g.k - g.k_split, g.m, 2ull * g.lda2)))
+        return WC_OK;
+    if (!encode_operand(&maps.a, g.a, g.a2 ? g.k_split : g.k, g.m, 2ull * g.lda) || !encode_operand(&maps.b, g.b, g.k, g.n, 2ull * g.ldb))
         return WC_OK;
     if (bf && !encode_operand(&maps.cb, g.c_bf16, g.n, g.m, 2ull * g.ldc, 32)) return WC_OK;
     if (f32 && !encode_operand(&maps.cf, g.c_f32, g.n, g.m, 4ull * g.ldc, 32, true)) return WC_OK;
@@ -1491,7 +1497,7 @@ wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s) {
         const uint32_t tiles = ((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
         const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
         const bool rb = g.n <= (uint32_t)BN && (g.k + BK - 1) / BK <= RB_MAX_SLICES;
-        if (rb && !g.a_rows && !g.a2) {
+        if (rb && !g.a_rows) {
             bool launched = false;
             WC_TRY(launch_tma(g, grid, err, s, &launched));
             if (launched) return WC_OK;
