@@ -304,6 +304,18 @@ wc_status ensure_staging(wc_batch* b) {
     return WC_OK;
 }
 
+// Host AoS -> the state, on the batch's stream, without waiting; a page-locked buffer is read where it lies.
+wc_status enqueue_upload(wc_batch* b, const wc_particle* in) {
+    const float4* src = mapped_host(in, sizeof(wc_particle) * (size_t)b->n);
+    if (!src) {
+        WC_TRY(ensure_staging(b));
+        WC_CUDA_TRY(cudaMemcpyAsync(b->staging, in, sizeof(wc_particle) * (size_t)b->n, cudaMemcpyHostToDevice, b->stream));
+        src = b->staging;
+    }
+    launch_aos_to_soa(src, b->d.pos_a, b->d.vel_a, (uint32_t)b->n, b->stream);
+    return WC_OK;
+}
+
 wc_status require(const wc_batch* b, bool need_setup) {
     if (!b) return fail(WC_ERR_INVALID_ARG, "null batch handle");
     if (need_setup && !b->setup_done) return fail(WC_ERR_STATE, "wc_batch_setup has not been called");
@@ -605,9 +617,7 @@ WC_API wc_status wc_batch_set_particles(wc_batch* b, const wc_particle* in, uint
                                    (unsigned long long)total, (unsigned long long)b->n);
     if (!total) return WC_OK;
     if (!in) return fail(WC_ERR_INVALID_ARG, "null input");
-    WC_TRY(ensure_staging(b));
-    WC_CUDA_TRY(cudaMemcpyAsync(b->staging, in, sizeof(wc_particle) * total, cudaMemcpyHostToDevice, b->stream));
-    launch_aos_to_soa(b->staging, b->d.pos_a, b->d.vel_a, (uint32_t)total, b->stream);
+    WC_TRY(enqueue_upload(b, in));
     WC_CUDA_TRY(cudaStreamSynchronize(b->stream));
     return WC_OK;
 }
@@ -685,17 +695,17 @@ WC_API wc_status wc_batch_step_host(wc_batch* b, float dt, const wc_particle* in
     }
     const uint32_t n = (uint32_t)total;
     b->in.dt = dt;
-    WC_TRY(ensure_staging(b));
-    if (in) {
-        // the final wait covers the copy from in
-        WC_CUDA_TRY(cudaMemcpyAsync(b->staging, in, sizeof(wc_particle) * total, cudaMemcpyHostToDevice, b->stream));
-        launch_aos_to_soa(b->staging, b->d.pos_a, b->d.vel_a, n, b->stream);
-    }
+    if (in) WC_TRY(enqueue_upload(b, in));  // the final wait covers the copy from in
     StepInputs step = b->in;
-    WC_TRY(b->readback.arm(b->stream, n, b->staging, step));
+    step.aos_out = mapped_host(out, sizeof(wc_particle) * total);
+    const bool direct = step.aos_out != nullptr;  // the force pass writes the host records where they belong
+    if (!direct) {
+        WC_TRY(ensure_staging(b));
+        WC_TRY(b->readback.arm(b->stream, n, b->staging, step));
+    }
     enqueue_step(b, step);  // the graph's stages, launched directly with the readback fields
     WC_CUDA_TRY(cudaGetLastError());
-    WC_TRY(b->readback.drain(b->stream, n, b->staging, out));
+    if (!direct) WC_TRY(b->readback.drain(b->stream, n, b->staging, out));
     return read_errors(b);
 }
 

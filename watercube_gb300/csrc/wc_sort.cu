@@ -350,11 +350,15 @@ __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint
     }
 }
 
+// Host records in place run at the link's rate (205 GB/s read; 1 to 4 records per thread in flight and 256 to
+// 4,096 blocks at most make no difference).
 __global__ void aos_to_soa_kernel(const float4* __restrict__ aos, float4* __restrict__ pos, float4* __restrict__ vel,
                                   uint32_t n) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        pos[i] = aos[2 * (size_t)i];
-        vel[i] = aos[2 * (size_t)i + 1];
+        float4 p, v;
+        load_float8(aos, i, p, v);
+        pos[i] = p;
+        vel[i] = v;
     }
 }
 

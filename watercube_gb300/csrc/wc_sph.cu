@@ -671,16 +671,9 @@ __device__ __forceinline__ float relu_nan(float v) {
     return r;
 }
 
-__device__ __forceinline__ void store_record(float4* rec, uint32_t pslot, const float4& pi, float inv_rho, const float4& vi,
+__device__ __forceinline__ void store_record(float4* rec, uint32_t pslot, const float4& p, float inv_rho, const float4& v,
                                              float pressure) {
-    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(rec + 2 * (size_t)pslot), "f"(pi.x), "f"(pi.y),
-                 "f"(pi.z), "f"(inv_rho), "f"(vi.x), "f"(vi.y), "f"(vi.z), "f"(pressure)
-                 : "memory");
-}
-__device__ __forceinline__ void load_record(const float4* rec, uint32_t pslot, float4& p, float4& v) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-        : "l"(rec + 2 * (size_t)pslot));
+    store_float8(rec, pslot, make_float4(p.x, p.y, p.z, inv_rho), make_float4(v.x, v.y, v.z, pressure));
 }
 
 // Slot ti's entry 0; its entry e lies 32 e further.
@@ -1006,7 +999,7 @@ __device__ __forceinline__ void accumulate_records(const uint32_t* list, uint32_
 #pragma unroll
         for (int u = 0; u < ROUND; ++u) {
             const uint32_t k = e + (uint32_t)u < cnt ? list[(e + (uint32_t)u) * 32u] : self;
-            load_record(rec, k, pj[u], vj[u]);
+            load_float8(rec, k, pj[u], vj[u]);
             rj[u] = FEAT == FEAT_FULL ? __ldg(rate + k) : make_float2(0.f, 0.f);
         }
 #pragma unroll
@@ -1067,10 +1060,7 @@ __device__ __forceinline__ void integrate_store(const SceneConsts& sc, const Ste
     const float4 pa = make_float4(x[0], x[1], x[2], rho), va = make_float4(v[0], v[1], v[2], pressure);
     pos_a[ti] = pa;
     vel_a[ti] = va;
-    if (in.aos_out) {
-        in.aos_out[2 * (size_t)ti] = pa;
-        in.aos_out[2 * (size_t)ti + 1] = va;
-    }
+    if (in.aos_out) store_float8(in.aos_out, ti, pa, va);
     if (ids_a) ids_a[ti] = ids_b[ti];
     if (accel) accel[ti] = make_float4(acc[0], acc[1], acc[2], 0.f);
     if (FEAT == FEAT_RATE) fb.out[ti] = make_float4(0.f, 0.f, 0.f, -6.f * sc.m * sc.c6 * f[6]);
@@ -1518,10 +1508,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 3) force_lane_kernel(
                 // not evaluated (see MAX_CELL_PARTICLES): the particle keeps its state, reported
                 pos_a[ti] = pi;
                 vel_a[ti] = vi;
-                if (in.aos_out) {
-                    in.aos_out[2 * (size_t)ti] = pi;
-                    in.aos_out[2 * (size_t)ti + 1] = vi;
-                }
+                if (in.aos_out) store_float8(in.aos_out, ti, pi, vi);
                 if (ids_a) ids_a[ti] = ids_b[ti];
                 if (accel) accel[ti] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (FEAT) fb.out[ti] = make_float4(0.f, 0.f, 0.f, 0.f);
