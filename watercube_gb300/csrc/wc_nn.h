@@ -52,6 +52,21 @@ bool gemm_tma_available();
 wc_status check_gemm(const GemmArgs& g);
 wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s);
 
+// out = LN(relu(a w1 + b1 (+ add1[add1_idx[row]] + add2[add2_idx[row]])) w2 + b2) gamma + beta, and + a where rows
+// are added: rows of k (a), 128 (the others); w1 [128 x k] and w2 [128 x 128] output-major. Not launched when
+// k > 128, an operand is not 16-byte aligned or tensor maps are not available (the caller runs the layers in turn).
+struct MlpArgs {
+    uint32_t m, k;
+    const __nv_bfloat16 *a, *w1, *w2;
+    const float *b1, *b2, *gamma, *beta;  // b1, b2 may be null
+    const __nv_bfloat16* add1;
+    const uint32_t* add1_idx;
+    const __nv_bfloat16* add2;  // both rows or neither
+    const uint32_t* add2_idx;
+    __nv_bfloat16* out;
+};
+wc_status launch_mlp(const MlpArgs& g, uint32_t* err, cudaStream_t s, bool* launched);
+
 }  // namespace nn
 }  // namespace wc
 

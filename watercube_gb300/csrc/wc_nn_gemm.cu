@@ -767,9 +767,60 @@ __device__ __forceinline__ void pair_sync(uint32_t quarter) {
     asm volatile("bar.sync %0, 64;" ::"r"(1u + quarter) : "memory");
 }
 
+// The LayerNorm of n = 128 columns by the two warps of a pair: x holds a thread's 64 columns (from col0) of its
+// row and becomes gamma (x - mean) rstd + beta, xs/xv/oks as in tma_epilogue. False when a wait of either warp
+// failed (both leave).
+template <bool VEC>
+__device__ __forceinline__ void ln_scale(const float* gamma, const float* beta, const float* x, float rstd, float* o) {
+    float gm[8], bt[8];
+    if (VEC) {
+#pragma unroll
+        for (int k = 0; k < 8; k += 4) {
+            const float4 g4 = __ldg(reinterpret_cast<const float4*>(gamma + k));
+            const float4 b4 = __ldg(reinterpret_cast<const float4*>(beta + k));
+            gm[k] = g4.x, gm[k + 1] = g4.y, gm[k + 2] = g4.z, gm[k + 3] = g4.w;
+            bt[k] = b4.x, bt[k + 1] = b4.y, bt[k + 2] = b4.z, bt[k + 3] = b4.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            gm[k] = __ldg(gamma + k);
+            bt[k] = __ldg(beta + k);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] = x[k] * rstd * gm[k] + bt[k];
+}
+__device__ __forceinline__ bool ln_centre(float (&x)[64], bool ok, float (*xs)[2][32], float (*xv)[2][32], int (*oks)[2],
+                                          volatile int* failed, uint32_t quarter, uint32_t half, uint32_t lane, float* rstd) {
+    constexpr float LN_EPSILON = 1e-5f;
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) sum += x[j];
+    xs[quarter][half][lane] = sum;
+    if (lane == 0) oks[quarter][half] = ok ? 1 : 0;
+    pair_sync(quarter);
+    if (!(oks[quarter][0] && oks[quarter][1])) {
+        if (lane == 0) *failed = 1;
+        return false;
+    }
+    const float mean = (xs[quarter][0][lane] + xs[quarter][1][lane]) * (1.f / 128.f);
+    float sq = 0.f;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+        x[j] -= mean;
+        sq += x[j] * x[j];
+    }
+    xv[quarter][half][lane] = sq;
+    pair_sync(quarter);
+    const float var = (xv[quarter][0][lane] + xv[quarter][1][lane]) * (1.f / 128.f);
+    *rstd = rsqrtf(var + LN_EPSILON);
+    return true;
+}
+
 // The epilogue of one warp: rows 32 quarter .., columns 64 half .. of every tile of the CTA.
 // LN (n = 128): the two warps that read the same 32 accumulator lanes hold a row's 128 columns
-// between them. Each thread sums its 64 values, the pair exchanges the sums through shared memory at
+// between them (ln_centre). Each thread sums its 64 values, the pair exchanges the sums through shared memory at
 // a named barrier of its 64 threads (ids 1 .. 4), then the squared deviations from the mean the
 // same way, and each thread normalises, scales and shifts its own columns and adds the residual
 // row. Both warps of a pair pass both barriers of every tile: whether each warp's waits succeeded is
@@ -938,48 +989,13 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
             }
             bias_add(x, col0);
             bias_add(x + 32, col0 + 32u);
-            float sum = 0.f;
-#pragma unroll
-            for (int j = 0; j < 64; ++j) sum += x[j];
-            xs[quarter][half][lane] = sum;
-            if (lane == 0) oks[quarter][half] = ok ? 1 : 0;
-            pair_sync(quarter);
-            if (!(oks[quarter][0] && oks[quarter][1])) {
-                if (lane == 0) *failed = 1;
-                break;
-            }
-            const float mean = (xs[quarter][0][lane] + xs[quarter][1][lane]) * (1.f / 128.f);
-            float sq = 0.f;
-#pragma unroll
-            for (int j = 0; j < 64; ++j) {
-                x[j] -= mean;
-                sq += x[j] * x[j];
-            }
-            xv[quarter][half][lane] = sq;
-            pair_sync(quarter);
-            const float var = (xv[quarter][0][lane] + xv[quarter][1][lane]) * (1.f / 128.f);
-            const float rstd = rsqrtf(var + LN_EPSILON);
+            float rstd;
+            if (!ln_centre(x, ok, xs, xv, oks, failed, quarter, half, lane, &rstd)) break;
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
-                float gm[8], bt[8];
-                if (vec) {
-#pragma unroll
-                    for (int k = 0; k < 8; k += 4) {
-                        const float4 g4 = __ldg(reinterpret_cast<const float4*>(g.ln_gamma + col0 + 8 * c + k));
-                        const float4 b4 = __ldg(reinterpret_cast<const float4*>(g.ln_beta + col0 + 8 * c + k));
-                        gm[k] = g4.x, gm[k + 1] = g4.y, gm[k + 2] = g4.z, gm[k + 3] = g4.w;
-                        bt[k] = b4.x, bt[k + 1] = b4.y, bt[k + 2] = b4.z, bt[k + 3] = b4.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        gm[k] = __ldg(g.ln_gamma + col0 + 8 * c + k);
-                        bt[k] = __ldg(g.ln_beta + col0 + 8 * c + k);
-                    }
-                }
                 float o[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) o[k] = x[8 * c + k] * rstd * gm[k] + bt[k];
+                if (vec) ln_scale<true>(g.ln_gamma + col0 + 8 * c, g.ln_beta + col0 + 8 * c, x + 8 * c, rstd, o);
+                else ln_scale<false>(g.ln_gamma + col0 + 8 * c, g.ln_beta + col0 + 8 * c, x + 8 * c, rstd, o);
                 const uint32_t at = stage + sw128(r, (uint32_t)c);
                 if (AUX == AUX_TMA) add8(o, lds128(at));
                 sts128(at, make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7])));
@@ -1219,6 +1235,308 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
     }
 }
 
+// ---- two layers and a LayerNorm in one kernel (inference) ----------------------------------------
+//
+// out = LN(relu(A W1 + b1 (+ P[i] + Q[j])) W2 + b2) gamma + beta (+ A), hidden and output width 128, k <= 128. As two
+// launches the hidden rows cross memory twice and a message layer reads its edges' rows again as the residual: 1,280
+// bytes per edge and layer where this kernel moves 512 (and the gathered rows, from L2).
+// A tile of 128 rows passes through a pipeline of warps: warp 0's TMA brings A into one of three slots; warp 1 issues
+// the first layer's MMAs; warps 8..15 add the bias and the gathered rows, apply the ReLU and write the hidden rows as
+// BF16 into the 128-byte-swizzled K-major layout that warp 2's MMAs of the second layer read; warps 16..23 normalise,
+// add the rows that the slot still holds, write the result over them and store it by TMA. Both layers' accumulators
+// are double (all 512 TMEM columns). Q's rows are copied by warps 4..7 into the place of the hidden rows; P's are
+// read straight into registers: edges are sorted by receiver, so the 32 rows of a warp share one or two of P's,
+// which L1 serves (any index is correct). Registers are moved from the copying warps to the normalising ones.
+// The arithmetic and its order are those of the two launches (the same results bit for bit).
+// 1.85 M edges: 312 us against 240 + 250 in two launches (345 us when one group of eight warps ran both epilogues
+// and both gathered rows were copied); bound by the epilogues' instructions (55 % of the issue slots) and L1 (72 %).
+constexpr uint32_t MLP_SLOTS = 3;
+constexpr int MLP_THREADS = 24 * 32;
+constexpr uint32_t MLP_TMEM_COLS = 512;
+// Registers per thread at launch, and by role (warpgroups 0, 1: 40, 2, 3: 80, 4, 5: 120) in the same total.
+constexpr int MLP_REGS = 80;
+static_assert(2 * 40 + 2 * 80 + 2 * 120 <= 6 * MLP_REGS, "the roles share what the block was launched with");
+constexpr uint32_t mlp_smem(uint32_t nslices) { return (nslices + 2u) * TILE_BYTES + (MLP_SLOTS + 2u) * AUX_BYTES; }
+
+struct MlpMaps {
+    CUtensorMap a, w1, w2, c;
+};
+
+// The MMAs of one 128 x 128 tile over nslices slices of 64 (operands TILE_BYTES apart), committed to `done`.
+__device__ __forceinline__ void mma_tile(uint32_t acc_addr, uint32_t a, uint32_t b, uint32_t nslices, uint64_t* done) {
+    for (uint32_t sl = 0; sl < nslices; ++sl) {
+#pragma unroll
+        for (uint32_t j = 0; j < BK / 16; ++j) {
+            const uint64_t ad = sw128_desc(a + sl * TILE_BYTES + 32u * j);
+            const uint64_t bd = sw128_desc(b + sl * TILE_BYTES + 32u * j);
+            const uint32_t acc = (sl > 0 || j > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc_addr),
+                "l"(ad), "l"(bd), "r"(IDESC), "r"(acc));
+        }
+    }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(done)) : "memory");
+}
+
+template <bool MP>
+__global__ void __launch_bounds__(MLP_THREADS, 1)
+    gemm_mlp_kernel(const MlpArgs g, const __grid_constant__ MlpMaps maps, uint32_t* err) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ uint64_t a_full[MLP_SLOTS], a_empty[MLP_SLOTS], acc1_full[2], acc1_empty[2], acc2_full[2], acc2_empty[2],
+        z_full[2], q_full[2], w_full;
+    __shared__ float s_lnx[4][2][32], s_lnv[4][2][32];
+    __shared__ int s_lnok[4][2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_failed;
+    volatile int* failed = &s_failed;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t ntiles = (g.m + BM - 1) / BM, nslices = (g.k + BK - 1) / BK;
+    const uint32_t mine = ntiles > blockIdx.x ? (ntiles - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;  // this CTA's tiles
+    const uint32_t w1 = smem_addr(smem_raw), w2 = w1 + nslices * TILE_BYTES;
+    unsigned char* const slots = smem_raw + (nslices + 2u) * TILE_BYTES;
+    const uint32_t z = smem_addr(slots) + MLP_SLOTS * AUX_BYTES;  // two stages of Q's, then the hidden rows
+
+    if (threadIdx.x == 0) {
+        for (uint32_t q = 0; q < MLP_SLOTS; ++q) {
+            mbar_init(&a_full[q], 1);
+            mbar_init(&a_empty[q], 8);
+        }
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(&acc1_full[q], 1);
+            mbar_init(&acc1_empty[q], 8);
+            mbar_init(&acc2_full[q], 1);
+            mbar_init(&acc2_empty[q], 8);
+            mbar_init(&z_full[q], 8);
+            mbar_init(&q_full[q], 4 * 32);
+        }
+        mbar_init(&w_full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_failed = 0;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
+                     "r"(MLP_TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;  // layer 1: columns 0 .., 128 ..; layer 2: 256 .., 384 ..
+
+    if (warp < 4u) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (lane == 0 && warp == 0) {
+            mbar_expect_tx(&w_full, (nslices + 2u) * TILE_BYTES);
+            for (uint32_t sl = 0; sl < nslices; ++sl) tma_load_box(&maps.w1, smem_raw + sl * TILE_BYTES, sl * BK, 0u, &w_full);
+            for (uint32_t sl = 0; sl < 2u; ++sl)
+                tma_load_box(&maps.w2, smem_raw + (nslices + sl) * TILE_BYTES, sl * BK, 0u, &w_full);
+            for (uint32_t t = 0; t < mine && !*failed; ++t) {
+                const uint32_t st = t % MLP_SLOTS, u = t / MLP_SLOTS;
+                if (u && !mbar_wait(smem_addr(&a_empty[st]), (u - 1u) & 1u)) {
+                    *failed = 1;
+                    break;
+                }
+                mbar_expect_tx(&a_full[st], nslices * TILE_BYTES);
+                for (uint32_t sl = 0; sl < nslices; ++sl)
+                    tma_load_box(&maps.a, slots + st * AUX_BYTES + sl * TILE_BYTES, sl * BK, (blockIdx.x + t * gridDim.x) * BM,
+                                 &a_full[st]);
+            }
+        } else if (lane == 0 && warp == 1) {
+            bool ok = mbar_wait(smem_addr(&w_full), 0u);
+            for (uint32_t t = 0; t < mine && ok; ++t) {
+                const uint32_t b = t & 1u, st = t % MLP_SLOTS;
+                ok = !*failed && (t < 2 || mbar_wait(smem_addr(&acc1_empty[b]), ((t >> 1) - 1u) & 1u)) &&
+                     mbar_wait(smem_addr(&a_full[st]), (t / MLP_SLOTS) & 1u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                mma_tile(tmem + b * (uint32_t)BN, smem_addr(slots) + st * AUX_BYTES, w1, nslices, &acc1_full[b]);
+            }
+            if (!ok) *failed = 1;
+        } else if (lane == 0 && warp == 2) {
+            bool ok = mbar_wait(smem_addr(&w_full), 0u);
+            for (uint32_t t = 0; t < mine && ok; ++t) {
+                const uint32_t b = t & 1u;
+                ok = !*failed && (t < 2 || mbar_wait(smem_addr(&acc2_empty[b]), ((t >> 1) - 1u) & 1u)) &&
+                     mbar_wait(smem_addr(&z_full[b]), (t >> 1) & 1u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                mma_tile(tmem + (2u + b) * (uint32_t)BN, z + b * AUX_BYTES, w2, 2u, &acc2_full[b]);
+            }
+            if (!ok) *failed = 1;
+        }
+        __syncwarp();
+    } else if (warp < 8u) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (MP) {
+            // Q's rows, two per instruction (16 lanes of 16 bytes each); rows past the matrix are zero-filled
+            const uint32_t r0 = 32u * (warp - 4u), chunk = lane & 15u;
+            auto index = [&](uint32_t t) {
+                const uint32_t row = (blockIdx.x + t * gridDim.x) * BM + r0 + lane;
+                return t < mine && row < g.m ? __ldg(g.add2_idx + row) : 0u;
+            };
+            uint32_t next = index(0);
+            for (uint32_t t = 0; t < mine; ++t) {
+                const uint32_t b = t & 1u, row0 = (blockIdx.x + t * gridDim.x) * BM + r0, at = next;
+                next = index(t + 1u);
+                // the stage's hidden rows of two tiles ago have been read
+                bool ok = !*failed && (t < 2 || mbar_wait(smem_addr(&acc2_full[b]), ((t >> 1) - 1u) & 1u));
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) {
+                    if (lane == 0) *failed = 1;
+                    break;
+                }
+                const uint32_t dst = z + b * AUX_BYTES + (chunk >> 3) * HALF_BYTES;
+#pragma unroll 8
+                for (uint32_t q = 0; q < 16u; ++q) {
+                    const uint32_t rr = 2u * q + (lane >> 4);
+                    const uint32_t k = __shfl_sync(0xffffffffu, at, (int)rr);
+                    const uint32_t bytes = row0 + rr < g.m ? 16u : 0u;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + sw128(r0 + rr, chunk & 7u)),
+                                 "l"(g.add2 + (size_t)k * 128u + 8u * chunk), "r"(bytes)
+                                 : "memory");
+                }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&q_full[b])) : "memory");
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        }
+    } else if (warp < 16u) {
+        const uint32_t quarter = warp & 3u, half = (warp - 8u) / 4u, col0 = 64u * half, r = 32u * quarter + lane;
+        auto index = [&](uint32_t t) {
+            const uint32_t row = (blockIdx.x + t * gridDim.x) * BM + r;
+            return MP && t < mine && row < g.m ? __ldg(g.add1_idx + row) : 0u;
+        };
+        uint32_t next = index(0);
+        for (uint32_t t = 0; t < mine; ++t) {
+            const uint32_t b = t & 1u;
+            const uint4* p_row = reinterpret_cast<const uint4*>(g.add1 + (size_t)next * 128u + col0);
+            uint4 p[4];
+            if (MP) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) p[c] = __ldg(p_row + c);
+            }
+            next = index(t + 1u);
+            bool ok = !*failed && mbar_wait(smem_addr(&acc1_full[b]), (t >> 1) & 1u);
+            if (MP) ok = ok && mbar_wait(smem_addr(&q_full[b]), (t >> 1) & 1u);
+            else if (t >= 2) ok = ok && mbar_wait(smem_addr(&acc2_full[b]), ((t >> 1) - 1u) & 1u);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+                if (lane == 0) *failed = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (uint32_t q = 0; q < 2; ++q) {
+                uint32_t v[32];
+                tmem_ld32(tmem + ((32u * quarter) << 16) + b * (uint32_t)BN + col0 + 32u * q, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (uint32_t c = 0; c < 4; ++c) {
+                    float y[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) y[k] = __uint_as_float(v[8 * c + k]);
+                    if (g.b1) {
+#pragma unroll
+                        for (int k = 0; k < 8; k += 4) {
+                            const float4 bb = __ldg(reinterpret_cast<const float4*>(g.b1 + col0 + 32u * q + 8u * c + k));
+                            y[k] += bb.x;
+                            y[k + 1] += bb.y;
+                            y[k + 2] += bb.z;
+                            y[k + 3] += bb.w;
+                        }
+                    }
+                    const uint32_t at = z + b * AUX_BYTES + half * HALF_BYTES + sw128(r, 4u * q + c);
+                    if (MP) {
+                        add8(y, p[c]);
+                        if (q == 0) p[c] = __ldg(p_row + 4 + c);
+                        add8(y, lds128(at));
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) y[k] = fmaxf(y[k], 0.f);
+                    sts128(at, make_uint4(pack2(y[0], y[1]), pack2(y[2], y[3]), pack2(y[4], y[5]), pack2(y[6], y[7])));
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&acc1_empty[b]);
+                mbar_arrive(&z_full[b]);
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+        const uint32_t quarter = warp & 3u, half = (warp - 16u) / 4u, col0 = 64u * half, r = 32u * quarter + lane;
+        for (uint32_t t = 0; t < mine; ++t) {
+            const uint32_t b = t & 1u, st = t % MLP_SLOTS;
+            bool ok = !*failed && mbar_wait(smem_addr(&acc2_full[b]), (t >> 1) & 1u) &&
+                      mbar_wait(smem_addr(&a_full[st]), (t / MLP_SLOTS) & 1u);
+            ok = __all_sync(0xffffffffu, ok);
+            if (lane == 0 && t) {  // the previous tile has left its slot
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                mbar_arrive(&a_empty[(t - 1u) % MLP_SLOTS]);
+            }
+            __syncwarp();
+            float x[64];
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint32_t v[32];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    tmem_ld32(tmem + ((32u * quarter) << 16) + (2u + b) * (uint32_t)BN + col0 + 32u * q, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) x[32 * q + j] = __uint_as_float(v[j]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc2_empty[b]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 64; ++j) x[j] = 0.f;
+            }
+            if (g.b2) {
+#pragma unroll
+                for (int j = 0; j < 64; j += 4) {
+                    const float4 bb = __ldg(reinterpret_cast<const float4*>(g.b2 + col0 + j));
+                    x[j] += bb.x;
+                    x[j + 1] += bb.y;
+                    x[j + 2] += bb.z;
+                    x[j + 3] += bb.w;
+                }
+            }
+            float rstd;
+            if (!ln_centre(x, ok, s_lnx, s_lnv, s_lnok, failed, quarter, half, lane, &rstd)) break;
+            const uint32_t out = smem_addr(slots) + st * AUX_BYTES + half * HALF_BYTES;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                float o[8];
+                ln_scale<true>(g.gamma + col0 + 8 * c, g.beta + col0 + 8 * c, x + 8 * c, rstd, o);
+                const uint32_t at = out + sw128(r, (uint32_t)c);
+                if (MP) add8(o, lds128(at));
+                sts128(at, make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7])));
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                const uint32_t row0 = (blockIdx.x + t * gridDim.x) * BM + 32u * quarter;
+                if (row0 < g.m) tma_store_box(&maps.c, out + 32u * quarter * 128u, col0, row0, false);
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            __syncwarp();
+        }
+        // the stores have left shared memory before the CTA gives it up
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        __syncwarp();
+    }
+    __syncthreads();
+    if (*failed && threadIdx.x == 0 && err) atomicOr(err, DEVERR_MMA_TIMEOUT);
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(MLP_TMEM_COLS));
+    }
+}
+
 // ---- weight gradients: C = X^T dY, both operands read along their rows ---------------------------
 //
 // A transposed and B row-major (m, n <= 128; X [k x m], dY [k x n]): a slice of 64 rows of either is
@@ -1411,6 +1729,16 @@ bool encode_operand(CUtensorMap* map, const void* base, uint64_t inner, uint64_t
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+int sm_count() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 1;
+    }();
+    return sms;
+}
+
 bool gemm_tma_available() { return encode_tiled() != nullptr; }
 
 namespace {
@@ -1475,7 +1803,37 @@ wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream
                : launch_tma_as<AUX_NONE, false, false, true>(g, maps, plan, grid, err, s);
 }
 
+template <bool MP>
+wc_status launch_mlp_as(const MlpArgs& g, const MlpMaps& maps, uint32_t* err, cudaStream_t s, bool* launched) {
+    // the roles' register shares assume MLP_REGS per thread at launch
+    static const bool usable = [] {
+        cudaFuncAttributes a{};
+        return cudaFuncGetAttributes(&a, gemm_mlp_kernel<MP>) == cudaSuccess && a.numRegs == MLP_REGS &&
+               cudaFuncSetAttribute(gemm_mlp_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem(2u)) ==
+                   cudaSuccess;
+    }();
+    if (!usable) return WC_OK;
+    const uint32_t tiles = (g.m + BM - 1) / BM, sms = (uint32_t)sm_count();
+    gemm_mlp_kernel<MP><<<std::min(tiles, sms), MLP_THREADS, mlp_smem((g.k + BK - 1) / BK), s>>>(g, maps, err);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(WC_ERR_CUDA, "mlp launch: %s", cudaGetErrorString(e));
+    *launched = true;
+    return WC_OK;
+}
+
 }  // namespace
+
+wc_status launch_mlp(const MlpArgs& g, uint32_t* err, cudaStream_t s, bool* launched) {
+    *launched = false;
+    const auto at16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16u == 0; };
+    MlpMaps maps;
+    if (!g.m || g.k % 8u || g.k == 0 || g.k > 128u || (g.add1 && g.k != 128u) || !at16(g.b1) || !at16(g.b2) || !at16(g.gamma) ||
+        !at16(g.beta) || !at16(g.add1) || !at16(g.add2) || !encode_operand(&maps.a, g.a, g.k, g.m, 2ull * g.k) ||
+        !encode_operand(&maps.w1, g.w1, g.k, 128, 2ull * g.k) || !encode_operand(&maps.w2, g.w2, 128, 128, 256) ||
+        !encode_operand(&maps.c, g.out, 128, g.m, 256, 32))
+        return WC_OK;
+    return g.add1 ? launch_mlp_as<true>(g, maps, err, s, launched) : launch_mlp_as<false>(g, maps, err, s, launched);
+}
 
 wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s) {
     const wc_status st = check_gemm(g);
@@ -1483,17 +1841,14 @@ wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s) {
     if (!g.a_transposed && !g.b_rowmajor && g.k_chunk >= g.k) {
         // row-major operands, no split of K: the persistent pipelined kernel, one CTA per SM;
         // B resident in shared memory when it is one column of tiles of at most RB_MAX_SLICES
-        static int sms = 0;
-        if (!sms) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (sms <= 0) sms = 1;
+        static std::once_flag pipe_once;
+        const int sms = sm_count();
+        std::call_once(pipe_once, [] {
             cudaFuncSetAttribute(gemm_pipe_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)pipe_smem_bytes(false, 0));
             cudaFuncSetAttribute(gemm_pipe_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)pipe_smem_bytes(true, RB_MAX_SLICES * BK));
-        }
+        });
         const uint32_t tiles = ((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
         const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
         const bool rb = g.n <= (uint32_t)BN && (g.k + BK - 1) / BK <= RB_MAX_SLICES;

@@ -539,15 +539,45 @@ wc_status layer_ln(wc_surrogate* s, bool keep, const Lin& l, uint32_t rows, cons
     return WC_OK;
 }
 
+// Two layers (hidden rows z) and their LayerNorm; with add, P's rows by receiver and Q's by sender in the first and
+// the residual a. Nothing kept: one kernel, which leaves z unwritten.
+wc_status mlp_ln(wc_surrogate* s, bool keep, const Lin& l1, const Lin& l2, const LNp& ln, uint32_t rows, const __nv_bfloat16* a,
+                 bool add, __nv_bfloat16* z, __nv_bfloat16* out, float* y, float* stats) {
+    const Work& w = s->work;
+    if (!keep) {
+        MlpArgs m{};
+        m.m = rows;
+        m.k = l1.kin;
+        m.a = a;
+        m.w1 = s->wb + l1.wt;
+        m.w2 = s->wb + l2.wt;
+        m.b1 = l1.b != NONE ? s->w + l1.b : nullptr;
+        m.b2 = l2.b != NONE ? s->w + l2.b : nullptr;
+        m.gamma = s->w + ln.g;
+        m.beta = s->w + ln.g + W;
+        if (add) {
+            m.add1 = w.P;
+            m.add1_idx = w.recv;
+            m.add2 = w.Q;
+            m.add2_idx = w.col;
+        }
+        m.out = out;
+        bool launched = false;
+        WC_TRY(launch_mlp(m, s->d_err, s->stream, &launched));
+        if (launched) return WC_OK;
+    }
+    if (add) WC_TRY(fwd(s, l1, rows, a, nullptr, true, nullptr, z, w.P, w.recv, w.Q, w.col));
+    else WC_TRY(fwd(s, l1, rows, a, nullptr, true, nullptr, z));
+    return layer_ln(s, keep, l2, rows, z, ln, add ? a : nullptr, out, y, stats);
+}
+
 // keep: the activations and LayerNorm statistics the backward pass reads (training).
 wc_status forward(wc_surrogate* s, bool keep) {
     if (s->cast_dirty) cast_all(s);
     Work& w = s->work;
     const uint32_t n = s->n, e = s->e;
-    WC_TRY(fwd(s, s->ne1, n, w.xn, nullptr, true, nullptr, w.zn0));
-    WC_TRY(layer_ln(s, keep, s->ne2, n, w.zn0, s->lnn0, nullptr, hbuf(w, 0), w.yn0, w.stn0));
-    WC_TRY(fwd(s, s->ee1, e, w.xe, nullptr, true, nullptr, w.ze0));
-    WC_TRY(layer_ln(s, keep, s->ee2, e, w.ze0, s->lne0, nullptr, ebuf(w, 0), w.ye0, w.ste0));
+    WC_TRY(mlp_ln(s, keep, s->ne1, s->ne2, s->lnn0, n, w.xn, false, w.zn0, hbuf(w, 0), w.yn0, w.stn0));
+    WC_TRY(mlp_ln(s, keep, s->ee1, s->ee2, s->lne0, e, w.xe, false, w.ze0, ebuf(w, 0), w.ye0, w.ste0));
     const size_t pn = (size_t)w.cap_n * W, pe = (size_t)w.cap_e * W;
     for (uint32_t l = 0; l < s->L; ++l) {
         const MPLayer& L = s->layers[l];
@@ -557,8 +587,8 @@ wc_status forward(wc_surrogate* s, bool keep) {
         __nv_bfloat16* zn = lbuf(w, w.zn, l, pn);
         WC_TRY(fwd(s, L.e1i, n, h, nullptr, false, nullptr, w.P));
         WC_TRY(fwd(s, L.e1s, n, h, nullptr, false, nullptr, w.Q));
-        WC_TRY(fwd(s, L.e1e, e, el, nullptr, true, nullptr, ze, w.P, w.recv, w.Q, w.col));
-        WC_TRY(layer_ln(s, keep, L.e2, e, ze, L.lne, el, e1, lbuf(w, w.ye, l, pe), lbuf(w, w.ste, l, 2 * (size_t)w.cap_e)));
+        WC_TRY(mlp_ln(s, keep, L.e1e, L.e2, L.lne, e, el, true, ze, e1, lbuf(w, w.ye, l, pe),
+                      lbuf(w, w.ste, l, 2 * (size_t)w.cap_e)));
         segment_sum_bf16(n, w.rowptr, nullptr, e1, nullptr, agg, s->stream);
         WC_TRY(fwd(s, L.n1, n, h, agg, true, nullptr, zn));
         WC_TRY(layer_ln(s, keep, L.n2, n, zn, L.lnn, h, h1, lbuf(w, w.yn, l, pn), lbuf(w, w.stn, l, 2 * (size_t)w.cap_n)));
