@@ -741,14 +741,14 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
     const __nv_bfloat162 q = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&q);
 }
-// x[0..8) += the eight BF16 of v
+// x[0..8) += the eight BF16 of v, one instruction each (BF16 widens exactly)
 __device__ __forceinline__ void add8(float* x, const uint4& v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        x[2 * k] += __uint_as_float(w[k] << 16);
-        x[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u);
-    }
+    for (int k = 0; k < 4; ++k)
+        asm("{\n .reg .b16 lo, hi;\n mov.b32 {lo, hi}, %2;\n add.rn.f32.bf16 %0, lo, %0;\n add.rn.f32.bf16 %1, hi, %1;\n}\n"
+            : "+f"(x[2 * k]), "+f"(x[2 * k + 1])
+            : "r"(w[k]));
 }
 
 // Shared memory of the TMA kernel: [B^T slices][A ring][two aux / BF16 output stages][FP32 output].
@@ -767,9 +767,23 @@ __device__ __forceinline__ void pair_sync(uint32_t quarter) {
     asm volatile("bar.sync %0, 64;" ::"r"(1u + quarter) : "memory");
 }
 
-// The LayerNorm of n = 128 columns by the two warps of a pair: x holds a thread's 64 columns (from col0) of its
-// row and becomes gamma (x - mean) rstd + beta, xs/xv/oks as in tma_epilogue. False when a wait of either warp
-// failed (both leave).
+// The packed FP32 instructions on (a[0], a[1]), each half rounded as the scalar ones.
+__device__ __forceinline__ void add_pair(float* a, float b0, float b1) {
+    asm("{\n .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n add.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}\n"
+        : "+f"(a[0]), "+f"(a[1])
+        : "f"(b0), "f"(b1));
+}
+// a = a m g + b
+__device__ __forceinline__ void scale_pair(float* a, float m, float g0, float g1, float b0, float b1) {
+    asm("{\n .reg .b64 a, m, g, b;\n mov.b64 a, {%0, %1};\n mov.b64 m, {%2, %2};\n mov.b64 g, {%3, %4};\n mov.b64 b, {%5, %6};\n"
+        " mul.rn.f32x2 a, a, m;\n fma.rn.f32x2 a, a, g, b;\n mov.b64 {%0, %1}, a;\n}\n"
+        : "+f"(a[0]), "+f"(a[1])
+        : "f"(m), "f"(g0), "f"(g1), "f"(b0), "f"(b1));
+}
+
+// The LayerNorm of n = 128 columns. ln_centre: by the two warps of a pair, x a thread's 64 columns of its row, which
+// becomes x - mean (xs, xv, oks as in tma_epilogue); false when a wait of either warp failed (both leave). ln_scale:
+// eight columns o = gamma x rstd + beta.
 template <bool VEC>
 __device__ __forceinline__ void ln_scale(const float* gamma, const float* beta, const float* x, float rstd, float* o) {
     float gm[8], bt[8];
@@ -807,9 +821,10 @@ __device__ __forceinline__ bool ln_centre(float (&x)[64], bool ok, float (*xs)[2
     const float mean = (xs[quarter][0][lane] + xs[quarter][1][lane]) * (1.f / 128.f);
     float sq = 0.f;
 #pragma unroll
-    for (int j = 0; j < 64; ++j) {
-        x[j] -= mean;
+    for (int j = 0; j < 64; j += 2) {
+        add_pair(x + j, -mean, -mean);
         sq += x[j] * x[j];
+        sq += x[j + 1] * x[j + 1];
     }
     xv[quarter][half][lane] = sq;
     pair_sync(quarter);
@@ -1248,8 +1263,10 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
 // read straight into registers: edges are sorted by receiver, so the 32 rows of a warp share one or two of P's,
 // which L1 serves (any index is correct). Registers are moved from the copying warps to the normalising ones.
 // The arithmetic and its order are those of the two launches (the same results bit for bit).
-// 1.85 M edges: 312 us against 240 + 250 in two launches (345 us when one group of eight warps ran both epilogues
-// and both gathered rows were copied); bound by the epilogues' instructions (55 % of the issue slots) and L1 (72 %).
+// 1.85 M edges: 262 us against 240 + 250 in two launches. Bound by L1 (86 %), most of it the loads of bias, gamma and
+// beta, which every warp needs for every tile. Slower: both epilogues in one group of eight warps with both gathered
+// rows copied, 345 us; FP32 arithmetic in scalar instructions, 312; the constants as kernel parameters (constant
+// cache misses), 352; the second layer's columns spread over the lanes so that a thread needs fewer of them, 286.
 constexpr uint32_t MLP_SLOTS = 3;
 constexpr int MLP_THREADS = 24 * 32;
 constexpr uint32_t MLP_TMEM_COLS = 512;
@@ -1261,6 +1278,17 @@ constexpr uint32_t mlp_smem(uint32_t nslices) { return (nslices + 2u) * TILE_BYT
 struct MlpMaps {
     CUtensorMap a, w1, w2, c;
 };
+
+// Eight consecutive values.
+__device__ __forceinline__ void load8(float* o, const float* p) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w, o[4] = b.x, o[5] = b.y, o[6] = b.z, o[7] = b.w;
+}
+// max(x, 0) of two BF16 (a NaN gives 0, as fmaxf before the rounding does)
+__device__ __forceinline__ uint32_t relu2(uint32_t w) {
+    const __nv_bfloat162 h = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&w), __floats2bfloat162_rn(0.f, 0.f));
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
 
 // The MMAs of one 128 x 128 tile over nslices slices of 64 (operands TILE_BYTES apart), committed to `done`.
 __device__ __forceinline__ void mma_tile(uint32_t acc_addr, uint32_t a, uint32_t b, uint32_t nslices, uint64_t* done) {
@@ -1436,14 +1464,10 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
                     for (int k = 0; k < 8; ++k) y[k] = __uint_as_float(v[8 * c + k]);
                     if (g.b1) {
+                        float bb[8];
+                        load8(bb, g.b1 + col0 + 32u * q + 8u * c);
 #pragma unroll
-                        for (int k = 0; k < 8; k += 4) {
-                            const float4 bb = __ldg(reinterpret_cast<const float4*>(g.b1 + col0 + 32u * q + 8u * c + k));
-                            y[k] += bb.x;
-                            y[k + 1] += bb.y;
-                            y[k + 2] += bb.z;
-                            y[k + 3] += bb.w;
-                        }
+                        for (int k = 0; k < 8; k += 2) add_pair(y + k, bb[k], bb[k + 1]);
                     }
                     const uint32_t at = z + b * AUX_BYTES + half * HALF_BYTES + sw128(r, 4u * q + c);
                     if (MP) {
@@ -1451,9 +1475,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
                         if (q == 0) p[c] = __ldg(p_row + 4 + c);
                         add8(y, lds128(at));
                     }
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) y[k] = fmaxf(y[k], 0.f);
-                    sts128(at, make_uint4(pack2(y[0], y[1]), pack2(y[2], y[3]), pack2(y[4], y[5]), pack2(y[6], y[7])));
+                    sts128(at, make_uint4(relu2(pack2(y[0], y[1])), relu2(pack2(y[2], y[3])), relu2(pack2(y[4], y[5])), relu2(pack2(y[6], y[7]))));
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1497,12 +1519,11 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
             }
             if (g.b2) {
 #pragma unroll
-                for (int j = 0; j < 64; j += 4) {
-                    const float4 bb = __ldg(reinterpret_cast<const float4*>(g.b2 + col0 + j));
-                    x[j] += bb.x;
-                    x[j + 1] += bb.y;
-                    x[j + 2] += bb.z;
-                    x[j + 3] += bb.w;
+                for (int j = 0; j < 64; j += 8) {
+                    float bb[8];
+                    load8(bb, g.b2 + col0 + j);
+#pragma unroll
+                    for (int k = 0; k < 8; k += 2) add_pair(x + j + k, bb[k], bb[k + 1]);
                 }
             }
             float rstd;
@@ -1511,7 +1532,14 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 float o[8];
-                ln_scale<true>(g.gamma + col0 + 8 * c, g.beta + col0 + 8 * c, x + 8 * c, rstd, o);
+                float gm[8], bt[8];
+                load8(gm, g.gamma + col0 + 8 * c);
+                load8(bt, g.beta + col0 + 8 * c);
+#pragma unroll
+                for (int k = 0; k < 8; k += 2) {
+                    o[k] = x[8 * c + k], o[k + 1] = x[8 * c + k + 1];
+                    scale_pair(o + k, rstd, gm[k], gm[k + 1], bt[k], bt[k + 1]);
+                }
                 const uint32_t at = out + sw128(r, (uint32_t)c);
                 if (MP) add8(o, lds128(at));
                 sts128(at, make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7])));
