@@ -140,9 +140,10 @@ __device__ __forceinline__ void store_tile(uint32_t* s, const uint32_t (&v)[SCAN
     }
 }
 
-// second: LANE ? the padded starts (+ total) : the list of non-empty cells.
+// second: LANE ? the padded starts (+ total) : the list of non-empty cells. Five blocks per SM: a batch of 23.8 M cells
+// waits at the blocks' barriers with three (72 registers), its step takes 3,305 us against 3,284; one scene's is the same.
 template <bool LANE>
-__global__ void __launch_bounds__(SCAN_THREADS) scan_cells_kernel(uint32_t* __restrict__ counts, uint32_t C,
+__global__ void __launch_bounds__(SCAN_THREADS, 5) scan_cells_kernel(uint32_t* __restrict__ counts, uint32_t C,
                                                                   uint32_t* __restrict__ start,
                                                                   uint32_t* __restrict__ second,
                                                                   uint32_t* __restrict__ num_nonempty,
