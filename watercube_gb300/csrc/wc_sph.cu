@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
         float judge = 0.f;  // FEAT with judge_part: this lane's |rho_carried / rho - 1|
         do {
             uint32_t ti[TARGETS];  // sorted slots (>= n: none)
-            if (TARGETS == 2) {
+            if constexpr (TARGETS == 2) {
                 const uint32_t p0 = (m << 6) + 2u * lane;
                 if (p0 >= padded) break;
                 const uint2 c2 = __ldg(reinterpret_cast<const uint2*>(cidx + p0));

@@ -463,7 +463,7 @@ WC_API wc_status wc_surface_extract(wc_surface* s, wc_fluid* f, uint64_t* num_tr
     const float radius = s->p.radius > 0.f ? s->p.radius : sc.h;
     if (radius > sc.bin) return fail(WC_ERR_INVALID_ARG, "field radius %g exceeds the cell edge %g", radius, sc.bin);
     const uint32_t G = s->G, C = G - 1;
-    const uint64_t V = (uint64_t)G * G * G, cubes = (uint64_t)C * C * C;
+    const uint64_t cubes = (uint64_t)C * C * C;
     Grid g{G, sc.size / (float)(G - 1)};
     s->spacing = g.spacing;
     s->iso = s->p.iso;
