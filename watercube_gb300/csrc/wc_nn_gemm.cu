@@ -756,6 +756,7 @@ struct TmaPlan {
     uint32_t stages;     // A ring slots
     uint32_t aux_bytes;  // per stage: operands of 32 KB (AUX_GATHER with two: 64 KB), 0 without BF16 output or aux
     uint32_t f32_bytes;
+    uint32_t one_stage;  // BF16 output, no aux rows: one stage instead of two
     uint32_t smem;
 };
 
@@ -867,13 +868,13 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
             if (lane == 0) *failed = 1;
             break;
         }
-        const uint32_t stage = aux_base + b * plan.aux_bytes + half * HALF_BYTES;
+        const uint32_t stage = aux_base + (AUX == AUX_NONE && plan.one_stage ? 0u : b) * plan.aux_bytes + half * HALF_BYTES;
         const uint32_t row0 = tile * BM + 32u * quarter;
         // The staging this warp is about to write has been read by its earlier stores: two tiles ago
         // (BF16, two stages), the previous tile's (FP32, one). With aux rows the previous tile's
         // stage, read by then, goes back to the producer, who fills it during this tile.
         if (lane == 0) {
-            if (F32 || (AUX != AUX_NONE && BF)) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            if (F32 || (AUX != AUX_NONE && BF) || plan.one_stage) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
             if (AUX != AUX_NONE && BF && t > 0) mbar_arrive(&aux_empty[b ^ 1u]);
         }
@@ -966,7 +967,7 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
                 g.ln_mean[row0 + lane] = mean;
                 g.ln_rstd[row0 + lane] = rstd;
             }
-            const uint32_t rows = aux_base + b * plan.aux_bytes;
+                const uint32_t rows = aux_base + (AUX == AUX_NONE && plan.one_stage ? 0u : b) * plan.aux_bytes;
 #pragma unroll
             for (uint32_t j = 0; j < 16; ++j) {
                 const float* y = x + 4 * j;
@@ -1095,7 +1096,7 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
     const uint32_t stages = plan.stages;
     unsigned char* const ring = smem_raw + nslices * TILE_BYTES;
     const uint32_t aux_base = smem_addr(ring) + stages * TILE_BYTES;
-    const uint32_t f32_base = aux_base + 2u * plan.aux_bytes;
+    const uint32_t f32_base = aux_base + (plan.one_stage ? 1u : 2u) * plan.aux_bytes;
 
     if (threadIdx.x == 0) {
         for (uint32_t q = 0; q < stages; ++q) {
@@ -1263,7 +1264,7 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
 // read straight into registers: edges are sorted by receiver, so the 32 rows of a warp share one or two of P's,
 // which L1 serves (any index is correct). Registers are moved from the copying warps to the normalising ones.
 // The arithmetic and its order are those of the two launches (the same results bit for bit).
-// 1.85 M edges: 262 us against 240 + 250 in two launches. Bound by L1 (86 %), most of it the loads of bias, gamma and
+// 1.85 M edges: 262 us against 203 + 231 in two launches. Bound by L1 (86 %), most of it the loads of bias, gamma and
 // beta, which every warp needs for every tile. Slower: both epilogues in one group of eight warps with both gathered
 // rows copied, 345 us; FP32 arithmetic in scalar instructions, 312; the constants as kernel parameters (constant
 // cache misses), 352; the second layer's columns spread over the lanes so that a thread needs fewer of them, 286.
@@ -1810,7 +1811,11 @@ wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream
     TmaPlan plan{};
     plan.aux_bytes = (g.add1 && g.add2) ? 2u * AUX_BYTES : (aux || bf) ? AUX_BYTES : 0u;
     plan.f32_bytes = f32 ? F32_OUT_BYTES : 0u;
-    const uint32_t fixed = nslices * TILE_BYTES + 2u * plan.aux_bytes + plan.f32_bytes;
+    // a second output stage only where it leaves the whole ring: at k = 384 it takes two of six slots (460,000 rows 81
+    // us against 74, 82 before the output went through shared memory); up to k = 256 both fit
+    plan.one_stage = !aux && bf &&
+                     nslices * TILE_BYTES + 2u * plan.aux_bytes + plan.f32_bytes + TMA_MAX_STAGES * TILE_BYTES > TMA_SMEM_LIMIT;
+    const uint32_t fixed = nslices * TILE_BYTES + (plan.one_stage ? 1u : 2u) * plan.aux_bytes + plan.f32_bytes;
     if (fixed + 2u * TILE_BYTES > TMA_SMEM_LIMIT) return WC_OK;
     plan.stages = std::min<uint32_t>(TMA_MAX_STAGES, (TMA_SMEM_LIMIT - fixed) / TILE_BYTES);
     plan.smem = fixed + plan.stages * TILE_BYTES;
