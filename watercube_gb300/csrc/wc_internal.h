@@ -147,7 +147,7 @@ constexpr uint32_t SCAN_SPIN_LIMIT = 1u << 22;  // ~0.3-1 s of polling before gi
 constexpr int SPH_THREADS = 256;
 // Candidates a warp stages in shared memory per cell in the density pass (padding included).
 constexpr int STAGE_CAP = 320;
-// 32-bit words of neighbour bit strings per particle (density pass -> force pass): room for 4,096
+// 32-bit words of neighbour bits per particle (density pass -> force pass): for the team passes room for 4,096
 // candidates, the 27-cell neighbourhoods of the 1M dam break's most compressed states (99th
 // percentile 3,731 at step 1,750); a target with more tests its candidates again in the force pass.
 constexpr int MASK_WORDS = 128;
@@ -195,7 +195,7 @@ struct DevBuffers {
     unsigned long long* scan_desc;  // [num_tiles]
     uint32_t* scan_tile_counter;
     uint32_t* ncount;  // [n] or null
-    uint32_t* hits;    // [n * MASK_WORDS] neighbour bit strings
+    uint32_t* hits;    // [n * MASK_WORDS] neighbours: bit strings (team passes) or entries (lane passes)
     // The lane passes' padded slots (see padded_capacity), written by the lane variant's scan and
     // gather: pstart is the exclusive prefix of the cells' counts rounded up to 4 (+ total), xyz the
     // sorted positions' x, y, z as three arrays of pcap elements, cidx the sorted slot of a padded
@@ -216,8 +216,7 @@ struct DevBuffers {
 // Neighbour pass variants (threads per cell): a 32-lane team per non-empty cell that splits the
 // cell's targets into (targets x slices) and stages candidates in shared memory (PASSES_TEAM), or
 // one lane per target walking its cell's 9 candidate rows (PASSES_LANE). The density pass of a
-// variant writes its neighbour bit strings in the layout the force pass of the same variant
-// reads; both variants select the same neighbour sets, their sums differ only in the order of
+// variant writes its neighbours in the layout the force pass of the same variant reads; both variants select the same neighbour sets, their sums differ only in the order of
 // the additions.
 enum : int { PASSES_TEAM = 0, PASSES_LANE = 1 };
 
