@@ -301,8 +301,10 @@ wc_status ensure_part(wc_surrogate* s, size_t count) {
 wc_status wgrad(wc_surrogate* s, const Lin& l, uint32_t rows, const __nv_bfloat16* x, uint32_t kcount, uint32_t k0,
                 const __nv_bfloat16* dy) {
     if (!rows) return WC_OK;
-    // one split per resident CTA (two on each of the 152 SMs), of two slices of 64 rows at least
-    const uint32_t chunk = std::max(128u, ((rows + 303u) / 304u + 63u) / 64u * 64u);
+    // One split per SM, of three slices of 64 rows at least: the partial sums are 64 KB per split, written and read
+    // again. Training passes over 16,384 / 2,048 particles: 8,330 / 3,400 us; 304 splits (two per SM) of two slices
+    // 8,445 / 3,430, 110 splits 8,375, 76 8,490.
+    const uint32_t chunk = std::max(192u, ((rows + 151u) / 152u + 63u) / 64u * 64u);
     const uint32_t splits = (rows + chunk - 1) / chunk;
     const size_t tile = (size_t)kcount * l.nout;
     WC_TRY(ensure_part(s, splits * tile));
@@ -434,9 +436,9 @@ wc_status ensure_work(wc_surrogate* s, uint32_t n, uint32_t e, bool saved) {
         WC_TRY(dalloc(&w.dPb, (size_t)cn * W));
         WC_TRY(dalloc(&w.dQb, (size_t)cn * W));
     }
-    // split-K partials of the weight gradients (<= 304 splits of a 128 x 128 tile), column-sum
+    // split-K partials of the weight gradients (<= 152 splits of a 128 x 128 tile), column-sum
     // and LayerNorm-backward partials
-    size_t need = std::max<size_t>(part_cap, 304u * (size_t)W * W);
+    size_t need = std::max<size_t>(part_cap, 152u * (size_t)W * W);
     need = std::max<size_t>(need, (size_t)layernorm_backward_blocks(ce) * 384);
     need = std::max<size_t>(need, (size_t)colsum_blocks(ce) * W);
     WC_TRY(ensure_part(s, need));
