@@ -110,6 +110,13 @@ void adam(size_t count, float* w, const float* g, float* m, float* v, float lr, 
           int step, float grad_scale, cudaStream_t s);
 void cast_weight(const float* w, uint32_t k_in, uint32_t n_out, uint32_t k_pad, uint32_t n_pad, __nv_bfloat16* wt,
                  __nv_bfloat16* wk, cudaStream_t s);
+// The same for `count` layers without padding in one launch: layer i's W (k_in x n_out) at w + l[i].w, its BF16 forms at
+// wb + l[i].wt and wb + l[i].wk; max_elements: the largest k_in n_out.
+struct CastLayer {
+    size_t w, wt, wk;
+    uint32_t k_in, n_out;
+};
+void cast_weights(const CastLayer* l, uint32_t count, uint32_t max_elements, const float* w, __nv_bfloat16* wb, cudaStream_t s);
 void gather4(uint32_t n, const uint32_t* perm, const float4* src, float4* dst, cudaStream_t s);
 void predictions(uint32_t n, const float* pred, uint32_t ldp, float scale, const float4* base, const uint32_t* perm,
                  float4* out, cudaStream_t s);

@@ -125,6 +125,8 @@ struct wc_surrogate {
     __nv_bfloat16* wb = nullptr;
     int adam_step = 0;
     bool cast_dirty = true;
+    CastLayer* cast_layers = nullptr;  // every layer's, on the device
+    uint32_t cast_count = 0, cast_max = 0;
     Work work;
     cudaStream_t stream = nullptr;
     uint32_t* d_err = nullptr;
@@ -205,7 +207,7 @@ void init_params(wc_surrogate* s, std::vector<float>& host) {
 }
 
 void cast_all(wc_surrogate* s) {
-    for_each_lin(s, [&](Lin& l) { cast_weight(s->w + l.w, l.kin, l.nout, l.kin, l.nout, s->wb + l.wt, s->wb + l.wk, s->stream); });
+    cast_weights(s->cast_layers, s->cast_count, s->cast_max, s->w, s->wb, s->stream);
     s->cast_dirty = false;
 }
 
@@ -1000,6 +1002,13 @@ WC_API wc_status wc_surrogate_create(const wc_surrogate_config* c, wc_surrogate*
     if (st == WC_OK) st = dalloc(&s->m, s->nparams);
     if (st == WC_OK) st = dalloc(&s->v, s->nparams);
     if (st == WC_OK) st = dalloc(&s->wb, s->nbf16);
+    std::vector<CastLayer> casts;
+    for_each_lin(s, [&](Lin& l) {
+        casts.push_back(CastLayer{l.w, l.wt, l.wk, l.kin, l.nout});
+        s->cast_max = std::max(s->cast_max, l.kin * l.nout);
+    });
+    s->cast_count = (uint32_t)casts.size();
+    if (st == WC_OK) st = dalloc(&s->cast_layers, casts.size());
     if (st == WC_OK) st = dalloc(&s->d_err, 1);
     if (st == WC_OK && cudaMallocHost(reinterpret_cast<void**>(&s->h_err), sizeof(uint32_t)) != cudaSuccess)
         st = fail(WC_ERR_OOM, "pinned allocation failed");
@@ -1007,6 +1016,7 @@ WC_API wc_status wc_surrogate_create(const wc_surrogate_config* c, wc_surrogate*
         std::vector<float> host;
         init_params(s, host);
         cudaMemcpy(s->w, host.data(), sizeof(float) * s->nparams, cudaMemcpyHostToDevice);
+        cudaMemcpy(s->cast_layers, casts.data(), sizeof(CastLayer) * casts.size(), cudaMemcpyHostToDevice);
         cudaMemset(s->g, 0, sizeof(float) * s->nparams);
         cudaMemset(s->m, 0, sizeof(float) * s->nparams);
         cudaMemset(s->v, 0, sizeof(float) * s->nparams);
@@ -1026,7 +1036,7 @@ WC_API void wc_surrogate_destroy(wc_surrogate* s) {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
     free_work(s->work);
-    void* ptrs[] = {s->w, s->g, s->m, s->v, s->wb, s->d_err, s->hist_in, s->target_in, s->stale_in, s->save_pos, s->save_vel,
+    void* ptrs[] = {s->w, s->g, s->m, s->v, s->wb, s->cast_layers, s->d_err, s->hist_in, s->target_in, s->stale_in, s->save_pos, s->save_vel,
                     s->alt_pos, s->alt_vel, s->stale, s->stale_tmp, s->rho_a, s->rho_b, s->err_part};
     for (void* p : ptrs)
         if (p) cudaFree(p);
