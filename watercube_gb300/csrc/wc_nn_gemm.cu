@@ -685,16 +685,6 @@ constexpr uint32_t AUX_BYTES = BM * 128u * 2u;      // 128 rows of 128 BF16: two
 constexpr uint32_t HALF_BYTES = AUX_BYTES / 2u;     // a half's rows of 128 bytes, swizzled
 constexpr uint32_t F32_OUT_BYTES = BM * 128u * 4u;  // per warp two boxes of 32 rows x 32 columns
 
-// A kernel launched by launch_after starts when the blocks of the kernel before it on the stream leave their SMs
-// (or have all called this): its prologue, barriers and tensor memory, runs beside that kernel's end. Every thread
-// calls it before its first access to global memory; what the kernel before wrote is visible then. A training
-// pass over 2,048 / 16,384 particles, ~320 launches: 3,378 -> 3,030 / 8,310 -> 7,965 us; a prediction of 2,500 particles
-// 537 -> 459.
-__device__ __forceinline__ void after_previous() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // Shared-memory descriptor of a K-major operand tile in the 128-byte swizzle layout: rows of
 // 128 bytes, 8-row groups 1,024 bytes apart (SBO), the leading-byte offset unused, version 1.
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
@@ -1785,21 +1775,6 @@ bool gemm_tma_available() { return encode_tiled() != nullptr; }
 
 namespace {
 
-template <class... P, class... A>
-cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, int threads, size_t smem, cudaStream_t s, const A&... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3((unsigned)threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, args...);
-}
-
 template <int AUX, bool LN, bool F32, bool BF>
 wc_status launch_tma_as(const GemmArgs& g, const TmaMaps& maps, const TmaPlan& plan, uint32_t grid, uint32_t* err,
                         cudaStream_t s) {
@@ -1809,7 +1784,8 @@ wc_status launch_tma_as(const GemmArgs& g, const TmaMaps& maps, const TmaPlan& p
                              (int)TMA_SMEM_LIMIT);
     });
     const int threads = TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER_WARPS : 0);
-    const cudaError_t e = launch_after(gemm_tma_kernel<AUX, LN, F32, BF>, grid, threads, plan.smem, s, g, maps, plan, err);
+    launch_after(gemm_tma_kernel<AUX, LN, F32, BF>, grid, threads, plan.smem, s, g, maps, plan, err);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(WC_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
     return WC_OK;
 }
@@ -1874,8 +1850,8 @@ wc_status launch_mlp_as(const MlpArgs& g, const MlpMaps& maps, uint32_t* err, cu
     }();
     if (!usable) return WC_OK;
     const uint32_t tiles = (g.m + BM - 1) / BM, sms = (uint32_t)sm_count();
-    const cudaError_t e =
-        launch_after(gemm_mlp_kernel<MP>, std::min(tiles, sms), MLP_THREADS, mlp_smem((g.k + BK - 1) / BK), s, g, maps, err);
+    launch_after(gemm_mlp_kernel<MP>, std::min(tiles, sms), MLP_THREADS, mlp_smem((g.k + BK - 1) / BK), s, g, maps, err);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(WC_ERR_CUDA, "mlp launch: %s", cudaGetErrorString(e));
     *launched = true;
     return WC_OK;
@@ -1935,8 +1911,8 @@ wc_status launch_gemm(const GemmArgs& g, uint32_t* err, cudaStream_t s) {
             std::call_once(once, [] {
                 cudaFuncSetAttribute(gemm_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM);
             });
-            const cudaError_t e =
-                launch_after(gemm_wgrad_kernel, (g.k + g.k_chunk - 1) / g.k_chunk, THREADS, WG_SMEM, s, g, ma, mb, err);
+            launch_after(gemm_wgrad_kernel, (g.k + g.k_chunk - 1) / g.k_chunk, THREADS, WG_SMEM, s, g, ma, mb, err);
+            const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return fail(WC_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
             return WC_OK;
         }

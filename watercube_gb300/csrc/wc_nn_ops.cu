@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(LNB_WARPS * 32) layernorm_backward_kernel(
     const uint32_t* __restrict__ add_idx, const float* __restrict__ add_src, int fresh, __nv_bfloat16* __restrict__ dy,
     float* __restrict__ part, float* __restrict__ part_dy) {
     __shared__ float s_sum[3][LNB_WARPS][128];
+    after_previous();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
     const float4 gm = reinterpret_cast<const float4*>(gamma)[lane];
@@ -330,6 +331,7 @@ __global__ void __launch_bounds__(CS_WARPS * 32) colsum_part_kernel(uint32_t row
                                                                    uint32_t rows_per_block, const float* __restrict__ x,
                                                                    float* __restrict__ part) {
     __shared__ float s[CS_WARPS][256];
+    after_previous();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
     const bool vec = (cols % 4u == 0) && (ld % 4u == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0);
@@ -374,6 +376,7 @@ __global__ void __launch_bounds__(256) colsum_final_kernel(uint32_t blocks, uint
                                                            float* __restrict__ out, int accumulate) {
     constexpr uint32_t G = 256 / Q;
     __shared__ float4 s[G][Q];
+    after_previous();
     const uint32_t q = threadIdx.x % Q, grp = threadIdx.x / Q, c = 4u * (blockIdx.x * Q + q);
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < cols) {
@@ -415,9 +418,9 @@ __global__ void __launch_bounds__(256) colsum_final_kernel(uint32_t blocks, uint
 // cols is a multiple of 4 and part, out are 16-byte aligned (the parameter blocks all are).
 void launch_colsum_final(uint32_t blocks, uint32_t cols, const float* part, float* out, int accumulate, cudaStream_t s) {
     if (cols <= 512u)
-        colsum_final_kernel<4><<<(cols + 15u) / 16u, 256, 0, s>>>(blocks, cols, part, out, accumulate);
+        launch_after(colsum_final_kernel<4>, (cols + 15u) / 16u, 256, 0, s, blocks, cols, part, out, accumulate);
     else
-        colsum_final_kernel<16><<<(cols + 63u) / 64u, 256, 0, s>>>(blocks, cols, part, out, accumulate);
+        launch_after(colsum_final_kernel<16>, (cols + 63u) / 64u, 256, 0, s, blocks, cols, part, out, accumulate);
 }
 
 // Mean squared error over 3 components: pred [n x ldp] (normalised), target [n] float4 / scale.
@@ -624,11 +627,11 @@ void layernorm_backward(uint32_t rows, float* dout, const float* y, const float*
     const uint32_t blocks = layernorm_backward_blocks(rows), rpb = layernorm_backward_rows(rows);
     if (!blocks) return;
     if (add_src)
-        layernorm_backward_kernel<true><<<blocks, LNB_WARPS * 32, 0, s>>>(rows, rpb, dout, y, mean, rstd, gamma, add_idx,
-                                                                          add_src, fresh, dy, part, part_dy);
+        launch_after(layernorm_backward_kernel<true>, blocks, LNB_WARPS * 32, 0, s, rows, rpb, dout, y, mean, rstd, gamma,
+                     add_idx, add_src, (int)fresh, dy, part, part_dy);
     else
-        layernorm_backward_kernel<false><<<blocks, LNB_WARPS * 32, 0, s>>>(rows, rpb, dout, y, mean, rstd, gamma, nullptr,
-                                                                           nullptr, 0, dy, part, part_dy);
+        launch_after(layernorm_backward_kernel<false>, blocks, LNB_WARPS * 32, 0, s, rows, rpb, dout, y, mean, rstd, gamma,
+                     add_idx, add_src, 0, dy, part, part_dy);
 }
 void relu_mask(size_t count, float* g, const __nv_bfloat16* z, __nv_bfloat16* out, cudaStream_t s) {
     if (count) relu_mask_kernel<<<(unsigned)std::min<size_t>(blocks_for(count, 256), 65535), 256, 0, s>>>(count, g, z, out);
@@ -653,7 +656,7 @@ void colsum(uint32_t rows, uint32_t cols, uint32_t ld, const float* x, float* pa
             cudaStream_t s) {
     const uint32_t blocks = colsum_blocks(rows);
     if (!blocks) return;
-    colsum_part_kernel<<<blocks, CS_WARPS * 32, 0, s>>>(rows, cols, ld, CS_ROWS, x, part);
+    launch_after(colsum_part_kernel, blocks, CS_WARPS * 32, 0, s, rows, cols, ld, CS_ROWS, x, part);
     launch_colsum_final(blocks, cols, part, out, accumulate, s);
 }
 void colsum_partials(uint32_t blocks, uint32_t cols, const float* part, float* out, int accumulate, cudaStream_t s) {
