@@ -313,13 +313,17 @@ __global__ void classify_kernel(uint32_t G, const float* __restrict__ phi, float
     }
 }
 
-// The triangles of the scan's list of non-empty cubes (most cubes have none: 2.0 million cubes took 26 us).
+// The triangles of the scan's list of non-empty cubes (most cubes have none: 2.0 million cubes took 26 us). It is
+// launched before the host has read the error word, so it looks itself: after a failed field or scan (whose list may
+// have holes) it writes nothing, and the mesh of the extraction before stays whole.
 __global__ void emit_kernel(Grid g, const float* __restrict__ phi, float iso, const uint32_t* __restrict__ offsets,
                             const uint32_t* __restrict__ list, const uint32_t* __restrict__ list_len,
-                            uint64_t max_tris, float* __restrict__ out) {
-    const uint32_t G = g.G, C = G - 1, len = *list_len;
+                            const uint32_t* __restrict__ err, uint64_t max_tris, float* __restrict__ out) {
+    if (*err) return;
+    const uint32_t G = g.G, C = G - 1, cubes = C * C * C, len = min(*list_len, cubes);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
         const uint32_t q = list[i];
+        if (q >= cubes) continue;
         const uint32_t ix = q % C, iy = (q / C) % C, iz = q / (C * C);
         const uint32_t cfg = cube_config(phi, G, ix, iy, iz, iso);
         const uint32_t nt = c_count[cfg];
@@ -512,7 +516,7 @@ WC_API wc_status wc_surface_extract(wc_surface* s, wc_fluid* f, uint64_t* num_tr
     auto emit = [&] {
         if (s->tri_cap)
             emit_kernel<<<grid_blocks(std::min<uint64_t>(cubes, 152ull * 8 * 256)), 256, 0, fi.stream>>>(
-                g, s->phi, s->p.iso, s->offsets, s->cell_list, s->words + 1, s->tri_cap, s->tris);
+                g, s->phi, s->p.iso, s->offsets, s->cell_list, s->words + 1, s->err, s->tri_cap, s->tris);
     };
     emit();
     cudaEventRecord(e2, fi.stream);
@@ -533,6 +537,7 @@ WC_API wc_status wc_surface_extract(wc_surface* s, wc_fluid* f, uint64_t* num_tr
         if (s->tris) cudaFree(s->tris);
         s->tris = nullptr;
         s->tri_cap = 0;
+        s->have = false;  // the mesh of the extraction before went with its buffer
         st = dalloc(&s->tris, (size_t)total * 9u);
         if (st == WC_OK) {
             s->tri_cap = total;
