@@ -16,6 +16,8 @@ namespace nn {
 // pass over 2,048 / 16,384 particles, ~320 launches, takes 3,378 / 8,310 us without, 3,040 / 7,970 with the GEMMs and
 // 2,755 / 7,890 with the sums and LayerNorms too; a prediction of 2,500 particles 537 -> 459. The segment sums are
 // launched as usual: the next GEMM's blocks would take places from their second wave (65,536 particles 3,375 -> 3,415).
+// Such a kernel is resident while its inputs are written, so they are not read-only for its lifetime: its loads are
+// plain ones, without __ldg (ld.global.nc) and without const __restrict__, from which the compiler makes the same.
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

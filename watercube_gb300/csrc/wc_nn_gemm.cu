@@ -175,7 +175,7 @@ __device__ __forceinline__ void add_row(float x[32], const __nv_bfloat16* r, uin
     if (ncols == 32u && (reinterpret_cast<uintptr_t>(r) & 15u) == 0) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(r) + q);
+            const uint4 v = reinterpret_cast<const uint4*>(r)[q];
             const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -199,10 +199,10 @@ __device__ __forceinline__ void epilogue_store(const GemmArgs& g, float x[32], u
     if (g.bias) {
 #pragma unroll
         for (int j = 0; j < 32; ++j)
-            if ((uint32_t)j < ncols) x[j] += __ldg(g.bias + col0 + j);
+            if ((uint32_t)j < ncols) x[j] += g.bias[col0 + j];
     }
-    if (g.add1) add_row(x, g.add1 + (size_t)__ldg(g.add1_idx + row) * g.ld_add + col0, ncols);
-    if (g.add2) add_row(x, g.add2 + (size_t)__ldg(g.add2_idx + row) * g.ld_add + col0, ncols);
+    if (g.add1) add_row(x, g.add1 + (size_t)g.add1_idx[row] * g.ld_add + col0, ncols);
+    if (g.add2) add_row(x, g.add2 + (size_t)g.add2_idx[row] * g.ld_add + col0, ncols);
     if (g.relu) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) x[j] = fmaxf(x[j], 0.f);
@@ -782,6 +782,12 @@ __device__ __forceinline__ void scale_pair(float* a, float m, float g0, float g1
         : "f"(m), "f"(g0), "f"(g1), "f"(b0), "f"(b1));
 }
 
+// Eight consecutive values.
+__device__ __forceinline__ void load8(float* o, const float* p) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = reinterpret_cast<const float4*>(p)[1];
+    o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w, o[4] = b.x, o[5] = b.y, o[6] = b.z, o[7] = b.w;
+}
+
 // The LayerNorm of n = 128 columns. ln_centre: by the two warps of a pair, x a thread's 64 columns of its row, which
 // becomes x - mean (xs, xv, oks as in tma_epilogue); false when a wait of either warp failed (both leave). ln_scale:
 // eight columns o = gamma x rstd + beta.
@@ -791,16 +797,16 @@ __device__ __forceinline__ void ln_scale(const float* gamma, const float* beta, 
     if (VEC) {
 #pragma unroll
         for (int k = 0; k < 8; k += 4) {
-            const float4 g4 = __ldg(reinterpret_cast<const float4*>(gamma + k));
-            const float4 b4 = __ldg(reinterpret_cast<const float4*>(beta + k));
+            const float4 g4 = *reinterpret_cast<const float4*>(gamma + k);
+            const float4 b4 = *reinterpret_cast<const float4*>(beta + k);
             gm[k] = g4.x, gm[k + 1] = g4.y, gm[k + 2] = g4.z, gm[k + 3] = g4.w;
             bt[k] = b4.x, bt[k + 1] = b4.y, bt[k + 2] = b4.z, bt[k + 3] = b4.w;
         }
     } else {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            gm[k] = __ldg(gamma + k);
-            bt[k] = __ldg(beta + k);
+            gm[k] = gamma[k];
+            bt[k] = beta[k];
         }
     }
 #pragma unroll
@@ -851,13 +857,25 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
                                              uint64_t* acc_full, uint64_t* acc_empty, uint64_t* aux_full,
                                              uint64_t* aux_empty, volatile int* failed, uint32_t ntiles, uint32_t quarter,
                                              uint32_t half, uint32_t lane, uint32_t aux_base, uint32_t f32_base,
-                                             float (*xs)[2][32], float (*xv)[2][32], int (*oks)[2]) {
+                                             float* s_bias, float (*xs)[2][32], float (*xv)[2][32], int (*oks)[2]) {
     constexpr float LN_EPSILON = 1e-5f;
     const uint32_t col0 = 64u * half, r = 32u * quarter + lane;
     const uint32_t f32_buf = f32_base + (quarter * 2u + half) * (F32_OUT_BYTES / 8u);  // this warp's two boxes
     // bias, gamma and beta four at a time when they allow 16-byte loads of whole tiles (uniform branch)
     const bool vec = g.n == 128u && ((reinterpret_cast<uintptr_t>(g.bias) | (LN ? reinterpret_cast<uintptr_t>(g.ln_gamma) |
                                       reinterpret_cast<uintptr_t>(g.ln_beta) : 0)) & 15u) == 0;
+    // The bias: from shared memory beside gathered rows, which leave it no room in L1 (460,000 rows 53.9 us; 57.9
+    // from global memory) and where it has no 16-byte loads; otherwise L1 is as fast and there is nothing to copy.
+    const bool staged = !LN && g.bias && (AUX == AUX_GATHER || !vec);
+    if (staged) {
+        const uint32_t c = threadIdx.x - 64u;
+        if (c < 128u) s_bias[c] = c < g.n ? g.bias[c] : 0.f;
+        asm volatile("bar.sync 5, 256;" ::: "memory");  // the epilogue's warps
+    }
+    auto bias8 = [&](float* o, uint32_t c) {  // eight columns from c
+        if (staged) load8(o, s_bias + c);
+        else load8(o, g.bias + c);
+    };
     uint32_t t = 0;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t) {
         const uint32_t b = t & 1u;
@@ -881,23 +899,6 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t taddr = tmem + ((32u * quarter) << 16) + b * (uint32_t)BN + col0;
-        auto bias_add = [&](float* x, uint32_t c) {  // 32 columns from c
-            if (!g.bias) return;
-            if (vec) {
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) {
-                    const float4 bb = __ldg(reinterpret_cast<const float4*>(g.bias + c + j));
-                    x[j] += bb.x;
-                    x[j + 1] += bb.y;
-                    x[j + 2] += bb.z;
-                    x[j + 3] += bb.w;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (c + j < g.n) x[j] += __ldg(g.bias + c + j);
-            }
-        };
         if constexpr (LN && F32) {
             float x[64];  // group j (0..15): columns 8 j + 4 half ..
             if (ok) {
@@ -919,7 +920,7 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
             }
             auto four = [&](const float* base, uint32_t j) {  // columns of group j
                 const float* q = base + 8u * j + 4u * half;
-                return vec ? __ldg(reinterpret_cast<const float4*>(q)) : make_float4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+                return vec ? *reinterpret_cast<const float4*>(q) : make_float4(*q, q[1], q[2], q[3]);
             };
             float s[16];
             auto tree = [&]() {  // the sum of s[0..16) in pairs 8, 4, 2, 1 apart
@@ -1003,8 +1004,20 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
 #pragma unroll
                 for (int j = 0; j < 64; ++j) x[j] = 0.f;
             }
-            bias_add(x, col0);
-            bias_add(x + 32, col0 + 32u);
+            if (g.bias) {
+#pragma unroll
+                for (int j = 0; j < 64; j += 8) {
+                    float bb[8];
+                    if (vec) {
+                        load8(bb, g.bias + col0 + j);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) bb[k] = g.bias[col0 + j + k];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) x[j + k] += bb[k];
+                }
+            }
             float rstd;
             if (!ln_centre(x, ok, xs, xv, oks, failed, quarter, half, lane, &rstd)) break;
 #pragma unroll
@@ -1020,16 +1033,21 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
 #pragma unroll
             for (uint32_t q = 0; q < 2; ++q) {
                 uint32_t v[32];
+                float x[32], bb[8];  // bb: the bias, eight columns ahead of its use
+                if (g.bias) bias8(bb, col0 + 32u * q);
                 tmem_ld32(taddr + 32u * q, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                float x[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) x[j] = g.k ? __uint_as_float(v[j]) : 0.f;
-                bias_add(x, col0 + 32u * q);
 #pragma unroll
                 for (uint32_t c = 0; c < 4; ++c) {
                     float* y = x + 8 * c;
                     const uint32_t at = stage + sw128(r, 4u * q + c);
+                    if (g.bias) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) y[k] += bb[k];
+                        if (c < 3u) bias8(bb, col0 + 32u * q + 8u * (c + 1u));
+                    }
                     if (AUX == AUX_GATHER) {
                         if (g.add1) add8(y, lds128(at));
                         if (g.add2) add8(y, lds128(at + (g.add1 ? AUX_BYTES : 0u)));
@@ -1087,6 +1105,7 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
     // LN: the warp pairs' exchanged row sums, squared deviations and wait outcomes
     __shared__ float s_lnx[LN ? 4 : 1][2][32], s_lnv[LN ? 4 : 1][2][32];
     __shared__ int s_lnok[LN ? 4 : 1][2];
+    __shared__ __align__(16) float s_bias[LN ? 4 : 128];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_failed;
     volatile int* failed = &s_failed;
@@ -1205,7 +1224,7 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
         // warps 2..9: quarter w % 4 (the accumulator lanes its position in the warpgroup may
         // address), columns 64 ((w - 2) / 4) ..
         tma_epilogue<AUX, LN, F32, BF>(g, maps, plan, tmem, acc_full, acc_empty, aux_full, aux_empty, failed, ntiles,
-                                       warp & 3u, (warp - 2u) / 4u, lane, aux_base, f32_base, s_lnx, s_lnv, s_lnok);
+                                       warp & 3u, (warp - 2u) / 4u, lane, aux_base, f32_base, s_bias, s_lnx, s_lnv, s_lnok);
     } else {
         // AUX_GATHER: warp w copies the gathered rows of tile rows 32 w .. + 31, two rows per
         // instruction, 16 lanes of 16 bytes each; every thread's copies arrive on the stage's
@@ -1213,12 +1232,17 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
         const uint32_t r0 = 32u * (warp - 2u - PIPE_EPILOGUE), chunk = lane & 15u;
         const __nv_bfloat16* const src[2] = {g.add1, g.add2};
         const uint32_t* const idx[2] = {g.add1_idx, g.add2_idx};
+        uint32_t next[2];  // this lane's row indices, a tile ahead
+        auto index = [&](uint32_t tile) {
+            const uint32_t row = tile * BM + r0 + lane;
+#pragma unroll
+            for (int o = 0; o < 2; ++o) next[o] = src[o] && tile < ntiles && row < g.m ? idx[o][row] : 0u;
+        };
+        index(blockIdx.x);
         uint32_t t = 0;
         for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t) {
-            const uint32_t b = t & 1u, row = tile * BM + r0 + lane;
-            uint32_t at[2];
-#pragma unroll
-            for (int o = 0; o < 2; ++o) at[o] = src[o] && row < g.m ? __ldg(idx[o] + row) : 0u;
+            const uint32_t b = t & 1u, at[2] = {next[0], next[1]};
+            index(tile + gridDim.x);
             bool ok = !*failed && (t < 2 || mbar_wait(smem_addr(&aux_empty[b]), ((t >> 1) - 1u) & 1u));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
@@ -1281,11 +1305,6 @@ struct MlpMaps {
     CUtensorMap a, w1, w2, c;
 };
 
-// Eight consecutive values.
-__device__ __forceinline__ void load8(float* o, const float* p) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w, o[4] = b.x, o[5] = b.y, o[6] = b.z, o[7] = b.w;
-}
 // max(x, 0) of two BF16 (a NaN gives 0, as fmaxf before the rounding does)
 __device__ __forceinline__ uint32_t relu2(uint32_t w) {
     const __nv_bfloat162 h = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&w), __floats2bfloat162_rn(0.f, 0.f));
@@ -1404,7 +1423,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
             const uint32_t r0 = 32u * (warp - 4u), chunk = lane & 15u;
             auto index = [&](uint32_t t) {
                 const uint32_t row = (blockIdx.x + t * gridDim.x) * BM + r0 + lane;
-                return t < mine && row < g.m ? __ldg(g.add2_idx + row) : 0u;
+                return t < mine && row < g.m ? g.add2_idx[row] : 0u;
             };
             uint32_t next = index(0);
             for (uint32_t t = 0; t < mine; ++t) {
@@ -1435,7 +1454,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         const uint32_t quarter = warp & 3u, half = (warp - 8u) / 4u, col0 = 64u * half, r = 32u * quarter + lane;
         auto index = [&](uint32_t t) {
             const uint32_t row = (blockIdx.x + t * gridDim.x) * BM + r;
-            return MP && t < mine && row < g.m ? __ldg(g.add1_idx + row) : 0u;
+            return MP && t < mine && row < g.m ? g.add1_idx[row] : 0u;
         };
         uint32_t next = index(0);
         for (uint32_t t = 0; t < mine; ++t) {
@@ -1444,7 +1463,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
             uint4 p[4];
             if (MP) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) p[c] = __ldg(p_row + c);
+                for (int c = 0; c < 4; ++c) p[c] = p_row[c];
             }
             next = index(t + 1u);
             bool ok = !*failed && mbar_wait(smem_addr(&acc1_full[b]), (t >> 1) & 1u);
@@ -1459,6 +1478,8 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
             for (uint32_t q = 0; q < 2; ++q) {
                 uint32_t v[32];
+                float next_b[8];  // eight columns ahead of their use, as the rows of P
+                if (g.b1) load8(next_b, g.b1 + col0 + 32u * q);
                 tmem_ld32(tmem + ((32u * quarter) << 16) + b * (uint32_t)BN + col0 + 32u * q, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -1467,15 +1488,14 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
                     for (int k = 0; k < 8; ++k) y[k] = __uint_as_float(v[8 * c + k]);
                     if (g.b1) {
-                        float bb[8];
-                        load8(bb, g.b1 + col0 + 32u * q + 8u * c);
 #pragma unroll
-                        for (int k = 0; k < 8; k += 2) add_pair(y + k, bb[k], bb[k + 1]);
+                        for (int k = 0; k < 8; k += 2) add_pair(y + k, next_b[k], next_b[k + 1]);
+                        if (c < 3u) load8(next_b, g.b1 + col0 + 32u * q + 8u * (c + 1u));
                     }
                     const uint32_t at = z + b * AUX_BYTES + half * HALF_BYTES + sw128(r, 4u * q + c);
                     if (MP) {
                         add8(y, p[c]);
-                        if (q == 0) p[c] = __ldg(p_row + 4 + c);
+                        if (q == 0) p[c] = p_row[4 + c];
                         add8(y, lds128(at));
                     }
                     sts128(at, make_uint4(relu2(pack2(y[0], y[1])), relu2(pack2(y[2], y[3])), relu2(pack2(y[4], y[5])), relu2(pack2(y[6], y[7]))));
@@ -1532,16 +1552,20 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
             float rstd;
             if (!ln_centre(x, ok, s_lnx, s_lnv, s_lnok, failed, quarter, half, lane, &rstd)) break;
             const uint32_t out = smem_addr(slots) + st * AUX_BYTES + half * HALF_BYTES;
+            float gm[8], bt[8];  // eight columns ahead of their use
+            load8(gm, g.gamma + col0);
+            load8(bt, g.beta + col0);
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 float o[8];
-                float gm[8], bt[8];
-                load8(gm, g.gamma + col0 + 8 * c);
-                load8(bt, g.beta + col0 + 8 * c);
 #pragma unroll
                 for (int k = 0; k < 8; k += 2) {
                     o[k] = x[8 * c + k], o[k + 1] = x[8 * c + k + 1];
                     scale_pair(o + k, rstd, gm[k], gm[k + 1], bt[k], bt[k + 1]);
+                }
+                if (c < 7) {
+                    load8(gm, g.gamma + col0 + 8 * (c + 1));
+                    load8(bt, g.beta + col0 + 8 * (c + 1));
                 }
                 const uint32_t at = out + sw128(r, (uint32_t)c);
                 if (MP) add8(o, lds128(at));

@@ -193,10 +193,9 @@ __global__ void layernorm_kernel(uint32_t rows, const float* __restrict__ y, con
 constexpr int LNB_WARPS = 8;
 template <bool ADD>
 __global__ void __launch_bounds__(LNB_WARPS * 32) layernorm_backward_kernel(
-    uint32_t rows, uint32_t rows_per_block, float* __restrict__ dout, const float* __restrict__ y,
-    const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ gamma,
-    const uint32_t* __restrict__ add_idx, const float* __restrict__ add_src, int fresh, __nv_bfloat16* __restrict__ dy,
-    float* __restrict__ part, float* __restrict__ part_dy) {
+    uint32_t rows, uint32_t rows_per_block, float* dout, const float* y, const float* mean, const float* rstd,
+    const float* gamma, const uint32_t* add_idx, const float* add_src, int fresh, __nv_bfloat16* dy, float* part,
+    float* part_dy) {
     __shared__ float s_sum[3][LNB_WARPS][128];
     after_previous();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -210,11 +209,11 @@ __global__ void __launch_bounds__(LNB_WARPS * 32) layernorm_backward_kernel(
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const uint32_t i = u && two ? row + LNB_WARPS : row;
-            if (ADD) s[u] = __ldg(reinterpret_cast<const float4*>(add_src + (size_t)__ldg(add_idx + i) * 128) + lane);
+            if (ADD) s[u] = reinterpret_cast<const float4*>(add_src + (size_t)add_idx[i] * 128)[lane];
             d[u] = ADD && fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4*>(dout + (size_t)i * 128)[lane];
-            v[u] = __ldg(reinterpret_cast<const float4*>(y + (size_t)i * 128) + lane);
-            mu[u] = __ldg(mean + i);
-            rs[u] = __ldg(rstd + i);
+            v[u] = reinterpret_cast<const float4*>(y + (size_t)i * 128)[lane];
+            mu[u] = mean[i];
+            rs[u] = rstd[i];
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
@@ -328,8 +327,8 @@ __global__ void segment_sum_kernel(uint32_t nodes, const uint32_t* __restrict__ 
 constexpr int CS_WARPS = 8;
 constexpr uint32_t CS_ROWS = 256;
 __global__ void __launch_bounds__(CS_WARPS * 32) colsum_part_kernel(uint32_t rows, uint32_t cols, uint32_t ld,
-                                                                   uint32_t rows_per_block, const float* __restrict__ x,
-                                                                   float* __restrict__ part) {
+                                                                   uint32_t rows_per_block, const float* x,
+                                                                   float* part) {
     __shared__ float s[CS_WARPS][256];
     after_previous();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -372,8 +371,8 @@ __global__ void __launch_bounds__(CS_WARPS * 32) colsum_part_kernel(uint32_t row
 // pairs. (One thread per column over all partials, one load in flight: 18 us for 257 tiles of
 // 128 x 128.)
 template <int Q>
-__global__ void __launch_bounds__(256) colsum_final_kernel(uint32_t blocks, uint32_t cols, const float* __restrict__ part,
-                                                           float* __restrict__ out, int accumulate) {
+__global__ void __launch_bounds__(256) colsum_final_kernel(uint32_t blocks, uint32_t cols, const float* part,
+                                                           float* out, int accumulate) {
     constexpr uint32_t G = 256 / Q;
     __shared__ float4 s[G][Q];
     after_previous();
@@ -382,7 +381,7 @@ __global__ void __launch_bounds__(256) colsum_final_kernel(uint32_t blocks, uint
     if (c < cols) {
 #pragma unroll 4
         for (uint32_t b = grp; b < blocks; b += G) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(part + (size_t)b * cols + c));
+            const float4 v = *reinterpret_cast<const float4*>(part + (size_t)b * cols + c);
             a.x += v.x;
             a.y += v.y;
             a.z += v.z;
