@@ -193,16 +193,16 @@ __device__ __forceinline__ void add_row(float x[32], const __nv_bfloat16* r, uin
 
 // Bias, gathered row adds, ReLU and the stores of 32 accumulator columns of one row:
 // x[0..ncols) belong to output columns col0 ..; kz: the split of the K range (partial outputs
-// split_stride apart).
+// split_stride apart); i1, i2: the row's indices into the gathered operands.
 __device__ __forceinline__ void epilogue_store(const GemmArgs& g, float x[32], uint32_t row, uint32_t col0,
-                                               uint32_t ncols, uint32_t kz) {
+                                               uint32_t ncols, uint32_t kz, uint32_t i1, uint32_t i2) {
     if (g.bias) {
 #pragma unroll
         for (int j = 0; j < 32; ++j)
             if ((uint32_t)j < ncols) x[j] += g.bias[col0 + j];
     }
-    if (g.add1) add_row(x, g.add1 + (size_t)g.add1_idx[row] * g.ld_add + col0, ncols);
-    if (g.add2) add_row(x, g.add2 + (size_t)g.add2_idx[row] * g.ld_add + col0, ncols);
+    if (g.add1) add_row(x, g.add1 + (size_t)i1 * g.ld_add + col0, ncols);
+    if (g.add2) add_row(x, g.add2 + (size_t)i2 * g.ld_add + col0, ncols);
     if (g.relu) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) x[j] = fmaxf(x[j], 0.f);
@@ -383,7 +383,8 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(const GemmArgs g, uint32_
         float x[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) x[j] = issued ? __uint_as_float(v[j]) : 0.f;
-        epilogue_store(g, x, row, n0 + c0, min(32u, g.n - (n0 + c0)), kz);
+        epilogue_store(g, x, row, n0 + c0, min(32u, g.n - (n0 + c0)), kz, g.add1 ? g.add1_idx[row] : 0u,
+                       g.add2 ? g.add2_idx[row] : 0u);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -466,6 +467,10 @@ __device__ __forceinline__ void drain_accumulators(const GemmArgs& g, uint32_t t
     uint32_t t = 0;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t) {
         const uint32_t b = t & 1u;
+        const uint32_t m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
+        const uint32_t row = m0 + 32u * quarter + lane;
+        const bool row_ok = row < g.m;
+        const uint32_t i1 = g.add1 && row_ok ? g.add1_idx[row] : 0u, i2 = g.add2 && row_ok ? g.add2_idx[row] : 0u;
         bool ok = !*failed && mbar_wait(smem_addr(&acc_full[b]), (t >> 1) & 1u);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
@@ -473,9 +478,6 @@ __device__ __forceinline__ void drain_accumulators(const GemmArgs& g, uint32_t t
             break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
-        const uint32_t row = m0 + 32u * quarter + lane;
-        const bool row_ok = row < g.m;
         for (uint32_t c0 = 64u * half; c0 < 64u * half + 64u; c0 += 32) {
             uint32_t v[32];
             const uint32_t taddr = tmem + ((32u * quarter) << 16) + b * (uint32_t)BN + c0;
@@ -493,7 +495,7 @@ __device__ __forceinline__ void drain_accumulators(const GemmArgs& g, uint32_t t
             float x[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) x[j] = nslices ? __uint_as_float(v[j]) : 0.f;
-            epilogue_store(g, x, row, n0 + c0, min(32u, g.n - (n0 + c0)), 0u);
+            epilogue_store(g, x, row, n0 + c0, min(32u, g.n - (n0 + c0)), 0u, i1, i2);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -672,7 +674,8 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1) gemm_pipe_kernel(const GemmAr
 // leave through shared memory and TMA stores, a 32-row box per warp (FP32 accumulation into C as
 // a TMA add), and what it reads per element arrives there first, 128 columns by 128 rows in two
 // stages — the residual rows of a LayerNorm by TMA (AUX_TMA), the gathered rows added to a layer by
-// four more warps with cp.async, 16 lanes to a row (AUX_GATHER). BF16 results are written over
+// four more warps with cp.async, 16 lanes to a row (AUX_GATHER). Forms that it cannot take are written from the
+// registers (AUX_DIRECT, see launch_tma). BF16 results are written over
 // the place of the values read. Bound by the traffic it cannot avoid: 460,000 rows of 128 with two
 // gathered rows each take 59 us against 134 us with row-per-thread accesses (62 % of the copy
 // bandwidth for A and C alone, the gathered rows come from L2 on top).
@@ -680,7 +683,7 @@ constexpr int TMA_THREADS = 32 * (2 + PIPE_EPILOGUE);
 constexpr int GATHER_WARPS = 4;
 constexpr int TMA_MAX_STAGES = 6;
 constexpr uint32_t TMA_SMEM_LIMIT = 224u * 1024u;  // dynamic; the barriers and row sums take up to 3 KB more
-enum : int { AUX_NONE = 0, AUX_TMA = 1, AUX_GATHER = 2 };
+enum : int { AUX_NONE = 0, AUX_TMA = 1, AUX_GATHER = 2, AUX_DIRECT = 3 };
 constexpr uint32_t AUX_BYTES = BM * 128u * 2u;      // 128 rows of 128 BF16: two halves of 64 columns
 constexpr uint32_t HALF_BYTES = AUX_BYTES / 2u;     // a half's rows of 128 bytes, swizzled
 constexpr uint32_t F32_OUT_BYTES = BM * 128u * 4u;  // per warp two boxes of 32 rows x 32 columns
@@ -861,24 +864,21 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
     constexpr float LN_EPSILON = 1e-5f;
     const uint32_t col0 = 64u * half, r = 32u * quarter + lane;
     const uint32_t f32_buf = f32_base + (quarter * 2u + half) * (F32_OUT_BYTES / 8u);  // this warp's two boxes
-    // bias, gamma and beta four at a time when they allow 16-byte loads of whole tiles (uniform branch)
-    const bool vec = g.n == 128u && ((reinterpret_cast<uintptr_t>(g.bias) | (LN ? reinterpret_cast<uintptr_t>(g.ln_gamma) |
-                                      reinterpret_cast<uintptr_t>(g.ln_beta) : 0)) & 15u) == 0;
-    // The bias: from shared memory beside gathered rows, which leave it no room in L1 (460,000 rows 53.9 us; 57.9
-    // from global memory) and where it has no 16-byte loads; otherwise L1 is as fast and there is nothing to copy.
-    const bool staged = !LN && g.bias && (AUX == AUX_GATHER || !vec);
-    if (staged) {
+    // LN: bias, gamma and beta four at a time when they allow 16-byte loads (uniform branch)
+    const bool vec = LN && ((reinterpret_cast<uintptr_t>(g.bias) | reinterpret_cast<uintptr_t>(g.ln_gamma) |
+                             reinterpret_cast<uintptr_t>(g.ln_beta)) & 15u) == 0;
+    // The bias from shared memory (16,384 rows 4.5 us, one chunk ahead from L1 5.4; beside gathered rows, which leave
+    // it no room in L1, 460,000 rows 54.9 against 57.9)
+    if (!LN && g.bias) {
         const uint32_t c = threadIdx.x - 64u;
         if (c < 128u) s_bias[c] = c < g.n ? g.bias[c] : 0.f;
         asm volatile("bar.sync 5, 256;" ::: "memory");  // the epilogue's warps
     }
-    auto bias8 = [&](float* o, uint32_t c) {  // eight columns from c
-        if (staged) load8(o, s_bias + c);
-        else load8(o, g.bias + c);
-    };
     uint32_t t = 0;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t) {
         const uint32_t b = t & 1u;
+        float bb[8];  // the bias, eight columns ahead of its use
+        if (!LN && g.bias) load8(bb, s_bias + col0);
         bool ok = !*failed && mbar_wait(smem_addr(&acc_full[b]), (t >> 1) & 1u);
         if (AUX != AUX_NONE) ok = ok && mbar_wait(smem_addr(&aux_full[b]), (t >> 1) & 1u);
         ok = __all_sync(0xffffffffu, ok);
@@ -1033,8 +1033,7 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
 #pragma unroll
             for (uint32_t q = 0; q < 2; ++q) {
                 uint32_t v[32];
-                float x[32], bb[8];  // bb: the bias, eight columns ahead of its use
-                if (g.bias) bias8(bb, col0 + 32u * q);
+                float x[32];
                 tmem_ld32(taddr + 32u * q, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -1046,7 +1045,7 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
                     if (g.bias) {
 #pragma unroll
                         for (int k = 0; k < 8; ++k) y[k] += bb[k];
-                        if (c < 3u) bias8(bb, col0 + 32u * q + 8u * (c + 1u));
+                        if (4u * q + c < 7u) load8(bb, s_bias + col0 + 32u * q + 8u * (c + 1u));
                     }
                     if (AUX == AUX_GATHER) {
                         if (g.add1) add8(y, lds128(at));
@@ -1223,7 +1222,9 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
     } else if (warp < 2u + PIPE_EPILOGUE) {
         // warps 2..9: quarter w % 4 (the accumulator lanes its position in the warpgroup may
         // address), columns 64 ((w - 2) / 4) ..
-        tma_epilogue<AUX, LN, F32, BF>(g, maps, plan, tmem, acc_full, acc_empty, aux_full, aux_empty, failed, ntiles,
+        if constexpr (AUX == AUX_DIRECT)
+            drain_accumulators(g, tmem, acc_full, acc_empty, failed, ntiles, 1u, nslices, warp & 3u, (warp - 2u) / 4u, lane);
+        else tma_epilogue<AUX, LN, F32, BF>(g, maps, plan, tmem, acc_full, acc_empty, aux_full, aux_empty, failed, ntiles,
                                        warp & 3u, (warp - 2u) / 4u, lane, aux_base, f32_base, s_bias, s_lnx, s_lnv, s_lnok);
     } else {
         // AUX_GATHER: warp w copies the gathered rows of tile rows 32 w .. + 31, two rows per
@@ -1706,7 +1707,8 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_wgrad_kernel(const GemmArgs g
         float x[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
-        epilogue_store(g, x, row, c0, min(32u, g.n - c0), blockIdx.x);
+        epilogue_store(g, x, row, c0, min(32u, g.n - c0), blockIdx.x, g.add1 ? g.add1_idx[row] : 0u,
+                       g.add2 ? g.add2_idx[row] : 0u);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -1816,9 +1818,13 @@ wc_status launch_tma_as(const GemmArgs& g, const TmaMaps& maps, const TmaPlan& p
 
 // The TMA kernel for row-major A (or [A | A2] split at a whole slice: the node layers' 65,536 x 256 take
 // 33 us with cp.async), n <= 128 and k <= 384, when every operand it moves by TMA has a
-// tensor map (16-byte aligned base and rows), the gathered rows are whole and aligned, and the shared
-// memory holds at least two A slots (all but k > 256 with two gathered operands, or with FP32 and
-// BF16 outputs together). Otherwise the caller runs the cp.async kernel.
+// tensor map (16-byte aligned base and rows). Its epilogue through shared memory needs tensor maps for the results
+// too, whole and aligned gathered rows (n = 128) and room for at least two A slots (all but k > 256 with two gathered
+// operands, or with FP32 and BF16 outputs together). The other forms write from the registers, a row per thread
+// (AUX_DIRECT), and so do results of at most eight columns or of 32 in BF16 alone, whose rows a thread writes in a few
+// whole accesses (460,000 rows, k = 16: 21.4 us against 25.6 at n = 8, 23.3 against 26.3 at n = 32; but 46 against 26
+// at n = 16, and 47 against 27 where FP32 results are added to). With cp.async operands instead of TMA's, two gathered
+// operands at k = 384 take 103 us per 200,000 rows (75 so), at n = 64 49 (37).
 wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream_t s, bool* launched) {
     *launched = false;
     const bool gather = g.add1 || g.add2, aux = gather || g.ln_resid || g.relu_z, f32 = g.c_f32 != nullptr, bf = g.c_bf16 != nullptr;
@@ -1826,13 +1832,6 @@ wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream
     if (g.a2 && (g.k_split % BK || g.k_split >= g.k || !encode_operand(&maps.a2, g.a2, g.k - g.k_split, g.m, 2ull * g.lda2)))
         return WC_OK;
     if (!encode_operand(&maps.a, g.a, g.a2 ? g.k_split : g.k, g.m, 2ull * g.lda) || !encode_operand(&maps.b, g.b, g.k, g.n, 2ull * g.ldb))
-        return WC_OK;
-    if (bf && !encode_operand(&maps.cb, g.c_bf16, g.n, g.m, 2ull * g.ldc, 32)) return WC_OK;
-    if (f32 && !encode_operand(&maps.cf, g.c_f32, g.n, g.m, 4ull * g.ldc, 32, true)) return WC_OK;
-    if (g.ln_resid && !encode_operand(&maps.aux, g.ln_resid, 128, g.m, 256)) return WC_OK;
-    if (g.relu_z && !encode_operand(&maps.aux, g.relu_z, 128, g.m, 256)) return WC_OK;
-    if (gather && (g.n != 128u || g.ld_add % 8u || reinterpret_cast<uintptr_t>(g.add1) % 16u ||
-                   reinterpret_cast<uintptr_t>(g.add2) % 16u))
         return WC_OK;
     const uint32_t nslices = (g.k + BK - 1) / BK;
     TmaPlan plan{};
@@ -1843,7 +1842,22 @@ wc_status launch_tma(const GemmArgs& g, uint32_t grid, uint32_t* err, cudaStream
     plan.one_stage = !aux && bf &&
                      nslices * TILE_BYTES + 2u * plan.aux_bytes + plan.f32_bytes + TMA_MAX_STAGES * TILE_BYTES > TMA_SMEM_LIMIT;
     const uint32_t fixed = nslices * TILE_BYTES + (plan.one_stage ? 1u : 2u) * plan.aux_bytes + plan.f32_bytes;
-    if (fixed + 2u * TILE_BYTES > TMA_SMEM_LIMIT) return WC_OK;
+    const bool narrow = !aux && !g.accumulate && (g.n <= 8u || (g.n == 32u && !f32)) && !g.ln_gamma;
+    const bool shared = !narrow && fixed + 2u * TILE_BYTES <= TMA_SMEM_LIMIT &&
+                        (!bf || encode_operand(&maps.cb, g.c_bf16, g.n, g.m, 2ull * g.ldc, 32)) &&
+                        (!f32 || encode_operand(&maps.cf, g.c_f32, g.n, g.m, 4ull * g.ldc, 32, true)) &&
+                        (!g.ln_resid || encode_operand(&maps.aux, g.ln_resid, 128, g.m, 256)) &&
+                        (!g.relu_z || encode_operand(&maps.aux, g.relu_z, 128, g.m, 256)) &&
+                        !(gather && (g.n != 128u || g.ld_add % 8u || reinterpret_cast<uintptr_t>(g.add1) % 16u ||
+                                     reinterpret_cast<uintptr_t>(g.add2) % 16u));
+    if (!shared) {
+        if (g.ln_gamma || g.relu_z) return WC_OK;
+        plan = TmaPlan{};
+        plan.stages = TMA_MAX_STAGES;
+        plan.smem = (nslices + TMA_MAX_STAGES) * TILE_BYTES;
+        *launched = true;
+        return launch_tma_as<AUX_DIRECT, false, false, false>(g, maps, plan, grid, err, s);
+    }
     plan.stages = std::min<uint32_t>(TMA_MAX_STAGES, (TMA_SMEM_LIMIT - fixed) / TILE_BYTES);
     plan.smem = fixed + plan.stages * TILE_BYTES;
     *launched = true;
