@@ -692,6 +692,22 @@ __device__ __forceinline__ void padded_row(const uint32_t* __restrict__ ptab, ui
     }
 }
 
+// Particles in the 27 cells around position p's.
+__device__ __forceinline__ uint32_t candidates(const uint32_t* __restrict__ tab, uint32_t n, const float4& p, float bin, int32_t R) {
+    int32_t cx, cy, cz;
+    bin_key(p.x, p.y, p.z, bin, R, &cx, &cy, &cz);
+    uint32_t total = 0;
+#pragma unroll 1
+    for (int r = 0; r < 9; ++r) {
+        const int yy = cy + (r % 3) - 1, zz = cz + (r / 3) - 1;
+        if (yy < 0 || yy >= R || zz < 0 || zz >= R) continue;
+        const uint32_t row = (uint32_t)((zz * R + yy) * R);
+        const uint32_t hi = min(__ldg(tab + row + (cx + 1 < R ? cx + 1 : R - 1) + 1), n);
+        total += hi - min(__ldg(tab + row + (cx > 0 ? cx - 1 : 0)), hi);
+    }
+    return total;
+}
+
 // The judge's pairs (FEAT_FULL): three blocks per SM, 78 registers without spills; two blocks, 96 registers, are
 // slower: 10 us per pass at 1,048,576 particles, 14 us at 200,000.
 template <bool BATCHED, int FEAT, int TARGETS>
@@ -866,6 +882,10 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
                 if (ti[t] >= n) continue;
                 const float4 v = FEAT == FEAT_FULL ? vi[t] : vel_in[ti[t]];
                 float pressure;
+                // a position that is not a number passes every test, also against the padding, which does not count
+                // (looked at where counts are wanted: in every target it costs 3 us of 125 at 1,048,576 particles)
+                if (ncount && (isnan(pi[t].x) || isnan(pi[t].y) || isnan(pi[t].z)))
+                    nh[t] = candidates(start + coff, n, pi[t], sc.bin, R);
                 const float rho_t = write_density(sc, acc[t], nh[t], pi[t], ti[t], rho_out, p_out, ncount, &pressure);
                 store_record(rec, pself + t, pi[t], __fdividef(1.0f, rho_t), v, pressure);
                 info[ti[t]] = make_uint2(ne[t] <= LANE_ENTRIES ? ne[t] : INFO_DENSE, pself + t);
