@@ -188,8 +188,8 @@ struct DevBuffers {
     uint32_t *keys, *ranks, *unordered, *perm;
     uint32_t *counts;     // [C] histogram (zero between steps)
     uint32_t *start;      // [C+1] exclusive prefix + total
-    uint32_t *cell_list;  // [C] non-empty cells, ascending
-    // [0]: non-empty cells (written by the scan); [1], [2]: the density and force passes' cell
+    uint32_t *cell_list;  // [C] non-empty cells (the team passes'), ascending from their scan
+    // [0]: non-empty cells (with the list); [1], [2]: the density and force passes' cell
     // counters (dynamic scheduling; each launch leaves its counter at zero)
     uint32_t *num_nonempty;
     unsigned long long* scan_desc;  // [num_tiles]
@@ -211,6 +211,9 @@ struct DevBuffers {
     uint32_t pcap;
     float4* accel;     // [n] acceleration of each particle in the last force pass, or null
     uint32_t* err;
+    // Host: whether cell_list belongs to the cell tables (the lane scan writes none; a team pass that
+    // follows it, in a stage call after a rollout, makes the list first).
+    mutable bool list_current;
 };
 
 // Neighbour pass variants (threads per cell): a 32-lane team per non-empty cell that splits the
@@ -246,6 +249,8 @@ void launch_bin_count(const DevBuffers& d, const SceneConsts& sc, const LaunchDi
 // lane: the tables of the lane passes (pstart, and the gather's padded arrays) instead of the team
 // passes' list of non-empty cells.
 void launch_scan_cells(const DevBuffers& d, cudaStream_t s, bool lane = false);
+// The list of non-empty cells from the cell tables, in any order (the cells of a team pass are independent).
+void launch_list_cells(const DevBuffers& d, cudaStream_t s);
 void launch_scatter(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s);
 // vxyz (optional, the learned rollout's judge steps): also the sorted velocities' x, y, z as three
 // arrays of d.pcap elements, in padded slots.

@@ -275,6 +275,17 @@ __global__ void __launch_bounds__(SCAN_THREADS, 5) scan_cells_kernel(uint32_t* _
     }
 }
 
+__global__ void __launch_bounds__(256) list_cells_kernel(uint32_t C, const uint32_t* __restrict__ start,
+                                                         uint32_t* __restrict__ list, uint32_t* __restrict__ count) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const bool some = c < C && start[c + 1] > start[c];
+    const uint32_t votes = __ballot_sync(0xffffffffu, some);
+    uint32_t at = 0;
+    if (lane == 0 && votes) at = atomicAdd(count, (uint32_t)__popc(votes));
+    at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(votes & ((1u << lane) - 1u));
+    if (some) list[at] = c;
+}
+
 // Tables are consistent unless a scan tile timed out (reported through DEVERR_SCAN_TIMEOUT);
 // the bounds checks below keep every access inside its buffer even then.
 __global__ void __launch_bounds__(256) scatter_cells_kernel(uint32_t n, const uint32_t* __restrict__ keys,
@@ -405,6 +416,7 @@ void launch_bin_count_batched(const DevBuffers& d, const BatchTables& bt, const 
 }
 
 void launch_scan_cells(const DevBuffers& d, cudaStream_t s, bool lane) {
+    d.list_current = !lane;
     if (lane)
         scan_cells_kernel<true><<<d.num_tiles, SCAN_THREADS, 0, s>>>(d.counts, d.num_cells, d.start, d.pstart,
                                                                      d.num_nonempty, d.scan_desc, d.scan_tile_counter,
@@ -413,6 +425,12 @@ void launch_scan_cells(const DevBuffers& d, cudaStream_t s, bool lane) {
         scan_cells_kernel<false><<<d.num_tiles, SCAN_THREADS, 0, s>>>(d.counts, d.num_cells, d.start, d.cell_list,
                                                                       d.num_nonempty, d.scan_desc, d.scan_tile_counter,
                                                                       d.num_tiles, d.err);
+}
+
+void launch_list_cells(const DevBuffers& d, cudaStream_t s) {
+    cudaMemsetAsync(d.num_nonempty, 0, sizeof(uint32_t), s);
+    list_cells_kernel<<<(d.num_cells + 255u) / 256u, 256, 0, s>>>(d.num_cells, d.start, d.cell_list, d.num_nonempty);
+    d.list_current = true;
 }
 
 void launch_scatter(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s) {

@@ -1601,6 +1601,7 @@ void launch_density_lane(const DevBuffers& d, const SceneConsts& sc, const Batch
 template <bool BATCHED>
 void launch_density_any(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
                         uint32_t* ncount, cudaStream_t s) {
+    if (ld.pass_variant != PASSES_LANE && !d.list_current) launch_list_cells(d, s);
     if (ld.pass_variant != PASSES_LANE)
         density_kernel<BATCHED><<<ld.grid_density, SPH_THREADS, 0, s>>>(
             sc, bt, d.n, d.num_cells, d.pos_b, reinterpret_cast<float*>(d.pos_b) + 3,
@@ -1636,6 +1637,7 @@ template <bool BATCHED, int FEAT>
 void launch_force_any(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const StepInputs& in,
                       const LaunchDims& ld, FeatureBuffers fb, cudaStream_t s) {
     const bool lane = FEAT != FEAT_NONE || ld.pass_variant == PASSES_LANE;
+    if (!lane && !d.list_current) launch_list_cells(d, s);
     int grid = ld.grid_force;
     if (FEAT != FEAT_NONE) {
         static int blocks = 0;

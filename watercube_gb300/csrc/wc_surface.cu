@@ -485,7 +485,6 @@ WC_API wc_status wc_surface_extract(wc_surface* s, wc_fluid* f, uint64_t* num_tr
     // sort the fluid's state (its cell tables then describe the sorted buffer), with the lane passes'
     // padded slots whatever its own pass variant
     WC_CUDA_TRY(cudaStreamSynchronize(s->stream));
-    if (fluid_target(f).ld.pass_variant != PASSES_LANE) fluid_enqueue_sort(f);
     fluid_enqueue_sort(f, PASSES_LANE);
     cudaEvent_t e0, e1, e2;
     cudaEventCreate(&e0);
