@@ -196,7 +196,7 @@ void apply_geometry(wc_batch* b, const wc_tuning& t) {
     const int variant = t.pass_variant == WC_PASSES_TEAM ? PASSES_TEAM : PASSES_LANE;
     if (variant != b->ld.pass_variant) {
         b->ld.pass_variant = variant;
-        sph_occupancy(true, &b->max_density_blocks, &b->max_force_blocks, variant, b->d.n);
+        sph_occupancy(true, &b->max_density_blocks, &b->max_force_blocks, variant, b->d.n, b->ld.sms);
     }
     b->tuning.pass_variant = (uint32_t)variant;
     b->ld.grid_density = b->ld.sms * (int)std::max(1u, std::min(t.density_blocks_per_sm, (uint32_t)b->max_density_blocks));
@@ -552,7 +552,7 @@ WC_API wc_status wc_batch_create(const wc_params* scenes, uint32_t num_scenes, w
     if (st == WC_OK) st = dalloc(&d.ids_a, n);
     if (st == WC_OK) st = dalloc(&d.ids_b, n);
     if (st == WC_OK) st = dalloc(&d.hits, hits_words(n));
-    d.pcap = padded_capacity(n, cells);
+    d.pcap = slot_capacity(n);
     if (st == WC_OK) st = dalloc(&d.xyz, 3 * (size_t)d.pcap);
     if (st == WC_OK) st = dalloc(&d.cidx, d.pcap);
     if (st == WC_OK) st = dalloc(&d.rec, 2 * (size_t)d.pcap);
@@ -585,7 +585,7 @@ WC_API wc_status wc_batch_create(const wc_params* scenes, uint32_t num_scenes, w
         // result bit for bit)
         const int variant = (b->base[0].flags & WC_FLAG_CELL_TEAMS) ? PASSES_TEAM : PASSES_LANE;
         b->ld = compute_launch_dims(b->device, variant, d.n);
-        sph_occupancy(true, &b->max_density_blocks, &b->max_force_blocks, variant, b->d.n);
+        sph_occupancy(true, &b->max_density_blocks, &b->max_force_blocks, variant, b->d.n, b->ld.sms);
         b->ld.grid_density = b->ld.sms * b->max_density_blocks;
         b->ld.grid_force = b->ld.sms * b->max_force_blocks;
         b->tuning = wc_tuning{(uint32_t)b->max_density_blocks, (uint32_t)b->max_force_blocks, 8u, 1.0f, 0.f, 0u,

@@ -103,7 +103,7 @@ wc_status allocate(wc_fluid* f) {
     WC_TRY(dalloc(&d.perm, n));
     if (f->params.flags & WC_FLAG_NEIGHBOR_COUNTS) WC_TRY(dalloc(&d.ncount, n));
     WC_TRY(dalloc(&d.hits, hits_words(n)));
-    d.pcap = padded_capacity(n, d.num_cells);
+    d.pcap = slot_capacity(n);
     WC_TRY(dalloc(&d.xyz, 3 * (size_t)d.pcap));
     WC_TRY(dalloc(&d.cidx, d.pcap));
     WC_TRY(dalloc(&d.rec, 2 * (size_t)d.pcap));

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "wc_lanes.h"
 #include "../../include/watercube.h"
 
 namespace wc {
@@ -166,17 +167,6 @@ constexpr uint32_t INFO_DENSE = 0xfffffffeu, INFO_OVERFULL = 0xffffffffu;
 // Words of DevBuffers::hits for n particles: whole chunks of 32.
 inline size_t hits_words(uint64_t n) { return (size_t)((n + 31u) & ~31ull) * MASK_WORDS; }
 
-// The padded slots of the lane passes: every cell's particles start at a multiple of 4 and the
-// places up to the next multiple hold PAD_POSITION in x, y and z, so that four consecutive slots
-// are one aligned 16-byte load per coordinate and never belong to two cells.
-// Far beyond any kernel radius, with a finite squared distance (a padding place contributes
-// 0 x finite = 0 to every sum, where an infinite one would contribute 0 x infinity).
-constexpr float PAD_POSITION = 3e18f;
-inline uint32_t padded_capacity(uint64_t n, uint64_t cells) {
-    const uint64_t c = n + 3u * (n < cells ? n : cells);
-    return (uint32_t)((c + 7u) & ~7ull) + 8u;
-}
-
 struct DevBuffers {
     uint32_t n;          // particles
     uint32_t num_cells;  // R^3
@@ -196,12 +186,12 @@ struct DevBuffers {
     uint32_t* scan_tile_counter;
     uint32_t* ncount;  // [n] or null
     uint32_t* hits;    // [n * MASK_WORDS] neighbours: bit strings (team passes) or entries (lane passes)
-    // The lane passes' padded slots (see padded_capacity), written by the lane variant's scan and
+    // The lane passes' slots (see slot_capacity), written by the lane variant's scan and
     // gather: pstart is the exclusive prefix of the cells' counts rounded up to 4 (+ total), xyz the
     // sorted positions' x, y, z as three arrays of pcap elements, cidx the sorted slot of a padded
-    // one (all ones: padding). rec: per padded slot (x, y, z, 1 / density) (v, pressure), 32 bytes
+    // one (all ones: padding). A total beyond pcap means packed slots. rec: per slot (x, y, z, 1 / density) (v, pressure), 32 bytes
     // written by the density pass and read by the force pass's neighbour gathers. info: per sorted
-    // slot (entries of its neighbour masks or INFO_*, its padded slot), from the density pass. Only
+    // slot (entries of its neighbour masks or INFO_*, its slot here), from the density pass. Only
     // pstart and info need a first value (zero: no candidates, no neighbours, nothing else read).
     uint32_t* pstart;  // [C+1]
     float* xyz;
@@ -236,7 +226,7 @@ LaunchDims compute_launch_dims(int device, int pass_variant = PASSES_LANE, uint3
 
 // The learned rollout's judge-step buffers of the force pass (sorted order): `out` receives
 // (J, density rate) per particle, `rate` holds the density pass's (density rate, pressure rate).
-// `rate` has one entry per padded slot; the density pass leaves the slot's own rates in out[ti].zw
+// `rate` has one entry per slot of the lane passes; the density pass leaves the slot's own rates in out[ti].zw
 // (pressure rate, density rate) until the force pass overwrites it.
 struct FeatureBuffers {
     float4* out;
@@ -253,7 +243,7 @@ void launch_scan_cells(const DevBuffers& d, cudaStream_t s, bool lane = false);
 void launch_list_cells(const DevBuffers& d, cudaStream_t s);
 void launch_scatter(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s);
 // vxyz (optional, the learned rollout's judge steps): also the sorted velocities' x, y, z as three
-// arrays of d.pcap elements, in padded slots.
+// arrays of d.pcap elements, in the lane passes' slots.
 void launch_rank_gather(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s, bool lane = false,
                         float* vxyz = nullptr);
 void launch_density(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, cudaStream_t s);
@@ -271,13 +261,20 @@ enum : int { FEAT_NONE = 0, FEAT_RATE = 1, FEAT_FULL = 2 };
 // The learned rollout's judge step runs the lane passes with their feature outputs, whatever
 // ld.pass_variant says: the density pass also writes the density and pressure rates (FeatureBuffers)
 // from the gather's velocity arrays vxyz and, when judge_part is given, the judge's sums
-// judge_part[m] = sum over the slots of chunk m (lane_chunks) of |rho_carried / rho_SPH - 1| (rho_carried:
-// the sorted buffer's .w before the pass); the force pass reads the neighbours' rates and writes
+// judge_part[m] = sum over the slots of chunk m of |rho_carried / rho_SPH - 1| (rho_carried:
+// the sorted buffer's .w before the pass; *judge_chunks of them, at most one per 32 particles); the force pass reads the neighbours' rates and writes
 // feat[ti] = (J, density rate), J the time derivative of the SPH acceleration (sorted order).
+struct FeatureInputs {
+    const float* vxyz = nullptr;
+    float2* rate = nullptr;
+    float4* feat = nullptr;
+    float* judge_part = nullptr;
+    uint32_t* judge_chunks = nullptr;
+};
 void launch_density_feat(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, int level,
-                         const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s);
+                         const FeatureInputs& fi, cudaStream_t s);
 void launch_density_batched_feat(const DevBuffers& d, const BatchTables& bt, const LaunchDims& ld, int level,
-                                 const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s);
+                                 const FeatureInputs& fi, cudaStream_t s);
 void launch_force_feat(const DevBuffers& d, const SceneConsts& sc, const StepInputs& in, const LaunchDims& ld,
                        int level, FeatureBuffers fb, cudaStream_t s);
 void launch_force_batched_feat(const DevBuffers& d, const BatchTables& bt, const StepInputs& in, const LaunchDims& ld,
@@ -323,23 +320,7 @@ void launch_density_batched(const DevBuffers& d, const BatchTables& bt, const La
 void launch_force_batched(const DevBuffers& d, const BatchTables& bt, const StepInputs& in, const LaunchDims& ld,
                           cudaStream_t s);
 
-// Targets per lane of the lane density pass over n particles: one, or the two of a pair of padded
-// slots, which share every candidate load and loop step (with ~1.2 padded slots per particle a
-// warp of pairs covers 1.65 times the targets in 1.5 times the time). Pairs halve the warps, so
-// the choice is by waves of the 152 x 32 resident ones, a last partial wave counted as half a
-// wave. Measured per step: 100,000 particles 94 us with one, 97 with pairs; 200,000 121 and 109;
-// 400,000 156 and 165; 1,048,576 (the pass alone) 138 and 125.
-inline uint32_t lane_targets(uint32_t n) {
-    const double resident = 152.0 * 32.0, one = n / (32.0 * resident), pairs = 1.2 * n / (64.0 * resident);
-    auto waves = [](double w) { return w <= 1.0 ? 1.0 : w + 0.5; };
-    return 1.5 * waves(pairs) < waves(one) ? 2u : 1u;
-}
-// Chunks of 32 lanes of that pass, at most (the judge's partial sums are per chunk).
-inline uint32_t lane_chunks(uint32_t n, uint32_t pcap) {
-    return lane_targets(n) == 2u ? (pcap + 63u) / 64u : (n + 31u) / 32u;
-}
-
-// What the lane force pass reads of the padded slots (DevBuffers).
+// What the lane force pass reads of the slots (DevBuffers).
 struct LaneTables {
     const float4* rec;
     const uint2* info;
@@ -384,7 +365,7 @@ struct ForceKernelArgs {
 const void* force_kernel_symbol(int pass_variant);
 const void* force_kernel_batched_symbol(int pass_variant);
 // Resident blocks per SM of the two neighbour passes (single-scene or batched variant).
-void sph_occupancy(bool batched, int* density_blocks, int* force_blocks, int pass_variant, uint32_t n);
+void sph_occupancy(bool batched, int* density_blocks, int* force_blocks, int pass_variant, uint32_t n, int sms);
 
 // Internals of a wc_fluid, for the surrogate (wc_surrogate.cu), which works on a fluid's buffers.
 struct FluidInternals {

@@ -583,17 +583,10 @@ __global__ void __launch_bounds__(32 * OUT) output_mean_kernel(uint32_t ctas, ui
 // kernel adds the chunk sums in a fixed order, FP32 per thread and warp (a relative
 // rounding of order 1e-6 against a tolerance of order 1e-2), FP64 across the warps.
 constexpr uint32_t JUDGE_THREADS = 1024;
-// padded: with two targets per lane, the number of padded slots (device memory), 64 to a chunk.
-struct JudgeChunks {
-    uint32_t chunks;
-    const uint32_t* padded;
-};
-JudgeChunks judge_chunks(const DevBuffers& d) {
-    return JudgeChunks{lane_chunks(d.n, d.pcap), lane_targets(d.n) == 2u ? d.pstart + d.num_cells : nullptr};
-}
-__global__ void __launch_bounds__(JUDGE_THREADS) judge_final_kernel(const JudgeChunks jc, const float* __restrict__ part,
-                                                                    double* __restrict__ out) {
-    const uint32_t chunks = jc.padded ? min(jc.chunks, (*jc.padded + 63u) / 64u) : jc.chunks;
+// num_chunks: how many (device memory, from the density pass).
+__global__ void __launch_bounds__(JUDGE_THREADS) judge_final_kernel(const uint32_t* __restrict__ num_chunks,
+                                                                    const float* __restrict__ part, double* __restrict__ out) {
+    const uint32_t chunks = *num_chunks;
     __shared__ float s[JUDGE_THREADS / 32];
     float a = 0.f;
     for (uint32_t b = threadIdx.x; b < chunks; b += JUDGE_THREADS) a += part[b];
@@ -798,7 +791,8 @@ struct wc_local {
     float* vxyz = nullptr;  // judge steps: the gather's sorted velocities (x, y, z arrays)
     float4 *save_pos[2] = {nullptr, nullptr}, *save_vel[2] = {nullptr, nullptr};
     uint32_t* save_ids[2] = {nullptr, nullptr};
-    float* judge_part = nullptr;  // per chunk of the density pass (lane_chunks)
+    float* judge_part = nullptr;  // per chunk of the density pass
+    uint32_t* judge_chunks = nullptr;  // their number
     double *judge_out = nullptr, *h_judge = nullptr;
     uint32_t cap_roll = 0;
 };
@@ -843,6 +837,7 @@ void free_local(wc_local* s) {
     dfree(s->vxyz);
     dfree(s->judge_part);
     dfree(s->judge_out);
+    dfree(s->judge_chunks);
     if (s->h_err) cudaFreeHost(s->h_err);
     if (s->h_judge) cudaFreeHost(s->h_judge);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -926,11 +921,12 @@ void enqueue_closing_judge(wc_local* s, const StepTarget& t) {
     launch_scan_cells(d, t.stream, true);
     launch_scatter(d, t.ld, t.stream);
     launch_rank_gather(d, t.ld, t.stream, true);
+    const FeatureInputs fi{nullptr, nullptr, nullptr, s->judge_part, s->judge_chunks};
     if (t.bt.num_scenes)
-        launch_density_batched_feat(d, t.bt, t.ld, FEAT_RATE, nullptr, nullptr, nullptr, s->judge_part, t.stream);
+        launch_density_batched_feat(d, t.bt, t.ld, FEAT_RATE, fi, t.stream);
     else
-        launch_density_feat(d, t.sc, t.ld, FEAT_RATE, nullptr, nullptr, nullptr, s->judge_part, t.stream);
-    judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(judge_chunks(d), s->judge_part, s->judge_out);
+        launch_density_feat(d, t.sc, t.ld, FEAT_RATE, fi, t.stream);
+    judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(s->judge_chunks, s->judge_part, s->judge_out);
 }
 
 // The judge step, on the target's stream: a plain SPH step whose force pass also writes s->feat
@@ -953,14 +949,15 @@ void enqueue_judge_step(wc_local* s, const StepTarget& t, float dt, bool judge, 
     launch_rank_gather(d, t.ld, t.stream, true, full ? s->vxyz : nullptr);
     const FeatureBuffers fb{s->feat, s->rate};
     float* jp = judge && d.n ? s->judge_part : nullptr;
+    const FeatureInputs fi{s->vxyz, s->rate, s->feat, jp, jp ? s->judge_chunks : nullptr};
     if (t.bt.num_scenes) {
-        launch_density_batched_feat(d, t.bt, t.ld, level, s->vxyz, s->rate, s->feat, jp, t.stream);
+        launch_density_batched_feat(d, t.bt, t.ld, level, fi, t.stream);
         launch_force_batched_feat(d, t.bt, in, t.ld, level, fb, t.stream);
     } else {
-        launch_density_feat(d, t.sc, t.ld, level, s->vxyz, s->rate, s->feat, jp, t.stream);
+        launch_density_feat(d, t.sc, t.ld, level, fi, t.stream);
         launch_force_feat(d, t.sc, in, t.ld, level, fb, t.stream);
     }
-    if (jp) judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(judge_chunks(d), jp, s->judge_out);
+    if (jp) judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(s->judge_chunks, jp, s->judge_out);
 }
 
 wc_status plain_step(const StepTarget& t, float dt) {
@@ -1280,6 +1277,7 @@ WC_API wc_status wc_local_create(const wc_local_config* c, wc_local** out) {
     if (st == WC_OK && cudaMallocHost(reinterpret_cast<void**>(&s->h_judge), sizeof(double)) != cudaSuccess)
         st = fail(WC_ERR_OOM, "pinned host allocation failed");
     if (st == WC_OK) st = dalloc(&s->judge_out, 1);
+    if (st == WC_OK) st = dalloc(&s->judge_chunks, 1);
     if (st == WC_OK) {
         std::vector<float> host;
         init_params(s, host);

@@ -303,9 +303,9 @@ __global__ void __launch_bounds__(256) scatter_cells_kernel(uint32_t n, const ui
 // its members in arrival order instead: the stable rank costs O(k) per member, O(k^2) per cell,
 // and an all-NaN state puts every particle in cell 0. Arrival ranks are unique in the cell, so
 // the permutation stays a permutation; the step reports the cell through DEVERR_CELL_OVERFLOW.
-// LANE: also the lane passes' padded slots (positions, slot index, and velocities with vxyz); the
+// LANE: also the lane passes' slots (positions, slot index, and velocities with vxyz). Padded: the
 // cell's last particle writes the places up to the next multiple of 4: a position far away, whose
-// distance never passes the neighbour test.
+// distance never passes the neighbour test. Packed (pstart's total beyond pcap): the sorted slots.
 template <bool IDS, bool VEL, bool LANE>
 __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint32_t* __restrict__ keys,
                                                           const uint32_t* __restrict__ ranks,
@@ -317,9 +317,10 @@ __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint
                                                           float4* __restrict__ pos_out, float4* __restrict__ vel_out,
                                                           uint32_t* __restrict__ ids_out, uint32_t* __restrict__ perm,
                                                           uint32_t* __restrict__ err,
-                                                          const uint32_t* __restrict__ pstart,
+                                                          uint32_t num_cells, const uint32_t* __restrict__ pstart,
                                                           uint32_t* __restrict__ cidx, float* __restrict__ xyz,
                                                           uint32_t pcap, float* __restrict__ vxyz) {
+    const bool packed = LANE && __ldg(pstart + num_cells) > pcap;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t key = keys[i];
         const uint32_t s = start[key], e = min(start[key + 1], n);
@@ -336,10 +337,10 @@ __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint
         const float4 p = pos_in[i];
         pos_out[dst] = p;
         if (LANE) {
-            const uint32_t pd = pstart[key] + r;
-            const uint32_t last = s + r + 1u == e ? ((r + 4u) & ~3u) - r : 1u;  // places this thread writes
+            const uint32_t pd = packed ? dst : pstart[key] + r;
+            const uint32_t last = !packed && s + r + 1u == e ? ((r + 4u) & ~3u) - r : 1u;  // places this thread writes
             if (pd + last <= pcap) {
-                cidx[pd] = dst;
+                if (!packed) cidx[pd] = dst;
                 xyz[pd] = p.x;
                 xyz[pcap + pd] = p.y;
                 xyz[2 * (size_t)pcap + pd] = p.z;
@@ -440,7 +441,8 @@ void launch_scatter(const DevBuffers& d, const LaunchDims& ld, cudaStream_t s) {
 template <bool IDS, bool VEL, bool LANE>
 static void launch_gather(const DevBuffers& d, int grid, cudaStream_t s, float* vxyz) {
     rank_gather_kernel<IDS, VEL, LANE><<<grid, 256, 0, s>>>(d.n, d.keys, d.ranks, d.unordered, d.start, d.pos_a, d.vel_a,
-                                                            d.ids_a, d.pos_b, d.vel_b, d.ids_b, d.perm, d.err, d.pstart,
+                                                            d.ids_a, d.pos_b, d.vel_b, d.ids_b, d.perm, d.err, d.num_cells,
+                                                            d.pstart,
                                                             d.cidx, d.xyz, d.pcap, vxyz);
 }
 

@@ -38,6 +38,8 @@
 // the same fused operations per element, so it agrees bit for bit.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "wc_internal.h"
 
 namespace wc {
@@ -629,7 +631,9 @@ __global__ void __launch_bounds__(SPH_THREADS, 5) density_kernel(const SceneCons
 // the 9 row ranges of the cell's 27 neighbour cells in padded slots, four candidates per 16-byte
 // load and coordinate; every cell starts at a multiple of 4 and its padding lies far away, so
 // no place needs a mask, and the sums do not depend on where a cell lies (a scene of a batch sees
-// the same sums as the scene alone, and a pair of targets the same as one).
+// the same sums as the scene alone, and a pair of targets the same as one). PACKED: where the padding would take
+// more slots than there are (DevBuffers::pcap), the slots are the sorted ones and the places of a quad outside the row
+// are masked, with the same sums and neighbours.
 // Per block of up to 32 candidates of a row, the misses' sign bits form a word, one funnel shift per
 // candidate; a block with hits other than the target itself becomes an entry (first candidate,
 // mask with candidate j at bit 31 - j) for the force pass.
@@ -679,62 +683,52 @@ __device__ __forceinline__ void store_record(float4* rec, uint32_t pslot, const 
 // Slot ti's entry 0; its entry e lies 32 e further.
 __device__ __forceinline__ size_t entry_index(uint32_t ti) { return (size_t)(ti >> 5) * (LANE_ENTRIES * 32u) + (ti & 31u); }
 
-// Row r = (dy, dz) = (r % 3 - 1, r / 3 - 1) of cell (cx, cy, cz): the padded slots [lo, hi) of its three
-// cells. A timed-out scan (reported) leaves inconsistent tables; the range stays in the buffers.
-__device__ __forceinline__ void padded_row(const uint32_t* __restrict__ ptab, uint32_t pcap, int32_t R, int cx, int cy,
-                                           int cz, int r, uint32_t& lo, uint32_t& hi) {
+// Row r = (dy, dz) = (r % 3 - 1, r / 3 - 1) of cell (cx, cy, cz): the slots [lo, hi) of its three cells, below
+// `limit`, from the cells' starts in the layout. A timed-out scan (reported) leaves inconsistent tables; the
+// range stays in the buffers.
+template <bool PACKED>
+__device__ __forceinline__ void slot_row(const uint32_t* __restrict__ tab, uint32_t limit, int32_t R, int cx, int cy,
+                                         int cz, int r, uint32_t& lo, uint32_t& hi) {
+    constexpr uint32_t whole = PACKED ? ~0u : ~3u;
     const int yy = cy + (r % 3) - 1, zz = cz + (r / 3) - 1;
     lo = hi = 0;
     if (yy >= 0 && yy < R && zz >= 0 && zz < R) {
         const uint32_t row = (uint32_t)((zz * R + yy) * R);
-        hi = min(__ldg(ptab + row + (cx + 1 < R ? cx + 1 : R - 1) + 1), pcap) & ~3u;
-        lo = min(__ldg(ptab + row + (cx > 0 ? cx - 1 : 0)) & ~3u, hi);
+        hi = min(__ldg(tab + row + (cx + 1 < R ? cx + 1 : R - 1) + 1), limit) & whole;
+        lo = min(__ldg(tab + row + (cx > 0 ? cx - 1 : 0)) & whole, hi);
     }
 }
 
 // Particles in the 27 cells around position p's.
-__device__ __forceinline__ uint32_t candidates(const uint32_t* __restrict__ tab, uint32_t n, const float4& p, float bin, int32_t R) {
+// (Not inlined: it is rarely called, and in line it costs every pass of pairs 2 %.)
+__device__ __noinline__ uint32_t candidates(const uint32_t* tab, uint32_t n, float4 p, float bin, int32_t R) {
     int32_t cx, cy, cz;
     bin_key(p.x, p.y, p.z, bin, R, &cx, &cy, &cz);
-    uint32_t total = 0;
+    uint32_t total = 0, lo, hi;
 #pragma unroll 1
     for (int r = 0; r < 9; ++r) {
-        const int yy = cy + (r % 3) - 1, zz = cz + (r / 3) - 1;
-        if (yy < 0 || yy >= R || zz < 0 || zz >= R) continue;
-        const uint32_t row = (uint32_t)((zz * R + yy) * R);
-        const uint32_t hi = min(__ldg(tab + row + (cx + 1 < R ? cx + 1 : R - 1) + 1), n);
-        total += hi - min(__ldg(tab + row + (cx > 0 ? cx - 1 : 0)), hi);
+        slot_row<true>(tab, n, R, cx, cy, cz, r, lo, hi);
+        total += hi - lo;
     }
     return total;
 }
 
-// The judge's pairs (FEAT_FULL): three blocks per SM, 78 registers without spills; two blocks, 96 registers, are
-// slower: 10 us per pass at 1,048,576 particles, 14 us at 200,000.
-template <bool BATCHED, int FEAT, int TARGETS>
-__global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL ? 3 : 4) density_lane_kernel(
-    const SceneConsts sc0, const BatchTables bt, const uint32_t n, const uint32_t num_cells,
-    const float4* pos_in,  // its .w lanes are the density output: read with coherent loads
-    const float4* vel_in,  // its .w lanes are the pressure output
-    float* rho_out, float* p_out, const uint32_t* __restrict__ start, const uint32_t* __restrict__ pstart,
-    const uint32_t* __restrict__ cidx, uint32_t* __restrict__ counter, uint32_t* __restrict__ ncount,
-    uint2* __restrict__ entries, uint2* __restrict__ info, uint32_t* __restrict__ err, const float* __restrict__ xyz,
-    const uint32_t pcap, float4* __restrict__ rec, const float* __restrict__ vxyz = nullptr,
-    float2* __restrict__ rate_out = nullptr, float4* __restrict__ feat = nullptr, float* __restrict__ judge_part = nullptr) {
-    __shared__ uint32_t s_poff[BATCHED ? MAX_SCENES + 1 : 1];
-    __shared__ uint32_t s_coff[BATCHED ? MAX_SCENES + 1 : 1];
-    if (BATCHED) {
-        for (uint32_t t = threadIdx.x; t <= bt.num_scenes; t += blockDim.x) {
-            s_poff[t] = bt.poff[t];
-            s_coff[t] = bt.coff[t];
-        }
-        __syncthreads();
-    }
+// A pass over all targets in one of its layouts: PACKED (one target per lane) or padded slots (one or a pair).
+template <bool BATCHED, int FEAT, int TARGETS, bool PACKED>
+__device__ __forceinline__ void density_walk(
+    const SceneConsts& sc0, const BatchTables& bt, const uint32_t* s_poff, const uint32_t* s_coff, const uint32_t n,
+    const uint32_t padded, const float4* pos_in, const float4* vel_in, float* rho_out, float* p_out,
+    const uint32_t* __restrict__ start, const uint32_t* __restrict__ pstart, const uint32_t* __restrict__ cidx,
+    uint32_t* __restrict__ counter, uint32_t* __restrict__ ncount, uint2* __restrict__ entries, uint2* __restrict__ info,
+    uint32_t* __restrict__ err, const float* __restrict__ xyz, const uint32_t pcap, float4* __restrict__ rec,
+    const float* __restrict__ vxyz, float2* __restrict__ rate_out, float4* __restrict__ feat,
+    float* __restrict__ judge_part, uint32_t* __restrict__ judge_chunks) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t padded = TARGETS == 2 ? min(__ldg(pstart + num_cells), pcap) : 0u;
     const uint32_t M = TARGETS == 2 ? (padded + 63u) >> 6 : (n + 31u) >> 5;
     const float* const X = xyz;
     const float* const Y = xyz + pcap;
     const float* const Z = xyz + 2 * (size_t)pcap;
+    if (FEAT && judge_chunks && blockIdx.x == 0 && threadIdx.x == 0) *judge_chunks = M;
     LaneChunks chunks(counter, M, lane);
     for (uint32_t m = chunks.first(); m < M; m = chunks.next()) {
         chunks.prefetch();
@@ -763,12 +757,14 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
             int32_t cx, cy, cz;
             const int32_t R = sc.R;
             const uint32_t c = bin_key(pi[0].x, pi[0].y, pi[0].z, sc.bin, R, &cx, &cy, &cz);
-            const uint32_t* const ptab = pstart + coff;
+            const uint32_t* const ptab = (PACKED ? start : pstart) + coff;
             const uint32_t cend = min(__ldg(start + coff + c + 1), n);
             const uint32_t cbeg = min(__ldg(start + coff + c), cend);
             // the lane's first padded slot (a slot outside its cell's range, which only a caller
             // who overwrote the sorted buffer leaves, is clamped into the buffers)
-            const uint32_t pself = TARGETS == 2 ? (m << 6) + 2u * lane : min(__ldg(ptab + c) + (ti[0] - cbeg), pcap - 1u);
+            const uint32_t pself = PACKED         ? ti[0]
+                                   : TARGETS == 2 ? (m << 6) + 2u * lane
+                                                  : min(__ldg(ptab + c) + (ti[0] - cbeg), pcap - 1u);
             if (cend - cbeg > MAX_CELL_PARTICLES) {
                 // not evaluated (see MAX_CELL_PARTICLES): NaN density and pressure, reported
                 const float nan = __int_as_float(0x7fc00000);
@@ -807,14 +803,15 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
                 if (FEAT == FEAT_FULL) vi[t] = vel_in[ti[t] < n ? ti[t] : ti[0]];
             }
             uint32_t lo, hi;
-            padded_row(ptab, pcap, R, cx, cy, cz, 0, lo, hi);
+            slot_row<PACKED>(ptab, PACKED ? n : pcap, R, cx, cy, cz, 0, lo, hi);
 #pragma unroll 1
             for (int r = 0; r < 9; ++r) {
-                uint32_t k = lo;
-                const uint32_t end = hi;
-                if (r < 8) padded_row(ptab, pcap, R, cx, cy, cz, r + 1, lo, hi);  // overlaps this row's tests
+                const uint32_t first = lo, end = hi;
+                uint32_t k = PACKED ? first & ~3u : first;
+                // overlaps this row's tests
+                if (r < 8) slot_row<PACKED>(ptab, PACKED ? n : pcap, R, cx, cy, cz, r + 1, lo, hi);
                 while (k < end) {
-                    const uint32_t base = k, stop = min(k + 32u, end);
+                    const uint32_t base = k, stop = min(k + 32u, PACKED ? (end + 3u) & ~3u : end);
                     uint32_t word[TARGETS];
 #pragma unroll
                     for (int t = 0; t < TARGETS; ++t) word[t] = 0u;
@@ -842,6 +839,13 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
                             float w0, w1, w2, w3;
                             upk(sub2(cull2, d01), w0, w1);
                             upk(sub2(cull2, d23), w2, w3);
+                            if (PACKED) {  // places outside the row are misses
+                                const uint32_t at0 = k - first, len = end - first;
+                                w0 = at0 < len ? w0 : -1.f;
+                                w1 = at0 + 1u < len ? w1 : -1.f;
+                                w2 = at0 + 2u < len ? w2 : -1.f;
+                                w3 = at0 + 3u < len ? w3 : -1.f;
+                            }
                             word[t] = __funnelshift_l(__float_as_uint(w0), word[t], 1);
                             word[t] = __funnelshift_l(__float_as_uint(w1), word[t], 1);
                             word[t] = __funnelshift_l(__float_as_uint(w2), word[t], 1);
@@ -859,6 +863,13 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
                                 float r0, r1, r2, r3;
                                 upk(ru01, r0, r1);
                                 upk(ru23, r2, r3);
+                                if (PACKED) {
+                                    const uint32_t at0 = k - first, len = end - first;
+                                    r0 = at0 < len ? r0 : 0.f;
+                                    r1 = at0 + 1u < len ? r1 : 0.f;
+                                    r2 = at0 + 2u < len ? r2 : 0.f;
+                                    r3 = at0 + 3u < len ? r3 : 0.f;
+                                }
                                 rr[t] = fmaf(q3, r3, fmaf(q2, r2, fmaf(q1, r1, fmaf(q0, r0, rr[t]))));
                             }
                         }
@@ -883,8 +894,8 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
                 const float4 v = FEAT == FEAT_FULL ? vi[t] : vel_in[ti[t]];
                 float pressure;
                 // a position that is not a number passes every test, also against the padding, which does not count
-                // (looked at where counts are wanted: in every target it costs 3 us of 125 at 1,048,576 particles)
-                if (ncount && (isnan(pi[t].x) || isnan(pi[t].y) || isnan(pi[t].z)))
+                // (looked at where counts are wanted; the judge's passes, which the call would cost 5 %: count_nan_kernel)
+                if (!PACKED && !FEAT && ncount && (isnan(pi[t].x) || isnan(pi[t].y) || isnan(pi[t].z)))
                     nh[t] = candidates(start + coff, n, pi[t], sc.bin, R);
                 const float rho_t = write_density(sc, acc[t], nh[t], pi[t], ti[t], rho_out, p_out, ncount, &pressure);
                 store_record(rec, pself + t, pi[t], __fdividef(1.0f, rho_t), v, pressure);
@@ -906,6 +917,55 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
             for (int off = 16; off > 0; off >>= 1) judge += __shfl_xor_sync(FULL, judge, off);
             if (lane == 0) judge_part[m] = judge;
         }
+    }
+}
+
+// The judge's pairs (FEAT_FULL): three blocks per SM, 78 registers without spills; two blocks, 96 registers, are
+// slower: 10 us per pass at 1,048,576 particles, 14 us at 200,000.
+template <bool BATCHED, int FEAT, int TARGETS>
+__global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL ? 3 : 4) density_lane_kernel(
+    const SceneConsts sc0, const BatchTables bt, const uint32_t n, const uint32_t num_cells,
+    const float4* pos_in,  // its .w lanes are the density output: read with coherent loads
+    const float4* vel_in,  // its .w lanes are the pressure output
+    float* rho_out, float* p_out, const uint32_t* __restrict__ start, const uint32_t* __restrict__ pstart,
+    const uint32_t* __restrict__ cidx, uint32_t* __restrict__ counter, uint32_t* __restrict__ ncount,
+    uint2* __restrict__ entries, uint2* __restrict__ info, uint32_t* __restrict__ err, const float* __restrict__ xyz,
+    const uint32_t pcap, float4* __restrict__ rec, const float* __restrict__ vxyz = nullptr,
+    float2* __restrict__ rate_out = nullptr, float4* __restrict__ feat = nullptr, float* __restrict__ judge_part = nullptr,
+    uint32_t* __restrict__ judge_chunks = nullptr) {
+    __shared__ uint32_t s_poff[BATCHED ? MAX_SCENES + 1 : 1];
+    __shared__ uint32_t s_coff[BATCHED ? MAX_SCENES + 1 : 1];
+    if (BATCHED) {
+        for (uint32_t t = threadIdx.x; t <= bt.num_scenes; t += blockDim.x) {
+            s_poff[t] = bt.poff[t];
+            s_coff[t] = bt.coff[t];
+        }
+        __syncthreads();
+    }
+    const uint32_t padded = __ldg(pstart + num_cells);
+    if (padded > pcap)
+        density_walk<BATCHED, FEAT, 1, true>(sc0, bt, s_poff, s_coff, n, padded, pos_in, vel_in, rho_out, p_out, start, pstart,
+                                             cidx, counter, ncount, entries, info, err, xyz, pcap, rec, vxyz, rate_out, feat,
+                                             judge_part, judge_chunks);
+    else
+        density_walk<BATCHED, FEAT, TARGETS, false>(sc0, bt, s_poff, s_coff, n, padded, pos_in, vel_in, rho_out, p_out, start,
+                                                    pstart, cidx, counter, ncount, entries, info, err, xyz, pcap, rec, vxyz,
+                                                    rate_out, feat, judge_part, judge_chunks);
+}
+
+// The neighbour counts of particles at NaN after a judge's density pass (see density_walk).
+template <bool BATCHED>
+__global__ void __launch_bounds__(256) count_nan_kernel(const SceneConsts sc0, const BatchTables bt, uint32_t n, const float4* __restrict__ pos,
+                                                        const uint32_t* __restrict__ start, uint32_t* __restrict__ ncount) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 p = pos[i];
+        if (!isnan(p.x) && !isnan(p.y) && !isnan(p.z)) continue;
+        const uint32_t s = BATCHED ? find_scene(bt.poff, bt.num_scenes, i) : 0u;
+        const SceneConsts& sc = BATCHED ? bt.scenes[s] : sc0;
+        const uint32_t* const tab = start + (BATCHED ? bt.coff[s] : 0u);
+        int32_t cx, cy, cz;
+        const uint32_t c = bin_key(p.x, p.y, p.z, sc.bin, sc.R, &cx, &cy, &cz);
+        if (tab[c + 1] - tab[c] <= MAX_CELL_PARTICLES) ncount[i] = candidates(tab, n, p, sc.bin, sc.R) - 1u;
     }
 }
 
@@ -1434,9 +1494,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 3) force_lane_kernel(
         for (uint32_t t = threadIdx.x; t <= bt.num_scenes; t += blockDim.x) s_poff[t] = bt.poff[t];
         __syncthreads();
     }
-    (void)start;
     (void)cell_list;
-    (void)num_cells;
     const uint2* const entries = reinterpret_cast<const uint2*>(hits);
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t* const list = s_list[threadIdx.x >> 5] + lane;
@@ -1484,7 +1542,26 @@ __global__ void __launch_bounds__(SPH_THREADS, 3) force_lane_kernel(
             take(cur.x, cur.y);
         }
         const bool dense = live && info.x == INFO_DENSE;
-        if (__any_sync(FULL, dense)) {
+        if (__any_sync(FULL, dense) && __ldg(lt.pstart + num_cells) > lt.pcap) {
+            // packed slots (dilute states, where such targets are rare): one candidate at a time
+            const uint32_t* const tab = start + (BATCHED ? __ldg(bt.coff + s) : 0u);
+            int32_t cx, cy, cz;
+            bin_key(pi.x, pi.y, pi.z, sc.bin, sc.R, &cx, &cy, &cz);
+#pragma unroll 1
+            for (int r = 0; r < 9; ++r) {
+                uint32_t lo = 0, hi = 0;
+                if (dense) slot_row<true>(tab, n, sc.R, cx, cy, cz, r, lo, hi);
+#pragma unroll 1
+                for (; __any_sync(FULL, lo < hi); ++lo) {
+                    uint32_t mask = 0;
+                    if (lo < hi && lo != self) {
+                        const float4 pj = __ldg(pos_b + lo);
+                        mask = dist2(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z) > cull ? 0u : 0x80000000u;
+                    }
+                    take(lo, mask);
+                }
+            }
+        } else if (__any_sync(FULL, dense)) {
             const uint32_t coff = BATCHED ? __ldg(bt.coff + s) : 0u;
             int32_t cx, cy, cz;
             bin_key(pi.x, pi.y, pi.z, sc.bin, sc.R, &cx, &cy, &cz);
@@ -1492,7 +1569,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 3) force_lane_kernel(
 #pragma unroll 1
             for (int r = 0; r < 9; ++r) {
                 uint32_t lo = 0, hi = 0;
-                if (dense) padded_row(lt.pstart + coff, lt.pcap, sc.R, cx, cy, cz, r, lo, hi);
+                if (dense) slot_row<false>(lt.pstart + coff, lt.pcap, sc.R, cx, cy, cz, r, lo, hi);
                 const uint32_t blocks = __reduce_max_sync(FULL, (hi - lo + 31u) >> 5);
 #pragma unroll 1
                 for (uint32_t b = 0; b < blocks; ++b, lo += 32u) {
@@ -1554,10 +1631,13 @@ static_assert(arity(&force_lane_kernel<true, FEAT_NONE>) == ForceKernelArgs::COU
 
 }  // namespace
 
+// Resident warps of the density pass with pairs of targets: four blocks per SM.
+static uint32_t resident_warps(int sms) { return (uint32_t)sms * 4u * (uint32_t)WARPS; }
+
 template <bool BATCHED>
-static void occupancy(int* bd, int* bf, int pass_variant, uint32_t n) {
+static void occupancy(int* bd, int* bf, int pass_variant, uint32_t n, int sms) {
     if (pass_variant == PASSES_LANE) {
-        if (lane_targets(n) == 2u)
+        if (lane_pairs(n, resident_warps(sms)))
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(bd, density_lane_kernel<BATCHED, FEAT_NONE, 2>, SPH_THREADS, 0);
         else
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(bd, density_lane_kernel<BATCHED, FEAT_NONE, 1>, SPH_THREADS, 0);
@@ -1568,10 +1648,10 @@ static void occupancy(int* bd, int* bf, int pass_variant, uint32_t n) {
     }
 }
 
-void sph_occupancy(bool batched, int* density_blocks, int* force_blocks, int pass_variant, uint32_t n) {
+void sph_occupancy(bool batched, int* density_blocks, int* force_blocks, int pass_variant, uint32_t n, int sms) {
     int bd = 0, bf = 0;
-    if (batched) occupancy<true>(&bd, &bf, pass_variant, n);
-    else occupancy<false>(&bd, &bf, pass_variant, n);
+    if (batched) occupancy<true>(&bd, &bf, pass_variant, n, sms);
+    else occupancy<false>(&bd, &bf, pass_variant, n, sms);
     *density_blocks = bd > 0 ? bd : 1;
     *force_blocks = bf > 0 ? bf : 1;
 }
@@ -1581,7 +1661,7 @@ LaunchDims compute_launch_dims(int device, int pass_variant, uint32_t n) {
     cudaDeviceGetAttribute(&ld.sms, cudaDevAttrMultiProcessorCount, device);
     if (ld.sms <= 0) ld.sms = 1;
     int bd = 1, bf = 1;
-    sph_occupancy(false, &bd, &bf, pass_variant, n);
+    sph_occupancy(false, &bd, &bf, pass_variant, n, ld.sms);
     ld.grid_density = ld.sms * bd;
     ld.grid_force = ld.sms * bf;
     ld.grid_stream = ld.sms * 8;
@@ -1592,11 +1672,12 @@ LaunchDims compute_launch_dims(int device, int pass_variant, uint32_t n) {
 namespace {
 template <bool BATCHED, int FEAT, int TARGETS>
 void launch_density_lane(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, int grid, uint32_t* ncount,
-                         const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
+                         const FeatureInputs& fi, cudaStream_t s) {
     density_lane_kernel<BATCHED, FEAT, TARGETS><<<grid, SPH_THREADS, 0, s>>>(
         sc, bt, d.n, d.num_cells, d.pos_b, d.vel_b, reinterpret_cast<float*>(d.pos_b) + 3,
         reinterpret_cast<float*>(d.vel_b) + 3, d.start, d.pstart, d.cidx, d.num_nonempty + 1, ncount,
-        reinterpret_cast<uint2*>(d.hits), d.info, d.err, d.xyz, d.pcap, d.rec, vxyz, rate, feat, judge_part);
+        reinterpret_cast<uint2*>(d.hits), d.info, d.err, d.xyz, d.pcap, d.rec, fi.vxyz, fi.rate, fi.feat,
+        fi.judge_part, fi.judge_chunks);
 }
 template <bool BATCHED>
 void launch_density_any(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
@@ -1606,10 +1687,10 @@ void launch_density_any(const DevBuffers& d, const SceneConsts& sc, const BatchT
         density_kernel<BATCHED><<<ld.grid_density, SPH_THREADS, 0, s>>>(
             sc, bt, d.n, d.num_cells, d.pos_b, reinterpret_cast<float*>(d.pos_b) + 3,
             reinterpret_cast<float*>(d.vel_b) + 3, d.start, d.cell_list, d.num_nonempty, ncount, d.hits, d.err);
-    else if (lane_targets(d.n) == 2u)
-        launch_density_lane<BATCHED, FEAT_NONE, 2>(d, sc, bt, ld.grid_density, ncount, nullptr, nullptr, nullptr, nullptr, s);
+    else if (lane_pairs(d.n, resident_warps(ld.sms)))
+        launch_density_lane<BATCHED, FEAT_NONE, 2>(d, sc, bt, ld.grid_density, ncount, FeatureInputs{}, s);
     else
-        launch_density_lane<BATCHED, FEAT_NONE, 1>(d, sc, bt, ld.grid_density, ncount, nullptr, nullptr, nullptr, nullptr, s);
+        launch_density_lane<BATCHED, FEAT_NONE, 1>(d, sc, bt, ld.grid_density, ncount, FeatureInputs{}, s);
 }
 }  // namespace
 
@@ -1688,7 +1769,7 @@ void launch_force_batched_feat(const DevBuffers& d, const BatchTables& bt, const
 // force pass's).
 template <bool BATCHED, int FEAT, int TARGETS>
 void launch_density_feat_as(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
-                            const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
+                            const FeatureInputs& fi, cudaStream_t s) {
     static int blocks = 0;
     if (!blocks) {
         int b = 0;
@@ -1696,29 +1777,31 @@ void launch_density_feat_as(const DevBuffers& d, const SceneConsts& sc, const Ba
         blocks = b > 0 ? b : 1;
     }
     uint32_t* nc = BATCHED ? d.ncount : ((sc.flags & WC_FLAG_NEIGHBOR_COUNTS) ? d.ncount : nullptr);
-    launch_density_lane<BATCHED, FEAT, TARGETS>(d, sc, bt, ld.sms * blocks, nc, vxyz, rate, feat, judge_part, s);
+    launch_density_lane<BATCHED, FEAT, TARGETS>(d, sc, bt, ld.sms * blocks, nc, fi, s);
+    if (nc && d.n)
+        count_nan_kernel<BATCHED><<<std::min((d.n + 255u) / 256u, (uint32_t)ld.grid_stream), 256, 0, s>>>(sc, bt, d.n, d.pos_b, d.start, nc);
 }
 
 template <bool BATCHED>
 void launch_density_feat_any(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
-                             int level, const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
-    const bool pairs = lane_targets(d.n) == 2u;
+                             int level, const FeatureInputs& fi, cudaStream_t s) {
+    const bool pairs = judge_pairs(d.n, resident_warps(ld.sms));
     if (level == FEAT_FULL)
-        pairs ? launch_density_feat_as<BATCHED, FEAT_FULL, 2>(d, sc, bt, ld, vxyz, rate, feat, judge_part, s)
-              : launch_density_feat_as<BATCHED, FEAT_FULL, 1>(d, sc, bt, ld, vxyz, rate, feat, judge_part, s);
+        pairs ? launch_density_feat_as<BATCHED, FEAT_FULL, 2>(d, sc, bt, ld, fi, s)
+              : launch_density_feat_as<BATCHED, FEAT_FULL, 1>(d, sc, bt, ld, fi, s);
     else
-        pairs ? launch_density_feat_as<BATCHED, FEAT_RATE, 2>(d, sc, bt, ld, vxyz, rate, feat, judge_part, s)
-              : launch_density_feat_as<BATCHED, FEAT_RATE, 1>(d, sc, bt, ld, vxyz, rate, feat, judge_part, s);
+        pairs ? launch_density_feat_as<BATCHED, FEAT_RATE, 2>(d, sc, bt, ld, fi, s)
+              : launch_density_feat_as<BATCHED, FEAT_RATE, 1>(d, sc, bt, ld, fi, s);
 }
 
 void launch_density_feat(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, int level,
-                         const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
-    launch_density_feat_any<false>(d, sc, BatchTables{}, ld, level, vxyz, rate, feat, judge_part, s);
+                         const FeatureInputs& fi, cudaStream_t s) {
+    launch_density_feat_any<false>(d, sc, BatchTables{}, ld, level, fi, s);
 }
 
 void launch_density_batched_feat(const DevBuffers& d, const BatchTables& bt, const LaunchDims& ld, int level,
-                                 const float* vxyz, float2* rate, float4* feat, float* judge_part, cudaStream_t s) {
-    launch_density_feat_any<true>(d, SceneConsts{}, bt, ld, level, vxyz, rate, feat, judge_part, s);
+                                 const FeatureInputs& fi, cudaStream_t s) {
+    launch_density_feat_any<true>(d, SceneConsts{}, bt, ld, level, fi, s);
 }
 
 const void* force_kernel_symbol(int pass_variant) {

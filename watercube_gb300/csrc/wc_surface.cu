@@ -25,6 +25,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "wc_internal.h"
@@ -209,15 +210,16 @@ __device__ __forceinline__ f2 mul2_alone(f2 a, f2 b, f2 minus_zero) {
 
 // phi at every vertex (x fastest). One thread per vertex; a warp takes 4 x 4 x 2 of them and a block
 // 8 x 8 x 4, so that its lanes lie in a cell or two and walk nearly the same candidates, four at a time
-// from the lane passes' padded slots (the padding lies far away and adds zero; the weights are added
-// in candidate order). Bound by the L1's data path: the lanes of a load lie in up to eight cells. 128^3
+// from the lane passes' slots (padding lies far away and adds zero, and so do the places of a load outside a packed
+// row; the weights are added in candidate order). Bound by the L1's data path: the lanes of a load lie in up to eight cells. 128^3
 // vertices over 262,144 particles: 154 us with 32 x 1 x 1 vertices per warp and one candidate per load,
 // 79 us in blocks, 65 us with the air left out block by block.
 __global__ void __launch_bounds__(256) field_kernel(Grid g, const float* __restrict__ xyz, uint32_t pcap, uint32_t n,
-                                                    const uint32_t* __restrict__ start,
+                                                    uint32_t num_cells, const uint32_t* __restrict__ start,
                                                     const uint32_t* __restrict__ pstart, float bin, int32_t R, float h2,
                                                     float scale, float minus_zero, float* __restrict__ phi,
                                                     uint32_t* __restrict__ err) {
+    const bool packed_slots = __ldg(pstart + num_cells) > pcap;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t ix = blockIdx.x * 8u + (warp & 1u) * 4u + (lane & 3u);
     const uint32_t iy = blockIdx.y * 8u + ((warp >> 1) & 1u) * 4u + ((lane >> 2) & 3u);
@@ -256,40 +258,53 @@ __global__ void __launch_bounds__(256) field_kernel(Grid g, const float* __restr
     const float* const Z = xyz + 2 * (size_t)pcap;
     const f2 vx = pk(px, px), vy = pk(py, py), vz = pk(pz, pz), hh = pk(h2, h2), nz = pk(minus_zero, minus_zero);
     float acc = 0.f;
-#pragma unroll
-    for (int r = 0; r < 9; ++r) {
-        const int y = cy + r % 3 - 1, z = cz + r / 3 - 1;
-        if (y < 0 || y >= R || z < 0 || z >= R) continue;
-        const uint32_t row = (uint32_t)((z * R + y) * R);
-        // a timed-out scan (reported) leaves inconsistent tables: keep the range in the buffers
-        const uint32_t hi = min(__ldg(pstart + row + x1 + 1), pcap) & ~3u;
-        const uint32_t lo = min(__ldg(pstart + row + x0) & ~3u, hi);
-        if (hi - lo > 3u * MAX_CELL_PARTICLES) {
-            const uint32_t e = min(__ldg(start + row + x1 + 1), n);
-            if (e - min(__ldg(start + row + x0), e) > 3u * MAX_CELL_PARTICLES) {  // a collapsed state: not evaluated
-                acc = __int_as_float(0x7fc00000);
-                atomicOr(err, DEVERR_CELL_OVERFLOW);
-                continue;
+    auto walk = [&](auto layout) {
+        constexpr bool packed = decltype(layout)::value;
+        const uint32_t* const tab = packed ? start : pstart;
+#pragma unroll(packed ? 1 : 9)
+        for (int r = 0; r < 9; ++r) {
+            const int y = cy + r % 3 - 1, z = cz + r / 3 - 1;
+            if (y < 0 || y >= R || z < 0 || z >= R) continue;
+            const uint32_t row = (uint32_t)((z * R + y) * R);
+            // a timed-out scan (reported) leaves inconsistent tables: keep the range in the buffers
+            const uint32_t hi = packed ? min(__ldg(tab + row + x1 + 1), n) : min(__ldg(tab + row + x1 + 1), pcap) & ~3u;
+            const uint32_t lo = min(packed ? __ldg(tab + row + x0) : __ldg(tab + row + x0) & ~3u, hi);
+            if (hi - lo > 3u * MAX_CELL_PARTICLES) {
+                const uint32_t e = min(__ldg(start + row + x1 + 1), n);
+                if (e - min(__ldg(start + row + x0), e) > 3u * MAX_CELL_PARTICLES) {  // a collapsed state: not evaluated
+                    acc = __int_as_float(0x7fc00000);
+                    atomicOr(err, DEVERR_CELL_OVERFLOW);
+                    continue;
+                }
+            }
+            for (uint32_t k = packed ? lo & ~3u : lo; k < hi; k += 4u) {
+                const ulonglong2 qx = *reinterpret_cast<const ulonglong2*>(X + k);
+                const ulonglong2 qy = *reinterpret_cast<const ulonglong2*>(Y + k);
+                const ulonglong2 qz = *reinterpret_cast<const ulonglong2*>(Z + k);
+                const f2 dx01 = sub2(vx, qx.x), dx23 = sub2(vx, qx.y);
+                const f2 dy01 = sub2(vy, qy.x), dy23 = sub2(vy, qy.y);
+                const f2 dz01 = sub2(vz, qz.x), dz23 = sub2(vz, qz.y);
+                // t = h2 - d2 > 0 exactly when d2 < h2; zero (or not a number, as the comparison has it)
+                // otherwise adds zero
+                float t0, t1, t2, t3, w0, w1, w2, w3;
+                upk(sub2(hh, add2(add2(mul2_alone(dx01, dx01, nz), mul2_alone(dy01, dy01, nz)), mul2_alone(dz01, dz01, nz))), t0, t1);
+                upk(sub2(hh, add2(add2(mul2_alone(dx23, dx23, nz), mul2_alone(dy23, dy23, nz)), mul2_alone(dz23, dz23, nz))), t2, t3);
+                if (packed) {
+                    const uint32_t at = k - lo, len = hi - lo;
+                    t0 = at < len ? t0 : 0.f;
+                    t1 = at + 1u < len ? t1 : 0.f;
+                    t2 = at + 2u < len ? t2 : 0.f;
+                    t3 = at + 3u < len ? t3 : 0.f;
+                }
+                const f2 t01 = pk(fmaxf(t0, 0.f), fmaxf(t1, 0.f)), t23 = pk(fmaxf(t2, 0.f), fmaxf(t3, 0.f));
+                upk(mul2_alone(mul2(t01, t01), t01, nz), w0, w1);
+                upk(mul2_alone(mul2(t23, t23), t23, nz), w2, w3);
+                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, w0), w1), w2), w3);
             }
         }
-        for (uint32_t k = lo; k < hi; k += 4u) {
-            const ulonglong2 qx = *reinterpret_cast<const ulonglong2*>(X + k);
-            const ulonglong2 qy = *reinterpret_cast<const ulonglong2*>(Y + k);
-            const ulonglong2 qz = *reinterpret_cast<const ulonglong2*>(Z + k);
-            const f2 dx01 = sub2(vx, qx.x), dx23 = sub2(vx, qx.y);
-            const f2 dy01 = sub2(vy, qy.x), dy23 = sub2(vy, qy.y);
-            const f2 dz01 = sub2(vz, qz.x), dz23 = sub2(vz, qz.y);
-            // t = h2 - d2 > 0 exactly when d2 < h2; zero (or not a number, as the comparison has it)
-            // otherwise adds zero
-            float t0, t1, t2, t3, w0, w1, w2, w3;
-            upk(sub2(hh, add2(add2(mul2_alone(dx01, dx01, nz), mul2_alone(dy01, dy01, nz)), mul2_alone(dz01, dz01, nz))), t0, t1);
-            upk(sub2(hh, add2(add2(mul2_alone(dx23, dx23, nz), mul2_alone(dy23, dy23, nz)), mul2_alone(dz23, dz23, nz))), t2, t3);
-            const f2 t01 = pk(fmaxf(t0, 0.f), fmaxf(t1, 0.f)), t23 = pk(fmaxf(t2, 0.f), fmaxf(t3, 0.f));
-            upk(mul2_alone(mul2(t01, t01), t01, nz), w0, w1);
-            upk(mul2_alone(mul2(t23, t23), t23, nz), w2, w3);
-            acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, w0), w1), w2), w3);
-        }
-    }
+    };
+    if (packed_slots) walk(std::true_type{});
+    else walk(std::false_type{});
     phi[(iz * g.G + iy) * g.G + ix] = __fmul_rn(acc, scale);
 }
 
@@ -492,7 +507,7 @@ WC_API wc_status wc_surface_extract(wc_surface* s, wc_fluid* f, uint64_t* num_tr
     cudaEventCreate(&e2);
     cudaEventRecord(e0, fi.stream);
     field_kernel<<<dim3((G + 7) / 8, (G + 7) / 8, (G + 3) / 4), 256, 0, fi.stream>>>(
-        g, d.xyz, d.pcap, d.n, d.start, d.pstart, sc.bin, sc.R, h2, scale, -0.0f, s->phi, s->err);
+        g, d.xyz, d.pcap, d.n, d.num_cells, d.start, d.pstart, sc.bin, sc.R, h2, scale, -0.0f, s->phi, s->err);
     cudaEventRecord(e1, fi.stream);
     classify_kernel<<<grid_blocks(cubes), 256, 0, fi.stream>>>(G, s->phi, s->p.iso, s->counts);
     DevBuffers sd{};
