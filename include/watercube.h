@@ -456,6 +456,24 @@ typedef struct wc_gemm_desc {
 
 WC_API wc_status wc_nn_gemm(const wc_gemm_desc* g, uint32_t* d_err, void* stream);
 
+/* Two layers of the surrogate and their LayerNorm in one kernel (inference):
+   out = LN(relu(a w1 + b1 (+ add1[add1_idx[row]] + add2[add2_idx[row]])) w2 + b2) gamma + beta, and + a where rows
+   are added (both operands or neither, k = 128). BF16 rows of k (a) and 128 (the others), w1 [128 x k] and
+   w2 [128 x 128] output-major, b1, b2 (may be null), gamma, beta FP32; device pointers, 16-byte aligned, k a multiple
+   of 8 up to 128. The results are those of two wc_nn_gemm calls, bit for bit. *launched: 0 when the kernel cannot take
+   the operands (nothing has run; the caller takes the two calls). d_err as for wc_nn_gemm. */
+typedef struct wc_mlp_desc {
+    uint32_t m, k;
+    const void *a, *w1, *w2;
+    const float *b1, *b2, *gamma, *beta;
+    const void* add1;
+    const uint32_t* add1_idx;
+    const void* add2;
+    const uint32_t* add2_idx;
+    void* out;
+} wc_mlp_desc;
+WC_API wc_status wc_nn_mlp(const wc_mlp_desc* g, uint32_t* d_err, void* stream, int* launched);
+
 /* ---- learned surrogate: network, training and judged rollout ---------------------------- */
 /*
  * No counterpart in the reference. A message-passing network over the radius-h graph of a

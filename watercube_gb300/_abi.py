@@ -167,6 +167,15 @@ class GemmDesc(C.Structure):
     ]
 
 
+class MlpDesc(C.Structure):
+    _fields_ = [
+        ("m", C.c_uint32), ("k", C.c_uint32), ("a", C.c_void_p), ("w1", C.c_void_p), ("w2", C.c_void_p),
+        ("b1", C.c_void_p), ("b2", C.c_void_p), ("gamma", C.c_void_p), ("beta", C.c_void_p),
+        ("add1", C.c_void_p), ("add1_idx", C.c_void_p), ("add2", C.c_void_p), ("add2_idx", C.c_void_p),
+        ("out", C.c_void_p),
+    ]
+
+
 class SnapshotHeader(C.Structure):
     _fields_ = [
         ("magic", C.c_char * 8),
@@ -281,6 +290,7 @@ def _declare(lib) -> None:
         "wc_batch_set_tuning": (S, [P, C.POINTER(Tuning)]),
         "wc_batch_get_tuning": (S, [P, C.POINTER(Tuning)]),
         "wc_nn_gemm": (S, [C.POINTER(GemmDesc), P, P]),
+        "wc_nn_mlp": (S, [C.POINTER(MlpDesc), P, P, C.POINTER(C.c_int)]),
         "wc_fluid_save_snapshot": (S, [P, C.c_char_p, C.c_uint64]),
         "wc_snapshot_read_header": (S, [C.c_char_p, C.POINTER(SnapshotHeader)]),
         "wc_fluid_load_snapshot": (S, [P, C.c_char_p]),

@@ -2005,3 +2005,33 @@ extern "C" WC_API wc_status wc_nn_gemm(const wc_gemm_desc* d, uint32_t* d_err, v
     g.ln_resid = static_cast<const __nv_bfloat16*>(d->ln_resid);
     return wc::nn::launch_gemm(g, d_err, static_cast<cudaStream_t>(stream));
 }
+
+extern "C" WC_API wc_status wc_nn_mlp(const wc_mlp_desc* d, uint32_t* d_err, void* stream, int* launched) {
+    wc::clear_error();
+    if (!d || !launched) return wc::fail(WC_ERR_INVALID_ARG, "wc_nn_mlp: null argument");
+    *launched = 0;
+    if (!d->m) return WC_OK;
+    if (!d->a || !d->w1 || !d->w2 || !d->gamma || !d->beta || !d->out) return wc::fail(WC_ERR_INVALID_ARG, "wc_nn_mlp: null operand");
+    if (!d->add1 != !d->add2 || (d->add1 && (!d->add1_idx || !d->add2_idx)))
+        return wc::fail(WC_ERR_INVALID_ARG, "wc_nn_mlp: both gathered operands with their indices, or neither");
+    using Row = const __nv_bfloat16*;
+    wc::nn::MlpArgs g{};
+    g.m = d->m;
+    g.k = d->k;
+    g.a = static_cast<Row>(d->a);
+    g.w1 = static_cast<Row>(d->w1);
+    g.w2 = static_cast<Row>(d->w2);
+    g.b1 = d->b1;
+    g.b2 = d->b2;
+    g.gamma = d->gamma;
+    g.beta = d->beta;
+    g.add1 = static_cast<Row>(d->add1);
+    g.add1_idx = d->add1_idx;
+    g.add2 = static_cast<Row>(d->add2);
+    g.add2_idx = d->add2_idx;
+    g.out = static_cast<__nv_bfloat16*>(d->out);
+    bool ran = false;
+    const wc_status st = wc::nn::launch_mlp(g, d_err, static_cast<cudaStream_t>(stream), &ran);
+    *launched = ran ? 1 : 0;
+    return st;
+}
