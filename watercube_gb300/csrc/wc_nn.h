@@ -122,7 +122,6 @@ void layernorm_backward(uint32_t rows, float* dout, const float* y, const float*
                         const float* gamma, const uint32_t* add_idx, const float* add_src, bool fresh, __nv_bfloat16* dy,
                         float* part, float* part_dy, cudaStream_t s);
 void relu_mask(size_t count, float* g_inout, const __nv_bfloat16* z, __nv_bfloat16* out, cudaStream_t s);
-void cast_bf16(size_t count, const float* x, __nv_bfloat16* out, cudaStream_t s);
 void segment_sum_bf16(uint32_t nodes, const uint32_t* rowptr, const uint32_t* idx, const __nv_bfloat16* src,
                       float* out_f32, __nv_bfloat16* out_bf16, cudaStream_t s);
 void segment_sum_f32(uint32_t nodes, const uint32_t* rowptr, const uint32_t* idx, const float* src, float* out_f32,

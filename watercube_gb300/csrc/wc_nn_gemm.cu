@@ -2,13 +2,17 @@
 //
 //   C[m, n] = sum_k A[m, k] * B[k, n]        (BF16 operands, FP32 accumulation in TMEM)
 //
-// One CTA (4 warps) computes a 128 x 128 tile of C. Per 64-deep slice of K, all threads stage
-// the A and B tiles into shared memory in the canonical no-swizzle K-major layout of the
-// tensor-core descriptors (8-row x 16-byte core matrices; the next core matrix along K is 128 B
-// away, the next 8-row group 1,024 B away), fence them into the async proxy, and one thread
-// issues four tcgen05.mma (K = 16 each) into a 128-column FP32 accumulator in tensor memory and
-// commits them to an mbarrier. The epilogue reads the accumulator with tcgen05.ld (warp w owns
-// rows 32w..32w+31, one row per thread) and applies bias, row gathers, ReLU and the store.
+// Five kernels, all with 128 x 128 tiles, operands in shared memory, tcgen05.mma issued by one thread into accumulators in
+// tensor memory and the results read back with tcgen05.ld:
+//   gemm_tma_kernel    row-major A (or two sources split at a whole slice of 64) and B^T, n <= 128, k <= 384: persistent,
+//                      operands by TMA; results through shared memory and TMA, or a row per thread (launch_tma)
+//   gemm_mlp_kernel    two layers and their LayerNorm, for inference
+//   gemm_wgrad_kernel  X^T dY with m, n <= 128, both operands by TMA along their rows
+//   gemm_pipe_kernel   the other row-major forms (A rows by index, a source split inside a slice, n > 128, k > 384,
+//                      operands that TMA cannot address): persistent, a cp.async operand ring
+//   gemm_kernel        the other transposed operands and splits of K, one tile per CTA: per 64-deep slice of K all
+//                      threads stage A and B in the no-swizzle K-major layout (8-row x 16-byte core matrices; the next
+//                      along K 128 B away, the next 8-row group 1,024 B away); warp w stores rows 32w .., one per thread
 //
 // Operand sources (staging policies):
 //   A row-major [m x k] (lda), optionally with a row index (gather) and a second source for
@@ -18,12 +22,6 @@
 //     [k x n] (the upstream gradient dY in X^T dY, and W in dY W^T).
 // Every wait on the mbarrier is bounded; a wait that runs out sets an error flag, and the
 // kernel still releases its tensor memory before it returns.
-//
-// Three kernels: gemm_tma_kernel (persistent, operands and results by TMA, see below) for the plain
-// forward layers and input gradients, gemm_pipe_kernel (persistent, warp-specialised, a cp.async
-// operand ring) for gathered or concatenated A, more than 128 columns and unaligned results, and
-// gemm_kernel (one tile per CTA, two operand buffers) for the transposed weight-gradient operands
-// and split-K.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -968,7 +966,7 @@ __device__ __forceinline__ void tma_epilogue(const GemmArgs& g, const TmaMaps& m
                 g.ln_mean[row0 + lane] = mean;
                 g.ln_rstd[row0 + lane] = rstd;
             }
-                const uint32_t rows = aux_base + (AUX == AUX_NONE && plan.one_stage ? 0u : b) * plan.aux_bytes;
+            const uint32_t rows = aux_base + (AUX == AUX_NONE && plan.one_stage ? 0u : b) * plan.aux_bytes;
 #pragma unroll
             for (uint32_t j = 0; j < 16; ++j) {
                 const float* y = x + 4 * j;

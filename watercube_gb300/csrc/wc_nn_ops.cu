@@ -272,11 +272,6 @@ __global__ void relu_mask_kernel(size_t count, float* __restrict__ g, const __nv
     }
 }
 
-__global__ void cast_kernel(size_t count, const float* __restrict__ x, __nv_bfloat16* __restrict__ out) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = __float2bfloat16_rn(x[i]);
-}
-
 // Four consecutive columns of a row.
 __device__ __forceinline__ float4 load4(const float* s) { return __ldg(reinterpret_cast<const float4*>(s)); }
 __device__ __forceinline__ float4 load4(const __nv_bfloat16* s) {
@@ -634,9 +629,6 @@ void layernorm_backward(uint32_t rows, float* dout, const float* y, const float*
 }
 void relu_mask(size_t count, float* g, const __nv_bfloat16* z, __nv_bfloat16* out, cudaStream_t s) {
     if (count) relu_mask_kernel<<<(unsigned)std::min<size_t>(blocks_for(count, 256), 65535), 256, 0, s>>>(count, g, z, out);
-}
-void cast_bf16(size_t count, const float* x, __nv_bfloat16* out, cudaStream_t s) {
-    if (count) cast_kernel<<<(unsigned)std::min<size_t>(blocks_for(count, 256), 65535), 256, 0, s>>>(count, x, out);
 }
 void segment_sum_bf16(uint32_t nodes, const uint32_t* rowptr, const uint32_t* idx, const __nv_bfloat16* src,
                       float* out_f32, __nv_bfloat16* out_bf16, cudaStream_t s) {
