@@ -148,8 +148,7 @@ void free_batch(wc_batch* b) {
                     d.unordered, d.perm,         d.counts,     d.start,  d.cell_list,    d.num_nonempty,
                     d.scan_desc, d.scan_tile_counter, d.err,   d.hits,   b->d_scenes,    b->d_poff,
                     b->d_coff,   b->d_diag,      b->staging,   b->flush_buf, b->flush_sink, d.ids_a,
-                    d.ids_b,     d.accel,        d.xyz,        d.pstart, d.cidx,         d.rec,
-                    d.info};
+                    d.ids_b,     d.accel,        d.slots};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (b->h_err) cudaFreeHost(b->h_err);
@@ -553,11 +552,9 @@ WC_API wc_status wc_batch_create(const wc_params* scenes, uint32_t num_scenes, w
     if (st == WC_OK) st = dalloc(&d.ids_b, n);
     if (st == WC_OK) st = dalloc(&d.hits, hits_words(n));
     d.pcap = slot_capacity(n);
-    if (st == WC_OK) st = dalloc(&d.xyz, 3 * (size_t)d.pcap);
-    if (st == WC_OK) st = dalloc(&d.cidx, d.pcap);
-    if (st == WC_OK) st = dalloc(&d.rec, 2 * (size_t)d.pcap);
-    if (st == WC_OK) st = dalloc(&d.info, n);
-    if (st == WC_OK) st = dalloc(&d.pstart, cells + 1);
+    char* slots = nullptr;
+    if (st == WC_OK) st = dalloc(&slots, place_slots(d, cells, nullptr));
+    if (st == WC_OK) place_slots(d, cells, slots);
     if (st == WC_OK) st = dalloc(&d.counts, cells);
     if (st == WC_OK) st = dalloc(&d.start, cells + 1);
     if (st == WC_OK) st = dalloc(&d.cell_list, cells);

@@ -69,9 +69,8 @@ void free_all(wc_fluid* f) {
     void* ptrs[] = {d.pos_a,     d.vel_a,        d.pos_b,     d.vel_b,    d.ids_a,           d.ids_b,
                     d.keys,      d.ranks,        d.unordered, d.perm,     d.counts,          d.start,
                     d.cell_list, d.num_nonempty, d.scan_desc, d.ncount,   d.scan_tile_counter, d.err,
-                    d.hits,      f->staging,     f->flush_buf, f->flush_sink, f->accel_store, d.xyz,
-                    f->diag_part,
-                    d.pstart,    d.cidx,         d.rec,       d.info};
+                    d.hits,      f->staging,     f->flush_buf, f->flush_sink, f->accel_store, d.slots,
+                    f->diag_part};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (f->h_err) cudaFreeHost(f->h_err);
@@ -104,11 +103,9 @@ wc_status allocate(wc_fluid* f) {
     if (f->params.flags & WC_FLAG_NEIGHBOR_COUNTS) WC_TRY(dalloc(&d.ncount, n));
     WC_TRY(dalloc(&d.hits, hits_words(n)));
     d.pcap = slot_capacity(n);
-    WC_TRY(dalloc(&d.xyz, 3 * (size_t)d.pcap));
-    WC_TRY(dalloc(&d.cidx, d.pcap));
-    WC_TRY(dalloc(&d.rec, 2 * (size_t)d.pcap));
-    WC_TRY(dalloc(&d.info, n));
-    WC_TRY(dalloc(&d.pstart, (size_t)d.num_cells + 1));
+    char* slots = nullptr;
+    WC_TRY(dalloc(&slots, place_slots(d, d.num_cells, nullptr)));
+    place_slots(d, d.num_cells, slots);
     WC_TRY(dalloc(&d.counts, d.num_cells));
     WC_TRY(dalloc(&d.start, (size_t)d.num_cells + 1));
     WC_TRY(dalloc(&d.cell_list, d.num_cells));
