@@ -943,14 +943,14 @@ __global__ void __launch_bounds__(SPH_THREADS, TARGETS == 2 && FEAT == FEAT_FULL
         __syncthreads();
     }
     const uint32_t padded = __ldg(pstart + num_cells);
-    if (padded > pcap)
-        density_walk<BATCHED, FEAT, 1, true>(sc0, bt, s_poff, s_coff, n, padded, pos_in, vel_in, rho_out, p_out, start, pstart,
-                                             cidx, counter, ncount, entries, info, err, xyz, pcap, rec, vxyz, rate_out, feat,
-                                             judge_part, judge_chunks);
-    else
+    if (__builtin_expect(padded <= pcap, 1))
         density_walk<BATCHED, FEAT, TARGETS, false>(sc0, bt, s_poff, s_coff, n, padded, pos_in, vel_in, rho_out, p_out, start,
                                                     pstart, cidx, counter, ncount, entries, info, err, xyz, pcap, rec, vxyz,
                                                     rate_out, feat, judge_part, judge_chunks);
+    else
+        density_walk<BATCHED, FEAT, 1, true>(sc0, bt, s_poff, s_coff, n, padded, pos_in, vel_in, rho_out, p_out, start, pstart,
+                                             cidx, counter, ncount, entries, info, err, xyz, pcap, rec, vxyz, rate_out, feat,
+                                             judge_part, judge_chunks);
 }
 
 // The neighbour counts of particles at NaN after a judge's density pass (see density_walk).
