@@ -14,7 +14,7 @@ namespace nn {
 // (or have all called this): its prologue, barriers and tensor memory, runs beside that kernel's end. Every thread
 // calls it before its first access to global memory; what the kernel before wrote is visible then. A training
 // pass over 2,048 / 16,384 particles, ~320 launches, takes 3,378 / 8,310 us without, 3,040 / 7,970 with the GEMMs and
-// 2,755 / 7,890 with the sums and LayerNorms too; a prediction of 2,500 particles 537 -> 459. The segment sums are
+// 2,670 / 7,770 with the sums and LayerNorms too; a prediction of 2,500 particles 537 -> 459. The segment sums are
 // launched as usual: the next GEMM's blocks would take places from their second wave (65,536 particles 3,375 -> 3,415).
 // Such a kernel is resident while its inputs are written, so they are not read-only for its lifetime: its loads are
 // plain ones, without __ldg (ld.global.nc) and without const __restrict__, from which the compiler makes the same.

@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1) gemm_pipe_kernel(const GemmAr
 // four more warps with cp.async, 16 lanes to a row (AUX_GATHER). Forms that it cannot take are written from the
 // registers (AUX_DIRECT, see launch_tma). BF16 results are written over
 // the place of the values read. Bound by the traffic it cannot avoid: 460,000 rows of 128 with two
-// gathered rows each take 59 us against 134 us with row-per-thread accesses (62 % of the copy
+// gathered rows each take 55 us against 134 us with row-per-thread accesses (66 % of the copy
 // bandwidth for A and C alone, the gathered rows come from L2 on top).
 constexpr int TMA_THREADS = 32 * (2 + PIPE_EPILOGUE);
 constexpr int GATHER_WARPS = 4;
@@ -1288,7 +1288,7 @@ __global__ void __launch_bounds__(TMA_THREADS + (AUX == AUX_GATHER ? 32 * GATHER
 // read straight into registers: edges are sorted by receiver, so the 32 rows of a warp share one or two of P's,
 // which L1 serves (any index is correct). Registers are moved from the copying warps to the normalising ones.
 // The arithmetic and its order are those of the two launches (the same results bit for bit).
-// 1.85 M edges: 262 us against 203 + 231 in two launches. Bound by L1 (86 %), most of it the loads of bias, gamma and
+// 1.85 M edges: 257 us against 203 + 231 in two launches. Bound by L1 (86 %), most of it the loads of bias, gamma and
 // beta, which every warp needs for every tile. Slower: both epilogues in one group of eight warps with both gathered
 // rows copied, 345 us; FP32 arithmetic in scalar instructions, 312; the constants as kernel parameters (constant
 // cache misses), 352; the second layer's columns spread over the lanes so that a thread needs fewer of them, 286.
