@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t key = keys[i];
         const uint32_t s = start[key], e = min(start[key + 1], n);
+        const uint32_t ps = LANE ? pstart[key] : 0u;  // (with the other loads, before it is known whether it counts)
         uint32_t r = 0;
         if (e - min(s, e) <= MAX_SORT_CELL_PARTICLES) {
             for (uint32_t q = s; q < e; ++q) r += unordered[q] < i ? 1u : 0u;
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(256) rank_gather_kernel(uint32_t n, const uint
         const float4 p = pos_in[i];
         pos_out[dst] = p;
         if (LANE) {
-            const uint32_t pd = packed ? dst : pstart[key] + r;
+            const uint32_t pd = packed ? dst : ps + r;
             const uint32_t last = !packed && s + r + 1u == e ? ((r + 4u) & ~3u) - r : 1u;  // places this thread writes
             if (pd + last <= pcap) {
                 if (!packed) cidx[pd] = dst;
