@@ -283,7 +283,7 @@ enum : int { FEAT_NONE = 0, FEAT_RATE = 1, FEAT_FULL = 2 };
 // ld.pass_variant says: the density pass also writes the density and pressure rates (FeatureBuffers)
 // from the gather's velocity arrays vxyz and, when judge_part is given, the judge's sums
 // judge_part[m] = sum over the slots of chunk m of |rho_carried / rho_SPH - 1| (rho_carried:
-// the sorted buffer's .w before the pass; *judge_chunks of them, at most one per 32 particles); the force pass reads the neighbours' rates and writes
+// the sorted buffer's .w before the pass; *judge_chunks of them, when given; at most one per 32 particles); the force pass reads the neighbours' rates and writes
 // feat[ti] = (J, density rate), J the time derivative of the SPH acceleration (sorted order).
 struct FeatureInputs {
     const float* vxyz = nullptr;
@@ -292,6 +292,8 @@ struct FeatureInputs {
     float* judge_part = nullptr;
     uint32_t* judge_chunks = nullptr;
 };
+// Whether those passes take pairs of targets (the number of chunks then depends on the state).
+bool feature_pairs(uint32_t n, const LaunchDims& ld);
 void launch_density_feat(const DevBuffers& d, const SceneConsts& sc, const LaunchDims& ld, int level,
                          const FeatureInputs& fi, cudaStream_t s);
 void launch_density_batched_feat(const DevBuffers& d, const BatchTables& bt, const LaunchDims& ld, int level,

@@ -583,10 +583,10 @@ __global__ void __launch_bounds__(32 * OUT) output_mean_kernel(uint32_t ctas, ui
 // kernel adds the chunk sums in a fixed order, FP32 per thread and warp (a relative
 // rounding of order 1e-6 against a tolerance of order 1e-2), FP64 across the warps.
 constexpr uint32_t JUDGE_THREADS = 1024;
-// num_chunks: how many (device memory, from the density pass).
-__global__ void __launch_bounds__(JUDGE_THREADS) judge_final_kernel(const uint32_t* __restrict__ num_chunks,
+// num_chunks: how many, from the density pass, where the host does not know (pairs of targets), else null.
+__global__ void __launch_bounds__(JUDGE_THREADS) judge_final_kernel(uint32_t chunks, const uint32_t* __restrict__ num_chunks,
                                                                     const float* __restrict__ part, double* __restrict__ out) {
-    const uint32_t chunks = *num_chunks;
+    if (num_chunks) chunks = *num_chunks;
     __shared__ float s[JUDGE_THREADS / 32];
     float a = 0.f;
     for (uint32_t b = threadIdx.x; b < chunks; b += JUDGE_THREADS) a += part[b];
@@ -792,7 +792,7 @@ struct wc_local {
     float4 *save_pos[2] = {nullptr, nullptr}, *save_vel[2] = {nullptr, nullptr};
     uint32_t* save_ids[2] = {nullptr, nullptr};
     float* judge_part = nullptr;  // per chunk of the density pass
-    uint32_t* judge_chunks = nullptr;  // their number
+    uint32_t* judge_chunks = nullptr;  // their number, behind judge_out
     double *judge_out = nullptr, *h_judge = nullptr;
     uint32_t cap_roll = 0;
 };
@@ -837,7 +837,6 @@ void free_local(wc_local* s) {
     dfree(s->vxyz);
     dfree(s->judge_part);
     dfree(s->judge_out);
-    dfree(s->judge_chunks);
     if (s->h_err) cudaFreeHost(s->h_err);
     if (s->h_judge) cudaFreeHost(s->h_judge);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -908,6 +907,9 @@ void enqueue_predict(wc_local* s, const StepTarget& t, float dt) {
             n, src, nullptr, weights(s), s->change, ldo, ldo, residual_scale(s, dt), s->d_err);
 }
 
+// Where the density pass writes its number of chunks: one target per lane makes one per 32 particles.
+uint32_t* chunks_word(wc_local* s, const StepTarget& t) { return feature_pairs(t.d->n, t.ld) ? s->judge_chunks : nullptr; }
+
 // The judge of the last cycle when the rollout ends after its skipped steps: the sort and the
 // judge step's density pass with its judge sums, without a force pass (the state does not
 // advance).
@@ -921,12 +923,12 @@ void enqueue_closing_judge(wc_local* s, const StepTarget& t) {
     launch_scan_cells(d, t.stream, true);
     launch_scatter(d, t.ld, t.stream);
     launch_rank_gather(d, t.ld, t.stream, true);
-    const FeatureInputs fi{nullptr, nullptr, nullptr, s->judge_part, s->judge_chunks};
+    const FeatureInputs fi{nullptr, nullptr, nullptr, s->judge_part, chunks_word(s, t)};
     if (t.bt.num_scenes)
         launch_density_batched_feat(d, t.bt, t.ld, FEAT_RATE, fi, t.stream);
     else
         launch_density_feat(d, t.sc, t.ld, FEAT_RATE, fi, t.stream);
-    judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(s->judge_chunks, s->judge_part, s->judge_out);
+    judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(blocks_for(d.n, 32), fi.judge_chunks, s->judge_part, s->judge_out);
 }
 
 // The judge step, on the target's stream: a plain SPH step whose force pass also writes s->feat
@@ -949,7 +951,7 @@ void enqueue_judge_step(wc_local* s, const StepTarget& t, float dt, bool judge, 
     launch_rank_gather(d, t.ld, t.stream, true, full ? s->vxyz : nullptr);
     const FeatureBuffers fb{s->feat, s->rate};
     float* jp = judge && d.n ? s->judge_part : nullptr;
-    const FeatureInputs fi{s->vxyz, s->rate, s->feat, jp, jp ? s->judge_chunks : nullptr};
+    const FeatureInputs fi{s->vxyz, s->rate, s->feat, jp, jp ? chunks_word(s, t) : nullptr};
     if (t.bt.num_scenes) {
         launch_density_batched_feat(d, t.bt, t.ld, level, fi, t.stream);
         launch_force_batched_feat(d, t.bt, in, t.ld, level, fb, t.stream);
@@ -957,7 +959,7 @@ void enqueue_judge_step(wc_local* s, const StepTarget& t, float dt, bool judge, 
         launch_density_feat(d, t.sc, t.ld, level, fi, t.stream);
         launch_force_feat(d, t.sc, in, t.ld, level, fb, t.stream);
     }
-    if (jp) judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(s->judge_chunks, jp, s->judge_out);
+    if (jp) judge_final_kernel<<<1, JUDGE_THREADS, 0, t.stream>>>(blocks_for(d.n, 32), fi.judge_chunks, jp, s->judge_out);
 }
 
 wc_status plain_step(const StepTarget& t, float dt) {
@@ -1276,8 +1278,8 @@ WC_API wc_status wc_local_create(const wc_local_config* c, wc_local** out) {
         st = fail(WC_ERR_OOM, "pinned host allocation failed");
     if (st == WC_OK && cudaMallocHost(reinterpret_cast<void**>(&s->h_judge), sizeof(double)) != cudaSuccess)
         st = fail(WC_ERR_OOM, "pinned host allocation failed");
-    if (st == WC_OK) st = dalloc(&s->judge_out, 1);
-    if (st == WC_OK) st = dalloc(&s->judge_chunks, 1);
+    if (st == WC_OK) st = dalloc(&s->judge_out, 2);
+    if (st == WC_OK) s->judge_chunks = reinterpret_cast<uint32_t*>(s->judge_out + 1);
     if (st == WC_OK) {
         std::vector<float> host;
         init_params(s, host);

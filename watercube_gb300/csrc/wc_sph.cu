@@ -1782,10 +1782,12 @@ void launch_density_feat_as(const DevBuffers& d, const SceneConsts& sc, const Ba
         count_nan_kernel<BATCHED><<<std::min((d.n + 255u) / 256u, (uint32_t)ld.grid_stream), 256, 0, s>>>(sc, bt, d.n, d.pos_b, d.start, nc);
 }
 
+bool feature_pairs(uint32_t n, const LaunchDims& ld) { return judge_pairs(n, resident_warps(ld.sms)); }
+
 template <bool BATCHED>
 void launch_density_feat_any(const DevBuffers& d, const SceneConsts& sc, const BatchTables& bt, const LaunchDims& ld,
                              int level, const FeatureInputs& fi, cudaStream_t s) {
-    const bool pairs = judge_pairs(d.n, resident_warps(ld.sms));
+    const bool pairs = feature_pairs(d.n, ld);
     if (level == FEAT_FULL)
         pairs ? launch_density_feat_as<BATCHED, FEAT_FULL, 2>(d, sc, bt, ld, fi, s)
               : launch_density_feat_as<BATCHED, FEAT_FULL, 1>(d, sc, bt, ld, fi, s);
